@@ -19,6 +19,8 @@
 //    32 coalesced entries per step.
 //  * Three step variants: push with one warp per frontier vertex (one
 //    launch), load-balanced push (above), pull (above).
+//  * One launch per search (bfs_search_kernel) under the fixed schedule; a graph
+//    of conditional nodes over the step kernels under a learned one.
 //  * Schedule: Beamer's alpha/beta rule (alpha = 14, beta = 24) over the
 //    balanced push and the pull, fed by the frontier and unexplored edge
 //    counts the steps emit; or, when a learned schedule is installed on the
@@ -74,11 +76,13 @@ struct BfsDevState {
     uint32_t failed;                // the loop stopped on a state no search can reach
 };
 
+struct BfsSearchState;
+
 struct BfsWork {
     DeviceBuffer<int32_t> dist;
     DeviceBuffer<uint32_t> visited;
     DeviceBuffer<uint32_t> bitmap[2];
-    DeviceBuffer<uint32_t> queue[2];
+    DeviceBuffer<uint32_t> queue[2];       // vertices, or the one-launch search's items (uint2)
     DeviceBuffer<uint32_t> degree_scan;  // V + 1
     DeviceBuffer<BfsCounters> counters;
     BfsCounters host_counters{};  // host copy, read after a synchronisation (plain memory)
@@ -86,6 +90,17 @@ struct BfsWork {
     DeviceBuffer<uint32_t> active;         // vertices with edges, ascending (symmetric graphs)
     uint32_t n_active = 0;
     bool pull_list = false;                // the pull walks `active` instead of every bitmap word
+    // one-launch search
+    DeviceBuffer<uint32_t> search_bitmaps;  // three
+    DeviceBuffer<uint4> search_segments;
+    uint32_t search_epoch = 0;
+    DeviceBuffer<BfsSearchState> search;
+    unsigned search_grid = 0;
+    struct {
+        uint32_t reached;
+        int32_t level;
+        uint32_t failed;
+    } host_search{};
     // device-driven level loop (built on first use, per schedule network)
     DeviceBuffer<BfsDevState> loop_state;
     DeviceBuffer<uint32_t> loop_scan_sums;
@@ -469,7 +484,846 @@ __global__ void bfs_decide_kernel(const __nv_bfloat16* __restrict__ w, BfsCounte
     }
 }
 
-// ---------------------------------------------------------------- device-driven level loop
+// ---------------------------------------------------------------- one launch per search
+//
+// The fixed schedule's search runs as one cooperative kernel: every block
+// holds the level loop's state in registers and the blocks meet at a grid
+// barrier (about 1.5 us) between levels, instead of a graph of conditional
+// nodes with four to six launches per level (about 25-30 us per level,
+// whatever the frontier's size).
+//  * Push levels work on items: ranges of at most kItemEdges list entries of
+//    the frontier's vertices, appended when a vertex is discovered. A hub is
+//    many items, so the edges are spread evenly with no degree scan; a warp
+//    takes up to 32 items at a time and walks their edges in order, found by
+//    a search over a warp scan of the item lengths.
+//  * While the frontier has at most kLocalEdges edges, block 0 runs the levels
+//    alone with its queue in shared memory and block barriers; up to
+//    kGroupEdges, the first kGroupBlocks blocks run them with a barrier of
+//    their own. A level there is a chain of dependent accesses (317 cycles for
+//    an L2 read, 511 for an atomic, measured), and one SM completes one
+//    scattered L2 access per cycle, so a frontier of thousands of edges wants
+//    a few SMs and a cheap barrier, not one SM and not all.
+//  * Pull levels keep no queue: a push that follows builds its items from the
+//    frontier bitmap, a pull that follows a push builds the bitmap from the
+//    distances (one coalesced pass, far below the level's own work).
+// Measured on one B200, a whole search through the Python module (the graph of
+// conditional nodes before, this kernel after): R-MAT 14 with distances 195 ->
+// 83 us; 1024 x 1024 grid with dropped edges, 1,640 levels, 56.7 -> 5.4 ms (a
+// level 31 -> 2.8 us: 1.7 of work, 0.9 of barrier); 16 searches of R-MAT 22
+// 9.33 -> 4.18 ms (one: init 9, pushes 14, bitmap 6, pulls 50 + 28 + 15, tail
+// 15 us). The same levels with block 0 alone: 5.4 us at 4,000 frontier edges,
+// 2.2 at 100, hence kLocalEdges. What bounds it: the levels' latency chains on
+// small frontiers, the L1's tag lookups of the pull's scattered probes on wide
+// ones (about 130 lookups per 32 vertices; reading a list's sector in one
+// 32-byte load and joining the bitmap atomics per word took a third away).
+// Level counters rotate over three slots: phase p adds into slot p % 3, reads
+// it after its barrier, and clears slot (p + 1) % 3, whose readers are done.
+constexpr int kSearchThreads = 1024;
+constexpr int kSearchCtasPerSm = 1;
+constexpr uint32_t kItemEdges = 1024;
+constexpr uint32_t kLogItemParts = 4;        // up to 2^4 warps share an item of a short queue
+constexpr uint32_t kLaneItems = 8;           // items a lane writes alone
+constexpr uint32_t kLocalEdges = 512;        // frontier edges block 0 handles alone
+constexpr uint32_t kGroupEdges = 16384;      // frontier edges the first kGroupBlocks blocks handle
+constexpr unsigned kLogGroupBlocks = 4, kGroupBlocks = 1u << kLogGroupBlocks;
+constexpr uint32_t kGroupItems = 4096;       // items per block of the group (more end the stretch)
+constexpr uint32_t kPullMinEdges = 8192;     // a push with fewer frontier edges is never turned into a pull
+constexpr uint32_t kLocalItems = 2048;       // items of a local level kept in shared memory (the rest spill)
+constexpr uint32_t kLocalMaxLevels = 32768;  // levels per local or group stretch (the other blocks wait at a barrier)
+constexpr int kPushUnroll = 4;               // edges per lane in flight in a push
+constexpr int kPullTiles = 1;                // 32-vertex tiles per warp in flight in a pull
+
+struct alignas(16) BfsSlot {
+    unsigned long long edges;     // out-edges of the new frontier
+    uint32_t discovered;          // vertices of the new frontier
+    uint32_t items;               // its items (push)
+    unsigned long long explored;  // stretch: out-edges of every vertex it labelled
+    uint32_t levels;              // stretch: levels it advanced
+    uint32_t reached;             // stretch: vertices it labelled
+};
+
+// 16-byte accesses that are single and bypass L1: a value and its tag arrive
+// together.
+__device__ __forceinline__ void st_relaxed_16(uint4* p, const uint4& v) {
+    asm volatile("{\n\t.reg .b128 q;\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+                 "mov.b128 q, {a, b};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p),
+                 "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+__device__ __forceinline__ uint4 ld_relaxed_16(const uint4* p) {
+    uint4 v;
+    asm volatile("{\n\t.reg .b128 q;\n\t.reg .b64 a, b;\n\tld.relaxed.gpu.global.b128 q, [%4];\n\tmov.b128 {a, b}, q;\n\t"
+                 "mov.b64 {%0, %1}, a;\n\tmov.b64 {%2, %3}, b;\n\t}"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+
+// Device memory of a search besides the graph-sized arrays, zeroed before it.
+struct BfsSearchState {
+    GridBarrier bar;
+    GridBarrier group_bar;
+    BfsSlot slot[3];
+    uint4 entry[2][kGroupBlocks];  // the group's barrier: items, vertices, edges, phase of every block
+    uint32_t overflow;             // the group's items beyond the blocks' segments (they end a stretch)
+    uint32_t reached;
+    int32_t level;
+    uint32_t failed;
+};
+
+struct BfsSearch {
+    const uint32_t* offsets;
+    const uint32_t* targets;
+    const uint32_t* active;  // list form of the pull
+    uint32_t V, E, n_active, source;
+    int symmetric;
+    int32_t* dist;
+    uint32_t* visited;
+    uint32_t* bitmaps;  // three of bitmap_words each
+    uint32_t bitmap_words;
+    uint2* queue0;
+    uint2* queue1;
+    uint4* segments;  // the group's items: [2][kGroupBlocks][kGroupItems] (start, end, phase, epoch)
+    uint32_t epoch;   // differs from search to search on the same buffers
+    BfsSearchState* st;
+};
+
+struct BfsLocal {
+    uint32_t found, edges, items;
+};
+
+struct BfsShared {
+    uint2 items[2][kLocalItems];
+    unsigned long long edges[kSearchThreads / 32];
+    uint32_t found[kSearchThreads / 32];
+    BfsSlot slot;
+    BfsLocal local[3];  // rotating like the slots: one block barrier per level
+    uint32_t counts[kGroupBlocks];  // items of every block's segment
+    BfsLocal all;                   // the group's counts of a level
+    uint32_t over, ok;
+};
+
+__device__ __forceinline__ uint32_t* search_bitmap(const BfsSearch& a, uint32_t i) {
+    return a.bitmaps + static_cast<size_t>(i) * a.bitmap_words;
+}
+__device__ __forceinline__ uint2* search_queue(const BfsSearch& a, uint32_t i) { return i ? a.queue1 : a.queue0; }
+
+// Expands the q items of the frontier with the warps warp, warp + nwarps, ...
+// of the blocks at work; new items go to slot `*count` onwards of g_out.
+__device__ __forceinline__ void push_items(const BfsSearch& a, const uint2* g_in, uint32_t q, uint2* g_out,
+                                           uint32_t* count, int32_t next_level, uint32_t warp, uint32_t nwarps,
+                                           Tally& tally) {
+    const unsigned lane = lane_id();
+    // Up to 32 items per warp at a time; with fewer items than warps, up to
+    // 2^kLogItemParts warps share each.
+    const uint32_t k = min(32u, max(1u, (q + nwarps - 1) / nwarps));
+    const uint32_t parts = q ? min(1u << kLogItemParts, max(1u, nwarps / q)) : 1u;
+    const uint32_t part = warp % parts;
+    for (uint64_t base = static_cast<uint64_t>(warp / parts) * k; base < q;
+         base += static_cast<uint64_t>(nwarps / parts) * k) {
+        const uint64_t i = base + lane;
+        uint2 it = make_uint2(0u, 0u);
+        if (lane < k && i < q) {
+            it = __ldcg(g_in + i);
+            if (parts > 1) {
+                const uint32_t piece = (it.y - it.x + parts - 1) / parts;
+                it.x = min(it.y, it.x + part * piece);
+                it.y = min(it.y, it.x + piece);
+            }
+        }
+        const uint32_t len = it.y - it.x;
+        const uint32_t inc = warp_inclusive_scan(len);
+        const uint32_t total = __shfl_sync(kFullMask, inc, 31);
+        const uint32_t shift = it.x - (inc - len);  // entry of edge e of this item = shift + e
+        for (uint32_t e0 = 0; e0 < total; e0 += 32 * kPushUnroll) {
+            uint32_t v[kPushUnroll], ls[kPushUnroll], deg[kPushUnroll];
+            bool found[kPushUnroll];
+#pragma unroll
+            for (int u = 0; u < kPushUnroll; ++u) {
+                const uint32_t e = e0 + u * 32 + lane;
+                // The item of edge e: the number of items that end at or before it.
+                uint32_t j = 0;
+                if (k > 1) {
+#pragma unroll
+                    for (uint32_t step = 16; step > 0; step >>= 1)
+                        if (__shfl_sync(kFullMask, inc, j + step - 1) <= e) j += step;
+                }
+                const uint32_t at = __shfl_sync(kFullMask, shift, j) + e;
+                found[u] = e < total;
+                v[u] = ld_nc_if(found[u], a.targets + at, 0u);
+            }
+            uint32_t word[kPushUnroll];
+#pragma unroll
+            for (int u = 0; u < kPushUnroll; ++u) {
+                word[u] = ld_cg_if(found[u], a.visited + (v[u] >> 5), 0xFFFFFFFFu);
+            }
+#pragma unroll
+            for (int u = 0; u < kPushUnroll; ++u) found[u] = !((word[u] >> (v[u] & 31)) & 1u);
+#pragma unroll
+            for (int u = 0; u < kPushUnroll; ++u)
+                word[u] = atomic_or_if(found[u], a.visited + (v[u] >> 5), 1u << (v[u] & 31), 0xFFFFFFFFu);
+#pragma unroll
+            for (int u = 0; u < kPushUnroll; ++u) found[u] = !((word[u] >> (v[u] & 31)) & 1u);
+#pragma unroll
+            for (int u = 0; u < kPushUnroll; ++u) {
+                ls[u] = ld_nc_if(found[u], a.offsets + v[u], 0u);
+                deg[u] = ld_nc_if(found[u], a.offsets + v[u] + 1, 0u);
+            }
+            uint32_t mine = 0;
+#pragma unroll
+            for (int u = 0; u < kPushUnroll; ++u) {
+                deg[u] = found[u] ? deg[u] - ls[u] : 0u;
+                if (found[u]) {
+                    a.dist[v[u]] = next_level;
+                    tally.found += 1;
+                    tally.edges += deg[u];
+                }
+                mine += (deg[u] + kItemEdges - 1) / kItemEdges;
+            }
+            const uint32_t upto = warp_inclusive_scan(mine);
+            const uint32_t all = __shfl_sync(kFullMask, upto, 31);
+            if (all == 0) continue;
+            uint32_t pos = 0;
+            if (lane == 0) pos = atomicAdd(count, all);
+            pos = __shfl_sync(kFullMask, pos, 0) + upto - mine;
+#pragma unroll
+            for (int u = 0; u < kPushUnroll; ++u) {
+                const uint32_t n = (deg[u] + kItemEdges - 1) / kItemEdges;
+                if (n <= kLaneItems)
+                    for (uint32_t c = 0; c < n; ++c)
+                        g_out[pos + c] = make_uint2(ls[u] + c * kItemEdges, ls[u] + min(deg[u], (c + 1) * kItemEdges));
+                // Longer lists: the warp writes their items together.
+                unsigned longs = __ballot_sync(kFullMask, n > kLaneItems);
+                while (longs) {
+                    const int l = __ffs(longs) - 1;
+                    longs &= longs - 1;
+                    const uint32_t s = __shfl_sync(kFullMask, ls[u], l), d = __shfl_sync(kFullMask, deg[u], l);
+                    const uint32_t p = __shfl_sync(kFullMask, pos, l);
+                    for (uint32_t c = lane; c * kItemEdges < d; c += 32)
+                        g_out[p + c] = make_uint2(s + c * kItemEdges, s + min(d, (c + 1) * kItemEdges));
+                }
+                pos += n;
+            }
+        }
+    }
+}
+
+// A stretch's level over the n items that read(i) gives, by 2^log_warps warps
+// of which this is number `index`. Items are spread over as many lanes as there
+// are: a warp takes k of them with 32 / k lanes each, and with fewer items
+// than warps several warps share one (a warp whose 32 lanes issue scattered
+// atomics waits about 9 cycles per lane for them, so few lanes per warp
+// shorten the level's chain). put(at, s, e) stores item `at`
+// of the new ones, numbered by the counter `count` in shared memory; when the
+// warp's numbers pass `room`, spill(lo, hi) is called by all lanes for the numbers
+// [lo, hi) past it, before their put().
+constexpr uint32_t kLocalSolo = 8;  // edges per lane of an item before the whole warp takes it
+constexpr int kStretchUnroll = 2;
+constexpr uint32_t kLogBlockWarps = 5;
+static_assert(kSearchThreads / 32 == 1 << kLogBlockWarps, "warps per block of a stretch");
+
+template <class Read, class Spill, class Put>
+__device__ __forceinline__ void stretch_items(const BfsSearch& a, uint32_t n, uint32_t index, uint32_t log_warps,
+                                              int32_t next_level, uint32_t* count, uint32_t room, BfsLocal* c,
+                                              Read read, Spill spill, Put put) {
+    const unsigned lane = lane_id();
+    uint32_t found_n = 0, found_m = 0;  // found_m: out-edges of a level's new vertices, below E < 2^32
+    // Labels up to kPushUnroll edges of the list entries at, at + stride, ...
+    // (all 32 lanes call it).
+    auto expand = [&](uint32_t at, uint32_t end, uint32_t stride) {
+        constexpr int kPushUnroll = kStretchUnroll;
+        uint32_t v[kPushUnroll], ls[kPushUnroll], deg[kPushUnroll];
+        bool ok[kPushUnroll];
+#pragma unroll
+        for (int u = 0; u < kPushUnroll; ++u) {
+            ok[u] = at < end && end - at > u * stride;
+            v[u] = ld_nc_if(ok[u], a.targets + at + u * stride, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < kPushUnroll; ++u) {
+            ls[u] = ld_nc_if(ok[u], a.offsets + v[u], 0u);
+            deg[u] = ld_nc_if(ok[u], a.offsets + v[u] + 1, 0u);
+        }
+        uint32_t word[kPushUnroll];
+#pragma unroll
+        for (int u = 0; u < kPushUnroll; ++u)
+            word[u] = atomic_or_if(ok[u], a.visited + (v[u] >> 5), 1u << (v[u] & 31), 0xFFFFFFFFu);
+#pragma unroll
+        for (int u = 0; u < kPushUnroll; ++u) ok[u] = !((word[u] >> (v[u] & 31)) & 1u);
+        uint32_t mine = 0;
+#pragma unroll
+        for (int u = 0; u < kPushUnroll; ++u) {
+            deg[u] = ok[u] ? deg[u] - ls[u] : 0u;
+            if (ok[u]) {
+                a.dist[v[u]] = next_level;
+                found_n += 1;
+                found_m += deg[u];
+            }
+            mine += (deg[u] + kItemEdges - 1) / kItemEdges;
+        }
+        if (__ballot_sync(kFullMask, mine) == 0) return;
+        const uint32_t upto = warp_inclusive_scan(mine);
+        uint32_t pos = 0;
+        if (lane == 31) pos = atomicAdd(count, upto);
+        const uint32_t lo = __shfl_sync(kFullMask, pos, 31), hi = lo + __shfl_sync(kFullMask, upto, 31);
+        if (hi > room) spill(max(lo, room), hi);
+        pos = lo + upto - mine;
+        bool one = true;  // at most one item per vertex
+#pragma unroll
+        for (int u = 0; u < kPushUnroll; ++u) one = one && deg[u] <= kItemEdges;
+        if (__all_sync(kFullMask, one)) {
+#pragma unroll
+            for (int u = 0; u < kPushUnroll; ++u)
+                if (deg[u]) put(pos++, ls[u], ls[u] + deg[u]);
+            return;
+        }
+#pragma unroll
+        for (int u = 0; u < kPushUnroll; ++u) {
+            const uint32_t n = (deg[u] + kItemEdges - 1) / kItemEdges;
+            if (n <= kLaneItems)
+                for (uint32_t k = 0; k < n; ++k)
+                    put(pos + k, ls[u] + k * kItemEdges, ls[u] + min(deg[u], (k + 1) * kItemEdges));
+            unsigned longs = __ballot_sync(kFullMask, n > kLaneItems);
+            while (longs) {
+                const int l = __ffs(longs) - 1;
+                longs &= longs - 1;
+                const uint32_t s = __shfl_sync(kFullMask, ls[u], l), d = __shfl_sync(kFullMask, deg[u], l);
+                const uint32_t p = __shfl_sync(kFullMask, pos, l);
+                for (uint32_t k = lane; k * kItemEdges < d; k += 32)
+                    put(p + k, s + k * kItemEdges, s + min(d, (k + 1) * kItemEdges));
+            }
+            pos += n;
+        }
+    };
+    // Powers of two throughout: a division is a chain of some twenty instructions.
+    const uint32_t warps = 1u << log_warps;
+    const uint32_t k = min(32u, max(1u, (n + warps - 1) >> log_warps));
+    const uint32_t log_parts = n == 0 || n > warps ? 0u : min(kLogItemParts, log_warps - (32 - __clz(n - 1)) % 32);
+    const uint32_t log_lanes = k <= 1 ? 5u : __clz(k - 1) - 27u;  // 32 >> ceil(log2 k) lanes per item
+    const uint32_t lanes = 1u << log_lanes;
+    const uint32_t mine = lane & (lanes - 1), slot = lane >> log_lanes, part = index & ((1u << log_parts) - 1);
+    for (uint32_t base = (index >> log_parts) * k; base < n; base += (warps >> log_parts) * k) {
+        uint2 it = make_uint2(0u, 0u);
+        if (slot < k && base + slot < n) {
+            it = read(base + slot);
+            if (log_parts) {
+                const uint32_t piece = ((it.y - it.x) >> log_parts) + 1;
+                it.x = min(it.y, it.x + part * piece);
+                it.y = min(it.y, it.x + piece);
+            }
+        }
+        const uint32_t len = it.y - it.x;
+        const bool together = lanes < 32 && len > kLocalSolo * lanes;  // by the whole warp, after the others
+        const uint32_t end = together ? it.x : it.y;
+        const uint32_t longest = __reduce_max_sync(kFullMask, end - it.x);
+        for (uint32_t o = 0; o < longest; o += lanes * kStretchUnroll) {
+            const uint32_t at = it.x + o + mine;
+            expand(min(at, end), end, lanes);
+        }
+        unsigned longs = __ballot_sync(kFullMask, together && mine == 0);
+        while (longs) {
+            const int l = __ffs(longs) - 1;
+            longs &= longs - 1;
+            const uint32_t s = __shfl_sync(kFullMask, it.x, l), e = __shfl_sync(kFullMask, it.y, l);
+            for (uint32_t b = s; b < e; b += 32 * kStretchUnroll) expand(min(b + lane, e), e, 32);
+        }
+    }
+    found_n = __reduce_add_sync(kFullMask, found_n);
+    found_m = __reduce_add_sync(kFullMask, found_m);
+    if (lane == 0 && found_n) {
+        atomicAdd(&c->found, found_n);
+        atomicAdd(&c->edges, found_m);
+    }
+}
+
+// Block 0 alone: item i of the frontier from s_in below kLocalItems and
+// `shared`, else from g_in; new items to s_out below kLocalItems, else g_out.
+__device__ __forceinline__ void local_level(const BfsSearch& a, const uint2* g_in, const uint2* s_in, bool shared,
+                                            uint32_t q, uint2* g_out, uint2* s_out, BfsLocal* c, int32_t next_level) {
+    stretch_items(
+        a, q, threadIdx.x >> 5, kLogBlockWarps, next_level, &c->items, kLocalItems, c,
+        [&](uint32_t i) { return shared && i < kLocalItems ? s_in[i] : __ldcg(g_in + i); },
+        [](uint32_t, uint32_t) {},
+        [&](uint32_t p, uint32_t s, uint32_t e) {
+            if (p < kLocalItems) s_out[p] = make_uint2(s, e);
+            else g_out[p] = make_uint2(s, e);
+        });
+}
+
+// The group: block b's new items go to its segment of `out` (and, past
+// kGroupItems, to g_out at positions from the shared counter `overflow`).
+// Warp w of block b reads segment (b + w) % group, so every segment is read by
+// warps of every block, whichever block filled it. An item carries the phase
+// that wrote it; a reader that comes before the item is there polls it, so the
+// group's barrier needs no memory fence (a release waits about a microsecond
+// for the level's scattered stores).
+__device__ __forceinline__ void group_level(const BfsSearch& a, const uint2* queue, const uint4* in,
+                                            const uint32_t* counts, bool first, uint32_t q, unsigned log_group, uint4* out,
+                                            uint2* g_out, uint32_t phase, BfsLocal* c, int32_t next_level) {
+    const uint32_t w = threadIdx.x >> 5;
+    const uint32_t seg = (blockIdx.x + w) & ((1u << log_group) - 1);
+    uint32_t shift = 0;  // g_out position of a spilled item less its number
+    // The first level's items are one list in the queue. The warps that share
+    // a segment: one of every block per `group` warps.
+    stretch_items(
+        a, first ? q : counts[seg], first ? (w << log_group) + blockIdx.x : w,
+        first ? kLogBlockWarps + log_group : kLogBlockWarps, next_level,
+        &c->items, kGroupItems, c,
+        [&](uint32_t i) {
+            if (first) return __ldcg(queue + i);
+            const uint4* p = in + static_cast<size_t>(seg) * kGroupItems + i;
+            uint4 v = ld_relaxed_16(p);
+            for (unsigned k = 0; (v.z != phase - 1 || v.w != a.epoch) && k < kGridSpinLimit; ++k) v = ld_relaxed_16(p);
+            if (v.z != phase - 1 || v.w != a.epoch) {
+                atomicExch(&a.st->bar.failed, 1u);
+                return make_uint2(0u, 0u);
+            }
+            return make_uint2(v.x, v.y);
+        },
+        [&](uint32_t lo, uint32_t hi) {
+            uint32_t at = 0;
+            if (lane_id() == 0) at = atomicAdd(&a.st->overflow, hi - lo);
+            shift = __shfl_sync(kFullMask, at, 0) - lo;
+        },
+        [&](uint32_t p, uint32_t s, uint32_t e) {
+            if (p < kGroupItems) st_relaxed_16(out + static_cast<size_t>(blockIdx.x) * kGroupItems + p,
+                                               make_uint4(s, e, phase, a.epoch));
+            else g_out[shift + p] = make_uint2(s, e);
+        });
+}
+
+// The group's barrier: every block posts its counts with the phase number in
+// one 16-byte store, and the first warp of every block polls all of them (one
+// lane each): no atomics, and the counts arrive with the last poll. It orders
+// nothing else: inside a stretch the blocks share the visited bitmap (atomics)
+// and tagged items only. Entries alternate by phase parity: a block posts
+// phase p + 2 only after barrier p + 1, when everyone has read phase p.
+// False: gave up (see grid_barrier).
+__device__ __forceinline__ bool group_barrier(BfsSearchState* st, unsigned group, uint32_t phase, const BfsLocal& mine,
+                                              BfsShared& sh) {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const unsigned lane = lane_id();
+        uint4* entry = st->entry[phase & 1];
+        if (lane == 0) st_relaxed_16(entry + blockIdx.x, make_uint4(mine.items, mine.found, mine.edges, phase));
+        bool ok = true;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (lane < group) {
+            v = ld_relaxed_16(entry + lane);
+            for (unsigned i = 0; v.w != phase; ++i) {
+                if (i >= kGridSpinLimit || ((i & 1023u) == 1023u && ld_relaxed(&st->bar.failed))) {
+                    atomicExch(&st->bar.failed, 1u);
+                    ok = false;
+                    break;
+                }
+                v = ld_relaxed_16(entry + lane);
+            }
+        }
+        ok = __all_sync(kFullMask, ok);
+        if (lane < group) sh.counts[lane] = v.x;
+        const uint32_t items = __reduce_add_sync(kFullMask, v.x), found = __reduce_add_sync(kFullMask, v.y);
+        const uint32_t edges = __reduce_add_sync(kFullMask, v.z);  // below E < 2^32
+        const uint32_t over = __reduce_add_sync(kFullMask, v.x > kGroupItems ? v.x - kGroupItems : 0u);
+        if (lane == 0) {
+            sh.all = BfsLocal{found, edges, items};
+            sh.over = over;
+            sh.ok = ok ? 1u : 0u;
+        }
+    }
+    __syncthreads();
+    return sh.ok != 0;
+}
+
+// Whether one of the sector's eight entries targets[at .. at + 7] that lie in
+// [s, e) is in the frontier (`at` a multiple of 8; the arrays are padded so
+// that the last sector can be read whole). Two probes at a time, then four:
+// lanes probe scattered words, so a probe costs the SM's L1 a tag lookup per
+// lane, and in a wide frontier one of the first entries is usually a parent.
+__device__ __forceinline__ bool probe_sector(uint32_t at, uint32_t s, uint32_t e, const uint32_t (&t)[8],
+                                             const uint32_t* frontier) {
+    uint32_t w[8];
+    auto probe = [&](int i) { w[i] = ld_if(at + i >= s && at + i < e, frontier + (t[i] >> 5), 0u) >> (t[i] & 31); };
+    probe(0), probe(1);
+    if ((w[0] | w[1]) & 1u) return true;
+    probe(2), probe(3);
+    if ((w[2] | w[3]) & 1u) return true;
+    probe(4), probe(5), probe(6), probe(7);
+    return (w[4] | w[5] | w[6] | w[7]) & 1u;
+}
+
+// Pull level: kPullTiles tiles of 32 vertices per warp at a time. A lane reads
+// its list in whole 32-byte sectors (8 entries, 8 frontier probes in flight),
+// up to kSoloSectors of them; the lists still open after that are walked by
+// the warp, 128 entries per step.
+constexpr uint32_t kSoloSectors = 4;
+
+template <bool kList>
+__device__ __forceinline__ void pull_level(const BfsSearch& a, const uint32_t* frontier, uint32_t* next_frontier,
+                                           int32_t next_level, uint32_t warp, uint32_t nwarps, Tally& tally) {
+    const unsigned lane = lane_id();
+    const uint64_t tiles = kList ? ceil_div_u64(a.n_active, 32) : ceil_div_u64(a.V, 32);
+    const uint64_t step = static_cast<uint64_t>(nwarps) * kPullTiles;
+    uint32_t nv[kPullTiles], ns[kPullTiles], ne[kPullTiles], nvis[kPullTiles];
+    // The next tiles' vertices, visited words and list bounds are loaded while
+    // the current ones are probed.
+    auto fetch = [&](uint64_t t) {
+#pragma unroll
+        for (int q = 0; q < kPullTiles; ++q) {
+            nv[q] = 0;
+            ns[q] = 0;
+            ne[q] = 0;
+            nvis[q] = 0xFFFFFFFFu;
+            const uint64_t i = (t + q) * 32 + lane;
+            if (i < (kList ? a.n_active : a.V)) {
+                nv[q] = kList ? __ldg(a.active + i) : static_cast<uint32_t>(i);
+                nvis[q] = a.visited[nv[q] >> 5];
+                ns[q] = __ldg(a.offsets + nv[q]);
+                ne[q] = __ldg(a.offsets + nv[q] + 1);
+            }
+        }
+    };
+    fetch(static_cast<uint64_t>(warp) * kPullTiles);
+    for (uint64_t t0 = static_cast<uint64_t>(warp) * kPullTiles; t0 < tiles; t0 += step) {
+        uint32_t v[kPullTiles], s[kPullTiles], e[kPullTiles], vis[kPullTiles];
+        bool found[kPullTiles];
+#pragma unroll
+        for (int q = 0; q < kPullTiles; ++q) {
+            v[q] = nv[q];
+            s[q] = ns[q];
+            e[q] = ne[q];
+            vis[q] = nvis[q];
+        }
+        uint32_t t[kPullTiles][8];
+#pragma unroll
+        for (int q = 0; q < kPullTiles; ++q) {
+            if ((vis[q] >> (v[q] & 31)) & 1u) e[q] = s[q];
+            if (e[q] > s[q]) ld_stream8(a.targets + (s[q] & ~7u), t[q]);
+        }
+        fetch(t0 + step);
+#pragma unroll
+        for (int q = 0; q < kPullTiles; ++q) {
+            found[q] = false;
+            if (e[q] > s[q]) found[q] = probe_sector(s[q] & ~7u, s[q], e[q], t[q], frontier);
+        }
+#pragma unroll
+        for (int q = 0; q < kPullTiles; ++q) {
+            // Rounded up in 64 bits: lists may end within a sector of 2^32.
+            uint64_t at = (static_cast<uint64_t>(s[q]) & ~7ull) + 8;
+            for (uint32_t k = 1; k < kSoloSectors && at < e[q] && !found[q]; ++k, at += 8) {
+                ld_stream8(a.targets + at, t[q]);
+                found[q] = probe_sector(static_cast<uint32_t>(at), s[q], e[q], t[q], frontier);
+            }
+            unsigned pending = __ballot_sync(kFullMask, !found[q] && at < e[q]);
+            while (pending) {
+                const int p = __ffs(pending) - 1;
+                pending &= pending - 1;
+                const uint64_t ps = __shfl_sync(kFullMask, static_cast<uint32_t>(at), p);
+                const uint64_t pe = __shfl_sync(kFullMask, e[q], p);
+                bool hit = false;
+                for (uint64_t b = ps; b < pe && !hit; b += 128) {
+                    const uint64_t j = b + 4 * lane;
+                    uint32_t h = 0;
+                    if (j < pe) {
+                        const uint4 z = ld_stream4(reinterpret_cast<const uint4*>(a.targets + j));
+                        const uint32_t h0 = ld_if(true, frontier + (z.x >> 5), 0u);
+                        const uint32_t h1 = ld_if(j + 1 < pe, frontier + (z.y >> 5), 0u);
+                        const uint32_t h2 = ld_if(j + 2 < pe, frontier + (z.z >> 5), 0u);
+                        const uint32_t h3 = ld_if(j + 3 < pe, frontier + (z.w >> 5), 0u);
+                        h = (h0 >> (z.x & 31)) | (h1 >> (z.y & 31)) | (h2 >> (z.z & 31)) | (h3 >> (z.w & 31));
+                    }
+                    hit = __any_sync(kFullMask, h & 1u);
+                }
+                if (static_cast<int>(lane) == p) found[q] = hit;
+            }
+            if (found[q]) {
+                a.dist[v[q]] = next_level;
+                tally.found += 1;
+                tally.edges += e[q] - s[q];
+            }
+            if (kList) {
+                // The tile's vertices ascend, so they share a few words: one
+                // pair of atomics per word.
+                if (__any_sync(kFullMask, found[q])) {
+                    const unsigned peers = __match_any_sync(kFullMask, v[q] >> 5);
+                    const uint32_t bits = __reduce_or_sync(peers, found[q] ? 1u << (v[q] & 31) : 0u);
+                    if (bits && lane == static_cast<unsigned>(__ffs(peers) - 1)) {
+                        atomicOr(next_frontier + (v[q] >> 5), bits);
+                        atomicOr(a.visited + (v[q] >> 5), bits);
+                    }
+                }
+            } else {
+                const unsigned mask = __ballot_sync(kFullMask, found[q]);
+                if (lane == 0 && t0 + q < tiles) {
+                    next_frontier[t0 + q] = mask;
+                    if (mask) a.visited[t0 + q] = vis[q] | mask;
+                }
+            }
+        }
+    }
+}
+
+// The block's tallies into the level's slot, one atomic pair per block.
+__device__ __forceinline__ void flush_block_tally(const Tally& tally, BfsShared& sh, BfsSlot* slot) {
+    const uint32_t found = warp_sum(tally.found);
+    const unsigned long long edges = warp_sum(tally.edges);
+    const unsigned warp = threadIdx.x >> 5;
+    if (lane_id() == 0) {
+        sh.found[warp] = found;
+        sh.edges[warp] = edges;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const unsigned lane = lane_id();
+        const uint32_t f = warp_sum(lane < kSearchThreads / 32 ? sh.found[lane] : 0u);
+        const unsigned long long m = warp_sum(lane < kSearchThreads / 32 ? sh.edges[lane] : 0ull);
+        if (lane == 0 && f) {
+            atomicAdd(&slot->discovered, f);
+            atomicAdd(&slot->edges, m);
+        }
+    }
+}
+
+__device__ __forceinline__ void fetch_slot(const BfsSlot* slot, BfsSlot* to) {
+    const uint4* p = reinterpret_cast<const uint4*>(slot);
+    const uint4 x = __ldcg(p), y = __ldcg(p + 1);
+    reinterpret_cast<uint4*>(to)[0] = x;
+    reinterpret_cast<uint4*>(to)[1] = y;
+}
+
+template <bool kList>
+__global__ void __launch_bounds__(kSearchThreads, kSearchCtasPerSm) bfs_search_kernel(const BfsSearch a) {
+    __shared__ BfsShared sh;
+    const unsigned lane = lane_id();
+    const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    // Warps of a block are spread over the grid's work (consecutive warps of
+    // the numbering sit on different SMs), so a frontier of few items is not
+    // left to one SM.
+    const uint32_t nwarps = static_cast<uint32_t>(nthreads >> 5);
+    const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const uint32_t words = (a.V >> 5) + ((a.V & 31) ? 1u : 0u);
+    unsigned barriers = 0;
+
+    for (uint64_t i = tid; i * 4 < a.V; i += nthreads) {
+        int4 d = make_int4(-1, -1, -1, -1);
+        if (i == a.source >> 2) {
+            const uint32_t c = a.source & 3;
+            d = make_int4(c == 0 ? 0 : -1, c == 1 ? 0 : -1, c == 2 ? 0 : -1, c == 3 ? 0 : -1);
+        }
+        reinterpret_cast<int4*>(a.dist)[i] = d;
+    }
+    for (uint64_t i = tid; i < words; i += nthreads) {
+        a.visited[i] = i == a.source >> 5 ? 1u << (a.source & 31) : 0u;
+        if (kList) {
+            search_bitmap(a, 0)[i] = 0;
+            search_bitmap(a, 1)[i] = 0;
+            search_bitmap(a, 2)[i] = 0;
+        }
+    }
+    const uint32_t s0 = __ldg(a.offsets + a.source), d0 = __ldg(a.offsets + a.source + 1) - s0;
+    uint32_t items = (d0 + kItemEdges - 1) / kItemEdges;
+    if (blockIdx.x == 0)
+        for (uint32_t c = threadIdx.x; c < items; c += blockDim.x)
+            a.queue0[c] = make_uint2(s0 + c * kItemEdges, s0 + min(d0, (c + 1) * kItemEdges));
+    if (!grid_barrier(&a.st->bar, barriers)) {
+        a.st->failed = 1;
+        return;
+    }
+
+    unsigned long long m = d0, unexplored = a.E - d0;  // frontier edges, edges of unlabelled vertices
+    uint32_t n = 1, reached = 1, cur = 0, bm = 0, phase = 0, group_phase = 0;
+    int32_t level = 0;
+    bool bottom_up = false, failed = false;
+    // Ends a phase: barrier, the phase's slot into shared memory.
+    auto end_phase = [&]() -> bool {
+        BfsSlot* slot = a.st->slot + phase % 3;
+        const bool ok = grid_barrier(&a.st->bar, gridDim.x, barriers, [&] { fetch_slot(slot, &sh.slot); });
+        ++phase;
+        if (tid == 0) a.st->slot[(phase + 1) % 3] = BfsSlot{};
+        if (!ok) a.st->failed = 1;
+        return ok;
+    };
+    while (m > 0) {
+        // A search labels each vertex once, so it ends within V levels with
+        // at most V vertices reached; anything else can only be a fault.
+        if (static_cast<uint32_t>(level) >= a.V || reached > a.V) {
+            failed = true;
+            break;
+        }
+        BfsSlot* slot = a.st->slot + phase % 3;
+        // A small frontier is cheaper to push by the group than to pull (which
+        // visits every vertex), whatever is left to explore.
+        const bool pull = bfs_fixed_variant(a.symmetric != 0, bottom_up, n, m, unexplored, a.V) == kPull &&
+                          (bottom_up || m > kPullMinEdges);
+        Tally tally;
+        bool local = false;
+        if (pull) {
+            if (!bottom_up) {  // the frontier bitmap from the distances
+                uint32_t* bitmap = search_bitmap(a, bm);
+                uint32_t* next = search_bitmap(a, (bm + 1) % 3);
+                for (uint64_t w0 = static_cast<uint64_t>(warp) * 8; w0 < words;
+                     w0 += static_cast<uint64_t>(nwarps) * 8) {
+                    int32_t d[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const uint64_t v = (w0 + q) * 32 + lane;
+                        d[q] = v < a.V ? a.dist[v] : -1;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const unsigned mask = __ballot_sync(kFullMask, d[q] == level);
+                        if (lane == 0 && w0 + q < words) {
+                            bitmap[w0 + q] = mask;
+                            if (kList) next[w0 + q] = 0;
+                        }
+                    }
+                }
+                if (!end_phase()) return;
+                slot = a.st->slot + phase % 3;
+            }
+            if (kList) {  // the bitmap the next pull fills
+                uint32_t* clear = search_bitmap(a, (bm + 2) % 3);
+                for (uint64_t i = tid; i < words; i += nthreads) clear[i] = 0;
+            }
+            pull_level<kList>(a, search_bitmap(a, bm), search_bitmap(a, (bm + 1) % 3), level + 1, warp, nwarps, tally);
+            flush_block_tally(tally, sh, slot);
+        } else {
+            if (bottom_up) {  // items of the frontier from its bitmap
+                for (uint64_t w0 = static_cast<uint64_t>(warp) * 32; w0 < words;
+                     w0 += static_cast<uint64_t>(nwarps) * 32) {
+                    const uint32_t bits = w0 + lane < words ? search_bitmap(a, bm)[w0 + lane] : 0u;
+                    // Each lane takes its word's vertices one by one.
+                    for (uint32_t left = bits; __any_sync(kFullMask, left != 0); left &= left - 1) {
+                        uint32_t s = 0, d = 0;
+                        if (left) {
+                            const uint32_t v = static_cast<uint32_t>((w0 + lane) * 32 + __ffs(left) - 1);
+                            s = __ldg(a.offsets + v);
+                            d = __ldg(a.offsets + v + 1) - s;
+                        }
+                        const uint32_t mine = (d + kItemEdges - 1) / kItemEdges;
+                        const uint32_t upto = warp_inclusive_scan(mine);
+                        uint32_t at = 0;
+                        if (lane == 31 && upto) at = atomicAdd(&slot->items, upto);
+                        at = __shfl_sync(kFullMask, at, 31) + upto - mine;
+                        for (uint32_t c = 0; c < mine; ++c)
+                            search_queue(a, cur)[at + c] = make_uint2(s + c * kItemEdges, s + min(d, (c + 1) * kItemEdges));
+                    }
+                }
+                if (!end_phase()) return;
+                items = sh.slot.items;
+                slot = a.st->slot + phase % 3;
+            }
+            local = m <= kGroupEdges;
+            if (!local) {
+                push_items(a, search_queue(a, cur), items, search_queue(a, cur ^ 1), &slot->items, level + 1,
+                                  warp, nwarps, tally);
+                flush_block_tally(tally, sh, slot);
+            } else {
+                // A stretch of levels by block 0 or by the group, until the
+                // frontier outgrows them or the search ends; the others wait.
+                const bool alone = m <= kLocalEdges;
+                const unsigned log_group = alone ? 0u : min(kLogGroupBlocks, 31 - __clz(gridDim.x));
+                const unsigned group = 1u << log_group;
+                if (blockIdx.x < group) {
+                    uint32_t lq = items, lcur = cur, steps = 0, lreached = 0, ln = n;
+                    unsigned long long lm = m, lexplored = 0;
+                    if (threadIdx.x < 3) sh.local[threadIdx.x] = BfsLocal{};
+                    __syncthreads();
+                    while (true) {
+                        const int32_t next_level = level + 1 + static_cast<int32_t>(steps);
+                        BfsLocal* c = sh.local + steps % 3;
+                        uint32_t found;
+                        if (alone) {
+                            // The frontier is in sh.items[steps & 1] (in the queue before the first level).
+                            local_level(a, search_queue(a, lcur), sh.items[steps & 1], steps > 0, lq,
+                                        search_queue(a, lcur ^ 1), sh.items[(steps & 1) ^ 1], c, next_level);
+                            __syncthreads();
+                            const BfsLocal r = *c;
+                            found = r.found;
+                            lm = r.edges;
+                            if (found) lq = r.items;
+                        } else {
+                            // The frontier is in segments[steps & 1] (in the queue before the first level).
+                            constexpr size_t kHalf = static_cast<size_t>(kGroupBlocks) * kGroupItems;
+                            ++group_phase;
+                            group_level(a, search_queue(a, lcur), a.segments + (steps & 1) * kHalf, sh.counts,
+                                        steps == 0, lq, log_group, a.segments + ((steps & 1) ^ 1) * kHalf,
+                                        search_queue(a, lcur ^ 1), group_phase, c, next_level);
+                            if (!group_barrier(a.st, group, group_phase, *c, sh)) {
+                                a.st->failed = 1;
+                                return;
+                            }
+                            found = sh.all.found;
+                            lm = sh.all.edges;
+                            if (found) lq = sh.all.items;
+                        }
+                        // Slot (steps + 2) % 3 was read a level ago.
+                        if (threadIdx.x == 0) sh.local[(steps + 2) % 3] = BfsLocal{};
+                        if (found == 0) break;
+                        steps += 1;
+                        lreached += found;
+                        lexplored += lm;
+                        ln = found;
+                        lcur ^= 1u;
+                        if (lm == 0 || lm > (alone ? kLocalEdges : kGroupEdges) || steps >= kLocalMaxLevels) break;
+                        // A frontier that has shrunk far enough is block 0's
+                        // again; one that has outgrown a segment, everyone's.
+                        if (!alone && (lm <= kLocalEdges / 2 || sh.over > 0)) break;
+                    }
+                    if (alone && steps > 0)
+                        for (uint32_t i = threadIdx.x; i < min(lq, kLocalItems); i += blockDim.x)
+                            search_queue(a, lcur)[i] = sh.items[steps & 1][i];
+                    if (!alone && steps > 0) {
+                        // The segments into the queue, after what overflowed.
+                        uint32_t at = sh.over;
+                        for (unsigned b = 0; b < blockIdx.x; ++b) at += min(sh.counts[b], kGroupItems);
+                        const uint32_t mine = min(sh.counts[blockIdx.x], kGroupItems);
+                        const uint4* from = a.segments + ((steps & 1) * kGroupBlocks + blockIdx.x) *
+                                                             static_cast<size_t>(kGroupItems);
+                        for (uint32_t i = threadIdx.x; i < mine; i += blockDim.x)
+                            search_queue(a, lcur)[at + i] = make_uint2(__ldcg(from + i).x, __ldcg(from + i).y);
+                    }
+                    if (tid == 0) {
+                        a.st->overflow = 0;
+                        slot->edges = lm;
+                        slot->explored = lexplored;
+                        slot->discovered = ln;
+                        slot->items = lq;
+                        slot->levels = steps;
+                        slot->reached = lreached;
+                    }
+                }
+            }
+        }
+        if (!end_phase()) return;
+        const BfsSlot r = sh.slot;
+        if (local) {
+            level += static_cast<int32_t>(r.levels);
+            reached += r.reached;
+            unexplored -= r.explored;
+            cur ^= r.levels & 1u;
+        } else {
+            if (r.discovered == 0) break;  // the step labelled nothing: level and reached stay
+            level += 1;
+            reached += r.discovered;
+            unexplored -= r.edges;
+            if (pull) bm = (bm + 1) % 3;
+            else cur ^= 1u;
+        }
+        n = r.discovered;
+        m = r.edges;
+        items = r.items;
+        bottom_up = pull;
+    }
+    if (tid == 0) {
+        a.st->reached = reached;
+        a.st->level = level;
+        if (failed) a.st->failed = 1;
+    }
+}
+
+// ---------------------------------------------------------------- device-driven level loop (learned schedule)
 //
 // The host-driven loop reads the level counters back after every step (one
 // copy and one synchronisation per level). The device-driven loop runs a
@@ -682,8 +1536,13 @@ static Error ensure_work(GraphImpl& g) {
     GCU_TRY(w->visited.allocate(dev, words));
     GCU_TRY(w->bitmap[0].allocate(dev, words));
     GCU_TRY(w->bitmap[1].allocate(dev, words));
-    GCU_TRY(w->queue[0].allocate(dev, V));
-    GCU_TRY(w->queue[1].allocate(dev, V));
+    GCU_TRY(w->search_bitmaps.allocate(dev, 3 * words));
+    // At most one item per labelled vertex plus one per kItemEdges entries.
+    const uint64_t queue_words = 2 * (V + static_cast<uint64_t>(g.num_edges) / kItemEdges + 1);
+    GCU_TRY(w->queue[0].allocate(dev, queue_words));
+    GCU_TRY(w->queue[1].allocate(dev, queue_words));
+    GCU_TRY(w->search_segments.allocate(dev, 2 * static_cast<size_t>(kGroupBlocks) * kGroupItems));
+    GCU_TRY(w->search.allocate(dev, 1));
     GCU_TRY(w->degree_scan.allocate(dev, V + 1));
     GCU_TRY(w->counters.allocate(dev, 1));
     // Bottom-up steps read in-neighbours; they equal the CSR lists only when
@@ -993,6 +1852,50 @@ Error run_loop(GraphImpl& g, BfsWork& w, uint32_t source, BfsDevState* final_sta
     return ok();
 }
 
+// Blocks of the one-launch search: all that are resident at once for a large
+// graph, one per kSearchVertices vertices or kSearchEntries entries for a
+// small one (fewer blocks meet faster at a barrier).
+constexpr uint64_t kSearchVertices = 2048;
+constexpr uint64_t kSearchEntries = 16384;
+
+// One search as one cooperative launch.
+Error run_search(GraphImpl& g, BfsWork& w, uint32_t source) {
+    DeviceImpl& dev = *g.dev;
+    const auto kernel = w.pull_list ? bfs_search_kernel<true> : bfs_search_kernel<false>;
+    if (!w.search_grid) {
+        int per_sm = 0;
+        GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSearchThreads, 0), "occupancy");
+        const uint64_t most = static_cast<uint64_t>(dev.sm_count) * std::max(1, std::min(per_sm, kSearchCtasPerSm));
+        const uint64_t want = std::max<uint64_t>(
+            {1, ceil_div_u64(g.num_nodes, kSearchVertices), ceil_div_u64(g.num_edges, kSearchEntries)});
+        w.search_grid = static_cast<unsigned>(std::min(want, most));
+    }
+    BfsSearch a{};
+    a.offsets = g.offsets.ptr;
+    a.targets = g.targets.ptr;
+    a.active = w.pull_list ? w.active.ptr : nullptr;
+    a.V = g.num_nodes;
+    a.E = g.num_edges;
+    a.n_active = w.n_active;
+    a.source = source;
+    a.symmetric = w.symmetric == 1 ? 1 : 0;
+    a.dist = w.dist.ptr;
+    a.visited = w.visited.ptr;
+    a.bitmaps = w.search_bitmaps.ptr;
+    a.bitmap_words = static_cast<uint32_t>(ceil_div_u64(g.num_nodes, 32));
+    a.queue0 = reinterpret_cast<uint2*>(w.queue[0].ptr);
+    a.queue1 = reinterpret_cast<uint2*>(w.queue[1].ptr);
+    a.segments = w.search_segments.ptr;
+    a.epoch = ++w.search_epoch;
+    a.st = w.search.ptr;
+    GCU_CUDA(cudaMemsetAsync(w.search.ptr, 0, sizeof(BfsSearchState), dev.stream), "memset");
+    GCU_LAUNCH_COOP(dev, "bfs_search", kernel, w.search_grid, kSearchThreads, 0, a);
+    GCU_CUDA(cudaMemcpyAsync(&w.host_search, &w.search.ptr->reached, sizeof(w.host_search), cudaMemcpyDeviceToHost,
+                             dev.stream),
+             "copy");
+    return ok();
+}
+
 uint64_t mix64(uint64_t z) {
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
@@ -1011,6 +1914,16 @@ Error bfs(GraphImpl& g, uint32_t source, int32_t* host_distances, uint32_t* reac
     DegreeStats stats;
     if (net) GCU_TRY(degree_stats(g, &stats));
 
+    if (dev.bfs_device_loop && !dev.kernel_timing && !net) {
+        GCU_TRY(run_search(g, w, source));
+        if (host_distances)
+            GCU_TRY(copy_to_host(dev, host_distances, w.dist.ptr, sizeof(int32_t) * g.num_nodes));
+        GCU_TRY(dev.sync());
+        if (w.host_search.failed) return kernel_error("BFS stopped on an impossible state");
+        *reachable = w.host_search.reached;
+        *max_depth = w.host_search.level;
+        return ok();
+    }
     if (dev.bfs_device_loop && !dev.kernel_timing && !w.loop_unavailable) {
         if (!w.loop_exec || w.loop_net != static_cast<const void*>(net)) {
             // A driver that cannot build the conditional graph leaves the

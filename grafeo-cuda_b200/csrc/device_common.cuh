@@ -79,6 +79,49 @@ __device__ __forceinline__ uint4 ld_stream4(const uint4* p) {
     return v;
 }
 
+// Predicated accesses (one instruction, no branch): several of them in a row
+// stay in flight together, where `if (p) x = atomicOr(...)` waits for each
+// result inside its own branch (1,790 cycles for four atomics in a row in
+// the BFS push, about 600 this way). Without `p` nothing is accessed and the
+// result is `other`.
+__device__ __forceinline__ uint32_t atomic_or_if(bool p, uint32_t* a, uint32_t bits, uint32_t other) {
+    uint32_t v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\tmov.u32 %0, %4;\n\t"
+                 "@q atom.global.or.b32 %0, [%2], %3;\n\t}"
+                 : "=&r"(v)
+                 : "r"(static_cast<uint32_t>(p)), "l"(a), "r"(bits), "r"(other)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_if(bool p, const uint32_t* a, uint32_t other) {
+    uint32_t v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\tmov.u32 %0, %3;\n\t@q ld.global.u32 %0, [%2];\n\t}"
+                 : "=&r"(v)
+                 : "r"(static_cast<uint32_t>(p)), "l"(a), "r"(other));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_cg_if(bool p, const uint32_t* a, uint32_t other) {
+    uint32_t v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\tmov.u32 %0, %3;\n\t@q ld.global.cg.u32 %0, [%2];\n\t}"
+                 : "=&r"(v)
+                 : "r"(static_cast<uint32_t>(p)), "l"(a), "r"(other));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_nc_if(bool p, const uint32_t* a, uint32_t other) {
+    uint32_t v;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\tmov.u32 %0, %3;\n\t@q ld.global.nc.u32 %0, [%2];\n\t}"
+        : "=&r"(v)
+        : "r"(static_cast<uint32_t>(p)), "l"(a), "r"(other));
+    return v;
+}
+
+// One 32-byte sector (sm_100's 256-bit load; p 32-byte aligned).
+__device__ __forceinline__ void ld_stream8(const uint32_t* p, uint32_t (&v)[8]) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(p));
+}
+
 // First index in [lo, hi) with a[idx] >= val.
 __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* a, uint32_t lo, uint32_t hi, uint32_t val) {
     while (lo < hi) {
@@ -103,6 +146,77 @@ __device__ __forceinline__ uint32_t row_of_entry(const uint32_t* offsets, uint32
             hi = mid;
     }
     return lo;
+}
+
+// ---------------------------------------------------------------- grid barrier
+// Barrier over the blocks of one cooperative launch (all resident at once).
+// `arrived` counts arrivals and only grows (zeroed before the launch), so a
+// phase needs one atomic per block and no reset; the comparison is by signed
+// difference, so the count may wrap. A block that waits for kGridSpinLimit
+// polls (seconds, against phases of at most milliseconds) gives up: it raises
+// `failed`, every block returns false from its barrier, and the kernel ends
+// with the flag set instead of hanging. Plain loads after the barrier see
+// what any block stored before it; data that changes inside the kernel must
+// not be read through the read-only (nc) path.
+struct GridBarrier {
+    unsigned arrived;
+    unsigned failed;
+};
+constexpr unsigned kGridSpinLimit = 1u << 25;
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void red_release_add(unsigned* p, unsigned x) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
+}
+
+// Every thread of the `blocks` blocks that share `bar` calls it; `phase` is the
+// block's count of barriers on `bar` so far; thread 0 of every block runs after() once all have arrived
+// (to fetch what the block needs into shared memory under the same block
+// barrier). False: another block is missing, the kernel must return.
+template <class After>
+__device__ __forceinline__ bool grid_barrier(GridBarrier* bar, unsigned blocks, unsigned& phase, After after) {
+    __shared__ unsigned s_ok;
+    ++phase;
+    if (blocks == 1) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();  // drops L1 lines that atomics have outdated
+            after();
+        }
+        __syncthreads();
+        return true;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned target = phase * blocks;
+        red_release_add(&bar->arrived, 1u);  // after every store of the block (the block barrier above)
+        unsigned ok = 1;
+        for (unsigned i = 0; static_cast<int>(ld_relaxed(&bar->arrived) - target) < 0; ++i) {
+            if (i >= kGridSpinLimit || ((i & 1023u) == 1023u && ld_relaxed(&bar->failed))) {
+                atomicExch(&bar->failed, 1u);
+                ok = 0;
+                break;
+            }
+        }
+        ld_acquire(&bar->arrived);
+        after();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+__device__ __forceinline__ bool grid_barrier(GridBarrier* bar, unsigned& phase) {
+    return grid_barrier(bar, gridDim.x, phase, [] {});
 }
 
 // ---------------------------------------------------------------- entry tiles

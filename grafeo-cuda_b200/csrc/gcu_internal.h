@@ -417,3 +417,28 @@ std::string batch_tuning(const BatchImpl& b);
             return ::gcu::kernel_error(std::string(name) + " launch failed: " +            \
                                        cudaGetErrorString(_le));                           \
     } while (0)
+
+// The same for a kernel whose blocks wait for one another (grid_barrier): a
+// cooperative launch, which the driver refuses unless every block is resident.
+#define GCU_LAUNCH_COOP(devref, name, kernel, grid, block, smem, ...)                      \
+    do {                                                                                   \
+        cudaEvent_t _ev = nullptr;                                                         \
+        (devref).before_launch(name, &_ev);                                                \
+        cudaLaunchAttribute _at[1];                                                        \
+        _at[0].id = cudaLaunchAttributeCooperative;                                        \
+        _at[0].val.cooperative = 1;                                                        \
+        cudaLaunchConfig_t _cfg = {};                                                      \
+        _cfg.gridDim = dim3(grid);                                                         \
+        _cfg.blockDim = dim3(block);                                                       \
+        _cfg.dynamicSmemBytes = (smem);                                                    \
+        _cfg.stream = (devref).stream;                                                     \
+        _cfg.attrs = _at;                                                                  \
+        _cfg.numAttrs = 1;                                                                 \
+        cudaError_t _le = cudaLaunchKernelEx(&_cfg, kernel, __VA_ARGS__);                  \
+        (devref).after_launch(name, _ev);                                                  \
+        if (_le != cudaSuccess) {                                                          \
+            cudaGetLastError();                                                            \
+            return ::gcu::kernel_error(std::string(name) + " launch failed: " +            \
+                                       cudaGetErrorString(_le));                           \
+        }                                                                                  \
+    } while (0)
