@@ -11,24 +11,27 @@
 //    else the fastest of the valid variants timed once on the batch); the
 //    wedge kernels add each DAG source's triangles into a per-vertex counter
 //    and a block per graph sums its vertices.
+//  * BFS and PageRank run over the union as a whole, one cooperative launch
+//    each: every level or iteration is one pass over the entries of all graphs
+//    that are still at work, and the blocks meet at a grid barrier. The entries
+//    are read as a stream of 256-entry chunks (8 consecutive entries per lane,
+//    a byte per entry says which row it belongs to), so a pass is spread evenly
+//    over the GPU whatever the sizes of the graphs; a graph has no CTA of its
+//    own to wait for. Rows that cross chunks leave parts that are joined after
+//    the pass.
 //  * BFS from S <= 32 sources per graph: multi-source BFS (Then et al., VLDB
-//    2015) with one S-bit mask per vertex for visited / frontier / next: a CTA
-//    owns a graph and runs all its levels itself (pull: a vertex ORs its
-//    neighbours' frontier masks, stopping once every missing bit is found),
-//    so there is no host round trip and no grid-wide barrier; bit k of a
-//    vertex's mask appearing at level L is distance L from source k.
+//    2015) with one S-bit mask per vertex. A level ORs the neighbours' masks
+//    into the vertex's own, from one mask array into another; a bit that is new
+//    at level L is distance L. (The masks hold every source seen so far, not
+//    the last level's only: an older bit of a neighbour has reached the vertex
+//    already.)
 //  * Personalised PageRank from K seeds per graph (teleport 1/K per seed,
-//    repeats add up; the formula of gcu_personalized_pagerank): a CTA owns a
-//    graph and iterates to its own convergence (L1 change < tol, FP64 block
-//    reductions of the residual and the dangling mass), FP32 row sums (a lane
-//    per short row, a warp per row of >= 32 entries).
-//  * CTAs take graphs from a queue ordered by entry count, largest first
-//    (longest-processing-time order). The CTA size of the BFS and PageRank
-//    kernels is autotuned per batch (256 / 512 / 1024 threads, each timed
-//    once on the whole batch, the fastest kept).
+//    repeats add up; the formula of gcu_personalized_pagerank): every graph
+//    iterates to its own convergence (L1 change < tol; the change and the
+//    dangling mass are summed per graph as 64-bit fixed-point integers, so the
+//    result does not depend on which warp did what), FP64 row sums.
 // No reference counterpart: the reference runs one graph per call.
 #include <algorithm>
-#include <numeric>
 
 #include "device_common.cuh"
 #include "gcu_internal.h"
@@ -93,198 +96,554 @@ __global__ void batch_extract_kernel(const uint32_t* __restrict__ offsets, const
     }
 }
 
-// Multi-source BFS, one CTA per graph at a time (see the file comment).
-template <int kThreads>
-__global__ void __launch_bounds__(kThreads) batch_bfs_kernel(
-    const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ vbase,
-    const uint32_t* __restrict__ order, uint32_t G, const uint32_t* __restrict__ sources, uint32_t S,
-    uint32_t* __restrict__ visited, uint32_t* buf_a, uint32_t* buf_b, int32_t* __restrict__ dist, uint64_t Vt,
-    uint32_t* __restrict__ reachable, int32_t* __restrict__ max_depth, uint32_t* __restrict__ next_graph) {
-    constexpr int kWarps = kThreads / 32;
-    __shared__ uint32_t s_item;
-    __shared__ uint32_t s_or[kWarps];
-    __shared__ uint32_t s_count[kMaxBatchSources];
-    __shared__ int32_t s_last[kMaxBatchSources];
-    const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-    const uint32_t full = S >= 32 ? 0xFFFFFFFFu : ((1u << S) - 1u);
-    while (true) {
-        if (tid == 0) s_item = atomicAdd(next_graph, 1u);
-        __syncthreads();
-        const uint32_t h = s_item;
-        if (h >= G) break;
-        const uint32_t g = order[h];
-        const uint32_t vb = vbase[g], ve = vbase[g + 1];
-        uint32_t* frontier = buf_a;
-        uint32_t* next = buf_b;
-        for (uint32_t v = vb + tid; v < ve; v += kThreads) {
-            visited[v] = 0;
-            frontier[v] = 0;
+// ---------------------------------------------------------------- passes over the union's entries
+
+constexpr uint32_t kBatchChunk = 256;     // entries per warp step
+constexpr int kBatchThreads = 512;
+constexpr int kBatchCtasPerSm = 3;
+constexpr uint32_t kBatchRun = 2;         // consecutive chunks per warp turn (neighbouring chunks share their graph's lines)
+constexpr uint32_t kNoGraph = 0xFFFFFFFFu;
+
+// Measured on one B200, 256 graphs of the generated corpus (6 M vertices, 106 M
+// entries), a CTA per graph before: BFS from 16 sources 49.1 -> 3.7 ms (the four
+// or five graphs of 4 M entries ran alone at the end), 20 PageRank iterations
+// 74.1 -> 8.1 ms (260 G entries/s; the bound is the L1's rate of scattered
+// gathers, as in the single-graph SpMV, plus eight words per finished row). CTA
+// shapes: 2 x 512 threads (64 registers) 8.8 / 4.0 ms, 3 x 512 (40) 8.1 / 3.7;
+// turns of 1 / 4 / 16 chunks 8.9 / 8.8 / 9.6 ms with two CTAs.
+
+// The union's rows with entries, packed ("rows" below are indices into this
+// list), and its vertices without.
+struct BatchRows {
+    const uint32_t* targets;
+    const uint32_t* row_vertex;  // union vertex of each row
+    const uint32_t* row_graph;
+    const uint32_t* row_start;   // first entry of each row; [n_rows] = E
+    const uint32_t* chunk_row;   // row of each chunk's first entry
+    const uint8_t* delta;        // per entry: its row minus its chunk's first row
+    const uint4* split;          // (row, first chunk, last chunk, 0) of the rows that cross chunks
+    const uint32_t* lone;        // vertices without entries
+    const uint32_t* lone_graph;
+    uint32_t E, n_rows, n_chunks, n_split, n_lone;
+};
+
+struct BatchRunState {
+    GridBarrier bar;
+    uint32_t active[3];  // graphs at work in this pass, rotating
+};
+
+__global__ void batch_row_flags_kernel(const uint32_t* __restrict__ offsets, uint32_t V, uint32_t* __restrict__ flag) {
+    for (uint64_t v = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < V;
+         v += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+        flag[v] = offsets[v + 1] > offsets[v] ? 1u : 0u;
+}
+
+__global__ void batch_rows_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ pos,
+                                  const uint32_t* __restrict__ vbase, uint32_t G, uint32_t V, uint32_t E,
+                                  uint32_t* __restrict__ row_vertex, uint32_t* __restrict__ row_graph,
+                                  uint32_t* __restrict__ row_start, uint32_t* __restrict__ lone,
+                                  uint32_t* __restrict__ lone_graph, uint32_t* __restrict__ lone_count) {
+    for (uint64_t v = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; v <= V;
+         v += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        if (v == V) {
+            row_start[pos[V]] = E;
+            continue;
         }
-        if (tid < kMaxBatchSources) {
-            s_count[tid] = 0;
-            s_last[tid] = 0;
+        // The last graph that begins at or before v (empty graphs share a base with their successor).
+        uint32_t lo = 0, hi = G;
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (vbase[mid] <= v) lo = mid;
+            else hi = mid;
         }
-        __syncthreads();
-        if (tid < S) {
-            const uint32_t s = vb + sources[static_cast<uint64_t>(g) * S + tid];
-            atomicOr(visited + s, 1u << tid);
-            atomicOr(frontier + s, 1u << tid);
-            if (dist) dist[tid * Vt + s] = 0;
+        const uint32_t r = pos[v], i = static_cast<uint32_t>(v) - r;
+        if (pos[v + 1] > r) {
+            row_vertex[r] = static_cast<uint32_t>(v);
+            row_graph[r] = lo;
+            row_start[r] = offsets[v];
+        } else {
+            lone[i] = static_cast<uint32_t>(v);
+            lone_graph[i] = lo;
+            atomicAdd(lone_count + lo, 1u);
         }
-        __syncthreads();
-        int32_t level = 0;
-        while (true) {
-            uint32_t any = 0;
-            for (uint32_t v = vb + tid; v < ve; v += kThreads) {
-                const uint32_t vis = visited[v];
-                uint32_t nw = 0;
-                if (vis != full) {
-                    uint32_t m = 0;
-                    const uint32_t e = offsets[v + 1];
-                    for (uint32_t j = offsets[v]; j < e; ++j) {
-                        m |= frontier[targets[j]];
-                        if ((m | vis) == full) break;
-                    }
-                    nw = m & ~vis;
-                    if (nw && dist) {
-                        uint32_t bits = nw;
-                        while (bits) {
-                            const uint32_t k = __ffs(bits) - 1;
-                            dist[k * Vt + v] = level + 1;
-                            bits &= bits - 1;
-                        }
-                    }
-                    any |= nw;
-                }
-                next[v] = nw;
-            }
-            any = __reduce_or_sync(kFullMask, any);
-            if (lane == 0) s_or[warp] = any;
-            __syncthreads();
-            uint32_t all = 0;
+    }
+}
+
+__global__ void batch_chunk_rows_kernel(const uint32_t* __restrict__ row_start, uint32_t n_rows,
+                                        uint32_t* __restrict__ chunk_row, uint32_t* __restrict__ split_flag) {
+    for (uint64_t r = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < n_rows;
+         r += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        const uint64_t s = row_start[r], e = row_start[r + 1];
+        const uint64_t c_first = s / kBatchChunk, c_last = (e - 1) / kBatchChunk;
+        for (uint64_t c = (s + kBatchChunk - 1) / kBatchChunk; c <= c_last; ++c) chunk_row[c] = static_cast<uint32_t>(r);
+        split_flag[r] = c_first != c_last ? 1u : 0u;
+    }
+}
+
+__global__ void batch_split_rows_kernel(const uint32_t* __restrict__ row_start, uint32_t n_rows,
+                                        const uint32_t* __restrict__ pos, uint4* __restrict__ split) {
+    for (uint64_t r = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < n_rows;
+         r += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+        if (pos[r + 1] > pos[r])
+            split[pos[r]] = make_uint4(static_cast<uint32_t>(r), row_start[r] / kBatchChunk,
+                                       (row_start[r + 1] - 1) / kBatchChunk, 0u);
+}
+
+__global__ void __launch_bounds__(256) batch_delta_kernel(const uint32_t* __restrict__ row_start, uint32_t n_rows,
+                                                          uint32_t E, const uint32_t* __restrict__ chunk_row,
+                                                          uint8_t* __restrict__ delta) {
+    for_each_entry<256, 4>(row_start, n_rows, E, [&](uint32_t j, uint32_t r) {
+        delta[j] = static_cast<uint8_t>(r - chunk_row[j / kBatchChunk]);
+    });
+}
+
+// One pass: chunk after chunk, a warp each (kBatchRun consecutive chunks per
+// turn), 8 consecutive entries per lane. op gives
+//   begin(g0, g1)      whether a graph in [g0, g1] is at work (else the chunk is skipped)
+//   want(row)          whether the row's entries have to be gathered
+//   gather(target), add(x, y), zero()
+//   finish(row, x)     the row's result
+//   part(i, x)         part i of a row that crosses chunks: 2c for the end of a row
+//                      begun before chunk c, 2c + 1 for a row that goes on after it
+//   flush()            after every turn (all lanes)
+// Runs of equal rows are joined per lane, then across lanes by a segmented
+// scan; the lane where a row ends finishes it.
+template <class Op>
+__device__ __forceinline__ void batch_pass(const BatchRows& R, Op& op) {
+    using T = typename Op::T;
+    const unsigned lane = lane_id();
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    for (uint64_t c0 = static_cast<uint64_t>(warp) * kBatchRun; c0 < R.n_chunks;
+         c0 += static_cast<uint64_t>(warps) * kBatchRun) {
+        const uint32_t c1 = static_cast<uint32_t>(min_u64(c0 + kBatchRun, R.n_chunks));
+        for (uint32_t c = static_cast<uint32_t>(c0); c < c1; ++c) {
+            const uint64_t e0 = static_cast<uint64_t>(c) * kBatchChunk;
+            const uint64_t eb = e0 + 8 * lane;
+            const uint32_t rbase = __ldg(R.chunk_row + c);
+            const uint2 dl = ld_stream2(reinterpret_cast<const uint2*>(R.delta + eb));
+            const bool any = eb < R.E;
+            uint32_t row[8];
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) all |= s_or[w];
-            if (all == 0) break;  // the same for every thread of the block
-            if (tid < S && ((all >> tid) & 1u)) s_last[tid] = level + 1;
-            for (uint32_t v = vb + tid; v < ve; v += kThreads) visited[v] |= next[v];
-            uint32_t* t = frontier;
-            frontier = next;
-            next = t;
-            ++level;
-            __syncthreads();
+            for (int i = 0; i < 8; ++i)
+                row[i] = eb + i < R.E ? rbase + (((i < 4 ? dl.x : dl.y) >> (8 * (i & 3))) & 0xFFu) : kNoGraph;
+            // The last row: of the last entry (only the last chunk can end early).
+            const uint64_t last = min_u64(e0 + kBatchChunk, R.E) - 1 - e0;
+            const uint32_t mine_last = rbase + ((last & 4 ? dl.y : dl.x) >> (8 * (last & 3)) & 0xFFu);
+            const uint32_t rlast = __shfl_sync(kFullMask, mine_last, static_cast<int>(last >> 3));
+            if (!op.begin(__ldg(R.row_graph + rbase), __ldg(R.row_graph + rlast))) continue;
+            const bool first_split = __ldg(R.row_start + rbase) < e0;
+            const bool last_split = __ldg(R.row_start + rlast + 1) > e0 + kBatchChunk;
+            bool want[8];
+            bool some = false;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (!Op::kSkips) want[i] = row[i] != kNoGraph;
+                else if (i > 0 && row[i] == row[i - 1]) want[i] = want[i - 1];
+                else want[i] = row[i] != kNoGraph && op.want(row[i]);
+                some = some || want[i];
+            }
+            uint32_t t[8] = {};
+            if (Op::kSkips ? some : any) ld_stream8(R.targets + eb, t);
+            T val[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) val[i] = op.gather(want[i], t[i]);
+            T head = Op::zero(), acc = Op::zero();
+            bool multi = false;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                acc = Op::add(acc, val[i]);
+                if (i < 7 && row[i + 1] != row[i]) {
+                    if (!multi) {
+                        head = acc;
+                        multi = true;
+                    } else {
+                        op.finish(row[i], acc);
+                    }
+                    acc = Op::zero();
+                }
+            }
+            const uint32_t rf = row[0], rl = row[7];
+            const uint32_t prev_last = __shfl_up_sync(kFullMask, rl, 1);
+            const uint32_t next_first = __shfl_down_sync(kFullMask, rf, 1);
+            const bool carry_in = lane > 0 && prev_last == rf;
+            bool head_flag = multi || !carry_in;
+            T S = acc;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const T su = __shfl_up_sync(kFullMask, S, d);
+                const bool fu = __shfl_up_sync(kFullMask, head_flag, d);
+                if (lane >= static_cast<unsigned>(d)) {
+                    if (!head_flag) S = Op::add(S, su);
+                    head_flag = head_flag || fu;
+                }
+            }
+            const T carry = __shfl_up_sync(kFullMask, S, 1);
+            if (multi && rf != kNoGraph) {  // the first run ends in this lane
+                const T total = carry_in ? Op::add(head, carry) : head;
+                if (rf == rbase && first_split) op.part(2 * static_cast<uint64_t>(c), total);
+                else op.finish(rf, total);
+            }
+            const bool continues = lane < 31 && next_first == rl;
+            if (!continues && rl != kNoGraph) {  // the last run ends at this lane's end
+                if (rl == rlast && last_split) op.part(2 * static_cast<uint64_t>(c) + 1, S);
+                else if (rl == rbase && first_split) op.part(2 * static_cast<uint64_t>(c), S);
+                else op.finish(rl, S);
+            }
         }
-        // Reached vertices per source: lane k of every warp counts bit k.
+        op.flush();
+    }
+}
+
+// The rows that cross chunks, a thread each: their parts in chunk order.
+template <class Op>
+__device__ __forceinline__ void batch_split_pass(const BatchRows& R, Op& op) {
+    using T = typename Op::T;
+    for (uint64_t b = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) & ~31ull; b < R.n_split;
+         b += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        const uint64_t i = b + lane_id();
+        if (i < R.n_split) {
+            const uint4 s = R.split[i];
+            const uint32_t g = __ldg(R.row_graph + s.x);
+            if (op.begin(g, g)) {
+                T x = op.parts(2 * static_cast<uint64_t>(s.y) + 1);
+                for (uint32_t c = s.y + 1; c < s.z; ++c) x = Op::add(x, op.parts(2 * static_cast<uint64_t>(c) + 1));
+                x = Op::add(x, op.parts(2 * static_cast<uint64_t>(s.z)));
+                op.finish(s.x, x);
+            }
+        }
+        op.flush();
+    }
+}
+
+// ---------------------------------------------------------------- multi-source BFS
+
+struct BatchBfs {
+    BatchRows rows;
+    const uint32_t* offsets;
+    const uint32_t* vbase;
+    const uint32_t* sources;
+    uint32_t G, V, S, full;
+    uint32_t *mask_a, *mask_b;
+    uint32_t* parts;
+    int32_t* dist;  // NULL: no distances
+    uint32_t* fresh;      // [3][G]: sources that reached something new, rotating by level
+    uint32_t* stop;       // [G]: the level a graph stopped before
+    uint32_t* reachable;
+    int32_t* max_depth;
+    BatchRunState* st;
+};
+
+struct BfsOp {
+    using T = uint32_t;
+    static constexpr bool kSkips = true;
+    const BatchBfs& a;
+    const uint32_t* in;
+    uint32_t* out;
+    const uint32_t* prev_fresh;  // [G], the level before (NULL at level 0)
+    uint32_t* fresh;
+    uint32_t level;
+    uint32_t my_graph = kNoGraph, my_fresh = 0;
+
+    static __device__ __forceinline__ T zero() { return 0u; }
+    static __device__ __forceinline__ T add(T x, T y) { return x | y; }
+    // A graph works on while the level before found something new.
+    __device__ __forceinline__ bool works(uint32_t g) const {
+        return a.stop[g] > level && (prev_fresh == nullptr || prev_fresh[g] != 0);
+    }
+    __device__ __forceinline__ bool begin(uint32_t g0, uint32_t g1) const {
+        for (uint32_t g = g0; g <= g1; ++g)
+            if (works(g)) return true;
+        return false;
+    }
+    __device__ __forceinline__ bool want(uint32_t r) const { return in[__ldg(a.rows.row_vertex + r)] != a.full; }
+    __device__ __forceinline__ T gather(bool p, uint32_t t) const { return ld_if(p, in + t, 0u); }
+    __device__ __forceinline__ void part(uint64_t i, T x) { a.parts[i] = x; }
+    __device__ __forceinline__ T parts(uint64_t i) const { return a.parts[i]; }
+    __device__ __forceinline__ void finish(uint32_t r, T m) {
+        const uint32_t v = __ldg(a.rows.row_vertex + r);
+        const uint32_t old = in[v], now = (m & ~old);
+        out[v] = old | m;
+        if (!now) return;
+        if (a.dist)
+            for (uint32_t bits = now; bits; bits &= bits - 1)
+                a.dist[static_cast<uint64_t>(__ffs(bits) - 1) * a.V + v] = static_cast<int32_t>(level) + 1;
+        const uint32_t g = __ldg(a.rows.row_graph + r);
+        if (g != my_graph) {
+            if (my_fresh) atomicOr(fresh + my_graph, my_fresh);
+            my_graph = g;
+            my_fresh = 0;
+        }
+        my_fresh |= now;
+    }
+    __device__ __forceinline__ void flush() {
+        const unsigned has = __ballot_sync(kFullMask, my_fresh != 0);
+        if (has) {
+            const uint32_t g = __shfl_sync(kFullMask, my_graph, __ffs(has) - 1);
+            const uint32_t bits = __reduce_or_sync(kFullMask, my_graph == g ? my_fresh : 0u);
+            if (lane_id() == static_cast<unsigned>(__ffs(has) - 1)) atomicOr(fresh + g, bits);
+            if (my_fresh && my_graph != g) atomicOr(fresh + my_graph, my_fresh);
+        }
+        my_graph = kNoGraph;
+        my_fresh = 0;
+    }
+};
+
+__global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_bfs_kernel(const BatchBfs a) {
+    __shared__ uint32_t s_active;
+    __shared__ uint32_t s_count[kMaxBatchSources];
+    const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    unsigned barriers = 0;
+    for (uint64_t v = tid; v < a.V; v += nthreads) {
+        a.mask_a[v] = 0;
+        a.mask_b[v] = 0;
+    }
+    for (uint64_t g = tid; g < a.G; g += nthreads) {
+        for (int q = 0; q < 3; ++q) a.fresh[static_cast<uint64_t>(q) * a.G + g] = 0;
+        a.stop[g] = a.vbase[g + 1] > a.vbase[g] ? 0xFFFFFFFFu : 0u;
+    }
+    for (uint64_t i = tid; i < static_cast<uint64_t>(a.G) * a.S; i += nthreads) {
+        a.reachable[i] = 0;
+        a.max_depth[i] = 0;
+    }
+    if (!grid_barrier(&a.st->bar, barriers)) return;
+    for (uint64_t i = tid; i < static_cast<uint64_t>(a.G) * a.S; i += nthreads) {
+        const uint32_t g = static_cast<uint32_t>(i / a.S), k = static_cast<uint32_t>(i % a.S);
+        const uint32_t v = a.vbase[g] + a.sources[i];
+        // Both arrays: a vertex without entries is never written again.
+        atomicOr(a.mask_a + v, 1u << k);
+        atomicOr(a.mask_b + v, 1u << k);
+        if (a.dist) a.dist[static_cast<uint64_t>(k) * a.V + v] = 0;
+    }
+    if (!grid_barrier(&a.st->bar, barriers)) return;
+    // Each level labels something in some graph, or is the last.
+    for (uint32_t level = 0;; ++level) {
+        BfsOp op{a, (level & 1) ? a.mask_b : a.mask_a, (level & 1) ? a.mask_a : a.mask_b,
+                 level ? a.fresh + static_cast<uint64_t>((level + 2) % 3) * a.G : nullptr,
+                 a.fresh + static_cast<uint64_t>(level % 3) * a.G, level};
+        for (uint64_t g = tid; g < a.G; g += nthreads) {
+            a.fresh[static_cast<uint64_t>((level + 1) % 3) * a.G + g] = 0;  // last read a level ago
+            if (a.stop[g] <= level) continue;
+            if (level) {
+                uint32_t bits = op.prev_fresh[g];
+                if (!bits) {
+                    a.stop[g] = level;
+                    continue;
+                }
+                for (; bits; bits &= bits - 1)
+                    a.max_depth[g * static_cast<uint64_t>(a.S) + __ffs(bits) - 1] = static_cast<int32_t>(level);
+            }
+            atomicAdd(a.st->active + level % 3, 1u);
+        }
+        if (tid == 0) a.st->active[(level + 1) % 3] = 0;
+        batch_pass(a.rows, op);
+        if (!grid_barrier(&a.st->bar, gridDim.x, barriers, [&] { s_active = __ldcg(a.st->active + level % 3); })) return;
+        if (s_active == 0) break;
+        batch_split_pass(a.rows, op);
+        if (!grid_barrier(&a.st->bar, barriers)) return;
+    }
+    // Reached vertices per source: lane k of every warp counts bit k of its
+    // graph's vertices. A graph that has stopped has the same masks in both arrays.
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    for (uint32_t g = blockIdx.x; g < a.G; g += gridDim.x) {
+        if (threadIdx.x < kMaxBatchSources) s_count[threadIdx.x] = 0;
+        __syncthreads();
         uint32_t cnt = 0;
-        for (uint32_t base = vb + warp * 32; base < ve; base += kThreads) {
+        const uint32_t ve = a.vbase[g + 1];
+        for (uint32_t base = a.vbase[g] + warp * 32; base < ve; base += kBatchThreads) {
             const uint32_t v = base + lane;
-            const uint32_t vis = v < ve ? visited[v] : 0u;
-            for (uint32_t k = 0; k < S; ++k) {
+            const uint32_t vis = v < ve ? a.mask_a[v] : 0u;
+            for (uint32_t k = 0; k < a.S; ++k) {
                 const unsigned b = __ballot_sync(kFullMask, (vis >> k) & 1u);
                 if (lane == k) cnt += __popc(b);
             }
         }
-        if (lane < S && cnt) atomicAdd(&s_count[lane], cnt);
+        if (lane < a.S && cnt) atomicAdd(&s_count[lane], cnt);
         __syncthreads();
-        if (tid < S) {
-            reachable[static_cast<uint64_t>(g) * S + tid] = s_count[tid];
-            max_depth[static_cast<uint64_t>(g) * S + tid] = s_last[tid];
-        }
+        if (threadIdx.x < a.S) a.reachable[static_cast<uint64_t>(g) * a.S + threadIdx.x] = s_count[threadIdx.x];
         __syncthreads();
     }
 }
 
-// Personalised PageRank, one CTA per graph at a time (see the file comment).
-template <int kThreads>
-__global__ void __launch_bounds__(kThreads) batch_ppr_kernel(
-    const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ vbase,
-    const uint32_t* __restrict__ order, uint32_t G, const float* __restrict__ tele, float damping,
-    uint32_t max_iterations, double tolerance, float* rank_a, float* rank_b, float* contrib_a, float* contrib_b,
-    float* __restrict__ ranks_out, uint32_t* __restrict__ iterations, uint8_t* __restrict__ converged,
-    uint32_t* __restrict__ next_graph) {
-    __shared__ uint32_t s_item;
-    __shared__ double scratch[32];
-    const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-    const double d = damping;
-    while (true) {
-        if (tid == 0) s_item = atomicAdd(next_graph, 1u);
-        __syncthreads();
-        const uint32_t h = s_item;
-        if (h >= G) break;
-        const uint32_t g = order[h];
-        const uint32_t vb = vbase[g], ve = vbase[g + 1], n = ve - vb;
-        if (n == 0) {
-            if (tid == 0) {
-                iterations[g] = 0;
-                converged[g] = 1;
+// ---------------------------------------------------------------- personalised PageRank
+
+// Sums of values in [0, 2] as 64-bit fixed-point integers (units of 2^-62).
+__device__ __forceinline__ unsigned long long batch_fixed(double x) { return __double2ull_rz(x * 4611686018427387904.0); }
+__device__ __forceinline__ double batch_from_fixed(unsigned long long q) {
+    return static_cast<double>(q) * (1.0 / 4611686018427387904.0);
+}
+
+struct BatchPpr {
+    BatchRows rows;
+    const uint32_t* vbase;
+    const uint32_t* lone_count;  // [G]
+    const float* tele;
+    uint32_t G, V;
+    double damp, tolerance;
+    uint32_t max_iterations;
+    float *contrib_a, *contrib_b;
+    float* ranks;
+    double* parts;
+    unsigned long long* diff;    // [3][G], rotating by iteration
+    unsigned long long* dangle;  // [3][G]
+    uint32_t* stop;              // [G]: iterations a graph has run when it stopped
+    uint32_t* iterations;
+    uint8_t* converged;
+    BatchRunState* st;
+};
+
+struct PprOp {
+    using T = double;
+    static constexpr bool kSkips = false;
+    const BatchPpr& a;
+    const float* in;
+    float* out;
+    const unsigned long long* prev_diff;    // [G], the iteration before
+    const unsigned long long* prev_dangle;  // [G]
+    unsigned long long* diff;
+    unsigned long long* dangle;
+    uint32_t it;
+    uint32_t my_graph = kNoGraph;
+    bool my_works = false;
+    double my_mass = 0.0;
+    unsigned long long my_diff = 0, my_dangle = 0;
+
+    static __device__ __forceinline__ T zero() { return 0.0; }
+    static __device__ __forceinline__ T add(T x, T y) { return x + y; }
+    __device__ __forceinline__ bool works(uint32_t g) const {
+        return a.stop[g] > it && (it == 0 || !(batch_from_fixed(prev_diff[g]) < a.tolerance));
+    }
+    __device__ __forceinline__ bool begin(uint32_t g0, uint32_t g1) const {
+        for (uint32_t g = g0; g <= g1; ++g)
+            if (works(g)) return true;
+        return false;
+    }
+    __device__ __forceinline__ bool want(uint32_t) const { return true; }
+    __device__ __forceinline__ T gather(bool p, uint32_t t) const {
+        return static_cast<double>(__uint_as_float(ld_if(p, reinterpret_cast<const uint32_t*>(in) + t, 0u)));
+    }
+    __device__ __forceinline__ void part(uint64_t i, T x) { a.parts[i] = x; }
+    __device__ __forceinline__ T parts(uint64_t i) const { return a.parts[i]; }
+    // Makes g the lane's graph (its sums so far go out if it was another).
+    __device__ __forceinline__ void enter(uint32_t g) {
+        if (g == my_graph) return;
+        if (my_graph != kNoGraph) spill();
+        my_graph = g;
+        my_works = works(g);
+        my_mass = batch_from_fixed(prev_dangle[g]);
+    }
+    __device__ __forceinline__ void spill() {
+        if (my_diff) atomicAdd(diff + my_graph, my_diff);
+        if (my_dangle) atomicAdd(dangle + my_graph, my_dangle);
+        my_diff = 0;
+        my_dangle = 0;
+    }
+    __device__ __forceinline__ float update(uint32_t v, double sum) {
+        const double p = a.tele[v];
+        const float x = static_cast<float>((1.0 - a.damp) * p + a.damp * (sum + my_mass * p));
+        my_diff += batch_fixed(fabs(static_cast<double>(x) - static_cast<double>(a.ranks[v])));
+        a.ranks[v] = x;
+        return x;
+    }
+    __device__ __forceinline__ void finish(uint32_t r, T sum) {
+        enter(__ldg(a.rows.row_graph + r));
+        if (!my_works) return;
+        const uint32_t v = __ldg(a.rows.row_vertex + r);
+        const float x = update(v, sum);
+        out[v] = x / static_cast<float>(__ldg(a.rows.row_start + r + 1) - __ldg(a.rows.row_start + r));
+    }
+    // A vertex without entries: its rank is dangling mass.
+    __device__ __forceinline__ void finish_lone(uint32_t i) {
+        enter(__ldg(a.rows.lone_graph + i));
+        if (!my_works) return;
+        my_dangle += batch_fixed(static_cast<double>(update(__ldg(a.rows.lone + i), 0.0)));
+    }
+    __device__ __forceinline__ void flush() {
+        const unsigned has = __ballot_sync(kFullMask, my_graph != kNoGraph);
+        if (has) {
+            // One graph per warp turn nearly always: one pair of atomics.
+            const uint32_t g = __shfl_sync(kFullMask, my_graph, __ffs(has) - 1);
+            const bool same = my_graph == g;
+            const unsigned long long d = warp_sum(same ? my_diff : 0ull), m = warp_sum(same ? my_dangle : 0ull);
+            if (lane_id() == static_cast<unsigned>(__ffs(has) - 1)) {
+                if (d) atomicAdd(diff + g, d);
+                if (m) atomicAdd(dangle + g, m);
             }
-            __syncthreads();
-            continue;
-        }
-        const float r0 = 1.0f / static_cast<float>(n);
-        double dang = 0.0;
-        for (uint32_t v = vb + tid; v < ve; v += kThreads) {
-            const uint32_t deg = offsets[v + 1] - offsets[v];
-            rank_a[v] = r0;
-            contrib_a[v] = deg ? r0 / static_cast<float>(deg) : 0.f;
-            if (!deg) dang += r0;
-        }
-        double dangling = block_sum(dang, scratch);
-        float *r = rank_a, *rn = rank_b, *c = contrib_a, *cn = contrib_b;
-        uint32_t it = 0;
-        bool conv = false;
-        while (it < max_iterations) {
-            double l1 = 0.0, dn = 0.0;
-            for (uint32_t base = vb + warp * 32; base < ve; base += kThreads) {
-                const uint32_t v = base + lane;
-                const bool valid = v < ve;
-                uint32_t s = 0, e = 0;
-                if (valid) {
-                    s = offsets[v];
-                    e = offsets[v + 1];
-                }
-                const uint32_t deg = e - s;
-                float sum = 0.f;
-                if (valid && deg < 32)
-                    for (uint32_t j = s; j < e; ++j) sum += c[targets[j]];
-                unsigned longs = __ballot_sync(kFullMask, valid && deg >= 32);
-                while (longs) {
-                    const int i = __ffs(longs) - 1;
-                    longs &= longs - 1;
-                    const uint32_t rs = __shfl_sync(kFullMask, s, i), re = __shfl_sync(kFullMask, e, i);
-                    float part = 0.f;
-                    for (uint32_t j = rs + lane; j < re; j += 32) part += c[targets[j]];
-                    part = warp_sum(part);
-                    if (static_cast<int>(lane) == i) sum = part;
-                }
-                if (valid) {
-                    const double p = tele[v];
-                    const float x = static_cast<float>((1.0 - d) * p + d * (static_cast<double>(sum) + dangling * p));
-                    l1 += fabs(static_cast<double>(x) - static_cast<double>(r[v]));
-                    rn[v] = x;
-                    cn[v] = deg ? x / static_cast<float>(deg) : 0.f;
-                    if (!deg) dn += x;
-                }
-            }
-            l1 = block_sum(l1, scratch);
-            dangling = block_sum(dn, scratch);
-            float* t = r;
-            r = rn;
-            rn = t;
-            t = c;
-            c = cn;
-            cn = t;
-            ++it;
-            if (l1 < tolerance) {
-                conv = true;
-                break;
+            if (same) {
+                my_diff = 0;
+                my_dangle = 0;
+            } else if (my_graph != kNoGraph) {
+                spill();
             }
         }
-        for (uint32_t v = vb + tid; v < ve; v += kThreads) ranks_out[v] = r[v];
-        if (tid == 0) {
-            iterations[g] = it;
-            converged[g] = conv ? 1 : 0;
+        my_graph = kNoGraph;
+    }
+};
+
+__global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kernel(const BatchPpr a) {
+    __shared__ uint32_t s_active;
+    const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    unsigned barriers = 0;
+    auto start = [&](uint32_t g) { return 1.0f / static_cast<float>(a.vbase[g + 1] - a.vbase[g]); };
+    for (uint64_t r = tid; r < a.rows.n_rows; r += nthreads) {
+        const uint32_t v = a.rows.row_vertex[r];
+        const float r0 = start(a.rows.row_graph[r]);
+        a.ranks[v] = r0;
+        a.contrib_a[v] = r0 / static_cast<float>(a.rows.row_start[r + 1] - a.rows.row_start[r]);
+    }
+    for (uint64_t i = tid; i < a.rows.n_lone; i += nthreads) {
+        // A CSR that is not symmetric may list such a vertex as a target.
+        const uint32_t v = a.rows.lone[i];
+        a.ranks[v] = start(a.rows.lone_graph[i]);
+        a.contrib_a[v] = 0.f;
+        a.contrib_b[v] = 0.f;
+    }
+    for (uint64_t g = tid; g < a.G; g += nthreads) {
+        const bool some = a.vbase[g + 1] > a.vbase[g];
+        for (uint64_t q = 0; q < 3; ++q) {
+            a.diff[q * a.G + g] = 0;
+            a.dangle[q * a.G + g] = 0;
         }
-        __syncthreads();
+        // Iteration 0 reads slot 2.
+        if (some) a.dangle[2ull * a.G + g] = batch_fixed(static_cast<double>(a.lone_count[g]) * static_cast<double>(start(static_cast<uint32_t>(g))));
+        a.stop[g] = some ? 0xFFFFFFFFu : 0u;
+    }
+    if (!grid_barrier(&a.st->bar, barriers)) return;
+    for (uint32_t it = 0; it < a.max_iterations; ++it) {
+        const uint64_t cur = static_cast<uint64_t>(it % 3) * a.G, prev = static_cast<uint64_t>((it + 2) % 3) * a.G;
+        const uint64_t next = static_cast<uint64_t>((it + 1) % 3) * a.G;
+        PprOp op{a, (it & 1) ? a.contrib_b : a.contrib_a, (it & 1) ? a.contrib_a : a.contrib_b,
+                 a.diff + prev, a.dangle + prev, a.diff + cur, a.dangle + cur, it};
+        for (uint64_t g = tid; g < a.G; g += nthreads) {
+            a.diff[next + g] = 0;  // last read an iteration ago
+            a.dangle[next + g] = 0;
+            if (a.stop[g] <= it) continue;
+            if (it && batch_from_fixed(op.prev_diff[g]) < a.tolerance) a.stop[g] = it;
+            else atomicAdd(a.st->active + it % 3, 1u);
+        }
+        if (tid == 0) a.st->active[(it + 1) % 3] = 0;
+        for (uint64_t b = tid & ~31ull; b < a.rows.n_lone; b += nthreads) {
+            if (b + lane_id() < a.rows.n_lone) op.finish_lone(static_cast<uint32_t>(b + lane_id()));
+            op.flush();
+        }
+        batch_pass(a.rows, op);
+        if (!grid_barrier(&a.st->bar, gridDim.x, barriers, [&] { s_active = __ldcg(a.st->active + it % 3); })) return;
+        if (s_active == 0) break;
+        batch_split_pass(a.rows, op);
+        if (!grid_barrier(&a.st->bar, barriers)) return;
+    }
+    // A graph whose last iteration met the tolerance has not been marked yet.
+    for (uint64_t g = tid; g < a.G; g += nthreads) {
+        uint32_t n = a.stop[g];
+        bool conv = n != 0xFFFFFFFFu;
+        if (!conv) {
+            n = a.max_iterations;
+            conv = n > 0 && batch_from_fixed(a.diff[static_cast<uint64_t>((n + 2) % 3) * a.G + g]) < a.tolerance;
+        }
+        a.iterations[g] = n;
+        a.converged[g] = conv ? 1 : 0;
     }
 }
 
@@ -295,24 +654,33 @@ struct BatchImpl {
     GraphImpl u;  // the union CSR
     uint32_t G = 0;
     std::vector<uint32_t> vbase, ebase;
-    DeviceBuffer<uint32_t> d_vbase, d_order, counters;
+    DeviceBuffer<uint32_t> d_vbase;
+    // rows of the union for the BFS and PageRank passes (built with the batch)
+    BatchRows rows{};
+    DeviceBuffer<uint32_t> row_vertex, row_graph, row_start, chunk_row, lone, lone_graph, lone_count;
+    DeviceBuffer<uint8_t> delta;
+    DeviceBuffer<uint4> split;
+    DeviceBuffer<BatchRunState> bfs_state, ppr_state;
+    unsigned bfs_grid = 0, ppr_grid = 0;
     BatchTcPlan* tc = nullptr;
     std::string tc_tuning;
     DeviceBuffer<unsigned long long> tri_vertex, tri_totals;
     // BFS
     uint32_t S = 0;
     bool keep_dist = true;
-    int bfs_threads = 0;
-    DeviceBuffer<uint32_t> sources, visited, mask_a, mask_b, reachable;
+    bool bfs_timed = false;
+    DeviceBuffer<uint32_t> sources, mask_a, mask_b, bfs_parts, fresh, bfs_stop, reachable;
     DeviceBuffer<int32_t> dist, max_depth;
     // personalised PageRank
     uint32_t K = 0;
     float damping = 0.85f, tolerance = 1e-6f;
     uint32_t max_iterations = 100;
-    int ppr_threads = 0;
-    DeviceBuffer<uint32_t> seeds, iterations;
+    bool ppr_timed = false;
+    DeviceBuffer<uint32_t> seeds, iterations, ppr_stop;
     DeviceBuffer<uint8_t> converged;
-    DeviceBuffer<float> tele, rank_a, rank_b, contrib_a, contrib_b, ranks;
+    DeviceBuffer<float> tele, contrib_a, contrib_b, ranks;
+    DeviceBuffer<double> ppr_parts;
+    DeviceBuffer<unsigned long long> sums;  // diff then dangle, [3][G] each
     // captured replay of the three
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -341,78 +709,145 @@ unsigned small_grid(const DeviceImpl& dev, uint64_t n, unsigned threads) {
         std::max<uint64_t>(1, std::min<uint64_t>(ceil_div_u64(n, threads), static_cast<uint64_t>(dev.sm_count) * 8)));
 }
 
-// vbase uploaded, ebase gathered, graphs ordered by entries (largest first).
+// vbase uploaded, ebase gathered, the rows of the BFS and PageRank passes.
 Error finish_layout(BatchImpl& b) {
     DeviceImpl& dev = *b.dev;
-    const uint32_t G = b.G;
+    const uint32_t G = b.G, V = b.u.num_nodes, E = b.u.num_edges;
     GCU_TRY(b.d_vbase.allocate(dev, G + 1));
     GCU_CUDA(cudaMemcpyAsync(b.d_vbase.ptr, b.vbase.data(), 4 * (G + 1), cudaMemcpyHostToDevice, dev.stream), "copy");
-    DeviceBuffer<uint32_t> d_ebase;
+    DeviceBuffer<uint32_t> d_ebase, pos, split_pos;
     GCU_TRY(d_ebase.allocate(dev, G + 1));
     GCU_LAUNCH(dev, "batch_entry_base", batch_entry_base_kernel, small_grid(dev, G + 1, 256), 256, 0, b.u.offsets.ptr,
                b.d_vbase.ptr, G, d_ebase.ptr);
     b.ebase.resize(G + 1);
     GCU_CUDA(cudaMemcpyAsync(b.ebase.data(), d_ebase.ptr, 4 * (G + 1), cudaMemcpyDeviceToHost, dev.stream), "copy");
+
+    GCU_TRY(pos.allocate(dev, static_cast<uint64_t>(V) + 1));
+    if (V)
+        GCU_LAUNCH(dev, "batch_row_flags", batch_row_flags_kernel, small_grid(dev, V, 256), 256, 0, b.u.offsets.ptr, V,
+                   pos.ptr);
+    GCU_TRY(exclusive_scan_u32(dev, pos.ptr, pos.ptr, V));
+    uint32_t n_rows = 0;
+    GCU_CUDA(cudaMemcpyAsync(&n_rows, pos.ptr + V, sizeof(uint32_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
     GCU_TRY(dev.sync());
-    std::vector<uint32_t> order(G);
-    std::iota(order.begin(), order.end(), 0u);
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
-        return b.ebase[x + 1] - b.ebase[x] > b.ebase[y + 1] - b.ebase[y];
-    });
-    GCU_TRY(b.d_order.allocate(dev, std::max<uint32_t>(G, 1)));
-    if (G) GCU_CUDA(cudaMemcpyAsync(b.d_order.ptr, order.data(), 4 * G, cudaMemcpyHostToDevice, dev.stream), "copy");
-    GCU_TRY(b.counters.allocate(dev, 2));
+    const uint32_t n_chunks = static_cast<uint32_t>(ceil_div_u64(E, kBatchChunk));
+    GCU_TRY(b.row_vertex.allocate(dev, n_rows));
+    GCU_TRY(b.row_graph.allocate(dev, n_rows));
+    GCU_TRY(b.row_start.allocate(dev, static_cast<uint64_t>(n_rows) + 1));
+    GCU_TRY(b.lone.allocate(dev, V - n_rows));
+    GCU_TRY(b.lone_graph.allocate(dev, V - n_rows));
+    GCU_TRY(b.lone_count.allocate(dev, std::max<uint32_t>(G, 1)));
+    GCU_CUDA(cudaMemsetAsync(b.lone_count.ptr, 0, 4ull * std::max<uint32_t>(G, 1), dev.stream), "memset");
+    GCU_LAUNCH(dev, "batch_rows", batch_rows_kernel, small_grid(dev, static_cast<uint64_t>(V) + 1, 256), 256, 0,
+               b.u.offsets.ptr, pos.ptr, b.d_vbase.ptr, G, V, E, b.row_vertex.ptr, b.row_graph.ptr, b.row_start.ptr,
+               b.lone.ptr, b.lone_graph.ptr, b.lone_count.ptr);
+    GCU_TRY(b.chunk_row.allocate(dev, n_chunks));
+    GCU_TRY(b.delta.allocate(dev, static_cast<uint64_t>(n_chunks) * kBatchChunk));
+    uint32_t n_split = 0;
+    if (n_rows) {
+        GCU_TRY(split_pos.allocate(dev, static_cast<uint64_t>(n_rows) + 1));
+        GCU_LAUNCH(dev, "batch_chunk_rows", batch_chunk_rows_kernel, small_grid(dev, n_rows, 256), 256, 0,
+                   b.row_start.ptr, n_rows, b.chunk_row.ptr, split_pos.ptr);
+        GCU_TRY(exclusive_scan_u32(dev, split_pos.ptr, split_pos.ptr, n_rows));
+        GCU_CUDA(cudaMemcpyAsync(&n_split, split_pos.ptr + n_rows, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                 dev.stream),
+                 "copy");
+        GCU_CUDA(cudaMemsetAsync(b.delta.ptr, 0, static_cast<size_t>(n_chunks) * kBatchChunk, dev.stream), "memset");
+        GCU_LAUNCH(dev, "batch_delta", batch_delta_kernel, small_grid(dev, E, 1024), 256, 0, b.row_start.ptr, n_rows,
+                   E, b.chunk_row.ptr, b.delta.ptr);
+        GCU_TRY(dev.sync());
+    }
+    GCU_TRY(b.split.allocate(dev, n_split));
+    if (n_split)
+        GCU_LAUNCH(dev, "batch_split_rows", batch_split_rows_kernel, small_grid(dev, n_rows, 256), 256, 0,
+                   b.row_start.ptr, n_rows, split_pos.ptr, b.split.ptr);
+    b.rows = BatchRows{b.u.targets.ptr, b.row_vertex.ptr, b.row_graph.ptr, b.row_start.ptr, b.chunk_row.ptr,
+                       b.delta.ptr, b.split.ptr, b.lone.ptr, b.lone_graph.ptr, E, n_rows, n_chunks, n_split,
+                       V - n_rows};
+    GCU_TRY(b.bfs_state.allocate(dev, 1));
+    GCU_TRY(b.ppr_state.allocate(dev, 1));
     return dev.sync();
 }
 
-template <int kThreads>
-Error launch_bfs_t(BatchImpl& b) {
-    DeviceImpl& dev = *b.dev;
+// Blocks of a pass kernel: all that are resident at once, fewer for a batch
+// too small to give every warp a turn.
+template <class Kernel>
+Error pass_grid(BatchImpl& b, Kernel kernel, unsigned* grid) {
+    if (*grid) return ok();
     int per_sm = 0;
-    GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_bfs_kernel<kThreads>, kThreads, 0),
-             "occupancy");
-    const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(
-        1, std::min<uint64_t>(b.G, static_cast<uint64_t>(dev.sm_count) * std::max(per_sm, 1))));
-    GCU_LAUNCH(dev, "batch_bfs", batch_bfs_kernel<kThreads>, grid, kThreads, 0, b.u.offsets.ptr, b.u.targets.ptr,
-               b.d_vbase.ptr, b.d_order.ptr, b.G, b.sources.ptr, b.S, b.visited.ptr, b.mask_a.ptr, b.mask_b.ptr,
-               b.keep_dist ? b.dist.ptr : nullptr, static_cast<uint64_t>(b.u.num_nodes), b.reachable.ptr,
-               b.max_depth.ptr, b.counters.ptr);
+    GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBatchThreads, 0), "occupancy");
+    const uint64_t most = static_cast<uint64_t>(b.dev->sm_count) * std::max(1, std::min(per_sm, kBatchCtasPerSm));
+    const uint64_t want = std::max<uint64_t>({1, ceil_div_u64(b.rows.n_chunks, kBatchThreads / 32),
+                                              ceil_div_u64(b.u.num_nodes, 4 * kBatchThreads)});
+    *grid = static_cast<unsigned>(std::min(want, most));
     return ok();
 }
 
-Error launch_bfs(BatchImpl& b, int threads) {
+Error launch_bfs(BatchImpl& b) {
     DeviceImpl& dev = *b.dev;
-    GCU_CUDA(cudaMemsetAsync(b.counters.ptr, 0, sizeof(uint32_t), dev.stream), "memset");
+    GCU_TRY(pass_grid(b, batch_bfs_kernel, &b.bfs_grid));
     if (b.keep_dist)
         GCU_CUDA(cudaMemsetAsync(b.dist.ptr, 0xFF, sizeof(int32_t) * b.S * static_cast<size_t>(b.u.num_nodes),
                                  dev.stream),
                  "memset");
-    if (threads == 256) return launch_bfs_t<256>(b);
-    if (threads == 512) return launch_bfs_t<512>(b);
-    return launch_bfs_t<1024>(b);
-}
-
-template <int kThreads>
-Error launch_ppr_t(BatchImpl& b) {
-    DeviceImpl& dev = *b.dev;
-    int per_sm = 0;
-    GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_ppr_kernel<kThreads>, kThreads, 0),
-             "occupancy");
-    const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(
-        1, std::min<uint64_t>(b.G, static_cast<uint64_t>(dev.sm_count) * std::max(per_sm, 1))));
-    GCU_LAUNCH(dev, "batch_ppr", batch_ppr_kernel<kThreads>, grid, kThreads, 0, b.u.offsets.ptr, b.u.targets.ptr,
-               b.d_vbase.ptr, b.d_order.ptr, b.G, b.tele.ptr, b.damping, b.max_iterations,
-               static_cast<double>(b.tolerance), b.rank_a.ptr, b.rank_b.ptr, b.contrib_a.ptr, b.contrib_b.ptr,
-               b.ranks.ptr, b.iterations.ptr, b.converged.ptr, b.counters.ptr + 1);
+    GCU_CUDA(cudaMemsetAsync(b.bfs_state.ptr, 0, sizeof(BatchRunState), dev.stream), "memset");
+    BatchBfs a{};
+    a.rows = b.rows;
+    a.offsets = b.u.offsets.ptr;
+    a.vbase = b.d_vbase.ptr;
+    a.sources = b.sources.ptr;
+    a.G = b.G;
+    a.V = b.u.num_nodes;
+    a.S = b.S;
+    a.full = b.S >= 32 ? 0xFFFFFFFFu : (1u << b.S) - 1u;
+    a.mask_a = b.mask_a.ptr;
+    a.mask_b = b.mask_b.ptr;
+    a.parts = b.bfs_parts.ptr;
+    a.dist = b.keep_dist ? b.dist.ptr : nullptr;
+    a.fresh = b.fresh.ptr;
+    a.stop = b.bfs_stop.ptr;
+    a.reachable = b.reachable.ptr;
+    a.max_depth = b.max_depth.ptr;
+    a.st = b.bfs_state.ptr;
+    GCU_LAUNCH_COOP(dev, "batch_bfs", batch_bfs_kernel, b.bfs_grid, kBatchThreads, 0, a);
     return ok();
 }
 
-Error launch_ppr(BatchImpl& b, int threads) {
+Error launch_ppr(BatchImpl& b) {
     DeviceImpl& dev = *b.dev;
-    GCU_CUDA(cudaMemsetAsync(b.counters.ptr + 1, 0, sizeof(uint32_t), dev.stream), "memset");
-    if (threads == 256) return launch_ppr_t<256>(b);
-    if (threads == 512) return launch_ppr_t<512>(b);
-    return launch_ppr_t<1024>(b);
+    GCU_TRY(pass_grid(b, batch_ppr_kernel, &b.ppr_grid));
+    GCU_CUDA(cudaMemsetAsync(b.ppr_state.ptr, 0, sizeof(BatchRunState), dev.stream), "memset");
+    BatchPpr a{};
+    a.rows = b.rows;
+    a.vbase = b.d_vbase.ptr;
+    a.lone_count = b.lone_count.ptr;
+    a.tele = b.tele.ptr;
+    a.G = b.G;
+    a.V = b.u.num_nodes;
+    a.damp = static_cast<double>(b.damping);
+    a.tolerance = static_cast<double>(b.tolerance);
+    a.max_iterations = b.max_iterations;
+    a.contrib_a = b.contrib_a.ptr;
+    a.contrib_b = b.contrib_b.ptr;
+    a.ranks = b.ranks.ptr;
+    a.parts = b.ppr_parts.ptr;
+    a.diff = b.sums.ptr;
+    a.dangle = b.sums.ptr + 3 * static_cast<size_t>(b.G);
+    a.stop = b.ppr_stop.ptr;
+    a.iterations = b.iterations.ptr;
+    a.converged = b.converged.ptr;
+    a.st = b.ppr_state.ptr;
+    GCU_LAUNCH_COOP(dev, "batch_ppr", batch_ppr_kernel, b.ppr_grid, kBatchThreads, 0, a);
+    return ok();
+}
+
+// Reads a pass kernel's error flag (the stream has been synchronized).
+Error check_run(BatchImpl& b, const DeviceBuffer<BatchRunState>& st, const char* what) {
+    BatchRunState h{};
+    GCU_CUDA(cudaMemcpyAsync(&h, st.ptr, sizeof(h), cudaMemcpyDeviceToHost, b.dev->stream), "copy");
+    GCU_TRY(b.dev->sync());
+    if (h.bar.failed) return kernel_error(std::string(what) + ": a block did not reach the grid barrier");
+    return ok();
 }
 
 Error launch_tc(BatchImpl& b) {
@@ -423,33 +858,23 @@ Error launch_tc(BatchImpl& b) {
     return ok();
 }
 
-// Times each candidate CTA size once on the whole batch and keeps the fastest.
+// Runs and times a pass kernel once on the whole batch (for batch_tuning).
 template <class Launch>
-Error autotune(BatchImpl& b, Launch launch, int* best, std::string* json) {
+Error timed_run(BatchImpl& b, Launch launch, std::string* json) {
     DeviceImpl& dev = *b.dev;
-    const int cand[3] = {256, 512, 1024};
     cudaEvent_t e0, e1;
     GCU_CUDA(cudaEventCreate(&e0), "cudaEventCreate");
     GCU_CUDA(cudaEventCreate(&e1), "cudaEventCreate");
-    float best_ms = 0.f;
-    *json = "{";
-    Error err = ok();
-    for (int i = 0; i < 3 && err.ok(); ++i) {
-        cudaEventRecord(e0, dev.stream);
-        err = launch(b, cand[i]);
-        cudaEventRecord(e1, dev.stream);
-        if (err.ok()) err = dev.sync();
-        float ms = 0.f;
-        if (err.ok()) cudaEventElapsedTime(&ms, e0, e1);
-        if (i == 0 || ms < best_ms) {
-            best_ms = ms;
-            *best = cand[i];
-        }
-        *json += (i ? ", \"" : "\"") + std::to_string(cand[i]) + "\": " + std::to_string(ms);
-    }
-    *json += ", \"chosen\": " + std::to_string(*best) + "}";
+    cudaEventRecord(e0, dev.stream);
+    Error err = launch(b);
+    cudaEventRecord(e1, dev.stream);
+    if (err.ok()) err = dev.sync();
+    float ms = 0.f;
+    if (err.ok()) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    const std::string threads = std::to_string(kBatchThreads);
+    *json = "{\"" + threads + "\": " + std::to_string(ms) + ", \"chosen\": " + threads + "}";
     return err;
 }
 
@@ -590,13 +1015,15 @@ Error batch_set_bfs(BatchImpl& b, const uint32_t* sources, uint32_t S, bool keep
     b.keep_dist = keep_distances;
     GCU_TRY(b.sources.allocate(dev, static_cast<uint64_t>(b.G) * S));
     GCU_CUDA(cudaMemcpyAsync(b.sources.ptr, sources, 4ull * b.G * S, cudaMemcpyHostToDevice, dev.stream), "copy");
-    GCU_TRY(b.visited.allocate(dev, V));
+    GCU_TRY(b.bfs_parts.allocate(dev, 2ull * b.rows.n_chunks));
+    GCU_TRY(b.fresh.allocate(dev, 3ull * b.G));
+    GCU_TRY(b.bfs_stop.allocate(dev, b.G));
     GCU_TRY(b.mask_a.allocate(dev, V));
     GCU_TRY(b.mask_b.allocate(dev, V));
     GCU_TRY(b.reachable.allocate(dev, static_cast<uint64_t>(b.G) * S));
     GCU_TRY(b.max_depth.allocate(dev, static_cast<uint64_t>(b.G) * S));
     if (keep_distances) GCU_TRY(b.dist.allocate(dev, V * S));
-    b.bfs_threads = 0;
+    b.bfs_timed = false;
     return dev.sync();
 }
 
@@ -622,8 +1049,9 @@ Error batch_set_ppr(BatchImpl& b, const uint32_t* seeds, uint32_t K, float dampi
     GCU_TRY(b.seeds.allocate(dev, static_cast<uint64_t>(b.G) * K));
     GCU_CUDA(cudaMemcpyAsync(b.seeds.ptr, seeds, 4ull * b.G * K, cudaMemcpyHostToDevice, dev.stream), "copy");
     GCU_TRY(b.tele.allocate(dev, V));
-    GCU_TRY(b.rank_a.allocate(dev, V));
-    GCU_TRY(b.rank_b.allocate(dev, V));
+    GCU_TRY(b.ppr_parts.allocate(dev, 2ull * b.rows.n_chunks));
+    GCU_TRY(b.sums.allocate(dev, 6ull * b.G));
+    GCU_TRY(b.ppr_stop.allocate(dev, b.G));
     GCU_TRY(b.contrib_a.allocate(dev, V));
     GCU_TRY(b.contrib_b.allocate(dev, V));
     GCU_TRY(b.ranks.allocate(dev, V));
@@ -632,7 +1060,7 @@ Error batch_set_ppr(BatchImpl& b, const uint32_t* seeds, uint32_t K, float dampi
     GCU_CUDA(cudaMemsetAsync(b.tele.ptr, 0, 4 * std::max<uint64_t>(V, 1), dev.stream), "memset");
     GCU_LAUNCH(dev, "batch_tele", batch_tele_kernel, small_grid(dev, static_cast<uint64_t>(b.G) * K, 256), 256, 0,
                b.seeds.ptr, b.d_vbase.ptr, b.G, K, b.tele.ptr);
-    b.ppr_threads = 0;
+    b.ppr_timed = false;
     return dev.sync();
 }
 
@@ -653,21 +1081,30 @@ Error batch_run_tc(BatchImpl& b, uint64_t* totals) {
 
 Error batch_run_bfs(BatchImpl& b) {
     if (!b.S) return kernel_error("batch BFS sources are not set");
-    if (!b.bfs_threads) return autotune(b, launch_bfs, &b.bfs_threads, &b.bfs_tuning);
-    GCU_TRY(launch_bfs(b, b.bfs_threads));
+    if (b.bfs_timed) {
+        GCU_TRY(launch_bfs(b));
+    } else {
+        GCU_TRY(timed_run(b, launch_bfs, &b.bfs_tuning));
+        b.bfs_timed = true;
+    }
     return b.dev->sync();
 }
 
 Error batch_run_ppr(BatchImpl& b) {
     if (!b.K) return kernel_error("batch PageRank seeds are not set");
-    if (!b.ppr_threads) return autotune(b, launch_ppr, &b.ppr_threads, &b.ppr_tuning);
-    GCU_TRY(launch_ppr(b, b.ppr_threads));
+    if (b.ppr_timed) {
+        GCU_TRY(launch_ppr(b));
+    } else {
+        GCU_TRY(timed_run(b, launch_ppr, &b.ppr_tuning));
+        b.ppr_timed = true;
+    }
     return b.dev->sync();
 }
 
 Error batch_read_bfs(BatchImpl& b, int32_t* distances, uint32_t* reachable, int32_t* max_depth) {
     DeviceImpl& dev = *b.dev;
     const uint64_t gs = static_cast<uint64_t>(b.G) * b.S;
+    GCU_TRY(check_run(b, b.bfs_state, "batch BFS"));
     if (distances && b.keep_dist) GCU_TRY(copy_to_host(dev, distances, b.dist.ptr, 4ull * b.S * b.u.num_nodes));
     if (reachable) GCU_CUDA(cudaMemcpyAsync(reachable, b.reachable.ptr, 4 * gs, cudaMemcpyDeviceToHost, dev.stream), "copy");
     if (max_depth) GCU_CUDA(cudaMemcpyAsync(max_depth, b.max_depth.ptr, 4 * gs, cudaMemcpyDeviceToHost, dev.stream), "copy");
@@ -676,6 +1113,7 @@ Error batch_read_bfs(BatchImpl& b, int32_t* distances, uint32_t* reachable, int3
 
 Error batch_read_ppr(BatchImpl& b, float* ranks, uint32_t* iterations, uint8_t* converged) {
     DeviceImpl& dev = *b.dev;
+    GCU_TRY(check_run(b, b.ppr_state, "batch PageRank"));
     if (ranks) GCU_TRY(copy_to_host(dev, ranks, b.ranks.ptr, 4ull * b.u.num_nodes));
     if (iterations)
         GCU_CUDA(cudaMemcpyAsync(iterations, b.iterations.ptr, 4ull * b.G, cudaMemcpyDeviceToHost, dev.stream), "copy");
@@ -690,15 +1128,15 @@ Error batch_capture(BatchImpl& b) {
     DeviceImpl& dev = *b.dev;
     if (!b.S || !b.K) return kernel_error("set the batch BFS sources and PageRank seeds before capturing");
     GCU_TRY(batch_ensure_tc(b));
-    if (!b.bfs_threads) GCU_TRY(autotune(b, launch_bfs, &b.bfs_threads, &b.bfs_tuning));
-    if (!b.ppr_threads) GCU_TRY(autotune(b, launch_ppr, &b.ppr_threads, &b.ppr_tuning));
+    if (!b.bfs_timed) GCU_TRY(batch_run_bfs(b));
+    if (!b.ppr_timed) GCU_TRY(batch_run_ppr(b));
     drop_capture(b);
     const bool timing = dev.kernel_timing;
     dev.kernel_timing = false;  // no event bookkeeping inside the capture
     GCU_CUDA(cudaStreamBeginCapture(dev.stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
     Error e = launch_tc(b);
-    if (e.ok()) e = launch_bfs(b, b.bfs_threads);
-    if (e.ok()) e = launch_ppr(b, b.ppr_threads);
+    if (e.ok()) e = launch_bfs(b);
+    if (e.ok()) e = launch_ppr(b);
     cudaGraph_t graph = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(dev.stream, &graph);
     dev.kernel_timing = timing;
