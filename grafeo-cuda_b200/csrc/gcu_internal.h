@@ -249,6 +249,22 @@ Error graph_symmetry(GraphImpl& g, bool* symmetric);
 Error build_dag(GraphImpl& g, bool by_degree, const uint32_t* rev, DeviceBuffer<uint32_t>* dag_offsets,
                 DeviceBuffer<uint32_t>* dag_targets, DeviceBuffer<uint32_t>* dag_eid, uint32_t* m);
 
+// N+(u) of every vertex of a symmetric CSR as (32-rank word, mask) pairs, and the
+// owners the count runs over (tri_words.cu).
+struct WordLists {
+    DeviceBuffer<uint32_t> rank;         // degree-class order
+    DeviceBuffer<uint2> lists;           // per vertex: first word, words
+    DeviceBuffer<uint2> words;           // (word, mask)
+    DeviceBuffer<uint32_t> warp_owners;
+    DeviceBuffer<uint2> items;           // (owner, slice of its row)
+    DeviceBuffer<uint32_t> counts;       // [2] warp owners, [3] items
+    uint64_t max_items = 0;
+};
+Error build_word_lists(GraphImpl& g, WordLists* w);
+// Adds the triangles to *total, or to per_vertex[owner] where that is given
+// (device memory). next: two words of scratch. Only enqueues (capturable).
+Error count_words(GraphImpl& g, const WordLists& w, uint32_t* next, unsigned long long* total,
+                  unsigned long long* per_vertex);
 Error triangle_count(GraphImpl& g, bool oriented, uint64_t* total);
 Error bfs(GraphImpl& g, uint32_t source, int32_t* host_distances, uint32_t* reachable,
           int32_t* max_depth);

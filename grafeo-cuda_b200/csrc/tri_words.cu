@@ -1,0 +1,567 @@
+// Triangle counting over word lists (symmetric CSRs, fixed schedule).
+//
+// Vertices are ranked by degree class (degree_class_order: hubs first), and
+// N+(u) is the set of u's neighbours that rank below it. Hubs take most of the
+// entries, so the ranks in an N+(u) crowd together: as bits of 32-rank words, a
+// list of R-MAT 22 has 0.79 words per entry, and weighted by the counting work
+// 2.5 times fewer words than entries (R-MAT 16: 4.3). A word costs what an entry
+// cost (a load, a table lookup), so the lists are kept as (word, mask) pairs and
+// an intersection is a sum of popcounts.
+//
+// The count is the sum over edges {u, v} of |N+(u) ∩ N+(v)|: every triangle
+// once, at the edge of its two highest-ranked vertices. Each edge is counted
+// from the end whose list has more words (ties: the larger id), the owner: the
+// owner's words go into a table in shared memory and the other end's words are
+// streamed against it, 4, 16 or 32 lanes per list. An owner reads its neighbours from its own CSR row, so there are no
+// in-lists and no oriented CSR to build.
+//  * owners of up to kWarpWords words and kWarpOwnerRow neighbours: a warp each,
+//    with a hash table of (word, mask);
+//  * the others: CTA items of kSlice neighbours; the table is a bitmap of the
+//    ranks below kBitmapRanks where the owner's rank allows, a hash table of up
+//    to kHashWords words elsewhere, and for longer lists the bitmap again, one
+//    window of kBitmapRanks ranks after the other.
+// Only the owner's words are ever set and cleared, not the whole bitmap.
+//
+// Measured on one B200 against the oriented-CSR form (triangle.cu): R-MAT 16
+// 3.13 -> 0.21 ms, R-MAT 22 30.7 -> 12.1 ms (count 9.9, lists 1.8), the triangles
+// of 256 batched graphs 9.5 -> 3.7 ms. On the way, R-MAT 22 count: one word per
+// lane and four lists in flight, 256-thread blocks 14.9 ms (76 instructions per
+// 32 words, 24 % of the stalls at the items' block barriers); two words per lane
+// 11.5; 128-thread blocks with a 16 KB bitmap 10.7; two lists in flight, 40
+// registers 10.1; lists by length, 4 / 16 / 32 lanes each, 9.9 (with four in
+// flight 13.3: a fifth fewer resident blocks). What bounds it is instruction
+// issue.
+#include <algorithm>
+
+#include "device_common.cuh"
+#include "gcu_internal.h"
+
+namespace gcu {
+
+namespace {
+
+constexpr int kTwThreads = 256;
+constexpr int kTwWarps = kTwThreads / 32;
+constexpr int kCountThreads = 128;       // of the count
+constexpr int kCountWarps = kCountThreads / 32;
+constexpr int kCountCtasPerSm = 12;
+constexpr uint32_t kNoWord = 0xFFFFFFFFu;
+constexpr uint32_t kWarpRow = 128;       // neighbours of a row that one warp turns into words
+// Words of an owner with a warp table: 64 on a large graph; 32 below
+// kSmallGraph vertices, where the last owners of a few warps would be the end
+// of the launch (R-MAT 16: 81 against 123 us; R-MAT 22: 10.2 against 9.9 ms).
+constexpr uint32_t kWarpWords = 64, kWarpWordsSmall = 32;
+constexpr uint32_t kSmallGraph = 1u << 19;
+constexpr uint32_t kWarpOwnerRow = 128;  // neighbours of such an owner
+constexpr uint32_t kWarpBits = 8;
+constexpr int kInFlight = 2;             // lists in flight per group of lanes in the count
+constexpr uint32_t kSlice = 2048;        // neighbours per CTA item
+constexpr uint32_t kBitmapWords = 4096;
+constexpr uint32_t kBitmapRanks = kBitmapWords * 32;
+constexpr uint32_t kHashBits = 11;       // 2048 (word, mask) slots: as many bytes as the bitmap
+constexpr uint32_t kHashWords = 1u << (kHashBits - 1);
+static_assert((1u << kHashBits) * 2 == kBitmapWords, "one shared array for both tables");
+static_assert(kCountWarps * (2u << kWarpBits) <= kBitmapWords, "the warps' tables fit the shared array");
+
+__device__ __forceinline__ uint32_t word_slot(uint32_t word, uint32_t bits) { return (word * 2654435761u) >> (32 - bits); }
+
+// ORs mask into the table entry of `word` (2^bits slots, never full).
+__device__ __forceinline__ void table_or(uint2* table, uint32_t bits, uint32_t word, uint32_t mask) {
+    const uint32_t wrap = (1u << bits) - 1;
+    uint32_t s = word_slot(word, bits);
+    for (uint32_t i = 0; i <= wrap; ++i) {
+        const uint32_t k = atomicCAS(&table[s].x, kNoWord, word);
+        if (k == kNoWord || k == word) {
+            atomicOr(&table[s].y, mask);
+            return;
+        }
+        s = (s + 1) & wrap;
+    }
+}
+
+// Mask of `word` in the table, 0 if absent.
+__device__ __forceinline__ uint32_t table_mask(const uint2* table, uint32_t bits, uint32_t word) {
+    const uint32_t wrap = (1u << bits) - 1;
+    uint32_t s = word_slot(word, bits);
+    for (uint32_t i = 0; i <= wrap; ++i) {
+        const uint2 e = table[s];
+        if (e.x == word) return e.y;
+        if (e.x == kNoWord) return 0u;
+        s = (s + 1) & wrap;
+    }
+    return 0u;
+}
+
+// ---------------------------------------------------------------- word lists
+
+// Room for a list of n words: it starts on 16 bytes and is padded to an even
+// length with an empty word, so that the count can read two words at a time.
+__device__ __forceinline__ unsigned long long take_words(uint2* words, unsigned long long* cursor, uint32_t n) {
+    const unsigned long long at = atomicAdd(cursor, static_cast<unsigned long long>(n + (n & 1)));
+    if (n & 1) words[at + n] = make_uint2(kNoWord, 0u);
+    return at;
+}
+
+// Rows of at most kWarpRow neighbours: up to 32 by matching equal words across
+// the lanes, longer ones through a hash table of the warp. A list's place
+// comes from a shared cursor (the order of the lists has no meaning).
+__global__ void __launch_bounds__(kTwThreads) tw_build_warp_kernel(const uint32_t* __restrict__ offsets,
+                                                                   const uint32_t* __restrict__ targets,
+                                                                   const uint32_t* __restrict__ rank, uint32_t V,
+                                                                   uint32_t turn, uint2* __restrict__ lists,
+                                                                   uint2* __restrict__ words,
+                                                                   unsigned long long* __restrict__ cursor) {
+    __shared__ uint2 s_table[kTwWarps][1u << kWarpBits];
+    __shared__ uint4 s_rows[kTwWarps][32];
+    const unsigned lane = lane_id();
+    uint2* table = s_table[threadIdx.x >> 5];
+    const uint64_t warps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
+    // `turn` vertices per warp turn (up to 32; fewer on a small graph, so that
+    // every warp has some).
+    for (uint64_t v0 = ((static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * turn; v0 < V;
+         v0 += warps * turn) {
+        const uint64_t my = v0 + lane;
+        uint32_t s = 0, d = 0, r = 0;
+        if (my < V && lane < turn) {
+            s = offsets[my];
+            d = offsets[my + 1] - s;
+            r = rank[my];
+            if (d == 0) lists[my] = make_uint2(0u, 0u);
+        }
+        // Rows of up to 32 neighbours: 8, 16 or 32 lanes each, so 4, 2 or 1 rows
+        // per step; equal words of a row find each other by a match over (row,
+        // word), and the step's rows take their room with one atomic.
+#pragma unroll
+        for (uint32_t log_size = 3; log_size <= 5; ++log_size) {
+            const uint32_t size = 1u << log_size, groups = 32u >> log_size;
+            const unsigned rows = __ballot_sync(kFullMask, d > (log_size == 3 ? 0u : size / 2) && d <= size);
+            if (rows == 0) continue;
+            __syncwarp();
+            if ((rows >> lane) & 1u) s_rows[threadIdx.x >> 5][__popc(rows & ((1u << lane) - 1))] = make_uint4(s, d, r, lane);
+            __syncwarp();
+            const uint32_t n_rows = __popc(rows), group = lane >> log_size, at = lane & (size - 1);
+            const unsigned mates = (size == 32 ? kFullMask : ((1u << size) - 1) << (group * size));
+            for (uint32_t b = 0; b < n_rows; b += groups) {
+                const bool real = b + group < n_rows;
+                const uint4 row = real ? s_rows[threadIdx.x >> 5][b + group] : make_uint4(0u, 0u, 0u, 0u);
+                const uint32_t x = at < row.y ? __ldg(rank + __ldg(targets + row.x + at)) : kNoWord;
+                const bool keep = x < row.z;
+                // Words are below 2^27: the row's group goes above.
+                const unsigned peers = __match_any_sync(kFullMask, keep ? x >> 5 | group << 27 : kNoWord);
+                const uint32_t mask = __reduce_or_sync(peers, keep ? 1u << (x & 31) : 0u);
+                const bool first = keep && lane == static_cast<unsigned>(__ffs(peers) - 1);
+                const unsigned firsts = __ballot_sync(kFullMask, first);
+                const uint32_t n = __popc(firsts & mates), padded = n + (n & 1);
+                const uint32_t upto = warp_inclusive_scan(at == 0 ? padded : 0u);
+                const uint32_t all = __shfl_sync(kFullMask, upto, 31);
+                unsigned long long base = 0;
+                if (all) {
+                    if (lane == 0) base = atomicAdd(cursor, static_cast<unsigned long long>(all));
+                    base = __shfl_sync(kFullMask, base, 0) + upto - padded;
+                    if (first) words[base + __popc(firsts & mates & ((1u << lane) - 1))] = make_uint2(x >> 5, mask);
+                    if (at == 0 && (n & 1)) words[base + n] = make_uint2(kNoWord, 0u);
+                }
+                // Positions stay below E / 2 + V: every edge is kept at one end.
+                if (real && at == 0) lists[v0 + row.w] = make_uint2(static_cast<uint32_t>(base), n);
+            }
+        }
+        unsigned todo = __ballot_sync(kFullMask, d > 32 && d <= kWarpRow);
+        while (todo) {
+            const int l = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t rs = __shfl_sync(kFullMask, s, l), rd = __shfl_sync(kFullMask, d, l);
+            const uint32_t ru = __shfl_sync(kFullMask, r, l);
+            uint32_t n = 0;
+            unsigned long long at = 0;
+            for (uint32_t k = lane; k < (1u << kWarpBits); k += 32) table[k] = make_uint2(kNoWord, 0u);
+            __syncwarp();
+            for (uint32_t k = lane; k < rd; k += 32) {
+                const uint32_t x = __ldg(rank + __ldg(targets + rs + k));
+                if (x < ru) table_or(table, kWarpBits, x >> 5, 1u << (x & 31));
+            }
+            __syncwarp();
+            for (uint32_t k = lane; k < (1u << kWarpBits); k += 32)
+                n += __popc(__ballot_sync(kFullMask, table[k].x != kNoWord));
+            if (n) {
+                if (lane == 0) at = take_words(words, cursor, n);
+                at = __shfl_sync(kFullMask, at, 0);
+                unsigned long long to = at;
+                for (uint32_t k = lane; k < (1u << kWarpBits); k += 32) {
+                    const uint2 e = table[k];
+                    const unsigned has = __ballot_sync(kFullMask, e.x != kNoWord);
+                    if (e.x != kNoWord) words[to + __popc(has & ((1u << lane) - 1))] = e;
+                    to += __popc(has);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) lists[v0 + l] = make_uint2(static_cast<uint32_t>(at), n);
+        }
+    }
+}
+
+// Appends, per warp, the vertices with `take` set.
+__device__ __forceinline__ void append_vertex(bool take, uint32_t v, uint32_t* __restrict__ list,
+                                              uint32_t* __restrict__ count) {
+    const unsigned mask = __ballot_sync(kFullMask, take);
+    if (mask == 0) return;
+    uint32_t at = 0;
+    const int leader = __ffs(mask) - 1;
+    if (lane_id() == static_cast<unsigned>(leader)) at = atomicAdd(count, static_cast<uint32_t>(__popc(mask)));
+    at = __shfl_sync(kFullMask, at, leader);
+    if (take) list[at + __popc(mask & ((1u << lane_id()) - 1))] = v;
+}
+
+__global__ void tw_long_rows_kernel(const uint32_t* __restrict__ offsets, uint32_t V, uint32_t* __restrict__ list,
+                                    uint32_t* __restrict__ count) {
+    for (uint64_t b = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) & ~31ull; b < V;
+         b += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        const uint64_t v = b + lane_id();
+        append_vertex(v < V && offsets[v + 1] - offsets[v] > kWarpRow, static_cast<uint32_t>(v), list, count);
+    }
+}
+
+// Longer rows, a CTA each: the ranks below the owner's are set in a bitmap,
+// kBitmapRanks of them at a time, and its non-zero words written out. Two
+// sweeps of the row where it has more than one window: the first counts.
+__global__ void __launch_bounds__(kTwThreads) tw_build_cta_kernel(
+    const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ rank,
+    const uint32_t* __restrict__ rows, const uint32_t* __restrict__ n_rows, uint32_t* __restrict__ next,
+    uint2* __restrict__ lists, uint2* __restrict__ words, unsigned long long* __restrict__ cursor) {
+    __shared__ uint32_t s_bits[kBitmapWords];
+    __shared__ uint32_t s_item, s_total, s_at;
+    __shared__ unsigned long long s_base;
+    const unsigned lane = lane_id();
+    for (uint32_t k = threadIdx.x; k < kBitmapWords; k += kTwThreads) s_bits[k] = 0;
+    const uint32_t n = *n_rows;
+    while (true) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s_item = atomicAdd(next, 1u);
+            s_total = 0;
+            s_at = 0;
+        }
+        __syncthreads();
+        if (s_item >= n) break;
+        const uint32_t u = rows[s_item];
+        const uint32_t s = offsets[u], e = offsets[u + 1], r = rank[u];
+        const uint32_t windows = (r + kBitmapRanks - 1) / kBitmapRanks;
+        for (uint32_t sweep = windows > 1 ? 0 : 1; sweep < 2; ++sweep) {
+            for (uint32_t w = 0; w < max(windows, 1u); ++w) {
+                const uint32_t lo = w * kBitmapRanks, hi = min(r - lo, kBitmapRanks) + lo;
+                for (uint64_t j = static_cast<uint64_t>(s) + threadIdx.x; j < e; j += kTwThreads) {
+                    const uint32_t x = __ldg(rank + ld_stream(targets + j));
+                    if (x >= lo && x < hi) atomicOr(s_bits + ((x - lo) >> 5), 1u << (x & 31));
+                }
+                __syncthreads();
+                const uint32_t used = (hi - lo + 31) / 32;
+                if (windows <= 1 || sweep == 0) {
+                    uint32_t mine = 0;
+                    for (uint32_t k = threadIdx.x; k < used; k += kTwThreads) {
+                        mine += s_bits[k] != 0 ? 1u : 0u;
+                        if (windows > 1) s_bits[k] = 0;
+                    }
+                    mine = warp_sum(mine);
+                    if (lane == 0 && mine) atomicAdd(&s_total, mine);
+                }
+                __syncthreads();
+                if (sweep == 1) {
+                    if (w == 0) {
+                        if (threadIdx.x == 0) {
+                            s_base = s_total ? take_words(words, cursor, s_total) : 0ull;
+                            lists[u] = make_uint2(static_cast<uint32_t>(s_base), s_total);
+                        }
+                        __syncthreads();
+                    }
+                    for (uint32_t k0 = threadIdx.x & ~31u; k0 < used; k0 += kTwThreads) {
+                        const uint32_t k = k0 + lane;
+                        const uint32_t m = k < used ? s_bits[k] : 0u;
+                        const unsigned has = __ballot_sync(kFullMask, m != 0);
+                        if (has == 0) continue;
+                        uint32_t at = 0;
+                        if (lane == 0) at = atomicAdd(&s_at, static_cast<uint32_t>(__popc(has)));
+                        at = __shfl_sync(kFullMask, at, 0);
+                        if (m) {
+                            words[s_base + at + __popc(has & ((1u << lane) - 1))] = make_uint2((lo >> 5) + k, m);
+                            s_bits[k] = 0;
+                        }
+                    }
+                }
+                __syncthreads();
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------- owners
+
+
+// Vertices with words: to the warp kernel's list, or as (vertex, slice) items
+// to the CTA kernel's.
+__global__ void tw_owners_kernel(const uint32_t* __restrict__ offsets, const uint2* __restrict__ lists, uint32_t V,
+                                 uint32_t warp_words,
+                                 uint32_t* __restrict__ warp_list, uint32_t* __restrict__ warp_count,
+                                 uint2* __restrict__ items, uint32_t* __restrict__ item_count) {
+    for (uint64_t b = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) & ~31ull; b < V;
+         b += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        const uint64_t v = b + lane_id();
+        uint32_t n = 0, d = 0;
+        if (v < V) {
+            n = lists[v].y;
+            d = offsets[v + 1] - offsets[v];
+        }
+        const bool alone = n <= warp_words && d <= kWarpOwnerRow;  // a warp's
+        append_vertex(n > 0 && alone, static_cast<uint32_t>(v), warp_list, warp_count);
+        if (n > 0 && !alone) {
+            const uint32_t slices = (d + kSlice - 1) / kSlice;
+            const uint32_t at = atomicAdd(item_count, slices);
+            for (uint32_t k = 0; k < slices; ++k) items[at + k] = make_uint2(static_cast<uint32_t>(v), k);
+        }
+    }
+}
+
+// ---------------------------------------------------------------- counting
+
+// Streams the lists e with `take` against mask(word), 2^kLogSize lanes per list
+// (a lane reads two words at a time) and kInFlight lists in flight per group of
+// lanes; with 32 lanes per list, lists may be longer than the group.
+template <uint32_t kLogSize, class Mask>
+__device__ __forceinline__ uint32_t stream_lists(bool take, const uint2 l, const uint2* __restrict__ words,
+                                                 uint2* s_list, Mask mask) {
+    const unsigned lane = lane_id();
+    const unsigned taken = __ballot_sync(kFullMask, take);
+    if (taken == 0) return 0;
+    constexpr uint32_t size = 1u << kLogSize, groups = 32u >> kLogSize;
+    const uint32_t count = __popc(taken), group = lane >> kLogSize, at = 2 * (lane & (size - 1));
+    __syncwarp();
+    if (take) s_list[__popc(taken & ((1u << lane) - 1))] = l;
+    __syncwarp();
+    uint32_t hits = 0;
+    auto add = [&](const uint4& p) {
+        hits += __popc(mask(p.x) & p.y);
+        hits += __popc(mask(p.z) & p.w);
+    };
+    for (uint32_t b = 0; b < count; b += kInFlight * groups) {
+        uint2 e[kInFlight];
+        uint4 p[kInFlight];
+#pragma unroll
+        for (int i = 0; i < kInFlight; ++i) {
+            const uint32_t k = b + i * groups + group;
+            e[i] = k < count ? s_list[k] : make_uint2(0u, 0u);
+        }
+#pragma unroll
+        for (int i = 0; i < kInFlight; ++i)
+            p[i] = at < e[i].y ? __ldg(reinterpret_cast<const uint4*>(words + e[i].x + at))
+                               : make_uint4(kNoWord, 0u, kNoWord, 0u);
+#pragma unroll
+        for (int i = 0; i < kInFlight; ++i)
+            if (at < e[i].y) add(p[i]);
+        if (kLogSize < 5) continue;
+#pragma unroll
+        for (int i = 0; i < kInFlight; ++i) {
+            uint32_t k = at + 64;
+            for (; k + 64 < e[i].y; k += 128) {
+                const uint4 x = __ldg(reinterpret_cast<const uint4*>(words + e[i].x + k));
+                const uint4 y = __ldg(reinterpret_cast<const uint4*>(words + e[i].x + k + 64));
+                add(x);
+                add(y);
+            }
+            if (k < e[i].y) add(__ldg(reinterpret_cast<const uint4*>(words + e[i].x + k)));
+        }
+    }
+    return hits;
+}
+
+// Up to 32 neighbours (v per lane, `valid`) of an owner with id u and n words:
+// the lists of those it owns the edge to (fewer words, or as many and a smaller
+// id), by length: up to 8 words 4 lanes each, up to 32 words 16, the others 32.
+template <class Mask>
+__device__ __forceinline__ uint32_t count_neighbours(bool valid, uint32_t v, uint32_t u, uint32_t n,
+                                                     const uint2* __restrict__ lists, const uint2* __restrict__ words,
+                                                     uint2* s_list, Mask mask) {
+    const uint2 l = valid ? __ldg(lists + v) : make_uint2(0u, 0u);
+    const bool take = l.y > 0 && (l.y < n || (l.y == n && v < u));
+    return stream_lists<2>(take && l.y <= 8, l, words, s_list, mask) +
+           stream_lists<4>(take && l.y > 8 && l.y <= 32, l, words, s_list, mask) +
+           stream_lists<5>(take && l.y > 32, l, words, s_list, mask);
+}
+
+// Total, or per owner (a union's graphs are told apart by their owners).
+__device__ __forceinline__ void add_owner(uint32_t u, uint32_t hits, unsigned long long* __restrict__ per_vertex,
+                                          unsigned long long& total) {
+    if (per_vertex) {
+        const uint32_t sum = __reduce_add_sync(kFullMask, hits);
+        if (lane_id() == 0 && sum) atomicAdd(per_vertex + u, static_cast<unsigned long long>(sum));
+    } else {
+        total += hits;
+    }
+}
+
+// Blocks take the CTA items first, then their warps take the warp owners: the
+// end of the one fills the idle warps with the other.
+__global__ void __launch_bounds__(kCountThreads, kCountCtasPerSm) tw_count_kernel(
+    const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ rank,
+    const uint2* __restrict__ lists, const uint2* __restrict__ words, const uint2* __restrict__ items,
+    const uint32_t* __restrict__ owners, const uint32_t* __restrict__ counts, uint32_t* __restrict__ next,
+    uint32_t batch, unsigned long long* __restrict__ total, unsigned long long* __restrict__ per_vertex) {
+    __shared__ uint32_t s_bits[kBitmapWords];
+    __shared__ uint2 s_list[kCountWarps][32];
+    __shared__ uint32_t s_item, s_chunk;
+    uint2* table = reinterpret_cast<uint2*>(s_bits);
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    const uint32_t n_items = counts[3], n_owners = counts[2];
+    unsigned long long sum = 0;
+    if (n_items)
+        for (uint32_t k = threadIdx.x; k < kBitmapWords; k += kCountThreads) s_bits[k] = 0;
+    while (true) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_item = atomicAdd(next, 1u);
+        __syncthreads();
+        if (s_item >= n_items) break;
+        const uint2 item = items[s_item];
+        const uint32_t u = item.x;
+        const uint2 own = __ldg(lists + u);
+        const uint32_t s = offsets[u] + item.y * kSlice, e = s + min(kSlice, offsets[u + 1] - s);
+        const uint32_t r = rank[u];
+        const bool hash = r > kBitmapRanks && own.y <= kHashWords;
+        const uint32_t windows = hash ? 1u : (r + kBitmapRanks - 1) / kBitmapRanks;
+        uint32_t hits = 0;
+        for (uint32_t win = 0; win < windows; ++win) {
+            const uint32_t lo = win * kBitmapWords;
+            if (hash) {
+                for (uint32_t k = threadIdx.x; k < (1u << kHashBits); k += kCountThreads)
+                    table[k] = make_uint2(kNoWord, 0u);
+                __syncthreads();
+            }
+            for (uint32_t k = threadIdx.x; k < own.y; k += kCountThreads) {
+                const uint2 w = __ldg(words + own.x + k);
+                if (hash) table_or(table, kHashBits, w.x, w.y);
+                else if (w.x - lo < kBitmapWords) s_bits[w.x - lo] = w.y;  // the words of a list are distinct
+            }
+            if (threadIdx.x == 0) s_chunk = 0;
+            __syncthreads();
+            while (true) {
+                uint32_t c = 0;
+                if (lane == 0) c = atomicAdd(&s_chunk, 32u);
+                c = __shfl_sync(kFullMask, c, 0);
+                if (c >= e - s) break;
+                const bool valid = e - s - c > lane;
+                const uint32_t v = valid ? ld_stream(targets + s + c + lane) : 0u;
+                if (hash)
+                    hits += count_neighbours(valid, v, u, own.y, lists, words, s_list[warp],
+                                             [&](uint32_t w) { return table_mask(table, kHashBits, w); });
+                else
+                    hits += count_neighbours(valid, v, u, own.y, lists, words, s_list[warp], [&](uint32_t w) {
+                        return w - lo < kBitmapWords ? s_bits[w - lo] : 0u;
+                    });
+            }
+            __syncthreads();
+            if (hash) {
+                for (uint32_t k = threadIdx.x; k < kBitmapWords; k += kCountThreads) s_bits[k] = 0;
+            } else {
+                for (uint32_t k = threadIdx.x; k < own.y; k += kCountThreads) {
+                    const uint32_t w = __ldg(words + own.x + k).x;
+                    if (w - lo < kBitmapWords) s_bits[w - lo] = 0;
+                }
+            }
+            if (win + 1 < windows) __syncthreads();
+        }
+        add_owner(u, hits, per_vertex, sum);
+    }
+    table += warp << kWarpBits;  // the warps' own tables from here on (after the loop's block barrier)
+    while (true) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(next + 1, batch);
+        base = __shfl_sync(kFullMask, base, 0);
+        if (base >= n_owners) break;
+        const uint32_t last = min(base + batch, n_owners);
+        for (uint32_t h = base; h < last; ++h) {
+            const uint32_t u = owners[h];
+            const uint2 own = __ldg(lists + u);
+            const uint32_t s = offsets[u], e = offsets[u + 1];
+            uint32_t bits = 5;  // load at most 3/8
+            while (bits < kWarpBits && (1u << bits) * 3 < own.y * 8) ++bits;
+            __syncwarp();
+            for (uint32_t k = lane; k < (1u << bits); k += 32) table[k] = make_uint2(kNoWord, 0u);
+            __syncwarp();
+            for (uint32_t k = lane; k < own.y; k += 32) {
+                const uint2 w = __ldg(words + own.x + k);
+                table_or(table, bits, w.x, w.y);
+            }
+            __syncwarp();
+            uint32_t hits = 0;
+            for (uint32_t j = s; j < e; j += 32) {
+                const bool valid = e - j > lane;
+                const uint32_t v = valid ? ld_stream(targets + j + lane) : 0u;
+                hits += count_neighbours(valid, v, u, own.y, lists, words, s_list[warp],
+                                         [&](uint32_t w) { return table_mask(table, bits, w); });
+            }
+            add_owner(u, hits, per_vertex, sum);
+        }
+    }
+    sum = warp_sum(sum);
+    if (lane == 0 && sum) atomicAdd(total, sum);
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------- host
+
+Error build_word_lists(GraphImpl& g, WordLists* w) {
+    DeviceImpl& dev = *g.dev;
+    const uint32_t V = g.num_nodes, E = g.num_edges;
+    const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
+    GCU_TRY(degree_class_order(dev, g.offsets.ptr, V, &w->rank));
+    GCU_TRY(w->lists.allocate(dev, V));
+    // Every edge's rank is kept at one end: E / 2 words at most, and a padding
+    // word per list (lists without words take no room).
+    const uint64_t room = static_cast<uint64_t>(E / 2) + std::min<uint64_t>(E / 2, V);
+    if (room > 0xFFFFFFFFull) return kernel_error("graph too large for the triangle count's word lists");
+    GCU_TRY(w->words.allocate(dev, std::max<uint64_t>(room, 1)));
+    GCU_TRY(w->warp_owners.allocate(dev, V));
+    // counters: [0] long rows, [1] next long row, [2] warp owners, [3] CTA items
+    GCU_TRY(w->counts.allocate(dev, 4));
+    DeviceBuffer<unsigned long long> cursor;
+    GCU_TRY(cursor.allocate(dev, 1));
+    GCU_CUDA(cudaMemsetAsync(w->counts.ptr, 0, 4 * sizeof(uint32_t), dev.stream), "memset");
+    GCU_CUDA(cudaMemsetAsync(cursor.ptr, 0, sizeof(unsigned long long), dev.stream), "memset");
+    const unsigned vgrid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(ceil_div_u64(V, 256), cap)));
+    uint32_t turn = 32;
+    while (turn > 4 && V / turn < static_cast<uint64_t>(dev.sm_count) * 8 * kTwWarps) turn /= 2;
+    const unsigned wgrid = static_cast<unsigned>(
+        std::max<uint64_t>(1, std::min<uint64_t>(ceil_div_u64(V, static_cast<uint64_t>(turn) * kTwWarps), cap)));
+    GCU_LAUNCH(dev, "tw_build_warp", tw_build_warp_kernel, wgrid, kTwThreads, 0, g.offsets.ptr, g.targets.ptr,
+               w->rank.ptr, V, turn, w->lists.ptr, w->words.ptr, cursor.ptr);
+    // The owner list is free until the owners are known: the long rows use it.
+    GCU_LAUNCH(dev, "tw_long_rows", tw_long_rows_kernel, vgrid, 256, 0, g.offsets.ptr, V, w->warp_owners.ptr,
+               w->counts.ptr);
+    const unsigned cgrid = static_cast<unsigned>(
+        std::max<uint64_t>(1, std::min<uint64_t>(E / kWarpRow, static_cast<uint64_t>(dev.sm_count) * 7)));
+    GCU_LAUNCH(dev, "tw_build_cta", tw_build_cta_kernel, cgrid, kTwThreads, 0, g.offsets.ptr, g.targets.ptr,
+               w->rank.ptr, w->warp_owners.ptr, w->counts.ptr, w->counts.ptr + 1, w->lists.ptr, w->words.ptr,
+               cursor.ptr);
+    // Items: at most one per kSlice entries plus one per vertex with more words,
+    // so more neighbours, than a warp owner.
+    const uint32_t warp_words = V < kSmallGraph ? kWarpWordsSmall : kWarpWords;
+    w->max_items = E / kSlice + E / warp_words + 1;
+    GCU_TRY(w->items.allocate(dev, w->max_items));
+    GCU_LAUNCH(dev, "tw_owners", tw_owners_kernel, vgrid, 256, 0, g.offsets.ptr, w->lists.ptr, V, warp_words,
+               w->warp_owners.ptr, w->counts.ptr + 2, w->items.ptr, w->counts.ptr + 3);
+    return ok();
+}
+
+Error count_words(GraphImpl& g, const WordLists& w, uint32_t* next, unsigned long long* total,
+                  unsigned long long* per_vertex) {
+    DeviceImpl& dev = *g.dev;
+    GCU_CUDA(cudaMemsetAsync(next, 0, 2 * sizeof(uint32_t), dev.stream), "memset");
+    const uint64_t want = std::max<uint64_t>(w.max_items, ceil_div_u64(g.num_nodes, kCountWarps));
+    const unsigned grid = static_cast<unsigned>(
+        std::max<uint64_t>(1, std::min<uint64_t>(want, static_cast<uint64_t>(dev.sm_count) * kCountCtasPerSm)));
+    // Owners per handout: several turns per warp, or one at a time on a small graph.
+    const uint32_t batch = static_cast<uint32_t>(
+        std::max<uint64_t>(1, std::min<uint64_t>(8, g.num_nodes / (static_cast<uint64_t>(grid) * kCountWarps * 8))));
+    GCU_LAUNCH(dev, "tw_count", tw_count_kernel, grid, kCountThreads, 0, g.offsets.ptr, g.targets.ptr, w.rank.ptr,
+               w.lists.ptr, w.words.ptr, w.items.ptr, w.warp_owners.ptr, w.counts.ptr, next, batch, total, per_vertex);
+    return ok();
+}
+
+}  // namespace gcu

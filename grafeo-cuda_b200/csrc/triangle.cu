@@ -1,4 +1,6 @@
-// Triangle counting over a degree-oriented DAG built on the device.
+// Triangle counting over a degree-oriented DAG built on the device: the form
+// for directed and already oriented CSRs, for traces and for a learned schedule
+// (a symmetric CSR under the fixed schedule is counted in tri_words.cu).
 //
 // Reference: crates/grafeo-cuda-algos/src/triangle_counting.rs:40-210 and
 // kernels/triangle_counting.cu. The reference's default path maps one warp to
@@ -591,6 +593,22 @@ Error triangle_count_ex(GraphImpl& g, bool oriented, uint64_t* total, std::vecto
     }
     bool symmetric = false;
     GCU_TRY(graph_symmetry(g, &symmetric));
+    if (symmetric && !trace && !g.dev->schedule) {
+        DeviceImpl& dev = *g.dev;
+        WordLists w;
+        DeviceBuffer<uint32_t> next;
+        DeviceBuffer<unsigned long long> sum;
+        GCU_TRY(next.allocate(dev, 2));
+        GCU_TRY(sum.allocate(dev, 1));
+        GCU_CUDA(cudaMemsetAsync(sum.ptr, 0, sizeof(unsigned long long), dev.stream), "memset");
+        GCU_TRY(build_word_lists(g, &w));
+        GCU_TRY(count_words(g, w, next.ptr, sum.ptr, nullptr));
+        unsigned long long host = 0;
+        GCU_CUDA(cudaMemcpyAsync(&host, sum.ptr, sizeof(host), cudaMemcpyDeviceToHost, dev.stream), "copy");
+        GCU_TRY(dev.sync());
+        *total = host;
+        return ok();
+    }
     DeviceBuffer<uint32_t> dag_offsets, dag_targets, rank, dag_rank;
     uint32_t m = 0;
     if (symmetric) {
@@ -639,6 +657,9 @@ struct VertexCountSink {
 }  // namespace
 
 struct BatchTcPlan {
+    // Symmetric union, no learned schedule: counted over word lists.
+    GraphImpl* word_graph = nullptr;
+    WordLists words;
     DeviceBuffer<uint32_t> dag_offsets, dag_targets;
     uint32_t m = 0;
     BucketPlan buckets;
@@ -651,6 +672,17 @@ void destroy_batch_tc_plan(BatchTcPlan* p) { delete p; }
 Error batch_tc_plan(GraphImpl& u, BatchTcPlan** out, std::string* tuning) {
     DeviceImpl& dev = *u.dev;
     auto p = std::make_unique<BatchTcPlan>();
+    bool symmetric = false;
+    GCU_TRY(graph_symmetry(u, &symmetric));
+    if (symmetric && !dev.schedule) {
+        p->word_graph = &u;
+        GCU_TRY(p->next.allocate(dev, 2));
+        GCU_TRY(build_word_lists(u, &p->words));
+        if (tuning) *tuning = "{\"variant\": \"word lists\"}";
+        GCU_TRY(dev.sync());
+        *out = p.release();
+        return ok();
+    }
     GCU_TRY(build_dag(u, true, nullptr, &p->dag_offsets, &p->dag_targets, nullptr, &p->m));
     DegreeStats stats;
     if (dev.schedule) GCU_TRY(degree_stats(u, &stats));
@@ -718,6 +750,7 @@ Error batch_tc_plan(GraphImpl& u, BatchTcPlan** out, std::string* tuning) {
 Error batch_tc_launch(DeviceImpl& dev, BatchTcPlan& p, unsigned long long* per_vertex, uint32_t num_nodes) {
     GCU_CUDA(cudaMemsetAsync(per_vertex, 0, sizeof(unsigned long long) * std::max<uint32_t>(num_nodes, 1), dev.stream),
              "memset");
+    if (p.word_graph) return count_words(*p.word_graph, p.words, p.next.ptr, nullptr, per_vertex);
     GCU_CUDA(cudaMemsetAsync(p.next.ptr, 0, sizeof(uint32_t) * kBuckets, dev.stream), "memset");
     for (int c = kBuckets - 1; c >= 0; --c) {
         if (p.buckets.host_counts[c] == 0) continue;
