@@ -42,7 +42,9 @@
 //    quarter of the L1TEX wavefronts); integer sums do not depend on the order, so the
 //    result is deterministic whatever the grid size (no float atomics);
 //    c'[v] = r'[v] / deg(v) is written for the next iteration.
-//  * The iteration loop stays on the device: each kernel reads a `done` flag
+//  * Graphs of up to kLoopEntries entries run all iterations in one cooperative
+//    launch (pr_loop_kernel): there the launches are most of the time.
+//  * Beyond, the iteration loop stays on the device: each kernel reads a `done` flag
 //    first, so the host queues iterations ahead and polls the flag once per
 //    chunk instead of syncing every iteration.
 #include <algorithm>
@@ -129,6 +131,18 @@ struct PrState {
     uint32_t pad;
 };
 
+// State of a run between launches, and the loop kernel's scratch.
+struct PrLoopState {
+    double dangling;   // sum of ranks of dangling vertices in the current ranks
+    double last_diff;  // L1 change of the last iteration
+    uint32_t iterations;
+    uint32_t done;
+    GridBarrier bar;   // zeroed before each launch, with the sums
+    unsigned long long sums[3][2];  // fixed-point L1 change and dangling mass, rotating by iteration
+};
+constexpr int kLoopThreads = 512;
+constexpr int kLoopCtasPerSm = 2;
+
 struct PageRankPlan {
     uint32_t long_rows = 0;   // rows [0, long_rows) of the relabelled CSR have >= 1024 entries
     uint32_t empty_rows = 0;  // rows without entries (the last class)
@@ -150,6 +164,10 @@ struct PageRankPlan {
     DeviceBuffer<unsigned long long> row_partials; // 2 fixed-point sums per CTA of the row kernel
     DeviceBuffer<unsigned long long> fin_partials; // 2 per block of the finishing kernel
     DeviceBuffer<PrState> state;
+    DeviceBuffer<PrLoopState> loop_state;
+    PrLoopState host_loop{};
+    uint32_t n_units = 0, empty_begin = 0;
+    unsigned loop_grid = 0;
     // Host copy of the state, read after each poll's synchronisation: plain
     // memory (a 32-byte copy needs no pinned page, and a graph's setup and
     // release then make no page-locking calls).
@@ -395,24 +413,29 @@ __global__ void pr_unpermute_kernel(const float* __restrict__ ranks, const uint3
 // outdeg[v] (pull over the transpose). Uniform teleport: r = (1-d)/N +
 // d (sum + dangling/N); with a personalisation vector p: r = (1-d) p[v] +
 // d (sum + dangling p[v]).
-__device__ __forceinline__ void pr_finish_row(uint32_t v, double sum, uint32_t row_len,
-                                              const float* __restrict__ rank_in, float* __restrict__ rank_out,
-                                              float* __restrict__ contrib_out, const uint32_t* __restrict__ outdeg,
-                                              const float* __restrict__ tele, double base, double damp,
-                                              double spread, double dangling, double& diff, double& dangle) {
-    const uint32_t deg = outdeg ? outdeg[v] : row_len;
+__device__ __forceinline__ void pr_update_row(uint32_t v, double sum, uint32_t deg, float old, bool personal, float tele,
+                                              float* __restrict__ rank_out, float* __restrict__ contrib_out,
+                                              double base, double damp, double spread, double dangling, double& diff,
+                                              double& dangle) {
     float r;
-    if (tele) {
-        const double pv = static_cast<double>(tele[v]);
+    if (personal) {
+        const double pv = static_cast<double>(tele);
         r = static_cast<float>((1.0 - damp) * pv + damp * (sum + dangling * pv));
     } else {
         r = static_cast<float>(base + damp * (sum + spread));
     }
-    const float old = rank_in[v];
     diff += fabs(static_cast<double>(r) - static_cast<double>(old));
     rank_out[v] = r;
     contrib_out[v] = deg > 0 ? r / static_cast<float>(deg) : 0.f;
     if (deg == 0) dangle += static_cast<double>(r);
+}
+
+__device__ __forceinline__ void pr_finish_row(uint32_t v, double sum, uint32_t row_len, const float* rank_in,
+                                              float* rank_out, float* contrib_out, const uint32_t* __restrict__ outdeg,
+                                              const float* __restrict__ tele, double base, double damp, double spread,
+                                              double dangling, double& diff, double& dangle) {
+    pr_update_row(v, sum, outdeg ? outdeg[v] : row_len, rank_in[v], tele != nullptr, tele ? tele[v] : 0.f, rank_out,
+                  contrib_out, base, damp, spread, dangling, diff, dangle);
 }
 
 // The L1 change and the dangling mass are summed as 64-bit fixed-point
@@ -833,6 +856,323 @@ __global__ void __launch_bounds__(256) pr_finish_kernel(
     }
 }
 
+// ---------------------------------------------------------------- the whole loop in one launch
+//
+// All iterations run in one cooperative launch. A pass deals the long rows'
+// segments, then the chunks, then the rows without entries round-robin to the
+// warps; after a grid barrier a second, short pass finishes the long rows and
+// the rows that cross chunks from their parts, and the barrier that follows
+// brings every block the iteration's L1 change and dangling mass, summed as
+// fixed-point integers. Ranks are updated in place (a rank is read by its own
+// row only); the contributions alternate between two arrays.
+// What the chunked rows are read from.
+struct PrChunks {
+    const uint32_t* poff;
+    const uint32_t* ptgt;
+    const uint8_t* delta;
+    const uint32_t* chunk_row;
+    uint32_t origin, lo, hi, n_chunks;
+    double* part;
+};
+
+// The loop kernel's form of a chunk: by one warp, 8 consecutive entries per
+// lane. Row
+// sums are FP64 (the contributions are FP32). A run of equal rows inside a lane
+// that is neither its first nor its last is a whole row; the first and last runs
+// are joined across lanes by a segmented scan. The lane where a row's run ends
+// puts its sum into s_sum (kChunk doubles of the warp's own), and then
+// consecutive lanes finish consecutive rows, so that what a row's update reads
+// and writes is coalesced and no lane finishes rows one after the other; the
+// first 32 rows' inputs are loaded beside the gathers. Parts of rows that cross
+// chunks go to part[2c] (chunk c's first row, when it began in an earlier chunk)
+// and part[2c + 1] (its last row, when that goes on into the next chunk; the
+// whole chunk when one row covers it).
+// gather(t): contribution of source t. load(row): a row's inputs, finish(row,
+// sum, length, inputs): its update.
+template <class Gather, class Load, class Finish>
+__device__ __forceinline__ void pr_chunk(const PrChunks& k, uint32_t c, double* s_sum, Gather gather, Load load,
+                                         Finish finish) {
+    const unsigned lane = lane_id();
+    const uint64_t e0 = k.origin + static_cast<uint64_t>(c) * kChunk;  // entries [e0, e0 + kChunk)
+    const uint64_t eb = e0 + 8 * lane;                                 // this lane's first (32-byte aligned)
+    const uint32_t rbase = __ldg(k.chunk_row + c);
+    const uint2 dl = ld_stream2(reinterpret_cast<const uint2*>(k.delta + (eb - k.origin)));
+    uint32_t t[8];
+    ld_stream8(k.ptgt + eb, t);
+    uint32_t row[8];  // minus rbase; kNoRow outside [lo, hi)
+    float val[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const bool ok = eb + i >= k.lo && eb + i < k.hi;
+        row[i] = ok ? ((i < 4 ? dl.x : dl.y) >> (8 * (i & 3))) & 0xFFu : kNoRow;
+        val[i] = gather(ok, t[i]);
+    }
+    const uint32_t last = static_cast<uint32_t>(min_u64(e0 + kChunk, k.hi) - 1 - e0);
+    const uint32_t n_rows =
+        1 + __shfl_sync(kFullMask, ((last & 4 ? dl.y : dl.x) >> (8 * (last & 3))) & 0xFFu, static_cast<int>(last >> 3));
+    uint32_t begin = 0, end = 0;
+    auto in = load(rbase, false);
+    if (lane < n_rows) {
+        begin = __ldg(k.poff + rbase + lane);
+        end = __ldg(k.poff + rbase + lane + 1);
+        in = load(rbase + lane, true);
+    }
+    double head = 0.0, acc = 0.0;
+    bool multi = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        acc += static_cast<double>(val[i]);
+        if (i < 7 && row[i + 1] != row[i]) {
+            if (!multi) {
+                head = acc;
+                multi = true;
+            } else {  // a whole row inside this lane (never kNoRow: those runs lead or trail)
+                s_sum[row[i]] = acc;
+            }
+            acc = 0.0;
+        }
+    }
+    // Segmented inclusive scan of the lanes' last runs: a lane continues the
+    // run of the lane before when it holds one row only and that row is the
+    // previous lane's last.
+    const uint32_t rf = row[0], rl = row[7];
+    const uint32_t prev_last = __shfl_up_sync(kFullMask, rl, 1);
+    const uint32_t next_first = __shfl_down_sync(kFullMask, rf, 1);
+    const bool carry_in = lane > 0 && prev_last == rf;
+    bool head_flag = multi || !carry_in;
+    double S = acc;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const double su = __shfl_up_sync(kFullMask, S, d);
+        const bool fu = __shfl_up_sync(kFullMask, head_flag, d);
+        if (lane >= static_cast<unsigned>(d)) {
+            if (!head_flag) S += su;
+            head_flag = head_flag || fu;
+        }
+    }
+    const double carry = __shfl_up_sync(kFullMask, S, 1);
+    if (multi && rf != kNoRow) s_sum[rf] = head + (carry_in ? carry : 0.0);  // the first run ends in this lane
+    if (!(lane < 31 && next_first == rl) && rl != kNoRow) s_sum[rl] = S;     // the last run ends at this lane's end
+    __syncwarp();
+    for (uint32_t r = lane; r < n_rows; r += 32) {
+        if (r >= 32) {
+            begin = __ldg(k.poff + rbase + r);
+            end = __ldg(k.poff + rbase + r + 1);
+            in = load(rbase + r, true);
+        }
+        const double sum = s_sum[r];
+        // Only a chunk's first row can have begun before it, only its last go on after it.
+        if (end > e0 + kChunk) k.part[2 * static_cast<uint64_t>(c) + 1] = sum;
+        else if (begin < e0) k.part[2 * static_cast<uint64_t>(c)] = sum;
+        else finish(rbase + r, sum, end - begin, in);
+    }
+    __syncwarp();  // s_sum is the next chunk's
+}
+
+// A row's inputs besides its sum.
+struct PrRowIn {
+    float old;
+    uint32_t deg;   // out-degree (pull over the transpose; else the row length is it)
+    float tele;
+};
+
+struct PrLoop {
+    const uint32_t* poff;
+    const uint32_t* ptgt;
+    PrChunks chunks;
+    const uint2* units;
+    const uint32_t* unit_begin;
+    const uint4* split_rows;
+    const uint32_t* outdeg;  // NULL: the row lengths
+    const float* tele;       // NULL: uniform
+    const uint32_t* inv;
+    float* ranks;            // relabelled order
+    float* contrib;          // 2 V
+    double* seg_partial;
+    float* out;              // original order
+    uint32_t V, long_rows, n_units, n_split, empty_begin;
+    float r0;
+    double base, damp, tolerance;
+    uint32_t first, last;    // iterations [first, last) of the run
+    PrLoopState* st;
+};
+
+// Sums of one lane over the rows it finished.
+struct PrSums {
+    unsigned long long diff = 0, dangle = 0;
+};
+
+struct PrPass {
+    const float* in;
+    float* out;
+    double mass, spread;  // dangling mass, its uniform share
+};
+
+__device__ __forceinline__ void pr_loop_row(const PrLoop& a, const PrPass& p, uint32_t row, double sum, uint32_t len,
+                                            PrSums& s) {
+    double d = 0.0, dg = 0.0;
+    pr_finish_row(row, sum, len, a.ranks, a.ranks, p.out, a.outdeg, a.tele, a.base, a.damp, p.spread, p.mass, d, dg);
+    s.diff += to_fixed(d);
+    s.dangle += to_fixed(dg);
+}
+
+// A 1024-entry segment of a long row: 32 entries per lane, kSegmentLoads in flight.
+constexpr int kSegmentLoads = 8;
+
+__device__ __forceinline__ float ld_contrib(const float* c, uint32_t t) {
+    return __uint_as_float(ld_if(true, reinterpret_cast<const uint32_t*>(c) + t, 0u));
+}
+
+__device__ __forceinline__ void pr_segment(const PrLoop& a, const PrPass& p, uint32_t u) {
+    const unsigned lane = lane_id();
+    const uint2 unit = __ldg(a.units + u);
+    const uint32_t row_start = __ldg(a.poff + unit.x), row_end = __ldg(a.poff + unit.x + 1);
+    const uint32_t s0 = row_start + unit.y * kSegment;
+    const uint32_t n = min(kSegment, row_end - s0);
+    float acc = 0.f, comp = 0.f;
+    uint32_t j = lane;
+    for (; j + (kSegmentLoads - 1) * 32 < n; j += kSegmentLoads * 32) {
+        uint32_t t[kSegmentLoads];
+#pragma unroll
+        for (int q = 0; q < kSegmentLoads; ++q) t[q] = ld_stream(a.ptgt + s0 + j + q * 32);
+        float c[kSegmentLoads];
+#pragma unroll
+        for (int q = 0; q < kSegmentLoads; ++q) c[q] = ld_contrib(p.in, t[q]);
+#pragma unroll
+        for (int q = 0; q < kSegmentLoads; ++q) kahan_add(acc, comp, c[q]);
+    }
+    for (; j < n; j += 32) kahan_add(acc, comp, ld_contrib(p.in, ld_stream(a.ptgt + s0 + j)));
+    const double part = warp_sum(static_cast<double>(acc) - static_cast<double>(comp));
+    if (lane == 0) a.seg_partial[u] = part;
+}
+
+// Finishes long row i from its segment partials (in segment order), or, past
+// the long rows, a row that crosses chunks from its parts: its part in its
+// first chunk (that chunk's last row), every chunk it covers whole, its part in
+// its last.
+__device__ __forceinline__ void pr_joined_row(const PrLoop& a, const PrPass& p, uint32_t i, PrSums& s) {
+    double sum = 0.0;
+    uint32_t row = i;
+    if (i < a.long_rows) {
+        const uint32_t e = __ldg(a.unit_begin + i + 1);
+        for (uint32_t u = __ldg(a.unit_begin + i); u < e; ++u) sum += a.seg_partial[u];
+    } else {
+        const uint4 sr = __ldg(a.split_rows + (i - a.long_rows));
+        row = sr.x;
+        sum = a.chunks.part[2 * static_cast<uint64_t>(sr.y) + 1];
+        for (uint32_t c = sr.y + 1; c < sr.z; ++c) sum += a.chunks.part[2 * static_cast<uint64_t>(c) + 1];
+        sum += a.chunks.part[2 * static_cast<uint64_t>(sr.z)];
+    }
+    pr_loop_row(a, p, row, sum, __ldg(a.poff + row + 1) - __ldg(a.poff + row), s);
+}
+
+__global__ void __launch_bounds__(kLoopThreads, kLoopCtasPerSm) pr_loop_kernel(const PrLoop a) {
+    constexpr int kWarps = kLoopThreads / 32;
+    __shared__ double s_rows[kWarps][kChunk];
+    __shared__ unsigned long long s_sum[2 * kWarps];
+    __shared__ unsigned long long s_total[2];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    // Consecutive warps of a block take consecutive units; the units of each
+    // kind start at the warp where the kind before ended.
+    const uint32_t W = static_cast<uint32_t>(nthreads >> 5), w0 = static_cast<uint32_t>(tid >> 5);
+    const uint32_t w1 = (w0 + W - a.n_units % W) % W;
+    const uint32_t w2 = (w1 + W - a.chunks.n_chunks % W) % W;
+    unsigned barriers = 0;
+    if (a.first == 0) {
+        for (uint64_t v = tid; v < a.V; v += nthreads) {
+            const uint32_t deg = a.outdeg ? a.outdeg[v] : a.poff[v + 1] - a.poff[v];
+            a.ranks[v] = a.r0;
+            a.contrib[v] = deg > 0 ? a.r0 / static_cast<float>(deg) : 0.f;
+        }
+        if (!grid_barrier(&a.st->bar, barriers)) return;
+    }
+    double mass = a.st->dangling, change = a.st->last_diff;
+    uint32_t done = 0, it = a.first;
+    // Adds the block's sums into the iteration's slot.
+    auto post = [&](const PrSums& s, unsigned long long* slot) {
+        const unsigned long long d = warp_sum(s.diff), g = warp_sum(s.dangle);
+        if (lane == 0) {
+            s_sum[2 * warp] = d;
+            s_sum[2 * warp + 1] = g;
+        }
+        __syncthreads();
+        if (warp < 2) {
+            const unsigned long long x = warp_sum(lane < kWarps ? s_sum[2 * lane + warp] : 0ull);
+            if (lane == 0 && x) atomicAdd(slot + warp, x);
+        }
+    };
+    while (it < a.last && !done) {
+        // Slot it % 3 takes this iteration's sums; the next one's is cleared
+        // here, two barriers after its last readers.
+        unsigned long long* slot = a.st->sums[it % 3];
+        if (tid < 2) a.st->sums[(it + 1) % 3][tid] = 0;
+        PrPass p;
+        p.in = a.contrib + ((it & 1) ? a.V : 0u);
+        p.out = a.contrib + ((it & 1) ? 0u : a.V);
+        p.mass = mass;
+        p.spread = mass / static_cast<double>(a.V);
+        {
+            PrSums s;
+            for (uint32_t u = w0; u < a.n_units; u += W) pr_segment(a, p, u);
+            for (uint32_t c = w1; c < a.chunks.n_chunks; c += W)
+                pr_chunk(
+                    a.chunks, c, s_rows[warp],
+                    [&](bool ok, uint32_t t) {
+                        return __uint_as_float(ld_if(ok, reinterpret_cast<const uint32_t*>(p.in) + t, 0u));
+                    },
+                    [&](uint32_t r, bool real) {
+                        PrRowIn in{0.f, 0u, 0.f};
+                        if (real) {
+                            in.old = a.ranks[r];
+                            if (a.outdeg) in.deg = __ldg(a.outdeg + r);
+                            if (a.tele) in.tele = __ldg(a.tele + r);
+                        }
+                        return in;
+                    },
+                    [&](uint32_t r, double sum, uint32_t len, const PrRowIn& in) {
+                        double d = 0.0, dg = 0.0;
+                        pr_update_row(r, sum, a.outdeg ? in.deg : len, in.old, a.tele != nullptr, in.tele, a.ranks,
+                                      p.out, a.base, a.damp, p.spread, p.mass, d, dg);
+                        s.diff += to_fixed(d);
+                        s.dangle += to_fixed(dg);
+                    });
+            for (uint64_t r = a.empty_begin + static_cast<uint64_t>(w2) * 32 + lane; r < a.V;
+                 r += static_cast<uint64_t>(W) * 32)
+                pr_loop_row(a, p, static_cast<uint32_t>(r), 0.0, 0, s);
+            post(s, slot);
+        }
+        if (!grid_barrier(&a.st->bar, barriers)) return;
+        {
+            PrSums s;
+            const uint64_t joined = static_cast<uint64_t>(a.long_rows) + a.n_split;
+            // 32 consecutive rows per warp, consecutive groups on different SMs.
+            for (uint64_t i = (static_cast<uint64_t>(warp) * gridDim.x + blockIdx.x) * 32 + lane; i < joined;
+                 i += nthreads)
+                pr_joined_row(a, p, static_cast<uint32_t>(i), s);
+            post(s, slot);
+        }
+        if (!grid_barrier(&a.st->bar, gridDim.x, barriers, [&] {
+                s_total[0] = __ldcg(slot);
+                s_total[1] = __ldcg(slot + 1);
+            }))
+            return;
+        change = from_fixed(s_total[0]);
+        mass = from_fixed(s_total[1]);
+        ++it;
+        done = change < a.tolerance ? 1u : 0u;
+    }
+    if (done || a.out)
+        for (uint64_t v = tid; v < a.V; v += nthreads) a.out[v] = a.ranks[__ldg(a.inv + v)];
+    if (tid == 0) {
+        a.st->dangling = mass;
+        a.st->last_diff = change;
+        a.st->iterations = it;
+        a.st->done = done;
+    }
+}
+
 // ---------------------------------------------------------------- host
 
 // Builds the relabelled pull CSR and the schedule for pulling over
@@ -1014,10 +1354,24 @@ static Error build_plan(GraphImpl& g, const uint32_t* pull_offsets, const uint32
     GCU_TRY(p.row_partials.allocate(dev, 2 * (static_cast<uint64_t>(p.row_ctas) + p.chunk_ctas)));
     GCU_TRY(p.fin_partials.allocate(dev, 2 * static_cast<uint64_t>(p.fin_blocks)));
     GCU_TRY(p.state.allocate(dev, 1));
+    GCU_TRY(p.loop_state.allocate(dev, 1));
+    p.n_units = n_units;
+    p.empty_begin = begin[0];
     GCU_TRY(dev.sync());
     *out = plan.release();
     return ok();
 }
+
+// The loop kernel runs graphs of up to this many entries. Measured per
+// iteration, launch per kernel against loop kernel (20 iterations, one B200):
+// R-MAT 10 22.9 / 8.7 us, 12 27.9 / 10.5, 14 28.5 / 12.0, 16 34.6 / 16.7, 18 (7.6 M
+// entries) 44.2 / 29.8, Erdos-Renyi 2^18 (8.4 M) 55 / 49; beyond, R-MAT 20 (31 M)
+// 97 / 120, R-MAT 22 373 / 553, Erdos-Renyi 2^20 167 / 172: there the gathers keep
+// the SMs busy, and the L1 that the loop kernel's row sums take (33 KB per block)
+// and the registers it shares between the phases cost more than the launches.
+constexpr uint32_t kLoopEntries = 16u << 20;
+// Iterations per launch (the host looks at the state in between).
+constexpr uint32_t kLoopIterations = 512;
 
 static Error ensure_plan(GraphImpl& g, bool directed, PageRankPlan** plan) {
     PageRankPlan*& slot = directed ? g.pr_plan_directed : g.pr_plan;
@@ -1141,8 +1495,74 @@ Error pagerank_ex(GraphImpl& g, bool directed, const float* tele_host, float dam
                    tele.ptr);
     }
     const float* d_tele = tele_host ? tele.ptr : nullptr;
+    const PrChunks chunks{p.poff.ptr,      p.ptgt.ptr, p.chunk_delta.ptr, p.chunk_row.ptr,
+                          p.chunk_origin, p.chunk_lo, p.chunk_hi,        p.n_chunks, p.chunk_part.ptr};
 
     const float r0 = 1.0f / static_cast<float>(V);  // pagerank.rs:83
+    if (p.n_chunks > 0 && g.num_edges <= kLoopEntries) {
+        if (!p.loop_grid) {
+            int per_sm = 0;
+            GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pr_loop_kernel, kLoopThreads, 0),
+                     "occupancy");
+            const uint64_t most = static_cast<uint64_t>(dev.sm_count) * std::max(1, std::min(per_sm, kLoopCtasPerSm));
+            // A warp per chunk or its equivalent where the graph is that small
+            // (half or a quarter of the warps measured 2-8 us an iteration slower).
+            const uint64_t warps = static_cast<uint64_t>(p.n_units) * (kSegment / kChunk) + p.n_chunks +
+                                   ceil_div_u64(p.empty_rows, 32);
+            p.loop_grid = static_cast<unsigned>(
+                std::max<uint64_t>(1, std::min<uint64_t>(most, ceil_div_u64(warps, kLoopThreads / 32))));
+        }
+        PrLoop a{};
+        a.poff = p.poff.ptr;
+        a.ptgt = p.ptgt.ptr;
+        a.chunks = chunks;
+        a.units = p.units.ptr;
+        a.unit_begin = p.unit_begin.ptr;
+        a.split_rows = p.split_rows.ptr;
+        a.outdeg = outdeg;
+        a.tele = d_tele;
+        a.inv = p.inv.ptr;
+        a.ranks = p.ranks.ptr;
+        a.contrib = p.contrib.ptr;
+        a.seg_partial = p.seg_partial.ptr;
+        a.out = p.ranks_out.ptr;
+        a.V = V;
+        a.long_rows = p.long_rows;
+        a.n_units = p.n_units;
+        a.n_split = p.n_split;
+        a.empty_begin = p.empty_begin;
+        a.r0 = r0;
+        a.damp = static_cast<double>(damping);
+        a.base = (1.0 - a.damp) / static_cast<double>(V);
+        a.tolerance = static_cast<double>(tolerance);
+        a.st = p.loop_state.ptr;
+        PrLoopState start{};
+        start.dangling = static_cast<double>(p.dangling_rows) * static_cast<double>(r0);
+        start.last_diff = INFINITY;
+        p.host_loop = start;
+        do {
+            p.host_loop.bar = GridBarrier{};
+            std::fill(&p.host_loop.sums[0][0], &p.host_loop.sums[0][0] + 6, 0ull);
+            GCU_CUDA(cudaMemcpyAsync(p.loop_state.ptr, &p.host_loop, sizeof(PrLoopState), cudaMemcpyHostToDevice,
+                                     dev.stream),
+                     "copy");
+            a.first = p.host_loop.iterations;
+            a.last = a.first + std::min<uint32_t>(max_iterations - a.first, kLoopIterations);
+            GCU_LAUNCH_COOP(dev, "pr_loop", pr_loop_kernel, p.loop_grid, kLoopThreads, 0, a);
+            GCU_CUDA(cudaMemcpyAsync(&p.host_loop, p.loop_state.ptr, sizeof(PrLoopState), cudaMemcpyDeviceToHost,
+                                     dev.stream),
+                     "copy");
+            if (host_ranks && a.last == max_iterations)
+                GCU_TRY(copy_to_host(dev, host_ranks, p.ranks_out.ptr, sizeof(float) * V));
+            GCU_TRY(dev.sync());
+            if (p.host_loop.bar.failed) return kernel_error("PageRank: a block did not reach the grid barrier");
+        } while (!p.host_loop.done && p.host_loop.iterations < max_iterations);
+        if (host_ranks && a.last != max_iterations)
+            GCU_TRY(copy_to_host(dev, host_ranks, p.ranks_out.ptr, sizeof(float) * V));
+        *iterations = p.host_loop.iterations;
+        *converged = p.host_loop.done != 0;
+        return ok();
+    }
     GCU_LAUNCH(dev, "pr_init", pr_init_kernel, vgrid, 256, 0, p.poff.ptr, outdeg, V, r0, ranks[0], contrib[0]);
     PrState init{};
     init.dangling = static_cast<double>(p.dangling_rows) * static_cast<double>(r0);
