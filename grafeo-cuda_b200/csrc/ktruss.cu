@@ -177,12 +177,11 @@ __global__ void kt_loops_kernel(const uint32_t* __restrict__ targets, const uint
 // Round r: every alive u < v entry whose support is below the threshold is
 // removed (state = r) and listed. With `loop` in round 1 a self-loop at either
 // end adds one to the support, as the reference's merge of the raw lists
-// does. With `truss`, every removed entry also gets truss_value there.
+// does.
 __global__ void kt_round_filter_kernel(const uint32_t* __restrict__ targets, const uint32_t* __restrict__ src,
                                        const uint8_t* __restrict__ loop, const uint32_t* __restrict__ support,
                                        uint32_t* __restrict__ state, uint32_t E, uint32_t threshold, uint32_t round,
-                                       uint32_t* __restrict__ removed, uint32_t* __restrict__ removed_count,
-                                       uint32_t* __restrict__ truss, uint32_t truss_value) {
+                                       uint32_t* __restrict__ removed, uint32_t* __restrict__ removed_count) {
     const unsigned lane = lane_id();
     for (uint64_t base = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) & ~31ull; base < E;
          base += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
@@ -194,7 +193,6 @@ __global__ void kt_round_filter_kernel(const uint32_t* __restrict__ targets, con
                 uint32_t s = support[j];
                 if (loop && round == 1) s += loop[u] + loop[v];
                 take = s < threshold;
-                if (take && truss) truss[j] = truss_value;
             }
         }
         const unsigned mask = __ballot_sync(kFullMask, take);
@@ -231,18 +229,17 @@ struct PeelEdge {
     uint32_t xs, xe, ys, ye;
 };
 
-// Lists of the live CSR `lv` (the graph's CSR, or its alive entries after a
-// compaction); e is an entry of the graph's CSR.
+// The graph's CSR (eid == nullptr), or its alive entries after a compaction with
+// the u < v entry of each one's edge.
 struct LiveCsr {
     const uint32_t* offsets;
     const uint32_t* targets;
-    const uint32_t* eid;  // graph entry of each live entry (nullptr: the graph's CSR itself)
-    __device__ __forceinline__ uint32_t entry(uint32_t p) const { return eid ? eid[p] : p; }
+    const uint32_t* eid;
 };
 
-__device__ __forceinline__ PeelEdge peel_edge(const LiveCsr& lv, const uint32_t* __restrict__ targets,
+__device__ __forceinline__ PeelEdge peel_edge(const uint32_t* __restrict__ offsets,
+                                              const uint32_t* __restrict__ targets,
                                               const uint32_t* __restrict__ src, uint32_t e) {
-    const uint32_t* __restrict__ offsets = lv.offsets;
     PeelEdge p;
     p.a = src[e];
     p.b = targets[e];
@@ -262,20 +259,20 @@ __device__ __forceinline__ PeelEdge peel_edge(const LiveCsr& lv, const uint32_t*
 }
 
 // chunks[i] = the walk chunks of removed edge i (at least one).
-__global__ void kt_peel_chunks_kernel(const LiveCsr lv, const uint32_t* __restrict__ targets,
+__global__ void kt_peel_chunks_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ targets,
                                       const uint32_t* __restrict__ src, const uint32_t* __restrict__ removed,
                                       const uint32_t* __restrict__ removed_count, uint32_t* __restrict__ chunks) {
     const uint32_t n = *removed_count;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const PeelEdge p = peel_edge(lv, targets, src, removed[i]);
+        const PeelEdge p = peel_edge(offsets, targets, src, removed[i]);
         chunks[i] = max(1u, (p.xe - p.xs + kPeelChunk - 1) / kPeelChunk);
     }
 }
 
 // Warp per chunk: chunk_start (n + 1 words) is the exclusive scan of the
 // chunk counts; each warp finds its edge by a binary search of it.
-__global__ void __launch_bounds__(256) kt_peel_kernel(const LiveCsr lv,
+__global__ void __launch_bounds__(256) kt_peel_kernel(const uint32_t* __restrict__ offsets,
                                                       const uint32_t* __restrict__ targets,
                                                       const uint32_t* __restrict__ src,
                                                       const uint32_t* __restrict__ rev,
@@ -301,20 +298,18 @@ __global__ void __launch_bounds__(256) kt_peel_kernel(const LiveCsr lv,
                 hi = mid;
         }
         const uint32_t e = removed[lo];
-        const PeelEdge pe = peel_edge(lv, targets, src, e);
+        const PeelEdge pe = peel_edge(offsets, targets, src, e);
         const uint32_t begin = pe.xs + (static_cast<uint32_t>(w) - chunk_start[lo]) * kPeelChunk;
         const uint32_t end = min(begin + kPeelChunk, pe.xe);
         for (uint32_t p = begin + lane; p < end; p += 32) {
-            const uint32_t wv = lv.targets[p];
+            const uint32_t wv = targets[p];
             if (wv == pe.a || wv == pe.b) continue;
-            const uint32_t j1 = lv.entry(p);
-            const uint32_t e1 = pe.x < wv ? j1 : rev[j1];
+            const uint32_t e1 = pe.x < wv ? p : rev[p];
             const uint32_t s1 = state[e1];
             if (s1 != 0 && s1 != round) continue;
-            const uint32_t q = lower_bound_u32(lv.targets, pe.ys, pe.ye, wv);
-            if (q == pe.ye || lv.targets[q] != wv) continue;
-            const uint32_t j2 = lv.entry(q);
-            const uint32_t e2 = pe.y < wv ? j2 : rev[j2];
+            const uint32_t q = lower_bound_u32(targets, pe.ys, pe.ye, wv);
+            if (q == pe.ye || targets[q] != wv) continue;
+            const uint32_t e2 = pe.y < wv ? q : rev[q];
             const uint32_t s2 = state[e2];
             if (s2 != 0 && s2 != round) continue;
             if ((s1 == round && e1 < e) || (s2 == round && e2 < e)) continue;
@@ -326,31 +321,32 @@ __global__ void __launch_bounds__(256) kt_peel_kernel(const LiveCsr lv,
 
 // One peel: chunk counts of the n removed edges, their scan, the chunk walk.
 // chunks holds n + 1 words.
-static Error launch_peel(DeviceImpl& dev, GraphImpl& g, const LiveCsr& lv, const uint32_t* src,
+static Error launch_peel(DeviceImpl& dev, GraphImpl& g, const uint32_t* src,
                          const uint32_t* rev, const uint32_t* state, uint32_t* support, const uint32_t* list,
                          const uint32_t* count, uint32_t n, uint32_t* chunks, uint32_t round, uint32_t threshold,
                          uint32_t* next, uint32_t* next_count) {
     const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
     const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(ceil_div_u64(n, 256), cap)));
-    GCU_LAUNCH(dev, "kt_peel_chunks", kt_peel_chunks_kernel, grid, 256, 0, lv, g.targets.ptr, src, list, count,
+    GCU_LAUNCH(dev, "kt_peel_chunks", kt_peel_chunks_kernel, grid, 256, 0, g.offsets.ptr, g.targets.ptr, src, list, count,
                chunks);
     GCU_TRY(exclusive_scan_u32(dev, chunks, chunks, n));
-    GCU_LAUNCH(dev, "kt_peel", kt_peel_kernel, static_cast<unsigned>(cap), 256, 0, lv, g.targets.ptr, src, rev,
+    GCU_LAUNCH(dev, "kt_peel", kt_peel_kernel, static_cast<unsigned>(cap), 256, 0, g.offsets.ptr, g.targets.ptr, src, rev,
                state, support, list, count, chunks, round, threshold, next, next_count);
     return ok();
 }
 
 // ---------------------------------------------------------------- live CSR compaction
 
-// keep[p] for every live entry p = u -> w: not a self-loop and its edge alive.
+// keep[p] for every live entry p = u -> w: not a self-loop and its edge alive
+// (state 0, or `pending`: removed in the next round only).
 __global__ void __launch_bounds__(256) kt_live_flag_kernel(const LiveCsr lv, uint32_t V, uint32_t L,
                                                            const uint32_t* __restrict__ rev,
-                                                           const uint32_t* __restrict__ state,
+                                                           const uint32_t* __restrict__ state, uint32_t pending,
                                                            uint32_t* __restrict__ keep) {
     for_each_entry<256, 4>(lv.offsets, V, L, [&](uint32_t p, uint32_t u) {
         const uint32_t w = lv.targets[p];
-        const uint32_t j = lv.entry(p);
-        keep[p] = (u != w && state[u < w ? j : rev[j]] == 0) ? 1u : 0u;
+        const uint32_t s = u != w ? state[lv.eid ? lv.eid[p] : u < w ? p : rev[p]] : 1u;
+        keep[p] = (u != w && (s == 0 || (pending && s == pending))) ? 1u : 0u;
     });
 }
 
@@ -361,15 +357,19 @@ __global__ void kt_live_offsets_kernel(const uint32_t* __restrict__ offsets, uin
         out[u] = pos[offsets[u]];
 }
 
-__global__ void kt_live_fill_kernel(const LiveCsr lv, uint32_t L, const uint32_t* __restrict__ pos,
-                                    uint32_t* __restrict__ targets, uint32_t* __restrict__ eid) {
-    for (uint64_t p = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < L;
-         p += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+// eid: the u < v entry, in the graph's CSR, of the edge of each live entry.
+__global__ void __launch_bounds__(256) kt_live_fill_kernel(const LiveCsr lv, uint32_t V, uint32_t L,
+                                                           const uint32_t* __restrict__ rev,
+                                                           const uint32_t* __restrict__ pos,
+                                                           uint32_t* __restrict__ targets,
+                                                           uint32_t* __restrict__ eid) {
+    for_each_entry<256, 4>(lv.offsets, V, L, [&](uint32_t p, uint32_t u) {
         const uint32_t at = pos[p];
-        if (pos[p + 1] == at) continue;
-        targets[at] = lv.targets[p];
-        eid[at] = lv.entry(p);
-    }
+        if (pos[p + 1] == at) return;
+        const uint32_t w = lv.targets[p];
+        targets[at] = w;
+        eid[at] = lv.eid ? lv.eid[p] : u < w ? p : rev[p];
+    });
 }
 
 // The alive entries of `lv` (L entries) in a new CSR (same order), so that
@@ -380,17 +380,16 @@ struct LiveBuffers {
 };
 
 static Error compact_live(DeviceImpl& dev, uint32_t V, const LiveCsr& lv, uint32_t L, const uint32_t* rev,
-                          const uint32_t* state, LiveBuffers* out) {
+                          const uint32_t* state, LiveBuffers* out, uint32_t pending = 0) {
     const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
     DeviceBuffer<uint32_t> pos;
     GCU_TRY(pos.allocate(dev, static_cast<uint64_t>(L) + 1));
     GCU_TRY(out->offsets.allocate(dev, static_cast<uint64_t>(V) + 1));
     const unsigned tiles = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(ceil_div_u64(L, 1024), cap)));
-    const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(ceil_div_u64(L, 256), cap)));
     const unsigned vgrid =
         static_cast<unsigned>(std::min<uint64_t>(ceil_div_u64(static_cast<uint64_t>(V) + 1, 256), cap));
     if (L > 0)
-        GCU_LAUNCH(dev, "kt_live_flag", kt_live_flag_kernel, tiles, 256, 0, lv, V, L, rev, state, pos.ptr);
+        GCU_LAUNCH(dev, "kt_live_flag", kt_live_flag_kernel, tiles, 256, 0, lv, V, L, rev, state, pending, pos.ptr);
     GCU_TRY(exclusive_scan_u32(dev, pos.ptr, pos.ptr, L));
     GCU_LAUNCH(dev, "kt_live_offsets", kt_live_offsets_kernel, vgrid, 256, 0, lv.offsets, V, pos.ptr,
                out->offsets.ptr);
@@ -400,24 +399,19 @@ static Error compact_live(DeviceImpl& dev, uint32_t V, const LiveCsr& lv, uint32
     GCU_TRY(out->targets.allocate(dev, std::max<uint32_t>(out->entries, 1)));
     GCU_TRY(out->eid.allocate(dev, std::max<uint32_t>(out->entries, 1)));
     if (out->entries > 0)
-        GCU_LAUNCH(dev, "kt_live_fill", kt_live_fill_kernel, grid, 256, 0, lv, L, pos.ptr, out->targets.ptr,
+        GCU_LAUNCH(dev, "kt_live_fill", kt_live_fill_kernel, tiles, 256, 0, lv, V, L, rev, pos.ptr, out->targets.ptr,
                    out->eid.ptr);
     GCU_TRY(dev.sync());  // pos is freed on return
     return ok();
 }
 
-// The entries listed for round r are removed in it (state = r); with truss,
-// they also get truss_value.
+// The entries listed for round r are removed in it (state = r).
 __global__ void kt_mark_kernel(const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
-                               uint32_t* __restrict__ state, uint32_t round, uint32_t* __restrict__ truss,
-                               uint32_t truss_value) {
+                               uint32_t* __restrict__ state, uint32_t round) {
     const uint32_t n = *count;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const uint32_t j = list[i];
-        state[j] = round;
-        if (truss) truss[j] = truss_value;
-    }
+         i += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+        state[list[i]] = round;
 }
 
 // Compacts the alive u < v entries, in CSR order, into host pairs.
@@ -576,8 +570,7 @@ static Error k_truss_symmetric(GraphImpl& g, uint32_t k, std::vector<uint32_t>* 
         if (scan) {
             GCU_CUDA(cudaMemsetAsync(scratch.ptr, 0, sizeof(uint32_t), dev.stream), "memset");
             GCU_LAUNCH(dev, "kt_round_filter", kt_round_filter_kernel, edge_grid, 256, 0, g.targets.ptr, src,
-                       c->loop.ptr, support.ptr, state.ptr, E, threshold, round, removed.ptr, scratch.ptr, nullptr,
-                       0u);
+                       c->loop.ptr, support.ptr, state.ptr, E, threshold, round, removed.ptr, scratch.ptr);
             GCU_CUDA(cudaMemcpyAsync(&n, scratch.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
             GCU_TRY(dev.sync());
         } else {
@@ -587,8 +580,7 @@ static Error k_truss_symmetric(GraphImpl& g, uint32_t k, std::vector<uint32_t>* 
             if (n > 0) {
                 const unsigned grid =
                     static_cast<unsigned>(std::min<uint64_t>(ceil_div_u64(n, 256), cap));
-                GCU_LAUNCH(dev, "kt_mark", kt_mark_kernel, grid, 256, 0, list, count, state.ptr, round,
-                           static_cast<uint32_t*>(nullptr), 0u);
+                GCU_LAUNCH(dev, "kt_mark", kt_mark_kernel, grid, 256, 0, list, count, state.ptr, round);
             }
         }
         // Round 1 also removes the self-loop entries (their support is 0).
@@ -597,8 +589,7 @@ static Error k_truss_symmetric(GraphImpl& g, uint32_t k, std::vector<uint32_t>* 
         uint32_t next_n = 0;
         GCU_CUDA(cudaMemsetAsync(scratch.ptr + 1 + cur, 0, sizeof(uint32_t), dev.stream), "memset");
         if (n > 0) {
-            GCU_TRY(launch_peel(dev, g, LiveCsr{g.offsets.ptr, g.targets.ptr, nullptr}, src, rev, state.ptr,
-                                support.ptr, list, count, n, chunks.ptr, round, threshold, lists[cur].ptr,
+            GCU_TRY(launch_peel(dev, g, src, rev, state.ptr, support.ptr, list, count, n, chunks.ptr, round, threshold, lists[cur].ptr,
                                 scratch.ptr + 1 + cur));
             GCU_CUDA(cudaMemcpyAsync(&next_n, scratch.ptr + 1 + cur, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                      dev.stream),
@@ -669,28 +660,208 @@ __global__ void kt_active_kernel(const uint32_t* __restrict__ targets, const uin
     }
 }
 
-// kt_round_filter_kernel over an active list: every listed entry still alive
-// with support < threshold is removed in this round (state = round), listed in
-// `removed` and given truss_value.
-__global__ void kt_active_filter_kernel(const uint32_t* __restrict__ active, uint32_t n,
-                                        const uint32_t* __restrict__ support, uint32_t* __restrict__ state,
-                                        uint32_t threshold, uint32_t round, uint32_t* __restrict__ removed,
-                                        uint32_t* __restrict__ removed_count, uint32_t* __restrict__ truss,
-                                        uint32_t truss_value) {
-    for (uint64_t base = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) & ~31ull; base < n;
-         base += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const uint64_t i = base + lane_id();
-        bool take = false;
-        uint32_t j = 0;
-        if (i < n) {
-            j = active[i];
-            take = state[j] == 0 && support[j] < threshold;
-            if (take) {
-                state[j] = round;
-                truss[j] = truss_value;
+// The decomposition's rounds run in one cooperative launch, from one compaction
+// of the live lists to the next; the blocks meet at a grid barrier after every
+// scan and every peel. State of an edge (its u < v entry): 0 alive, r removed in
+// round r; the peel of round r marks what round r + 1 removes with r + 1 when it
+// lists it, so during round r an edge is alive if its state is 0 or r + 1.
+struct TrussState {
+    GridBarrier bar;
+    uint32_t count[3];  // entries listed by the phase, rotating (slot p % 3 is phase p's)
+    uint32_t least[3];  // smallest support a scan left alive
+    // carried from launch to launch
+    uint32_t k, round, top, phase, level_start, list, n;
+    uint32_t alive;
+};
+
+struct TrussLoop {
+    const uint32_t* offsets;  // live CSR
+    const uint32_t* targets;
+    const uint32_t* eid;      // u < v entry (in the graph's CSR) of each live entry
+    const uint32_t* g_targets;
+    const uint32_t* src;
+    uint32_t* state;
+    uint32_t* support;
+    uint32_t* truss;
+    const uint32_t* active;
+    uint32_t listed;
+    uint32_t* list0;
+    uint32_t* list1;
+    TrussState* st;
+};
+
+constexpr int kTrussThreads = 1024;
+constexpr uint32_t kStage = 512;  // entries of the searched list a warp stages in shared memory
+constexpr int kTrussUnroll = 2;   // walked entries per lane in flight
+
+// One removed edge (or the part-th of 2^log_parts slices of its walk): the
+// shorter live list is walked, the longer one searched, in shared memory where
+// it fits kStage entries. A triangle with several edges removed in this round is
+// handled once, by the one with the smallest id; the edges of it that survive
+// the round lose one support, and one that falls below the threshold is listed
+// for the next round.
+__device__ __forceinline__ void truss_peel(const TrussLoop& a, uint32_t e, uint32_t part, uint32_t log_parts,
+                                           uint32_t round, uint32_t k, uint32_t* s_y, uint32_t* next,
+                                           uint32_t* next_count) {
+    const unsigned lane = lane_id();
+    const uint32_t u = __ldg(a.src + e), v = __ldg(a.g_targets + e);
+    uint32_t xs = __ldg(a.offsets + u), xn = __ldg(a.offsets + u + 1) - xs;
+    uint32_t ys = __ldg(a.offsets + v), yn = __ldg(a.offsets + v + 1) - ys;
+    if (xn > yn) {
+        uint32_t t = xs; xs = ys; ys = t;
+        t = xn; xn = yn; yn = t;
+    }
+    const bool staged = yn <= kStage;
+    if (staged) {
+        __syncwarp();
+#pragma unroll 4
+        for (uint32_t i = lane; i < yn; i += 32) s_y[i] = __ldg(a.targets + ys + i);
+        __syncwarp();
+    }
+    const uint32_t steps = yn ? 32 - __clz(yn) : 0;
+    const uint32_t stride = 32u << log_parts;
+    for (uint32_t i0 = part * 32 + lane; i0 < xn; i0 += kTrussUnroll * stride) {
+        uint32_t w[kTrussUnroll], q[kTrussUnroll];
+        bool hit[kTrussUnroll];
+#pragma unroll
+        for (int c = 0; c < kTrussUnroll; ++c) {
+            hit[c] = xn - i0 > c * stride;
+            w[c] = hit[c] ? __ldg(a.targets + xs + i0 + c * stride) : 0u;
+            q[c] = 0;
+        }
+        // q = entries of the list below w: the list's first entry >= w.
+        for (uint32_t b = steps; b-- > 0;) {
+#pragma unroll
+            for (int c = 0; c < kTrussUnroll; ++c) {
+                const uint32_t m = q[c] + (1u << b);
+                if (hit[c] && m <= yn && (staged ? s_y[m - 1] : __ldg(a.targets + ys + m - 1)) < w[c]) q[c] = m;
             }
         }
-        kt_append(take, j, removed, removed_count);
+#pragma unroll
+        for (int c = 0; c < kTrussUnroll; ++c)
+            hit[c] = hit[c] && q[c] < yn && (staged ? s_y[q[c]] : __ldg(a.targets + ys + q[c])) == w[c];
+        uint32_t e1[kTrussUnroll], e2[kTrussUnroll], s1[kTrussUnroll], s2[kTrussUnroll];
+#pragma unroll
+        for (int c = 0; c < kTrussUnroll; ++c) {
+            e1[c] = ld_nc_if(hit[c], a.eid + xs + i0 + c * stride, 0u);
+            e2[c] = ld_nc_if(hit[c], a.eid + ys + q[c], 0u);
+        }
+#pragma unroll
+        for (int c = 0; c < kTrussUnroll; ++c) {
+            s1[c] = ld_if(hit[c], a.state + e1[c], 1u);
+            s2[c] = ld_if(hit[c], a.state + e2[c], 1u);
+        }
+#pragma unroll
+        for (int c = 0; c < kTrussUnroll; ++c) {
+            if (!hit[c]) continue;
+            const bool live1 = s1[c] == 0 || s1[c] == round + 1, live2 = s2[c] == 0 || s2[c] == round + 1;
+            if ((!live1 && s1[c] != round) || (!live2 && s2[c] != round)) continue;   // destroyed earlier
+            if ((!live1 && e1[c] < e) || (!live2 && e2[c] < e)) continue;             // another edge's triangle
+            if (live1 && atomicSub(a.support + e1[c], 1u) == k - 2) {
+                a.state[e1[c]] = round + 1;
+                a.truss[e1[c]] = k - 1;
+                next[atomicAdd(next_count, 1u)] = e1[c];
+            }
+            if (live2 && atomicSub(a.support + e2[c], 1u) == k - 2) {
+                a.state[e2[c]] = round + 1;
+                a.truss[e2[c]] = k - 1;
+                next[atomicAdd(next_count, 1u)] = e2[c];
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kTrussThreads, 1) kt_truss_loop_kernel(const TrussLoop a) {
+    extern __shared__ uint32_t s_stage[];
+    __shared__ uint32_t s_count, s_least;
+    const unsigned lane = lane_id();
+    uint32_t* s_y = s_stage + (threadIdx.x >> 5) * kStage;
+    const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    const uint32_t nwarps = static_cast<uint32_t>(nthreads >> 5);
+    const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // neighbours on different SMs
+    uint32_t k = a.st->k, round = a.st->round, top = a.st->top, phase = a.st->phase, alive = a.st->alive;
+    uint32_t list = a.st->list, n = a.st->n;  // the entries this round removes: lists[list][0 .. n)
+    bool level_start = a.st->level_start != 0;
+    unsigned barriers = 0;
+    // Ends a phase: its counts to every block, the slot after next cleared.
+    auto end_phase = [&]() -> bool {
+        const uint32_t slot = phase % 3;
+        const bool ok = grid_barrier(&a.st->bar, gridDim.x, barriers, [&] {
+            s_count = __ldcg(a.st->count + slot);
+            s_least = __ldcg(a.st->least + slot);
+        });
+        ++phase;
+        // Slot (phase + 1) % 3 was read two barriers ago.
+        if (tid == 0) {
+            a.st->count[(phase + 1) % 3] = 0;
+            a.st->least[(phase + 1) % 3] = 0xFFFFFFFFu;
+        }
+        return ok;
+    };
+    // Half of the active list gone: the host compacts it and the live lists.
+    while (alive > 0 && 2ull * alive >= a.listed) {
+        ++round;
+        if (level_start) {
+            uint32_t least = 0xFFFFFFFFu;
+            for (uint64_t b = tid & ~31ull; b < a.listed; b += nthreads) {
+                const uint64_t i = b + lane;
+                bool take = false;
+                uint32_t j = 0;
+                if (i < a.listed) {
+                    j = __ldg(a.active + i);
+                    if (a.state[j] == 0) {
+                        const uint32_t s = a.support[j];
+                        take = s < k - 2;
+                        if (take) {
+                            a.state[j] = round;
+                            a.truss[j] = k - 1;
+                        } else {
+                            least = min(least, s);
+                        }
+                    }
+                }
+                kt_append(take, j, list ? a.list1 : a.list0, a.st->count + phase % 3);
+            }
+            least = __reduce_min_sync(kFullMask, least);
+            if (lane == 0 && least != 0xFFFFFFFFu) atomicMin(a.st->least + phase % 3, least);
+            if (!end_phase()) return;
+            n = s_count;
+            if (n == 0) {
+                // Every alive edge is in the k-truss, and in those up to k =
+                // least + 2: a round each that removes nothing.
+                top = s_least + 2;
+                round += top - k;
+                k = top + 1;
+                continue;
+            }
+        } else if (n == 0) {
+            top = k;
+            k += 1;
+            level_start = true;
+            continue;
+        }
+        alive -= n;
+        // With fewer edges than warps, up to 16 warps share one.
+        const uint32_t log_parts = n >= nwarps ? 0u : min(4u, 31 - __clz(nwarps / n));
+        for (uint64_t w = warp; w < static_cast<uint64_t>(n) << log_parts; w += nwarps)
+            truss_peel(a, __ldcg((list ? a.list1 : a.list0) + (w >> log_parts)),
+                       static_cast<uint32_t>(w) & ((1u << log_parts) - 1), log_parts, round, k, s_y,
+                       list ? a.list0 : a.list1, a.st->count + phase % 3);
+        if (!end_phase()) return;
+        n = s_count;
+        list ^= 1u;
+        level_start = false;
+    }
+    if (tid == 0) {
+        a.st->k = k;
+        a.st->round = round;
+        a.st->top = top;
+        a.st->phase = phase;
+        a.st->level_start = level_start ? 1u : 0u;
+        a.st->list = list;
+        a.st->n = n;
+        a.st->alive = alive;
     }
 }
 
@@ -724,16 +895,23 @@ Error truss_decomposition(GraphImpl& g, uint32_t* host_truss, uint32_t* max_trus
     GCU_TRY(ensure_kt_cache(g, &c));
     const uint32_t* src = c->src.ptr;
     const uint32_t* rev = c->rev.ptr;
-    DeviceBuffer<uint32_t> support, state, removed, truss, scratch, active[2], lists[2];
+    DeviceBuffer<uint32_t> support, state, truss, count, active[2], lists[2];
+    DeviceBuffer<TrussState> loop_state;
+    // Undirected edges: in a symmetric CSR every edge but a self-loop has two
+    // entries. The active list holds the alive ones' u < v entries and, with the
+    // live lists, is compacted whenever half of it has been peeled, so late
+    // rounds only touch the remaining core.
+    const uint32_t edges = (E - c->loops) / 2;
+    const uint64_t list_cap = std::max<uint32_t>(edges, 1);
     GCU_TRY(support.allocate(dev, E));
     GCU_TRY(state.allocate(dev, E));
-    GCU_TRY(removed.allocate(dev, E));
     GCU_TRY(truss.allocate(dev, E));
-    GCU_TRY(lists[0].allocate(dev, E));
-    GCU_TRY(lists[1].allocate(dev, E));
-    DeviceBuffer<uint32_t> chunks;  // peel chunk counts, then their scan
-    GCU_TRY(chunks.allocate(dev, static_cast<uint64_t>(E) + 1));
-    GCU_TRY(scratch.allocate(dev, 4));  // [0] removed by a scan, [1] active count, [2 + b] entries of lists[b]
+    GCU_TRY(lists[0].allocate(dev, list_cap));
+    GCU_TRY(lists[1].allocate(dev, list_cap));
+    GCU_TRY(active[0].allocate(dev, list_cap));
+    GCU_TRY(active[1].allocate(dev, list_cap));
+    GCU_TRY(count.allocate(dev, 1));
+    GCU_TRY(loop_state.allocate(dev, 1));
     const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
     const unsigned edge_grid = static_cast<unsigned>(std::min<uint64_t>(ceil_div_u64(E, 256), cap));
     GCU_CUDA(cudaMemcpyAsync(support.ptr, c->support.ptr, sizeof(uint32_t) * static_cast<size_t>(E),
@@ -741,85 +919,57 @@ Error truss_decomposition(GraphImpl& g, uint32_t* host_truss, uint32_t* max_trus
              "copy");
     GCU_CUDA(cudaMemsetAsync(state.ptr, 0, sizeof(uint32_t) * static_cast<size_t>(E), dev.stream), "memset");
     GCU_CUDA(cudaMemsetAsync(truss.ptr, 0, sizeof(uint32_t) * static_cast<size_t>(E), dev.stream), "memset");
-    // Undirected edges alive: in a symmetric CSR every edge but a self-loop
-    // has two entries, so there are (E - self-loop entries) / 2 of them; the
-    // active list holds their u < v entries and is compacted whenever half
-    // of it has been peeled, so late rounds only touch the remaining core.
-    uint64_t alive = (static_cast<uint64_t>(E) - c->loops) / 2;
-    const uint64_t list_cap = std::max<uint64_t>(alive, 1);
-    GCU_TRY(active[0].allocate(dev, list_cap));
-    GCU_TRY(active[1].allocate(dev, list_cap));
-    GCU_CUDA(cudaMemsetAsync(scratch.ptr + 1, 0, sizeof(uint32_t), dev.stream), "memset");
+    GCU_CUDA(cudaMemsetAsync(count.ptr, 0, sizeof(uint32_t), dev.stream), "memset");
     GCU_LAUNCH(dev, "kt_active", kt_active_kernel, edge_grid, 256, 0, g.targets.ptr, src, state.ptr,
-               static_cast<const uint32_t*>(nullptr), E, active[0].ptr, scratch.ptr + 1);
-    int cur = 0;              // active list in use
-    int out = 0;              // the peel lists the next round's removals in lists[out]
-    LiveCsr live{g.offsets.ptr, g.targets.ptr, nullptr};  // the peel's lists
-    uint32_t live_entries = E;
-    LiveBuffers live_bufs[2];
-    int live_cur = 0;
-    uint64_t listed = alive;  // entries in active[cur]
-    uint32_t round = 0, k = 3, top = alive > 0 ? 2 : 0;
-    // The first round of every level scans the active list for the edges
-    // below the new threshold; every later round of the level removes
-    // exactly the edges that the previous peel brought below it.
-    bool level_start = true;
-    uint32_t n = 0;  // entries removed in this round
-    while (alive > 0) {
-        round += 1;
-        const unsigned grid =
-            static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(ceil_div_u64(listed, 256), cap)));
-        const uint32_t* list = removed.ptr;
-        const uint32_t* count = scratch.ptr;
-        if (level_start) {
-            GCU_CUDA(cudaMemsetAsync(scratch.ptr, 0, sizeof(uint32_t), dev.stream), "memset");
-            GCU_LAUNCH(dev, "kt_active_filter", kt_active_filter_kernel, grid, 256, 0, active[cur].ptr,
-                       static_cast<uint32_t>(listed), support.ptr, state.ptr, k - 2, round, removed.ptr,
-                       scratch.ptr, truss.ptr, k - 1);
-            GCU_CUDA(cudaMemcpyAsync(&n, scratch.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
-            GCU_TRY(dev.sync());
-        } else {
-            list = lists[out ^ 1].ptr;
-            count = scratch.ptr + 2 + (out ^ 1);
-            if (n > 0) {
-                const unsigned mark_grid = static_cast<unsigned>(std::min<uint64_t>(ceil_div_u64(n, 256), cap));
-                GCU_LAUNCH(dev, "kt_mark", kt_mark_kernel, mark_grid, 256, 0, list, count, state.ptr, round,
-                           truss.ptr, k - 1);
-            }
-        }
-        if (n == 0) {
-            // Every alive edge has at least k - 2 alive triangles: it is in the k-truss.
-            top = k;
-            k += 1;
-            level_start = true;
-            continue;
-        }
-        alive -= n;
-        GCU_CUDA(cudaMemsetAsync(scratch.ptr + 2 + out, 0, sizeof(uint32_t), dev.stream), "memset");
-        GCU_TRY(launch_peel(dev, g, live, src, rev, state.ptr, support.ptr, list, count, n, chunks.ptr, round, k - 2,
-                            lists[out].ptr, scratch.ptr + 2 + out));
-        GCU_CUDA(cudaMemcpyAsync(&n, scratch.ptr + 2 + out, sizeof(uint32_t), cudaMemcpyDeviceToHost, dev.stream),
-                 "copy");
+               static_cast<const uint32_t*>(nullptr), E, active[0].ptr, count.ptr);
+    LiveBuffers live[2];
+    GCU_TRY(compact_live(dev, g.num_nodes, LiveCsr{g.offsets.ptr, g.targets.ptr, nullptr}, E, rev, state.ptr, &live[0]));
+
+    constexpr size_t kSmem = sizeof(uint32_t) * kStage * (kTrussThreads / 32);
+    GCU_CUDA(cudaFuncSetAttribute(kt_truss_loop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(kSmem)),
+             "cudaFuncSetAttribute");
+    int per_sm = 0;
+    GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kt_truss_loop_kernel, kTrussThreads, kSmem),
+             "occupancy");
+    if (per_sm < 1) return kernel_error("truss decomposition: the loop kernel does not fit an SM");
+    TrussState st{};
+    st.k = 3;
+    st.top = edges > 0 ? 2 : 0;
+    st.level_start = 1;
+    st.alive = edges;
+    uint32_t listed = edges;
+    int cur = 0;
+    while (st.alive > 0) {
+        st.bar = GridBarrier{};
+        std::fill(st.count, st.count + 3, 0u);
+        std::fill(st.least, st.least + 3, 0xFFFFFFFFu);
+        st.phase = 0;
+        GCU_CUDA(cudaMemcpyAsync(loop_state.ptr, &st, sizeof(st), cudaMemcpyHostToDevice, dev.stream), "copy");
+        const TrussLoop a{live[cur].offsets.ptr, live[cur].targets.ptr, live[cur].eid.ptr, g.targets.ptr, src, state.ptr,
+                          support.ptr, truss.ptr, active[cur].ptr, listed, lists[0].ptr, lists[1].ptr, loop_state.ptr};
+        // One block per SM; fewer for a core too small to use them.
+        const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(
+            1, std::min<uint64_t>(dev.sm_count, ceil_div_u64(listed, kTrussThreads / 32))));
+        GCU_LAUNCH_COOP(dev, "kt_truss_loop", kt_truss_loop_kernel, grid, kTrussThreads, kSmem, a);
+        GCU_CUDA(cudaMemcpyAsync(&st, loop_state.ptr, sizeof(st), cudaMemcpyDeviceToHost, dev.stream), "copy");
         GCU_TRY(dev.sync());
-        out ^= 1;
-        level_start = false;
-        if (alive > 0 && 2 * alive < listed) {
-            GCU_CUDA(cudaMemsetAsync(scratch.ptr + 1, 0, sizeof(uint32_t), dev.stream), "memset");
-            GCU_LAUNCH(dev, "kt_active", kt_active_kernel, grid, 256, 0, g.targets.ptr, src, state.ptr,
-                       active[cur].ptr, static_cast<uint32_t>(listed), active[cur ^ 1].ptr, scratch.ptr + 1);
-            cur ^= 1;
-            listed = alive;
-            // The peel's lists too: the alive entries only (the removals
-            // listed for the next round are still alive and stay).
-            GCU_TRY(compact_live(dev, g.num_nodes, live, live_entries, rev, state.ptr, &live_bufs[live_cur ^ 1]));
-            live_cur ^= 1;
-            live = LiveCsr{live_bufs[live_cur].offsets.ptr, live_bufs[live_cur].targets.ptr,
-                           live_bufs[live_cur].eid.ptr};
-            live_entries = live_bufs[live_cur].entries;
-        }
+        if (st.bar.failed) return kernel_error("truss decomposition: a block did not reach the grid barrier");
+        if (st.alive == 0) break;
+        // The removals listed for the next round count as alive (state round +
+        // 1), and their lists stay.
+        GCU_CUDA(cudaMemsetAsync(count.ptr, 0, sizeof(uint32_t), dev.stream), "memset");
+        const unsigned grid_l = static_cast<unsigned>(std::min<uint64_t>(ceil_div_u64(listed, 256), cap));
+        GCU_LAUNCH(dev, "kt_active", kt_active_kernel, grid_l, 256, 0, g.targets.ptr, src, state.ptr, active[cur].ptr,
+                   listed, active[cur ^ 1].ptr, count.ptr);
+        GCU_CUDA(cudaMemcpyAsync(&listed, count.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
+        GCU_TRY(compact_live(dev, g.num_nodes,
+                             LiveCsr{live[cur].offsets.ptr, live[cur].targets.ptr, live[cur].eid.ptr},
+                             live[cur].entries, rev, state.ptr, &live[cur ^ 1], st.n > 0 ? st.round + 1 : 0));
+        cur ^= 1;
     }
-    *max_truss = top;
-    *rounds = round;
+    *max_truss = st.top;
+    *rounds = st.round;
     if (host_truss) {
         GCU_LAUNCH(dev, "kt_truss_spread", kt_truss_spread_kernel, edge_grid, 256, 0, g.targets.ptr, src, rev,
                    truss.ptr, E, support.ptr);
