@@ -690,6 +690,15 @@ struct TrussLoop {
     TrussState* st;
 };
 
+// What bounds the loop: R-MAT scale 19 (14.3 M entries, trussness up to 187,
+// 1,697 rounds) takes 132 scans and about 1,300 peels. A round of a few edges is
+// one peel's chain of dependent loads and the barrier, 6 to 8 us; rounds of 1 K
+// to 12 K edges, most of the time, are bound by the searches, which take the
+// SM's issue slots and bank conflicts rather than bandwidth. Measured there:
+// 40.7 ms for the whole decomposition after the support, 109.5 ms when each
+// round was four launches and a count read by the host. 1,024 staged entries
+// take 40.1 ms, one or four walked entries in flight 40 to 41 ms, so the smaller
+// stage stays, which leaves the L1 the rest.
 constexpr int kTrussThreads = 1024;
 constexpr uint32_t kStage = 512;  // entries of the searched list a warp stages in shared memory
 constexpr int kTrussUnroll = 2;   // walked entries per lane in flight
