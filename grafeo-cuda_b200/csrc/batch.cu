@@ -938,9 +938,9 @@ Error batch_from_csr(DeviceImpl& dev, std::shared_ptr<DeviceImpl> owner, const u
     u.num_edges = static_cast<uint32_t>(n_targets);
     GCU_TRY(u.offsets.allocate(dev, n_offsets));
     GCU_TRY(u.targets.allocate(dev, n_targets));
-    GCU_CUDA(cudaMemcpyAsync(u.offsets.ptr, offsets, 4 * n_offsets, cudaMemcpyHostToDevice, dev.stream), "copy");
+    GCU_TRY(copy_to_device(dev, u.offsets.ptr, offsets, 4 * n_offsets, dev.stream));
     if (n_targets)
-        GCU_CUDA(cudaMemcpyAsync(u.targets.ptr, targets, 4 * n_targets, cudaMemcpyHostToDevice, dev.stream), "copy");
+        GCU_TRY(copy_to_device(dev, u.targets.ptr, targets, 4 * n_targets, dev.stream));
     uint32_t bad = UINT32_MAX;
     GCU_TRY(validate_csr_device(dev, u.offsets.ptr, u.targets.ptr, u.num_nodes, u.num_edges, &bad));
     if (bad != UINT32_MAX) {

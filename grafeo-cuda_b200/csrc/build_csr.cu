@@ -420,9 +420,7 @@ Error build_graph_from_pairs(DeviceImpl& dev, const uint32_t* host_pairs, uint64
     GCU_TRY(check_capacity(capacity));
     DeviceBuffer<uint32_t> d_pairs;
     GCU_TRY(d_pairs.allocate(dev, std::max<uint64_t>(2 * n_pairs, 1)));
-    if (n_pairs)
-        GCU_CUDA(cudaMemcpyAsync(d_pairs.ptr, host_pairs, 8 * n_pairs, cudaMemcpyHostToDevice, dev.stream),
-                 "copy edge pairs to device");
+    GCU_TRY(copy_to_device(dev, d_pairs.ptr, host_pairs, 8 * n_pairs, dev.stream));
     KeyScratch ks;
     GCU_TRY(ks.allocate(dev, capacity));
     GCU_LAUNCH(dev, "build_pairs_to_keys", pairs_to_keys_kernel, grid_for(dev, n_pairs), kBuildThreads, 0, d_pairs.ptr,

@@ -16,6 +16,7 @@
 #include <chrono>
 #include <cstdint>
 #include <cstdio>
+#include <cstdlib>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -80,6 +81,10 @@ struct KernelStat {
     double total_ms = 0.0;
 };
 
+// Page-locked slots of a device's staged host copies (64 MB in all).
+constexpr unsigned kStageSlots = 64;
+constexpr size_t kStageSlot = size_t(1) << 20;
+
 struct DeviceImpl {
     int ordinal = 0;
     std::string name;
@@ -111,12 +116,13 @@ struct DeviceImpl {
     // NULL: the fixed rules (alpha/beta BFS direction, degree-range buckets).
     uint16_t* schedule = nullptr;
 
-    // Two page-locked staging buffers for large device-to-host copies into
-    // pageable memory (copy_to_host), allocated with the device (NULL if
-    // page-locked memory ran out: those copies then go straight to the caller).
+    // Page-locked slots (kStageSlots of kStageSlot bytes) for large copies from
+    // and to pageable memory, allocated with the device (NULL if page-locked
+    // memory ran out: those copies then go straight through the driver). A
+    // slot's event is recorded after the last copy that used it.
     std::mutex stage_mu;
-    void* stage[2] = {nullptr, nullptr};
-    cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+    char* stage = nullptr;
+    cudaEvent_t stage_ev[kStageSlots] = {};
 
     ~DeviceImpl();
 
@@ -131,13 +137,41 @@ struct DeviceImpl {
 };
 
 // Copies `bytes` of device memory to pageable host memory and waits for it.
-// Up to kStageMin bytes: one copy. Beyond: chunks of kStageChunk bytes go
-// through two page-locked staging buffers, the DMA of the next chunk
-// overlapping the host copy of the current one, which is split over up to
-// kStageThreads threads. Measured on the B200 box: 67 MB in 5.1 ms against
-// 13.5 ms for the driver's pageable copy (2.7x), 396 MB of batch ranks in
-// about a third of the time; one host thread instead of four gained 7 %.
+// The driver's pageable copy is bound by one host thread that also takes the
+// page faults of a result array the caller has just allocated, so copies of
+// more than kStageMin bytes go through the page-locked slots, each worker
+// keeping DMAs into its own slots in flight while it empties others. Measured
+// (16-core host, fresh array of 4 KB pages / warm array): 128 MB in 12.3 / 4.3
+// ms, 32 MB in 3.7 / 1.0 ms; with two 32 MB buffers emptied by four threads
+// 19 / 5.5 and 5.2 / 1.5 ms; the driver's copy into the warm one 7.1 and 1.7 ms.
 Error copy_to_host(DeviceImpl& dev, void* dst, const void* src, size_t bytes);
+
+// Copies `bytes` of host memory to the device in `stream` order; the source may
+// be changed on return. Pageable sources of kStageUploadMin bytes or more are
+// copied into the page-locked slots by several workers, the DMAs following:
+// 128 MB in 4.2 ms, 32 MB in 1.2 ms, against 12.2 and 2.7 ms for the driver's
+// copy (2.4 and 0.6 ms from page-locked memory). Below, the workers cost what
+// they gain (6 MB: 0.33 ms either way). Up to kStageUploadFew bytes four of
+// them are faster than eight, which then hold each other up.
+Error copy_to_device(DeviceImpl& dev, void* dst, const void* src, size_t bytes, cudaStream_t stream);
+
+// Host memory for a result, left uninitialised (its first writers are the
+// workers of copy_to_host). Large ones ask for huge pages: 32 MB of 4 KB pages
+// cost 8,192 faults.
+class HostArray {
+public:
+    HostArray() = default;
+    HostArray(const HostArray&) = delete;
+    HostArray& operator=(const HostArray&) = delete;
+    ~HostArray() { std::free(data_); }
+    Error resize(size_t n);  // contents are lost
+    uint32_t* data() const { return data_; }
+    size_t size() const { return size_; }
+
+private:
+    uint32_t* data_ = nullptr;
+    size_t size_ = 0;
+};
 
 // Stream-ordered device allocation that reports OutOfMemory with the
 // reference's required/available fields (error.rs:18-26).
@@ -270,7 +304,7 @@ Error bfs(GraphImpl& g, uint32_t source, int32_t* host_distances, uint32_t* reac
           int32_t* max_depth);
 Error pagerank(GraphImpl& g, float damping, uint32_t max_iterations, float tolerance,
                float* host_ranks, uint32_t* iterations, bool* converged);
-Error k_truss(GraphImpl& g, uint32_t k, std::vector<uint32_t>* edges, uint32_t* iterations);
+Error k_truss(GraphImpl& g, uint32_t k, HostArray* edges, uint32_t* iterations);
 // Trussness of every CSR entry's edge (host_truss may be NULL), symmetric CSR.
 Error truss_decomposition(GraphImpl& g, uint32_t* host_truss, uint32_t* max_truss, uint32_t* rounds);
 

@@ -417,7 +417,7 @@ __global__ void kt_mark_kernel(const uint32_t* __restrict__ list, const uint32_t
 // Compacts the alive u < v entries, in CSR order, into host pairs.
 template <class Alive>
 static Error emit_edges(DeviceImpl& dev, GraphImpl& g, const uint32_t* src, Alive alive, uint32_t* flag,
-                        uint32_t* pos, std::vector<uint32_t>* edges) {
+                        uint32_t* pos, HostArray* edges) {
     const uint32_t E = g.num_edges;
     const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
     const unsigned edge_grid = static_cast<unsigned>(std::min<uint64_t>(ceil_div_u64(E, 256), cap));
@@ -431,7 +431,7 @@ static Error emit_edges(DeviceImpl& dev, GraphImpl& g, const uint32_t* src, Aliv
         GCU_TRY(out.allocate(dev, count));
         GCU_LAUNCH(dev, "kt_emit", kt_emit_kernel<Alive>, edge_grid, 256, 0, g.targets.ptr, src, alive, E, pos,
                    out.ptr);
-        edges->resize(2 * static_cast<size_t>(count));
+        GCU_TRY(edges->resize(2 * static_cast<size_t>(count)));
         GCU_TRY(copy_to_host(dev, edges->data(), out.ptr, sizeof(uint2) * count));
     }
     return ok();
@@ -439,7 +439,7 @@ static Error emit_edges(DeviceImpl& dev, GraphImpl& g, const uint32_t* src, Aliv
 
 // Any CSR: the reference's rounds, recomputing every support each round.
 static Error k_truss_general(GraphImpl& g, uint32_t k, const uint32_t* src, const uint32_t* rev,
-                             std::vector<uint32_t>* edges, uint32_t* iterations) {
+                             HostArray* edges, uint32_t* iterations) {
     DeviceImpl& dev = *g.dev;
     const uint32_t E = g.num_edges;
     const uint32_t threshold = k - 2;
@@ -531,7 +531,7 @@ static Error ensure_kt_cache(GraphImpl& g, KtCache** out) {
 // incremental peeling. Every round removes exactly the entries the
 // reference's round removes, so the edge list and the round count are the
 // same.
-static Error k_truss_symmetric(GraphImpl& g, uint32_t k, std::vector<uint32_t>* edges, uint32_t* iterations) {
+static Error k_truss_symmetric(GraphImpl& g, uint32_t k, HostArray* edges, uint32_t* iterations) {
     DeviceImpl& dev = *g.dev;
     const uint32_t E = g.num_edges;
     const uint32_t threshold = k - 2;
@@ -605,8 +605,8 @@ static Error k_truss_symmetric(GraphImpl& g, uint32_t k, std::vector<uint32_t>* 
     return emit_edges(dev, g, src, RoundState{state.ptr}, removed.ptr, support.ptr, edges);
 }
 
-Error k_truss(GraphImpl& g, uint32_t k, std::vector<uint32_t>* edges, uint32_t* iterations) {
-    edges->clear();
+Error k_truss(GraphImpl& g, uint32_t k, HostArray* edges, uint32_t* iterations) {
+    GCU_TRY(edges->resize(0));
     *iterations = 0;
     const uint32_t E = g.num_edges, V = g.num_nodes;
     // k_truss.rs:53-60: no edges, no truss.

@@ -6,11 +6,13 @@
 // runs on the device's own stream and synchronizes before returning, like the
 // reference's default-stream calls (device.rs:38).
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <cstring>
 #include <functional>
 #include <sstream>
+#include <system_error>
 #include <thread>
 
 #include "gcu_internal.h"
@@ -70,69 +72,155 @@ DeviceImpl::~DeviceImpl() {
         cudaStreamDestroy(copy_stream);
     }
     if (copy_event) cudaEventDestroy(copy_event);
-    for (int i = 0; i < 2; ++i) {
-        if (stage[i]) cudaFreeHost(stage[i]);
-        if (stage_ev[i]) cudaEventDestroy(stage_ev[i]);
-    }
+    if (stage) cudaFreeHost(stage);
+    for (auto e : stage_ev)
+        if (e) cudaEventDestroy(e);
     if (stream) cudaStreamDestroy(stream);
 }
 
 namespace {
 constexpr size_t kStageMin = size_t(4) << 20;
-constexpr size_t kStageChunk = size_t(32) << 20;
-constexpr unsigned kStageThreads = 4;
+constexpr size_t kStageUploadMin = size_t(16) << 20;
+constexpr size_t kStageUploadFew = size_t(64) << 20;
+constexpr unsigned kStageWorkers = 8;
 
-// memcpy split into contiguous parts over up to kStageThreads threads.
-void parallel_copy(void* dst, const void* src, size_t bytes) {
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const unsigned parts = std::min<unsigned>(kStageThreads, hw);
-    const size_t part = (bytes + parts - 1) / parts;
-    std::vector<std::thread> workers;
-    for (unsigned i = 1; i < parts; ++i) {
-        const size_t off = std::min(bytes, i * part);
-        const size_t len = std::min(part, bytes - off);
-        if (len == 0) break;
-        workers.emplace_back([=] { std::memcpy(static_cast<char*>(dst) + off, static_cast<const char*>(src) + off, len); });
+// Runs work(worker, workers) on the calling thread and up to workers - 1 others;
+// fewer where a thread cannot be started (each takes chunks until none is left).
+template <class Work>
+void run_workers(unsigned workers, const Work& work) {
+    std::thread pool[kStageWorkers];
+    for (unsigned t = 1; t < workers; ++t) {
+        try {
+            pool[t] = std::thread([&work, t] { work(t); });
+        } catch (const std::system_error&) {
+            break;
+        }
     }
-    std::memcpy(dst, src, std::min(part, bytes));
-    for (auto& w : workers) w.join();
+    work(0);
+    for (auto& t : pool)
+        if (t.joinable()) t.join();
 }
+
+unsigned stage_workers(unsigned wanted) {
+    return std::min({wanted, kStageWorkers, std::max(1u, std::thread::hardware_concurrency())});
+}
+
+// Shared state of one staged copy: the chunk handout and the first error.
+struct StagedCopy {
+    std::atomic<size_t> next{0};
+    std::atomic<int> error{cudaSuccess};
+    bool check(cudaError_t e) {
+        int expected = cudaSuccess;
+        if (e != cudaSuccess) error.compare_exchange_strong(expected, e);
+        return error.load(std::memory_order_relaxed) == cudaSuccess;
+    }
+};
 }  // namespace
 
 Error copy_to_host(DeviceImpl& dev, void* dst, const void* src, size_t bytes) {
     if (bytes == 0) return ok();
-    if (bytes <= kStageMin) {
-        GCU_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, dev.stream), "copy to host");
-        return dev.sync();
-    }
-    if (!dev.stage[0] || !dev.stage[1]) {
+    if (bytes <= kStageMin || !dev.stage) {
         GCU_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, dev.stream), "copy to host");
         return dev.sync();
     }
     std::lock_guard<std::mutex> lock(dev.stage_mu);
-    const size_t chunks = (bytes + kStageChunk - 1) / kStageChunk;
-    auto issue = [&](size_t k) -> Error {
-        const size_t off = k * kStageChunk;
-        const size_t len = std::min(kStageChunk, bytes - off);
-        GCU_CUDA(cudaMemcpyAsync(dev.stage[k & 1], static_cast<const char*>(src) + off, len, cudaMemcpyDeviceToHost,
-                                 dev.stream),
-                 "copy to host");
-        GCU_CUDA(cudaEventRecord(dev.stage_ev[k & 1], dev.stream), "cudaEventRecord");
-        return ok();
-    };
-    Error err = [&]() -> Error {
-        GCU_TRY(issue(0));
-        for (size_t k = 0; k < chunks; ++k) {
-            if (k + 1 < chunks) GCU_TRY(issue(k + 1));  // buffer (k + 1) & 1 was emptied at step k - 1
-            GCU_CUDA(cudaEventSynchronize(dev.stage_ev[k & 1]), "cudaEventSynchronize");
-            const size_t off = k * kStageChunk;
-            parallel_copy(static_cast<char*>(dst) + off, dev.stage[k & 1], std::min(kStageChunk, bytes - off));
+    const size_t chunks = (bytes + kStageSlot - 1) / kStageSlot;
+    const unsigned workers = stage_workers(kStageWorkers);
+    const unsigned own = kStageSlots / workers;
+    StagedCopy c;
+    run_workers(workers, [&](unsigned t) {
+        if (!c.check(cudaSetDevice(dev.ordinal))) return;
+        size_t held[kStageSlots];  // chunk of each slot of the ring
+        size_t issued = 0, done = 0;
+        bool more = true;
+        while (more || done < issued) {
+            // A share of the chunks in flight per worker, so that all get some of a short copy.
+            while (more && issued - done < own && (issued - done) * workers < chunks) {
+                const size_t k = c.next.fetch_add(1, std::memory_order_relaxed);
+                if (k >= chunks) {
+                    more = false;
+                    break;
+                }
+                const unsigned s = t * own + static_cast<unsigned>(issued % own);
+                const size_t off = k * kStageSlot;
+                if (!c.check(cudaEventSynchronize(dev.stage_ev[s]))) return;
+                if (!c.check(cudaMemcpyAsync(dev.stage + s * kStageSlot, static_cast<const char*>(src) + off,
+                                             std::min(kStageSlot, bytes - off), cudaMemcpyDeviceToHost, dev.stream)))
+                    return;
+                if (!c.check(cudaEventRecord(dev.stage_ev[s], dev.stream))) return;
+                held[issued++ % own] = k;
+            }
+            if (done == issued) break;
+            const unsigned s = t * own + static_cast<unsigned>(done % own);
+            const size_t off = held[done % own] * kStageSlot;
+            if (!c.check(cudaEventSynchronize(dev.stage_ev[s]))) return;
+            std::memcpy(static_cast<char*>(dst) + off, dev.stage + s * kStageSlot, std::min(kStageSlot, bytes - off));
+            ++done;
         }
-        return ok();
-    }();
-    if (!err.ok()) cudaStreamSynchronize(dev.stream);  // no copy into the staging buffers outlives the lock
-    GCU_TRY(err);
+    });
+    const auto e = static_cast<cudaError_t>(c.error.load());
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(dev.stream);  // no copy into the slots outlives the lock
+        return driver_error(e, "copy to host");
+    }
     return dev.sync();
+}
+
+Error copy_to_device(DeviceImpl& dev, void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+    if (bytes == 0) return ok();
+    cudaPointerAttributes attr{};
+    const bool pageable = bytes >= kStageUploadMin && dev.stage &&
+                          cudaPointerGetAttributes(&attr, src) == cudaSuccess &&
+                          attr.type == cudaMemoryTypeUnregistered;
+    if (!pageable) {
+        GCU_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream), "copy to device");
+        return ok();
+    }
+    std::lock_guard<std::mutex> lock(dev.stage_mu);
+    const size_t chunks = (bytes + kStageSlot - 1) / kStageSlot;
+    const unsigned workers = stage_workers(bytes < kStageUploadFew ? kStageWorkers / 2 : kStageWorkers);
+    const unsigned own = kStageSlots / workers;
+    StagedCopy c;
+    run_workers(workers, [&](unsigned t) {
+        if (!c.check(cudaSetDevice(dev.ordinal))) return;
+        for (unsigned i = 0;; ++i) {
+            const size_t k = c.next.fetch_add(1, std::memory_order_relaxed);
+            if (k >= chunks) return;
+            const unsigned s = t * own + i % own;
+            const size_t off = k * kStageSlot, len = std::min(kStageSlot, bytes - off);
+            if (!c.check(cudaEventSynchronize(dev.stage_ev[s]))) return;
+            std::memcpy(dev.stage + s * kStageSlot, static_cast<const char*>(src) + off, len);
+            if (!c.check(cudaMemcpyAsync(static_cast<char*>(dst) + off, dev.stage + s * kStageSlot, len,
+                                         cudaMemcpyHostToDevice, stream)))
+                return;
+            if (!c.check(cudaEventRecord(dev.stage_ev[s], stream))) return;
+        }
+    });
+    const auto e = static_cast<cudaError_t>(c.error.load());
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(stream);
+        return driver_error(e, "copy to device");
+    }
+    return ok();
+}
+
+Error HostArray::resize(size_t n) {
+    constexpr size_t kHuge = size_t(2) << 20;
+    std::free(data_);
+    data_ = nullptr;
+    size_ = 0;
+    if (n == 0) return ok();
+    const size_t bytes = n * sizeof(uint32_t);
+    if (bytes < 2 * kHuge) {
+        data_ = static_cast<uint32_t*>(std::malloc(bytes));
+    } else {
+        const size_t rounded = (bytes + kHuge - 1) / kHuge * kHuge;
+        data_ = static_cast<uint32_t*>(std::aligned_alloc(kHuge, rounded));
+        if (data_) madvise(data_, rounded, MADV_HUGEPAGE);  // a hint: small pages work as well
+    }
+    if (!data_) return kernel_error("out of host memory for " + std::to_string(bytes) + " bytes");
+    size_ = n;
+    return ok();
 }
 
 Error DeviceImpl::activate() const {
@@ -268,16 +356,14 @@ static Error create_device(int ordinal, std::shared_ptr<DeviceImpl>* out) {
         uint64_t threshold = UINT64_MAX;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
     }
-    // The staging pair of copy_to_host, page-locked once here (about 70 ms for
-    // 64 MB) rather than in the first call that copies a large result; without
-    // it (no page-locked memory left) large copies go straight to the caller.
-    for (int i = 0; i < 2; ++i) {
-        if (cudaMallocHost(&dev->stage[i], kStageChunk) != cudaSuccess) {
-            cudaGetLastError();
-            dev->stage[i] = nullptr;
-        }
-        GCU_CUDA(cudaEventCreateWithFlags(&dev->stage_ev[i], cudaEventDisableTiming), "cudaEventCreate");
+    // The slots of the staged copies, page-locked once here (about 70 ms for
+    // 64 MB) rather than in the first call that copies much; without them (no
+    // page-locked memory left) large copies go straight through the driver.
+    if (cudaMallocHost(reinterpret_cast<void**>(&dev->stage), kStageSlots * kStageSlot) != cudaSuccess) {
+        cudaGetLastError();
+        dev->stage = nullptr;
     }
+    for (auto& e : dev->stage_ev) GCU_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
     *out = dev;
     return ok();
 }
@@ -293,7 +379,7 @@ struct gcu_graph {
     std::unique_ptr<GraphImpl> impl;
 };
 struct gcu_edge_list {
-    std::vector<uint32_t> data;
+    gcu::HostArray data;
 };
 struct gcu_batch {
     BatchImpl* impl = nullptr;
@@ -460,8 +546,8 @@ GCU_API gcu_status gcu_graph_from_csr(gcu_device* dev, const uint32_t* offsets, 
     e = g->offsets.allocate(d, n_offsets);
     if (e.ok()) e = g->targets.allocate(d, n_targets);
     if (!e.ok()) return fail(e);
-    cudaError_t c = cudaMemcpyAsync(g->offsets.ptr, offsets, n_offsets * 4, cudaMemcpyHostToDevice, d.stream);
-    if (c != cudaSuccess) return fail(driver_error(c, "copy CSR to device"));
+    e = copy_to_device(d, g->offsets.ptr, offsets, n_offsets * 4, d.stream);
+    if (!e.ok()) return fail(e);
 
     // The targets are copied in chunks that the entry checks follow.
     uint32_t bad = UINT32_MAX;
@@ -987,7 +1073,7 @@ GCU_API size_t gcu_batch_tuning(const gcu_batch* b, char* buf, size_t buflen) {
 
 GCU_API size_t gcu_edge_list_len(const gcu_edge_list* list) { return list ? list->data.size() / 2 : 0; }
 GCU_API const uint32_t* gcu_edge_list_data(const gcu_edge_list* list) {
-    return list && !list->data.empty() ? list->data.data() : nullptr;
+    return list ? list->data.data() : nullptr;
 }
 GCU_API void gcu_edge_list_free(gcu_edge_list* list) { delete list; }
 

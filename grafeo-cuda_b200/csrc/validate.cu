@@ -107,9 +107,9 @@ static Error check_csr(DeviceImpl& dev, const uint32_t* d_offsets, uint32_t* d_t
         Error err = ok();
         for (uint64_t c0 = 0; c0 < num_edges && err.ok(); c0 += kUploadChunk) {
             const uint64_t c1 = std::min<uint64_t>(c0 + kUploadChunk, num_edges);
-            cudaError_t c = cudaMemcpyAsync(d_targets + c0, h_targets + c0, sizeof(uint32_t) * (c1 - c0),
-                                            cudaMemcpyHostToDevice, dev.copy_stream);
-            if (c == cudaSuccess) c = cudaEventRecord(dev.copy_event, dev.copy_stream);
+            err = copy_to_device(dev, d_targets + c0, h_targets + c0, sizeof(uint32_t) * (c1 - c0), dev.copy_stream);
+            if (!err.ok()) break;
+            cudaError_t c = cudaEventRecord(dev.copy_event, dev.copy_stream);
             if (c == cudaSuccess) c = cudaStreamWaitEvent(dev.stream, dev.copy_event, 0);
             if (c != cudaSuccess) {
                 err = driver_error(c, "copy CSR to device");

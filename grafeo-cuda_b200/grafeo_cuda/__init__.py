@@ -272,6 +272,21 @@ def generate_erdos_renyi(num_nodes: int, num_pairs: int, seed: int = 3) -> CsrAr
 # ---------------------------------------------------------------- device graph
 
 
+class _EdgeList:
+    """Owner of a library edge list; arrays over it keep it alive."""
+
+    def __init__(self, handle: C.c_void_p):
+        self._h = handle
+        self._free = lib.gcu_edge_list_free
+        m = int(lib.gcu_edge_list_len(handle))
+        data = C.cast(lib.gcu_edge_list_data(handle), C.c_void_p).value
+        self.__array_interface__ = {"shape": (m, 2), "typestr": np.dtype(np.uint32).str, "data": (data or 0, False),
+                                    "version": 3}
+
+    def __del__(self):
+        self._free(self._h)
+
+
 class GpuGraph:
     """A graph stored in GPU memory as CSR (gpu_graph.rs:15-26)."""
 
@@ -506,14 +521,9 @@ class GpuGraph:
         it = C.c_uint32()
         secs = C.c_double()
         check(lib.gcu_k_truss(self._h, k, C.byref(h), C.byref(it), C.byref(secs)))
-        try:
-            m = int(lib.gcu_edge_list_len(h))
-            if m:
-                edges = np.ctypeslib.as_array(lib.gcu_edge_list_data(h), shape=(2 * m,)).copy().reshape(m, 2)
-            else:
-                edges = np.zeros((0, 2), dtype=np.uint32)
-        finally:
-            lib.gcu_edge_list_free(h)
+        # The list as the library allocated it, not a copy.
+        kept = _EdgeList(h)
+        edges = np.asarray(kept) if kept.__array_interface__["shape"][0] else np.zeros((0, 2), dtype=np.uint32)
         return {"edges": edges, "k": k, "iterations": int(it.value), "time_seconds": float(secs.value)}
 
     def bfs_trace(self, source: int, explore_seed: int = 0, capacity: int = 65536) -> dict:
