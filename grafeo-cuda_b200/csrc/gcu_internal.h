@@ -278,27 +278,29 @@ Error degree_class_order(DeviceImpl& dev, const uint32_t* offsets, uint32_t V, D
 Error graph_symmetry(GraphImpl& g, bool* symmetric);
 
 // Degree-oriented (by_degree) or id-oriented DAG of the CSR: every undirected
-// edge once, lists still sorted. With `rev` (reverse-entry index) and dag_eid,
-// also the CSR index of each DAG edge's u < v entry. *m = DAG edges.
-Error build_dag(GraphImpl& g, bool by_degree, const uint32_t* rev, DeviceBuffer<uint32_t>* dag_offsets,
-                DeviceBuffer<uint32_t>* dag_targets, DeviceBuffer<uint32_t>* dag_eid, uint32_t* m);
+// edge once, lists still sorted. *m = DAG edges.
+Error build_dag(GraphImpl& g, bool by_degree, DeviceBuffer<uint32_t>* dag_offsets,
+                DeviceBuffer<uint32_t>* dag_targets, uint32_t* m);
 
-// N+(u) of every vertex of a symmetric CSR as (32-rank word, mask) pairs, and the
-// owners the count runs over (tri_words.cu).
+// N+(u), or (full) all neighbours, of every vertex of a symmetric CSR as (32-rank
+// word, mask) pairs, and the owners the count runs over (tri_words.cu).
 struct WordLists {
     DeviceBuffer<uint32_t> rank;         // degree-class order
-    DeviceBuffer<uint2> lists;           // per vertex: first word, words
+    DeviceBuffer<uint2> lists;           // per vertex: first word / 2, words
     DeviceBuffer<uint2> words;           // (word, mask)
     DeviceBuffer<uint32_t> warp_owners;
     DeviceBuffer<uint2> items;           // (owner, slice of its row)
     DeviceBuffer<uint32_t> counts;       // [2] warp owners, [3] items
     uint64_t max_items = 0;
 };
-Error build_word_lists(GraphImpl& g, WordLists* w);
+Error build_word_lists(GraphImpl& g, bool full, WordLists* w);
 // Adds the triangles to *total, or to per_vertex[owner] where that is given
 // (device memory). next: two words of scratch. Only enqueues (capturable).
 Error count_words(GraphImpl& g, const WordLists& w, uint32_t* next, unsigned long long* total,
                   unsigned long long* per_vertex);
+// support[j] = triangles of the edge whose u < v entry is j, for every edge in
+// one (symmetric CSR, rev = reverse-entry index); the others are not written.
+Error edge_support(GraphImpl& g, const uint32_t* rev, uint32_t* support);
 Error triangle_count(GraphImpl& g, bool oriented, uint64_t* total);
 Error bfs(GraphImpl& g, uint32_t source, int32_t* host_distances, uint32_t* reachable,
           int32_t* max_depth);

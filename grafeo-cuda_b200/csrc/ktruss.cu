@@ -11,9 +11,9 @@
 // sets round by round, hence the same edges and round count:
 //
 //  * Symmetric CSR (every graph exported from Grafeo): the support of every
-//    undirected edge is its triangle count, found once by enumerating the
-//    triangles of the degree-oriented DAG (wedge.cuh) with three atomic adds
-//    per triangle; round 1 adds one for a self-loop at either end. After a
+//    undirected edge is its triangle count, found once as the popcount of its
+//    ends' neighbour bits (edge_support, tri_words.cu); round 1 adds one for a
+//    self-loop at either end. After a
 //    round removes a set R of edges, each triangle with an edge in R that was
 //    alive at the start of the round is destroyed once (credited to its
 //    removed edge with the smallest id) and its surviving edges lose one
@@ -29,7 +29,6 @@
 
 #include "device_common.cuh"
 #include "gcu_internal.h"
-#include "wedge.cuh"
 
 namespace gcu {
 
@@ -143,23 +142,6 @@ __global__ void kt_emit_kernel(const uint32_t* __restrict__ targets, const uint3
 }
 
 // ---------------------------------------------------------------- symmetric CSR: incremental peeling
-
-namespace {
-
-// Adds each triangle found on the DAG to the support of its three edges.
-struct SupportSink {
-    static constexpr bool kNeedsPos = true;
-    const uint32_t* dag_eid;
-    uint32_t* support;
-    __device__ __forceinline__ void hit(uint32_t base, uint32_t pv, uint32_t pw, uint32_t evw) {
-        atomicAdd(support + dag_eid[base + pv], 1u);
-        atomicAdd(support + dag_eid[base + pw], 1u);
-        atomicAdd(support + dag_eid[evw], 1u);
-    }
-    __device__ __forceinline__ void finish() {}
-};
-
-}  // namespace
 
 // loop[u] = 1 for every vertex with a self-loop entry; counts them in *loops.
 __global__ void kt_loops_kernel(const uint32_t* __restrict__ targets, const uint32_t* __restrict__ src, uint32_t E,
@@ -470,19 +452,6 @@ static Error k_truss_general(GraphImpl& g, uint32_t k, const uint32_t* src, cons
     return emit_edges(dev, g, src, LiveFlag{live.ptr}, support.ptr, pos.ptr, edges);
 }
 
-// support[j] += triangles of the undirected edge whose u < v entry is j,
-// counted once on the degree DAG (symmetric CSR).
-static Error triangle_support(GraphImpl& g, const uint32_t* rev, uint32_t* support) {
-    DeviceBuffer<uint32_t> dag_offsets, dag_targets, dag_eid;
-    uint32_t m = 0;
-    GCU_TRY(build_dag(g, true, rev, &dag_offsets, &dag_targets, &dag_eid, &m));
-    if (m > 0) {
-        GCU_TRY(run_wedges(*g.dev, dag_offsets.ptr, dag_targets.ptr, g.num_nodes, 2,
-                           SupportSink{dag_eid.ptr, support}, "kt"));
-    }
-    return ok();
-}
-
 // Per-graph state of the symmetric k-truss: row of every entry, reverse
 // entries, self-loop flags and the triangle support of every u < v entry. It
 // depends only on the graph, so it is computed once and reused by every
@@ -518,7 +487,7 @@ static Error ensure_kt_cache(GraphImpl& g, KtCache** out) {
         GCU_LAUNCH(dev, "kt_loops", kt_loops_kernel, edge_grid, 256, 0, g.targets.ptr, c->src.ptr, E, c->loop.ptr,
                    count.ptr);
         GCU_CUDA(cudaMemsetAsync(c->support.ptr, 0, sizeof(uint32_t) * static_cast<size_t>(E), dev.stream), "memset");
-        GCU_TRY(triangle_support(g, c->rev.ptr, c->support.ptr));
+        GCU_TRY(edge_support(g, c->rev.ptr, c->support.ptr));
         GCU_CUDA(cudaMemcpyAsync(&c->loops, count.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
         GCU_TRY(dev.sync());
         g.kt_cache = c.release();
@@ -527,7 +496,7 @@ static Error ensure_kt_cache(GraphImpl& g, KtCache** out) {
     return ok();
 }
 
-// Symmetric CSR: per-edge triangle counts from the DAG (cached), then
+// Symmetric CSR: per-edge triangle counts (cached), then
 // incremental peeling. Every round removes exactly the entries the
 // reference's round removes, so the edge list and the round count are the
 // same.

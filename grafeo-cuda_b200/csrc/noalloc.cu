@@ -42,7 +42,6 @@ static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocHeader + kNo
 namespace {
 
 struct NoAllocCountSink {
-    static constexpr bool kNeedsPos = false;
     unsigned long long* total;
     unsigned long long count;
     __device__ __forceinline__ void hit(uint32_t, uint32_t, uint32_t, uint32_t) { ++count; }

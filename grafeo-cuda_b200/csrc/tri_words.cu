@@ -1,4 +1,5 @@
-// Triangle counting over word lists (symmetric CSRs, fixed schedule).
+// Triangle counting (symmetric CSRs, fixed schedule) and edge supports (k-truss)
+// over word lists.
 //
 // Vertices are ranked by degree class (degree_class_order: hubs first), and
 // N+(u) is the set of u's neighbours that rank below it. Hubs take most of the
@@ -12,8 +13,8 @@
 // once, at the edge of its two highest-ranked vertices. Each edge is counted
 // from the end whose list has more words (ties: the larger id), the owner: the
 // owner's words go into a table in shared memory and the other end's words are
-// streamed against it, 4, 16 or 32 lanes per list. An owner reads its neighbours from its own CSR row, so there are no
-// in-lists and no oriented CSR to build.
+// streamed against it, 4, 16 or 32 lanes per list. An owner reads its neighbours
+// from its own CSR row, so there are no in-lists and no oriented CSR to build.
 //  * owners of up to kWarpWords words and kWarpOwnerRow neighbours: a warp each,
 //    with a hash table of (word, mask);
 //  * the others: CTA items of kSlice neighbours; the table is a bitmap of the
@@ -31,6 +32,15 @@
 // registers 10.1; lists by length, 4 / 16 / 32 lanes each, 9.9 (with four in
 // flight 13.3: a fifth fewer resident blocks). What bounds it is instruction
 // issue.
+//
+// The support of an edge {u, v} is |N(u) ∩ N(v)|: the same sum of popcounts, kept
+// per edge, over lists of all neighbours. R-MAT 18 has 622 M words to stream that
+// way, 6.8 times those of the N+ lists, but each edge's sum is stored once, where
+// enumerating the triangles of the oriented CSR takes three scattered atomics per
+// triangle: 0.94 ms (and 0.25 ms for the lists) against 5.6 (and 0.35 for the
+// CSR). A full list reaches all ranks, so the bitmap covers all vertices while it
+// fits an SM's shared memory, 1.7 M of them, with the blocks as wide as it is
+// large: 128 threads with 16 KB, 1024 with 208 KB.
 #include <algorithm>
 
 #include "device_common.cuh"
@@ -60,6 +70,12 @@ constexpr uint32_t kBitmapWords = 4096;
 constexpr uint32_t kBitmapRanks = kBitmapWords * 32;
 constexpr uint32_t kHashBits = 11;       // 2048 (word, mask) slots: as many bytes as the bitmap
 constexpr uint32_t kHashWords = 1u << (kHashBits - 1);
+constexpr size_t kSmemPerSm = size_t(227) << 10;
+// Of the support's blocks (bitmap, lists in hand and 1 KB reserved each): 12 of
+// 128 threads, 6 of 256, 3 of 512 or one of 1024 in an SM, by the bitmap's bytes.
+constexpr size_t kBitmap128 = size_t(16) << 10, kBitmap256 = size_t(33) << 10, kBitmap512 = size_t(66) << 10;
+constexpr uint32_t kMaxBitmapWords = 52u << 10;  // 1.7 M ranks
+constexpr uint32_t kMaxTableWords = (1024 / 32) * (2u << kWarpBits);
 static_assert((1u << kHashBits) * 2 == kBitmapWords, "one shared array for both tables");
 static_assert(kCountWarps * (2u << kWarpBits) <= kBitmapWords, "the warps' tables fit the shared array");
 
@@ -94,6 +110,10 @@ __device__ __forceinline__ uint32_t table_mask(const uint2* table, uint32_t bits
 
 // ---------------------------------------------------------------- word lists
 
+// Whether a vertex whose neighbour ranks x is in that one's list: below it, or
+// any neighbour (not itself: a self-loop is in no triangle).
+__device__ __forceinline__ bool in_list(uint32_t x, uint32_t own, bool full) { return full ? x != own : x < own; }
+
 // Room for a list of n words: it starts on 16 bytes and is padded to an even
 // length with an empty word, so that the count can read two words at a time.
 __device__ __forceinline__ unsigned long long take_words(uint2* words, unsigned long long* cursor, uint32_t n) {
@@ -108,7 +128,7 @@ __device__ __forceinline__ unsigned long long take_words(uint2* words, unsigned 
 __global__ void __launch_bounds__(kTwThreads) tw_build_warp_kernel(const uint32_t* __restrict__ offsets,
                                                                    const uint32_t* __restrict__ targets,
                                                                    const uint32_t* __restrict__ rank, uint32_t V,
-                                                                   uint32_t turn, uint2* __restrict__ lists,
+                                                                   bool full, uint32_t turn, uint2* __restrict__ lists,
                                                                    uint2* __restrict__ words,
                                                                    unsigned long long* __restrict__ cursor) {
     __shared__ uint2 s_table[kTwWarps][1u << kWarpBits];
@@ -145,7 +165,7 @@ __global__ void __launch_bounds__(kTwThreads) tw_build_warp_kernel(const uint32_
                 const bool real = b + group < n_rows;
                 const uint4 row = real ? s_rows[threadIdx.x >> 5][b + group] : make_uint4(0u, 0u, 0u, 0u);
                 const uint32_t x = at < row.y ? __ldg(rank + __ldg(targets + row.x + at)) : kNoWord;
-                const bool keep = x < row.z;
+                const bool keep = x != kNoWord && in_list(x, row.z, full);
                 // Words are below 2^27: the row's group goes above.
                 const unsigned peers = __match_any_sync(kFullMask, keep ? x >> 5 | group << 27 : kNoWord);
                 const uint32_t mask = __reduce_or_sync(peers, keep ? 1u << (x & 31) : 0u);
@@ -161,8 +181,7 @@ __global__ void __launch_bounds__(kTwThreads) tw_build_warp_kernel(const uint32_
                     if (first) words[base + __popc(firsts & mates & ((1u << lane) - 1))] = make_uint2(x >> 5, mask);
                     if (at == 0 && (n & 1)) words[base + n] = make_uint2(kNoWord, 0u);
                 }
-                // Positions stay below E / 2 + V: every edge is kept at one end.
-                if (real && at == 0) lists[v0 + row.w] = make_uint2(static_cast<uint32_t>(base), n);
+                if (real && at == 0) lists[v0 + row.w] = make_uint2(static_cast<uint32_t>(base / 2), n);
             }
         }
         unsigned todo = __ballot_sync(kFullMask, d > 32 && d <= kWarpRow);
@@ -177,7 +196,7 @@ __global__ void __launch_bounds__(kTwThreads) tw_build_warp_kernel(const uint32_
             __syncwarp();
             for (uint32_t k = lane; k < rd; k += 32) {
                 const uint32_t x = __ldg(rank + __ldg(targets + rs + k));
-                if (x < ru) table_or(table, kWarpBits, x >> 5, 1u << (x & 31));
+                if (in_list(x, ru, full)) table_or(table, kWarpBits, x >> 5, 1u << (x & 31));
             }
             __syncwarp();
             for (uint32_t k = lane; k < (1u << kWarpBits); k += 32)
@@ -194,7 +213,7 @@ __global__ void __launch_bounds__(kTwThreads) tw_build_warp_kernel(const uint32_
                 }
             }
             __syncwarp();
-            if (lane == 0) lists[v0 + l] = make_uint2(static_cast<uint32_t>(at), n);
+            if (lane == 0) lists[v0 + l] = make_uint2(static_cast<uint32_t>(at / 2), n);
         }
     }
 }
@@ -220,18 +239,20 @@ __global__ void tw_long_rows_kernel(const uint32_t* __restrict__ offsets, uint32
     }
 }
 
-// Longer rows, a CTA each: the ranks below the owner's are set in a bitmap,
-// kBitmapRanks of them at a time, and its non-zero words written out. Two
+// Longer rows, a CTA each: the ranks of the list are set in a bitmap,
+// bitmap_words * 32 of them at a time, and its non-zero words written out. Two
 // sweeps of the row where it has more than one window: the first counts.
-__global__ void __launch_bounds__(kTwThreads) tw_build_cta_kernel(
+__global__ void __launch_bounds__(1024) tw_build_cta_kernel(
     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ rank,
-    const uint32_t* __restrict__ rows, const uint32_t* __restrict__ n_rows, uint32_t* __restrict__ next,
-    uint2* __restrict__ lists, uint2* __restrict__ words, unsigned long long* __restrict__ cursor) {
-    __shared__ uint32_t s_bits[kBitmapWords];
+    uint32_t V, bool full, uint32_t bitmap_words, const uint32_t* __restrict__ rows,
+    const uint32_t* __restrict__ n_rows, uint32_t* __restrict__ next, uint2* __restrict__ lists,
+    uint2* __restrict__ words, unsigned long long* __restrict__ cursor) {
+    extern __shared__ uint32_t s_bits[];
     __shared__ uint32_t s_item, s_total, s_at;
     __shared__ unsigned long long s_base;
     const unsigned lane = lane_id();
-    for (uint32_t k = threadIdx.x; k < kBitmapWords; k += kTwThreads) s_bits[k] = 0;
+    const uint32_t window = bitmap_words * 32;
+    for (uint32_t k = threadIdx.x; k < bitmap_words; k += blockDim.x) s_bits[k] = 0;
     const uint32_t n = *n_rows;
     while (true) {
         __syncthreads();
@@ -244,19 +265,20 @@ __global__ void __launch_bounds__(kTwThreads) tw_build_cta_kernel(
         if (s_item >= n) break;
         const uint32_t u = rows[s_item];
         const uint32_t s = offsets[u], e = offsets[u + 1], r = rank[u];
-        const uint32_t windows = (r + kBitmapRanks - 1) / kBitmapRanks;
+        const uint32_t end = full ? V : r;  // of the ranks in the list
+        const uint32_t windows = static_cast<uint32_t>(ceil_div_u64(end, window));
         for (uint32_t sweep = windows > 1 ? 0 : 1; sweep < 2; ++sweep) {
             for (uint32_t w = 0; w < max(windows, 1u); ++w) {
-                const uint32_t lo = w * kBitmapRanks, hi = min(r - lo, kBitmapRanks) + lo;
-                for (uint64_t j = static_cast<uint64_t>(s) + threadIdx.x; j < e; j += kTwThreads) {
+                const uint32_t lo = w * window, hi = min(end - lo, window) + lo;
+                for (uint64_t j = static_cast<uint64_t>(s) + threadIdx.x; j < e; j += blockDim.x) {
                     const uint32_t x = __ldg(rank + ld_stream(targets + j));
-                    if (x >= lo && x < hi) atomicOr(s_bits + ((x - lo) >> 5), 1u << (x & 31));
+                    if (x >= lo && x < hi && x != r) atomicOr(s_bits + ((x - lo) >> 5), 1u << (x & 31));
                 }
                 __syncthreads();
                 const uint32_t used = (hi - lo + 31) / 32;
                 if (windows <= 1 || sweep == 0) {
                     uint32_t mine = 0;
-                    for (uint32_t k = threadIdx.x; k < used; k += kTwThreads) {
+                    for (uint32_t k = threadIdx.x; k < used; k += blockDim.x) {
                         mine += s_bits[k] != 0 ? 1u : 0u;
                         if (windows > 1) s_bits[k] = 0;
                     }
@@ -268,11 +290,11 @@ __global__ void __launch_bounds__(kTwThreads) tw_build_cta_kernel(
                     if (w == 0) {
                         if (threadIdx.x == 0) {
                             s_base = s_total ? take_words(words, cursor, s_total) : 0ull;
-                            lists[u] = make_uint2(static_cast<uint32_t>(s_base), s_total);
+                            lists[u] = make_uint2(static_cast<uint32_t>(s_base / 2), s_total);
                         }
                         __syncthreads();
                     }
-                    for (uint32_t k0 = threadIdx.x & ~31u; k0 < used; k0 += kTwThreads) {
+                    for (uint32_t k0 = threadIdx.x & ~31u; k0 < used; k0 += blockDim.x) {
                         const uint32_t k = k0 + lane;
                         const uint32_t m = k < used ? s_bits[k] : 0u;
                         const unsigned has = __ballot_sync(kFullMask, m != 0);
@@ -293,7 +315,6 @@ __global__ void __launch_bounds__(kTwThreads) tw_build_cta_kernel(
 }
 
 // ---------------------------------------------------------------- owners
-
 
 // Vertices with words: to the warp kernel's list, or as (vertex, slice) items
 // to the CTA kernel's.
@@ -321,51 +342,91 @@ __global__ void tw_owners_kernel(const uint32_t* __restrict__ offsets, const uin
 
 // ---------------------------------------------------------------- counting
 
-// Streams the lists e with `take` against mask(word), 2^kLogSize lanes per list
+// Two words from word `at` (even) of a list, whose place is kept in units of two
+// words.
+__device__ __forceinline__ uint4 word_pair(const uint2* __restrict__ words, const uint2 l, uint32_t at) {
+    return __ldg(reinterpret_cast<const uint4*>(words) + (l.x + at / 2));
+}
+
+// First word of a list.
+__device__ __forceinline__ const uint2* list_words(const uint2* __restrict__ words, const uint2 l) {
+    return words + 2ull * l.x;
+}
+
+// The warp's neighbours in hand: their lists and, for the support, the entries
+// whose support their counts are.
+template <bool kSupport>
+struct ListBox {
+    uint2 list[32];
+    uint32_t entry[kSupport ? 32 : 1];
+};
+
+// Streams the lists l with `take` against mask(word), 2^kLogSize lanes per list
 // (a lane reads two words at a time) and kInFlight lists in flight per group of
-// lanes; with 32 lanes per list, lists may be longer than the group.
-template <uint32_t kLogSize, class Mask>
-__device__ __forceinline__ uint32_t stream_lists(bool take, const uint2 l, const uint2* __restrict__ words,
-                                                 uint2* s_list, Mask mask) {
+// lanes; with 32 lanes per list, lists may be longer than the group. The hits
+// are summed over all lists (the lane's part is returned), or, with kSupport,
+// over the lanes of each list and given to store(entry, sum).
+template <uint32_t kLogSize, bool kSupport, class Mask, class Store>
+__device__ __forceinline__ uint32_t stream_lists(bool take, const uint2 l, uint32_t entry,
+                                                 const uint2* __restrict__ words, ListBox<kSupport>& box, Mask mask,
+                                                 Store store) {
     const unsigned lane = lane_id();
     const unsigned taken = __ballot_sync(kFullMask, take);
     if (taken == 0) return 0;
     constexpr uint32_t size = 1u << kLogSize, groups = 32u >> kLogSize;
     const uint32_t count = __popc(taken), group = lane >> kLogSize, at = 2 * (lane & (size - 1));
     __syncwarp();
-    if (take) s_list[__popc(taken & ((1u << lane) - 1))] = l;
+    if (take) {
+        const uint32_t k = __popc(taken & ((1u << lane) - 1));
+        box.list[k] = l;
+        if constexpr (kSupport) box.entry[k] = entry;
+    }
     __syncwarp();
     uint32_t hits = 0;
-    auto add = [&](const uint4& p) {
-        hits += __popc(mask(p.x) & p.y);
-        hits += __popc(mask(p.z) & p.w);
-    };
+    auto popcounts = [&](const uint4& p) { return __popc(mask(p.x) & p.y) + __popc(mask(p.z) & p.w); };
     for (uint32_t b = 0; b < count; b += kInFlight * groups) {
         uint2 e[kInFlight];
         uint4 p[kInFlight];
+        uint32_t sum[kInFlight];
 #pragma unroll
         for (int i = 0; i < kInFlight; ++i) {
             const uint32_t k = b + i * groups + group;
-            e[i] = k < count ? s_list[k] : make_uint2(0u, 0u);
+            e[i] = k < count ? box.list[k] : make_uint2(0u, 0u);
         }
 #pragma unroll
         for (int i = 0; i < kInFlight; ++i)
-            p[i] = at < e[i].y ? __ldg(reinterpret_cast<const uint4*>(words + e[i].x + at))
+            p[i] = at < e[i].y ? word_pair(words, e[i], at)
                                : make_uint4(kNoWord, 0u, kNoWord, 0u);
 #pragma unroll
-        for (int i = 0; i < kInFlight; ++i)
-            if (at < e[i].y) add(p[i]);
-        if (kLogSize < 5) continue;
-#pragma unroll
         for (int i = 0; i < kInFlight; ++i) {
-            uint32_t k = at + 64;
-            for (; k + 64 < e[i].y; k += 128) {
-                const uint4 x = __ldg(reinterpret_cast<const uint4*>(words + e[i].x + k));
-                const uint4 y = __ldg(reinterpret_cast<const uint4*>(words + e[i].x + k + 64));
-                add(x);
-                add(y);
+            if constexpr (kSupport) sum[i] = 0;
+            if (at < e[i].y) (kSupport ? sum[i] : hits) += popcounts(p[i]);
+        }
+        if (kLogSize == 5) {
+#pragma unroll
+            for (int i = 0; i < kInFlight; ++i) {
+                uint32_t k = at + 64;
+                for (; k + 64 < e[i].y; k += 128) {
+                    const uint4 x = word_pair(words, e[i], k);
+                    const uint4 y = word_pair(words, e[i], k + 64);
+                    (kSupport ? sum[i] : hits) += popcounts(x);
+                    (kSupport ? sum[i] : hits) += popcounts(y);
+                }
+                if (k < e[i].y) (kSupport ? sum[i] : hits) += popcounts(word_pair(words, e[i], k));
             }
-            if (k < e[i].y) add(__ldg(reinterpret_cast<const uint4*>(words + e[i].x + k)));
+        }
+        if constexpr (kSupport) {
+#pragma unroll
+            for (int i = 0; i < kInFlight; ++i) {
+                if (kLogSize == 5) {
+                    sum[i] = __reduce_add_sync(kFullMask, sum[i]);
+                } else {
+#pragma unroll
+                    for (uint32_t d = size / 2; d > 0; d /= 2) sum[i] += __shfl_xor_sync(kFullMask, sum[i], d);
+                }
+                const uint32_t k = b + i * groups + group;
+                if (at == 0 && k < count && sum[i]) store(box.entry[k], sum[i]);
+            }
         }
     }
     return hits;
@@ -374,15 +435,20 @@ __device__ __forceinline__ uint32_t stream_lists(bool take, const uint2 l, const
 // Up to 32 neighbours (v per lane, `valid`) of an owner with id u and n words:
 // the lists of those it owns the edge to (fewer words, or as many and a smaller
 // id), by length: up to 8 words 4 lanes each, up to 32 words 16, the others 32.
-template <class Mask>
-__device__ __forceinline__ uint32_t count_neighbours(bool valid, uint32_t v, uint32_t u, uint32_t n,
+// j: the CSR entry of the neighbour; the support of an edge is kept at its
+// entry in the smaller vertex's row.
+template <bool kSupport, class Mask, class Store>
+__device__ __forceinline__ uint32_t count_neighbours(bool valid, uint32_t j, uint32_t v, uint32_t u, uint32_t n,
                                                      const uint2* __restrict__ lists, const uint2* __restrict__ words,
-                                                     uint2* s_list, Mask mask) {
+                                                     const uint32_t* __restrict__ rev, ListBox<kSupport>& box,
+                                                     Mask mask, Store store) {
     const uint2 l = valid ? __ldg(lists + v) : make_uint2(0u, 0u);
     const bool take = l.y > 0 && (l.y < n || (l.y == n && v < u));
-    return stream_lists<2>(take && l.y <= 8, l, words, s_list, mask) +
-           stream_lists<4>(take && l.y > 8 && l.y <= 32, l, words, s_list, mask) +
-           stream_lists<5>(take && l.y > 32, l, words, s_list, mask);
+    uint32_t entry = 0;
+    if constexpr (kSupport) entry = take ? (u < v ? j : __ldg(rev + j)) : 0u;
+    return stream_lists<2, kSupport>(take && l.y <= 8, l, entry, words, box, mask, store) +
+           stream_lists<4, kSupport>(take && l.y > 8 && l.y <= 32, l, entry, words, box, mask, store) +
+           stream_lists<5, kSupport>(take && l.y > 32, l, entry, words, box, mask, store);
 }
 
 // Total, or per owner (a union's graphs are told apart by their owners).
@@ -396,22 +462,37 @@ __device__ __forceinline__ void add_owner(uint32_t u, uint32_t hits, unsigned lo
     }
 }
 
+// What the kernel counts: triangles, in total or per owner, or the support of
+// every edge (full lists).
+struct WordCount {
+    unsigned long long* total;
+    unsigned long long* per_vertex;
+    uint32_t V;
+    uint32_t bitmap_words;  // of the support's dynamic shared array
+    const uint32_t* rev;
+    uint32_t* support;
+};
+
 // Blocks take the CTA items first, then their warps take the warp owners: the
 // end of the one fills the idle warps with the other.
-__global__ void __launch_bounds__(kCountThreads, kCountCtasPerSm) tw_count_kernel(
+template <bool kSupport, int kThreads, int kCtasPerSm>
+__global__ void __launch_bounds__(kThreads, kCtasPerSm) tw_count_kernel(
     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ rank,
     const uint2* __restrict__ lists, const uint2* __restrict__ words, const uint2* __restrict__ items,
     const uint32_t* __restrict__ owners, const uint32_t* __restrict__ counts, uint32_t* __restrict__ next,
-    uint32_t batch, unsigned long long* __restrict__ total, unsigned long long* __restrict__ per_vertex) {
-    __shared__ uint32_t s_bits[kBitmapWords];
-    __shared__ uint2 s_list[kCountWarps][32];
+    uint32_t batch, const WordCount out) {
+    __shared__ uint32_t s_fixed[kSupport ? 1 : kBitmapWords];
+    extern __shared__ uint32_t s_dynamic[];
+    __shared__ ListBox<kSupport> s_box[kThreads / 32];
     __shared__ uint32_t s_item, s_chunk;
+    uint32_t* s_bits = kSupport ? s_dynamic : s_fixed;
+    const uint32_t bitmap_words = kSupport ? out.bitmap_words : kBitmapWords;
     uint2* table = reinterpret_cast<uint2*>(s_bits);
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     const uint32_t n_items = counts[3], n_owners = counts[2];
     unsigned long long sum = 0;
     if (n_items)
-        for (uint32_t k = threadIdx.x; k < kBitmapWords; k += kCountThreads) s_bits[k] = 0;
+        for (uint32_t k = threadIdx.x; k < bitmap_words; k += kThreads) s_bits[k] = 0;
     while (true) {
         __syncthreads();
         if (threadIdx.x == 0) s_item = atomicAdd(next, 1u);
@@ -421,53 +502,59 @@ __global__ void __launch_bounds__(kCountThreads, kCountCtasPerSm) tw_count_kerne
         const uint32_t u = item.x;
         const uint2 own = __ldg(lists + u);
         const uint32_t s = offsets[u] + item.y * kSlice, e = s + min(kSlice, offsets[u + 1] - s);
-        const uint32_t r = rank[u];
-        const bool hash = r > kBitmapRanks && own.y <= kHashWords;
-        const uint32_t windows = hash ? 1u : (r + kBitmapRanks - 1) / kBitmapRanks;
+        const uint32_t end = kSupport ? out.V : rank[u];  // of the ranks in the owner's list
+        const uint32_t window = bitmap_words * 32;
+        const bool hash = end > window && own.y <= kHashWords;
+        const uint32_t windows = hash ? 1u : static_cast<uint32_t>(ceil_div_u64(end, window));
         uint32_t hits = 0;
         for (uint32_t win = 0; win < windows; ++win) {
-            const uint32_t lo = win * kBitmapWords;
+            const uint32_t lo = win * bitmap_words;
             if (hash) {
-                for (uint32_t k = threadIdx.x; k < (1u << kHashBits); k += kCountThreads)
+                for (uint32_t k = threadIdx.x; k < (1u << kHashBits); k += kThreads)
                     table[k] = make_uint2(kNoWord, 0u);
                 __syncthreads();
             }
-            for (uint32_t k = threadIdx.x; k < own.y; k += kCountThreads) {
-                const uint2 w = __ldg(words + own.x + k);
+            for (uint32_t k = threadIdx.x; k < own.y; k += kThreads) {
+                const uint2 w = __ldg(list_words(words, own) + k);
                 if (hash) table_or(table, kHashBits, w.x, w.y);
-                else if (w.x - lo < kBitmapWords) s_bits[w.x - lo] = w.y;  // the words of a list are distinct
+                else if (w.x - lo < bitmap_words) s_bits[w.x - lo] = w.y;  // the words of a list are distinct
             }
             if (threadIdx.x == 0) s_chunk = 0;
             __syncthreads();
+            // A later window adds to what the block stored before the barrier.
+            auto store = [&](uint32_t entry, uint32_t h) { out.support[entry] = win ? out.support[entry] + h : h; };
             while (true) {
                 uint32_t c = 0;
                 if (lane == 0) c = atomicAdd(&s_chunk, 32u);
                 c = __shfl_sync(kFullMask, c, 0);
                 if (c >= e - s) break;
                 const bool valid = e - s - c > lane;
-                const uint32_t v = valid ? ld_stream(targets + s + c + lane) : 0u;
+                const uint32_t j = s + c + lane;
+                const uint32_t v = valid ? ld_stream(targets + j) : 0u;
                 if (hash)
-                    hits += count_neighbours(valid, v, u, own.y, lists, words, s_list[warp],
-                                             [&](uint32_t w) { return table_mask(table, kHashBits, w); });
+                    hits += count_neighbours<kSupport>(
+                        valid, j, v, u, own.y, lists, words, out.rev, s_box[warp],
+                        [&](uint32_t w) { return table_mask(table, kHashBits, w); }, store);
                 else
-                    hits += count_neighbours(valid, v, u, own.y, lists, words, s_list[warp], [&](uint32_t w) {
-                        return w - lo < kBitmapWords ? s_bits[w - lo] : 0u;
-                    });
+                    hits += count_neighbours<kSupport>(
+                        valid, j, v, u, own.y, lists, words, out.rev, s_box[warp],
+                        [&](uint32_t w) { return w - lo < bitmap_words ? s_bits[w - lo] : 0u; }, store);
             }
             __syncthreads();
             if (hash) {
-                for (uint32_t k = threadIdx.x; k < kBitmapWords; k += kCountThreads) s_bits[k] = 0;
+                for (uint32_t k = threadIdx.x; k < (2u << kHashBits); k += kThreads) s_bits[k] = 0;
             } else {
-                for (uint32_t k = threadIdx.x; k < own.y; k += kCountThreads) {
-                    const uint32_t w = __ldg(words + own.x + k).x;
-                    if (w - lo < kBitmapWords) s_bits[w - lo] = 0;
+                for (uint32_t k = threadIdx.x; k < own.y; k += kThreads) {
+                    const uint32_t w = __ldg(list_words(words, own) + k).x;
+                    if (w - lo < bitmap_words) s_bits[w - lo] = 0;
                 }
             }
             if (win + 1 < windows) __syncthreads();
         }
-        add_owner(u, hits, per_vertex, sum);
+        if (!kSupport) add_owner(u, hits, out.per_vertex, sum);
     }
     table += warp << kWarpBits;  // the warps' own tables from here on (after the loop's block barrier)
+    auto store = [&](uint32_t entry, uint32_t h) { out.support[entry] = h; };
     while (true) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(next + 1, batch);
@@ -484,7 +571,7 @@ __global__ void __launch_bounds__(kCountThreads, kCountCtasPerSm) tw_count_kerne
             for (uint32_t k = lane; k < (1u << bits); k += 32) table[k] = make_uint2(kNoWord, 0u);
             __syncwarp();
             for (uint32_t k = lane; k < own.y; k += 32) {
-                const uint2 w = __ldg(words + own.x + k);
+                const uint2 w = __ldg(list_words(words, own) + k);
                 table_or(table, bits, w.x, w.y);
             }
             __syncwarp();
@@ -492,30 +579,45 @@ __global__ void __launch_bounds__(kCountThreads, kCountCtasPerSm) tw_count_kerne
             for (uint32_t j = s; j < e; j += 32) {
                 const bool valid = e - j > lane;
                 const uint32_t v = valid ? ld_stream(targets + j + lane) : 0u;
-                hits += count_neighbours(valid, v, u, own.y, lists, words, s_list[warp],
-                                         [&](uint32_t w) { return table_mask(table, bits, w); });
+                hits += count_neighbours<kSupport>(
+                    valid, j + lane, v, u, own.y, lists, words, out.rev, s_box[warp],
+                    [&](uint32_t w) { return table_mask(table, bits, w); }, store);
             }
-            add_owner(u, hits, per_vertex, sum);
+            if (!kSupport) add_owner(u, hits, out.per_vertex, sum);
         }
     }
-    sum = warp_sum(sum);
-    if (lane == 0 && sum) atomicAdd(total, sum);
+    if (!kSupport) {
+        sum = warp_sum(sum);
+        if (lane == 0 && sum) atomicAdd(out.total, sum);
+    }
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------- host
 
-Error build_word_lists(GraphImpl& g, WordLists* w) {
+namespace {
+
+// Bitmap of the full lists' ranks: all of them, or as many as fit an SM.
+uint32_t support_bitmap_words(uint32_t V) {
+    // Room for the warps' tables too (1024 threads: 32 tables).
+    const uint64_t words = ceil_div_u64(V, 32);
+    const uint64_t tables = words * sizeof(uint32_t) <= kBitmap256 ? kBitmapWords : kMaxTableWords;
+    return static_cast<uint32_t>(std::min<uint64_t>(std::max(words, tables), kMaxBitmapWords));
+}
+
+}  // namespace
+
+Error build_word_lists(GraphImpl& g, bool full, WordLists* w) {
     DeviceImpl& dev = *g.dev;
     const uint32_t V = g.num_nodes, E = g.num_edges;
     const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
     GCU_TRY(degree_class_order(dev, g.offsets.ptr, V, &w->rank));
     GCU_TRY(w->lists.allocate(dev, V));
-    // Every edge's rank is kept at one end: E / 2 words at most, and a padding
-    // word per list (lists without words take no room).
-    const uint64_t room = static_cast<uint64_t>(E / 2) + std::min<uint64_t>(E / 2, V);
-    if (room > 0xFFFFFFFFull) return kernel_error("graph too large for the triangle count's word lists");
+    // An edge's ranks are kept at one end, or at both: E / 2 or E words at most,
+    // and a padding word per list (lists without words take no room).
+    const uint64_t kept = full ? E : E / 2;
+    const uint64_t room = kept + std::min<uint64_t>(kept, V);
     GCU_TRY(w->words.allocate(dev, std::max<uint64_t>(room, 1)));
     GCU_TRY(w->warp_owners.allocate(dev, V));
     // counters: [0] long rows, [1] next long row, [2] warp owners, [3] CTA items
@@ -530,18 +632,26 @@ Error build_word_lists(GraphImpl& g, WordLists* w) {
     const unsigned wgrid = static_cast<unsigned>(
         std::max<uint64_t>(1, std::min<uint64_t>(ceil_div_u64(V, static_cast<uint64_t>(turn) * kTwWarps), cap)));
     GCU_LAUNCH(dev, "tw_build_warp", tw_build_warp_kernel, wgrid, kTwThreads, 0, g.offsets.ptr, g.targets.ptr,
-               w->rank.ptr, V, turn, w->lists.ptr, w->words.ptr, cursor.ptr);
+               w->rank.ptr, V, full, turn, w->lists.ptr, w->words.ptr, cursor.ptr);
     // The owner list is free until the owners are known: the long rows use it.
     GCU_LAUNCH(dev, "tw_long_rows", tw_long_rows_kernel, vgrid, 256, 0, g.offsets.ptr, V, w->warp_owners.ptr,
                w->counts.ptr);
+    // Full lists: all ranks in one window while the bitmap fits an SM.
+    const uint32_t bitmap_words = full ? support_bitmap_words(V) : kBitmapWords;
+    const unsigned threads = bitmap_words * sizeof(uint32_t) > kBitmap512 ? 1024u : kTwThreads;
+    const size_t smem = sizeof(uint32_t) * bitmap_words;
+    GCU_CUDA(cudaFuncSetAttribute(tw_build_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(sizeof(uint32_t) * kMaxBitmapWords)),
+             "cudaFuncSetAttribute");
+    const unsigned resident = static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(7, kSmemPerSm / (smem + 2048))));
     const unsigned cgrid = static_cast<unsigned>(
-        std::max<uint64_t>(1, std::min<uint64_t>(E / kWarpRow, static_cast<uint64_t>(dev.sm_count) * 7)));
-    GCU_LAUNCH(dev, "tw_build_cta", tw_build_cta_kernel, cgrid, kTwThreads, 0, g.offsets.ptr, g.targets.ptr,
-               w->rank.ptr, w->warp_owners.ptr, w->counts.ptr, w->counts.ptr + 1, w->lists.ptr, w->words.ptr,
-               cursor.ptr);
+        std::max<uint64_t>(1, std::min<uint64_t>(E / kWarpRow, static_cast<uint64_t>(dev.sm_count) * resident)));
+    GCU_LAUNCH(dev, "tw_build_cta", tw_build_cta_kernel, cgrid, threads, smem, g.offsets.ptr, g.targets.ptr,
+               w->rank.ptr, V, full, bitmap_words, w->warp_owners.ptr, w->counts.ptr, w->counts.ptr + 1, w->lists.ptr,
+               w->words.ptr, cursor.ptr);
     // Items: at most one per kSlice entries plus one per vertex with more words,
     // so more neighbours, than a warp owner.
-    const uint32_t warp_words = V < kSmallGraph ? kWarpWordsSmall : kWarpWords;
+    const uint32_t warp_words = !full && V < kSmallGraph ? kWarpWordsSmall : kWarpWords;
     w->max_items = E / kSlice + E / warp_words + 1;
     GCU_TRY(w->items.allocate(dev, w->max_items));
     GCU_LAUNCH(dev, "tw_owners", tw_owners_kernel, vgrid, 256, 0, g.offsets.ptr, w->lists.ptr, V, warp_words,
@@ -549,19 +659,50 @@ Error build_word_lists(GraphImpl& g, WordLists* w) {
     return ok();
 }
 
-Error count_words(GraphImpl& g, const WordLists& w, uint32_t* next, unsigned long long* total,
-                  unsigned long long* per_vertex) {
+namespace {
+
+template <bool kSupport, int kThreads, int kCtasPerSm>
+Error launch_count(GraphImpl& g, const WordLists& w, uint32_t* next, const WordCount& out) {
     DeviceImpl& dev = *g.dev;
+    constexpr int kWarps = kThreads / 32;
+    const size_t smem = sizeof(uint32_t) * out.bitmap_words;
+    const auto kernel = tw_count_kernel<kSupport, kThreads, kCtasPerSm>;
+    if (smem)
+        GCU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+                 "cudaFuncSetAttribute");
     GCU_CUDA(cudaMemsetAsync(next, 0, 2 * sizeof(uint32_t), dev.stream), "memset");
-    const uint64_t want = std::max<uint64_t>(w.max_items, ceil_div_u64(g.num_nodes, kCountWarps));
+    const uint64_t want = std::max<uint64_t>(w.max_items, ceil_div_u64(g.num_nodes, kWarps));
     const unsigned grid = static_cast<unsigned>(
-        std::max<uint64_t>(1, std::min<uint64_t>(want, static_cast<uint64_t>(dev.sm_count) * kCountCtasPerSm)));
+        std::max<uint64_t>(1, std::min<uint64_t>(want, static_cast<uint64_t>(dev.sm_count) * kCtasPerSm)));
     // Owners per handout: several turns per warp, or one at a time on a small graph.
     const uint32_t batch = static_cast<uint32_t>(
-        std::max<uint64_t>(1, std::min<uint64_t>(8, g.num_nodes / (static_cast<uint64_t>(grid) * kCountWarps * 8))));
-    GCU_LAUNCH(dev, "tw_count", tw_count_kernel, grid, kCountThreads, 0, g.offsets.ptr, g.targets.ptr, w.rank.ptr,
-               w.lists.ptr, w.words.ptr, w.items.ptr, w.warp_owners.ptr, w.counts.ptr, next, batch, total, per_vertex);
+        std::max<uint64_t>(1, std::min<uint64_t>(8, g.num_nodes / (static_cast<uint64_t>(grid) * kWarps * 8))));
+    GCU_LAUNCH(dev, kSupport ? "tw_support" : "tw_count", kernel, grid, kThreads, smem, g.offsets.ptr, g.targets.ptr,
+               w.rank.ptr, w.lists.ptr, w.words.ptr, w.items.ptr, w.warp_owners.ptr, w.counts.ptr, next, batch, out);
     return ok();
+}
+
+}  // namespace
+
+Error count_words(GraphImpl& g, const WordLists& w, uint32_t* next, unsigned long long* total,
+                  unsigned long long* per_vertex) {
+    return launch_count<false, kCountThreads, kCountCtasPerSm>(
+        g, w, next, WordCount{total, per_vertex, g.num_nodes, 0, nullptr, nullptr});
+}
+
+Error edge_support(GraphImpl& g, const uint32_t* rev, uint32_t* support) {
+    DeviceImpl& dev = *g.dev;
+    WordLists w;
+    GCU_TRY(build_word_lists(g, true, &w));
+    DeviceBuffer<uint32_t> next;
+    GCU_TRY(next.allocate(dev, 2));
+    WordCount out{nullptr, nullptr, g.num_nodes, support_bitmap_words(g.num_nodes), rev, support};
+    const size_t bytes = sizeof(uint32_t) * out.bitmap_words;
+    if (bytes <= kBitmap128) GCU_TRY((launch_count<true, 128, 12>(g, w, next.ptr, out)));
+    else if (bytes <= kBitmap256) GCU_TRY((launch_count<true, 256, 6>(g, w, next.ptr, out)));
+    else if (bytes <= kBitmap512) GCU_TRY((launch_count<true, 512, 3>(g, w, next.ptr, out)));
+    else GCU_TRY((launch_count<true, 1024, 1>(g, w, next.ptr, out)));
+    return dev.sync();  // the lists are freed on return
 }
 
 }  // namespace gcu

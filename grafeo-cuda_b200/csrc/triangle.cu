@@ -94,25 +94,16 @@ __global__ void __launch_bounds__(kOrientThreads) tc_orient_flag_kernel(const ui
     }
 }
 
-// Kept entries to their DAG positions; with dag_eid, also the CSR index of
-// the edge's u < v entry (the undirected edge id); with dag_rank, the rank of
-// each kept target.
-__global__ void __launch_bounds__(kOrientThreads) tc_orient_fill_kernel(const uint32_t* __restrict__ offsets,
-                                                                        const uint32_t* __restrict__ targets,
-                                                                        uint32_t V, uint32_t E,
-                                                                        const uint32_t* __restrict__ pos,
+// Kept entries to their DAG positions; with dag_rank, also the rank of each
+// kept target.
+__global__ void __launch_bounds__(kOrientThreads) tc_orient_fill_kernel(const uint32_t* __restrict__ targets,
+                                                                        uint32_t E, const uint32_t* __restrict__ pos,
                                                                         uint32_t* __restrict__ dag_targets,
-                                                                        const uint32_t* __restrict__ rev,
-                                                                        uint32_t* __restrict__ dag_eid,
                                                                         const uint32_t* __restrict__ rank,
                                                                         uint32_t* __restrict__ dag_rank) {
-    __shared__ uint32_t s_start[kOrientTile];
-    __shared__ uint32_t s_meta[2];
     for (uint64_t e0 = static_cast<uint64_t>(blockIdx.x) * kOrientTile; e0 < E;
          e0 += static_cast<uint64_t>(gridDim.x) * kOrientTile) {
         const uint64_t e1 = min_u64(e0 + kOrientTile, E);
-        const bool staged = dag_eid ? stage_tile_rows<kOrientTile>(offsets, V, e0, e1, s_start, s_meta) : false;
-        const uint32_t r0 = dag_eid ? s_meta[0] : 0, nrows = dag_eid ? s_meta[1] - r0 + 1 : 0;
 #pragma unroll
         for (int q = 0; q < kOrientItems; ++q) {
             const uint64_t j = e0 + q * kOrientThreads + threadIdx.x;
@@ -122,12 +113,7 @@ __global__ void __launch_bounds__(kOrientThreads) tc_orient_fill_kernel(const ui
             const uint32_t v = ld_stream(targets + j);
             dag_targets[at] = v;
             if (dag_rank) dag_rank[at] = __ldg(rank + v);
-            if (dag_eid) {
-                const uint32_t u = tile_row(offsets, V, s_start, staged, r0, nrows, static_cast<uint32_t>(j));
-                dag_eid[at] = u < v ? static_cast<uint32_t>(j) : rev[j];
-            }
         }
-        if (dag_eid) __syncthreads();
     }
 }
 
@@ -145,7 +131,6 @@ namespace {
 
 // Counts every triangle reported by the wedge kernels.
 struct CountSink {
-    static constexpr bool kNeedsPos = false;
     unsigned long long* total;
     unsigned long long count;
     __device__ __forceinline__ void hit(uint32_t, uint32_t, uint32_t, uint32_t) { ++count; }
@@ -160,9 +145,8 @@ struct CountSink {
 
 // With `rank`: oriented by that vertex order, and dag_rank (when given) holds
 // the rank of every DAG target.
-static Error build_dag_impl(GraphImpl& g, bool by_degree, const uint32_t* rank, const uint32_t* rev,
-                            DeviceBuffer<uint32_t>* dag_offsets, DeviceBuffer<uint32_t>* dag_targets,
-                            DeviceBuffer<uint32_t>* dag_eid, DeviceBuffer<uint32_t>* dag_rank, uint32_t* m) {
+static Error build_dag_impl(GraphImpl& g, bool by_degree, const uint32_t* rank, DeviceBuffer<uint32_t>* dag_offsets,
+                            DeviceBuffer<uint32_t>* dag_targets, DeviceBuffer<uint32_t>* dag_rank, uint32_t* m) {
     DeviceImpl& dev = *g.dev;
     const uint32_t V = g.num_nodes, E = g.num_edges;
     GCU_TRY(dag_offsets->allocate(dev, static_cast<uint64_t>(V) + 1));
@@ -181,19 +165,17 @@ static Error build_dag_impl(GraphImpl& g, bool by_degree, const uint32_t* rank, 
     GCU_CUDA(cudaMemcpyAsync(m, pos.ptr + E, sizeof(uint32_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
     GCU_TRY(dev.sync());
     GCU_TRY(dag_targets->allocate(dev, std::max<uint32_t>(*m, 1)));
-    if (dag_eid) GCU_TRY(dag_eid->allocate(dev, std::max<uint32_t>(*m, 1)));
     if (dag_rank) GCU_TRY(dag_rank->allocate(dev, std::max<uint32_t>(*m, 1)));
     if (*m == 0) return ok();
-    GCU_LAUNCH(dev, "tc_orient_fill", tc_orient_fill_kernel, tiles, kOrientThreads, 0, g.offsets.ptr, g.targets.ptr,
-               V, E, pos.ptr, dag_targets->ptr, rev, dag_eid ? dag_eid->ptr : nullptr, rank,
-               dag_rank ? dag_rank->ptr : nullptr);
+    GCU_LAUNCH(dev, "tc_orient_fill", tc_orient_fill_kernel, tiles, kOrientThreads, 0, g.targets.ptr,
+               E, pos.ptr, dag_targets->ptr, rank, dag_rank ? dag_rank->ptr : nullptr);
     GCU_TRY(dev.sync());  // pos is freed on return
     return ok();
 }
 
-Error build_dag(GraphImpl& g, bool by_degree, const uint32_t* rev, DeviceBuffer<uint32_t>* dag_offsets,
-                DeviceBuffer<uint32_t>* dag_targets, DeviceBuffer<uint32_t>* dag_eid, uint32_t* m) {
-    return build_dag_impl(g, by_degree, nullptr, rev, dag_offsets, dag_targets, dag_eid, nullptr, m);
+Error build_dag(GraphImpl& g, bool by_degree, DeviceBuffer<uint32_t>* dag_offsets,
+                DeviceBuffer<uint32_t>* dag_targets, uint32_t* m) {
+    return build_dag_impl(g, by_degree, nullptr, dag_offsets, dag_targets, nullptr, m);
 }
 
 // ---------------------------------------------------------------- out-degree buckets
@@ -601,7 +583,7 @@ Error triangle_count_ex(GraphImpl& g, bool oriented, uint64_t* total, std::vecto
         GCU_TRY(next.allocate(dev, 2));
         GCU_TRY(sum.allocate(dev, 1));
         GCU_CUDA(cudaMemsetAsync(sum.ptr, 0, sizeof(unsigned long long), dev.stream), "memset");
-        GCU_TRY(build_word_lists(g, &w));
+        GCU_TRY(build_word_lists(g, false, &w));
         GCU_TRY(count_words(g, w, next.ptr, sum.ptr, nullptr));
         unsigned long long host = 0;
         GCU_CUDA(cudaMemcpyAsync(&host, sum.ptr, sizeof(host), cudaMemcpyDeviceToHost, dev.stream), "copy");
@@ -616,9 +598,9 @@ Error triangle_count_ex(GraphImpl& g, bool oriented, uint64_t* total, std::vecto
         // out-neighbour ranks below its owner, so an owner's table can be a
         // bitmap of the ranks below its own.
         GCU_TRY(degree_class_order(*g.dev, g.offsets.ptr, g.num_nodes, &rank));
-        GCU_TRY(build_dag_impl(g, true, rank.ptr, nullptr, &dag_offsets, &dag_targets, nullptr, &dag_rank, &m));
+        GCU_TRY(build_dag_impl(g, true, rank.ptr, &dag_offsets, &dag_targets, &dag_rank, &m));
     } else {
-        GCU_TRY(build_dag(g, false, nullptr, &dag_offsets, &dag_targets, nullptr, &m));
+        GCU_TRY(build_dag(g, false, &dag_offsets, &dag_targets, &m));
     }
     if (m == 0) return ok();
     // A DAG vertex needs two out-neighbours to close a triangle.
@@ -642,7 +624,6 @@ namespace {
 
 // Triangles per DAG source vertex: each warp adds its lanes' count for u.
 struct VertexCountSink {
-    static constexpr bool kNeedsPos = false;
     unsigned long long* per_vertex;
     unsigned long long count;
     __device__ __forceinline__ void hit(uint32_t, uint32_t, uint32_t, uint32_t) { ++count; }
@@ -677,13 +658,13 @@ Error batch_tc_plan(GraphImpl& u, BatchTcPlan** out, std::string* tuning) {
     if (symmetric && !dev.schedule) {
         p->word_graph = &u;
         GCU_TRY(p->next.allocate(dev, 2));
-        GCU_TRY(build_word_lists(u, &p->words));
+        GCU_TRY(build_word_lists(u, false, &p->words));
         if (tuning) *tuning = "{\"variant\": \"word lists\"}";
         GCU_TRY(dev.sync());
         *out = p.release();
         return ok();
     }
-    GCU_TRY(build_dag(u, true, nullptr, &p->dag_offsets, &p->dag_targets, nullptr, &p->m));
+    GCU_TRY(build_dag(u, true, &p->dag_offsets, &p->dag_targets, &p->m));
     DegreeStats stats;
     if (dev.schedule) GCU_TRY(degree_stats(u, &stats));
     GCU_TRY(plan_buckets(dev, p->dag_offsets.ptr, u.num_nodes, 2, p->m, stats, false, p->buckets));

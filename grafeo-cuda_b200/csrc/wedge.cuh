@@ -1,6 +1,6 @@
 // Wedge enumeration over a DAG CSR with shared-memory tables.
 //
-// Shared by triangle counting and k-truss support counting. For a vertex u
+// Used by triangle counting over oriented CSRs. For a vertex u
 // with out-list N+(u), the keys of N+(u) go into a table in shared memory: an
 // open-addressing hash table (multiplicative hashing, linear probing, load
 // <= 1/2, <= 1/4 where the slots allow) or, when the DAG is oriented by a
@@ -38,30 +38,22 @@ __device__ __forceinline__ uint32_t hash_home(uint32_t key, uint32_t bits) {
 // Inserts a key that is not yet present. Keys are distinct (sorted lists), so
 // only the slot claim needs an atomic. Gives up after one sweep of the table,
 // which cannot happen below load 1.
-template <bool kWithPos>
-__device__ __forceinline__ void hash_insert(uint32_t* keys, uint32_t* pos, uint32_t bits, uint32_t key,
-                                            uint32_t value) {
+__device__ __forceinline__ void hash_insert(uint32_t* keys, uint32_t bits, uint32_t key) {
     const uint32_t mask = (1u << bits) - 1;
     uint32_t s = hash_home(key, bits);
     for (uint32_t i = 0; i <= mask; ++i) {
-        if (atomicCAS(keys + s, kEmptyKey, key) == kEmptyKey) {
-            if (kWithPos) pos[s] = value;
-            return;
-        }
+        if (atomicCAS(keys + s, kEmptyKey, key) == kEmptyKey) return;
         s = (s + 1) & mask;
     }
 }
 
-// Position stored with `key`, kNotFound if absent (1 when kWithPos is false
-// and the key is present).
-template <bool kWithPos>
-__device__ __forceinline__ uint32_t hash_find(const uint32_t* keys, const uint32_t* pos, uint32_t bits,
-                                              uint32_t key) {
+// 1 if the key is present, kNotFound if absent.
+__device__ __forceinline__ uint32_t hash_find(const uint32_t* keys, uint32_t bits, uint32_t key) {
     const uint32_t mask = (1u << bits) - 1;
     uint32_t s = hash_home(key, bits);
     for (uint32_t i = 0; i <= mask; ++i) {
         const uint32_t k = keys[s];
-        if (k == key) return kWithPos ? pos[s] : 1u;
+        if (k == key) return 1u;
         if (k == kEmptyKey) return kNotFound;
         s = (s + 1) & mask;
     }
@@ -166,15 +158,13 @@ struct CtaTable {
     const uint32_t* values;    // what the probes look up (ranks or targets)
 };
 
-template <bool kPos>
-__device__ __forceinline__ CtaTable build_cta_table(uint32_t* s_keys, uint32_t* pos,
-                                                    const uint32_t* __restrict__ targets,
+__device__ __forceinline__ CtaTable build_cta_table(uint32_t* s_keys, const uint32_t* __restrict__ targets,
                                                     const uint32_t* __restrict__ rank,
                                                     const uint32_t* __restrict__ vrank, uint32_t x, uint32_t s,
                                                     uint32_t d, int search) {
     CtaTable t{kSearch, 0, 0, targets};
     if (search) return t;
-    if (!kPos && rank) {
+    if (rank) {
         t.values = rank;
         const uint32_t r = vrank[x];
         if (r <= kCtaSlots * 32) {
@@ -196,7 +186,7 @@ __device__ __forceinline__ CtaTable build_cta_table(uint32_t* s_keys, uint32_t* 
         for (uint32_t k = threadIdx.x; k < (1u << t.bits); k += kWedgeThreads) s_keys[k] = kEmptyKey;
         __syncthreads();
         for (uint32_t k = threadIdx.x; k < d; k += kWedgeThreads)
-            hash_insert<kPos>(s_keys, pos, t.bits, t.values[s + k], k);
+            hash_insert(s_keys, t.bits, t.values[s + k]);
         __syncthreads();
         return t;
     }
@@ -204,20 +194,17 @@ __device__ __forceinline__ CtaTable build_cta_table(uint32_t* s_keys, uint32_t* 
     return t;
 }
 
-// Position of the probed value w in the owner's list (kNotFound if absent; 0
-// for any hit in a bitmap, which keeps no positions).
-template <bool kPos>
-__device__ __forceinline__ uint32_t cta_find(const CtaTable& t, const uint32_t* s_keys, const uint32_t* pos,
-                                             const uint32_t* sorted_list, uint32_t d, uint32_t w) {
+// kNotFound unless the probed value w is in the owner's list.
+__device__ __forceinline__ uint32_t cta_find(const CtaTable& t, const uint32_t* s_keys, const uint32_t* sorted_list,
+                                             uint32_t d, uint32_t w) {
     if (t.kind == kBitmap) return (w < t.limit && ((s_keys[w >> 5] >> (w & 31)) & 1u)) ? 0u : kNotFound;
-    if (t.kind == kHash) return hash_find<kPos>(s_keys, pos, t.bits, w);
+    if (t.kind == kHash) return hash_find(s_keys, t.bits, w);
     return sorted_find(sorted_list, d, w);
 }
 
 // A Sink receives every triangle: hit(row_base, pos_v, pos_w, entry_vw) with
 // row_base = offsets[u] (so row_base + pos_v is the entry u -> v) and
-// finish() once per thread at the end. Sink::kNeedsPos says whether the hash
-// table has to keep the positions of the keys.
+// finish() once per thread at the end.
 
 // Warp per vertex for out-lists of [min_deg, kWarpMaxDeg] entries; vertices
 // are handed out dynamically kVertexBatch at a time.
@@ -226,14 +213,11 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_warp_kernel(const uint32_
                                                                    const uint32_t* __restrict__ targets, uint32_t V,
                                                                    uint32_t min_deg, uint32_t* __restrict__ next_vertex,
                                                                    Sink sink) {
-    constexpr bool kPos = Sink::kNeedsPos;
     __shared__ uint32_t s_keys[kWedgeWarps][kWarpSlots];
-    __shared__ uint32_t s_pos[kPos ? kWedgeWarps : 1][kPos ? kWarpSlots : 1];
     __shared__ uint32_t s_excl[kWedgeWarps][33];
     __shared__ uint32_t s_start[kWedgeWarps][32];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     uint32_t* keys = s_keys[warp];
-    uint32_t* pos = kPos ? s_pos[warp] : nullptr;
     while (true) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(next_vertex, kVertexBatch);
@@ -247,12 +231,12 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_warp_kernel(const uint32_
             __syncwarp();
             for (uint32_t k = lane; k < (1u << bits); k += 32) keys[k] = kEmptyKey;
             __syncwarp();
-            for (uint32_t k = lane; k < du; k += 32) hash_insert<kPos>(keys, pos, bits, targets[s + k], k);
+            for (uint32_t k = lane; k < du; k += 32) hash_insert(keys, bits, targets[s + k]);
             __syncwarp();
             for (uint32_t c = 0; c < du; c += 32)
                 wedge_chunk(
                     offsets, targets, targets + s, du, c, s_excl[warp], s_start[warp], 0xFFFFFFFFu,
-                    [&](uint32_t w) { return hash_find<kPos>(keys, pos, bits, w); },
+                    [&](uint32_t w) { return hash_find(keys, bits, w); },
                     [&](uint32_t pv, uint32_t pw, uint32_t evw) { sink.hit(s, pv, pw, evw); });
         }
     }
@@ -277,15 +261,12 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_cta_kernel(const uint32_t
                                                                   const uint32_t* __restrict__ long_list,
                                                                   const uint32_t* __restrict__ long_count,
                                                                   uint32_t* __restrict__ next_item, Sink sink) {
-    constexpr bool kPos = Sink::kNeedsPos;
     __shared__ uint32_t s_keys[kCtaSlots];
-    __shared__ uint32_t s_pos[kPos ? kCtaSlots : 1];
     __shared__ uint32_t s_excl[kWedgeWarps][33];
     __shared__ uint32_t s_start[kWedgeWarps][32];
     __shared__ uint32_t s_item, s_chunk;
     const unsigned warp = threadIdx.x >> 5;
     const uint32_t n = *long_count;
-    uint32_t* pos = kPos ? s_pos : nullptr;
     while (true) {
         if (threadIdx.x == 0) {
             s_item = atomicAdd(next_item, 1u);
@@ -302,14 +283,14 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_cta_kernel(const uint32_t
         if (use_table) {
             for (uint32_t k = threadIdx.x; k < (1u << bits); k += kWedgeThreads) s_keys[k] = kEmptyKey;
             __syncthreads();
-            for (uint32_t k = threadIdx.x; k < du; k += kWedgeThreads) hash_insert<kPos>(s_keys, pos, bits, list[k], k);
+            for (uint32_t k = threadIdx.x; k < du; k += kWedgeThreads) hash_insert(s_keys, bits, list[k]);
             __syncthreads();
         }
         for (uint32_t c = next_chunk(&s_chunk); c < du; c = next_chunk(&s_chunk))
             wedge_chunk(
                 offsets, targets, list, du, c, s_excl[warp], s_start[warp], 0xFFFFFFFFu,
                 [&](uint32_t w) {
-                    return use_table ? hash_find<kPos>(s_keys, pos, bits, w) : sorted_find(list, du, w);
+                    return use_table ? hash_find(s_keys, bits, w) : sorted_find(list, du, w);
                 },
                 [&](uint32_t pv, uint32_t pw, uint32_t evw) { sink.hit(s, pv, pw, evw); });
         __syncthreads();  // the table and s_item are reused by the next list
@@ -336,14 +317,11 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_warp_list_kernel(const ui
                                                                         const uint32_t* __restrict__ list, uint32_t n,
                                                                         uint32_t* __restrict__ next, bool split,
                                                                         Sink sink) {
-    constexpr bool kPos = Sink::kNeedsPos;
     __shared__ uint32_t s_keys[kWedgeWarps][kWarpSlots];
-    __shared__ uint32_t s_pos[kPos ? kWedgeWarps : 1][kPos ? kWarpSlots : 1];
     __shared__ uint32_t s_excl[kWedgeWarps][33];
     __shared__ uint32_t s_start[kWedgeWarps][32];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     uint32_t* keys = s_keys[warp];
-    uint32_t* pos = kPos ? s_pos[warp] : nullptr;
     while (true) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(next, kVertexBatch);
@@ -359,7 +337,7 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_warp_list_kernel(const ui
             if (use_table) {
                 for (uint32_t k = lane; k < (1u << bits); k += 32) keys[k] = kEmptyKey;
                 __syncwarp();
-                for (uint32_t k = lane; k < du; k += 32) hash_insert<kPos>(keys, pos, bits, targets[s + k], k);
+                for (uint32_t k = lane; k < du; k += 32) hash_insert(keys, bits, targets[s + k]);
                 __syncwarp();
             }
             const uint32_t* ulist = targets + s;
@@ -368,7 +346,7 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_warp_list_kernel(const ui
                 wedge_chunk(
                     offsets, targets, ulist, du, c, s_excl[warp], s_start[warp], max_dv,
                     [&](uint32_t w) {
-                        return use_table ? hash_find<kPos>(keys, pos, bits, w) : sorted_find(ulist, du, w);
+                        return use_table ? hash_find(keys, bits, w) : sorted_find(ulist, du, w);
                     },
                     [&](uint32_t pv, uint32_t pw, uint32_t evw) { sink.hit(s, pv, pw, evw); });
             sink.end_vertex(u);
@@ -388,14 +366,11 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_cta_list_kernel(const uin
                                                                        uint32_t* __restrict__ next, int search,
                                                                        bool split, const uint32_t* __restrict__ rank,
                                                                        const uint32_t* __restrict__ vrank, Sink sink) {
-    constexpr bool kPos = Sink::kNeedsPos;
     __shared__ uint32_t s_keys[kCtaSlots];
-    __shared__ uint32_t s_pos[kPos ? kCtaSlots : 1];
     __shared__ uint32_t s_excl[kWedgeWarps][33];
     __shared__ uint32_t s_start[kWedgeWarps][32];
     __shared__ uint32_t s_item, s_chunk;
     const unsigned warp = threadIdx.x >> 5;
-    uint32_t* pos = kPos ? s_pos : nullptr;
     while (true) {
         if (threadIdx.x == 0) {
             s_item = atomicAdd(next, 1u);
@@ -407,12 +382,12 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_cta_list_kernel(const uin
         const uint32_t u = list[h];
         const uint32_t s = offsets[u], du = offsets[u + 1] - s;
         const uint32_t* ulist = targets + s;
-        const CtaTable tab = build_cta_table<kPos>(s_keys, pos, targets, rank, vrank, u, s, du, search);
+        const CtaTable tab = build_cta_table(s_keys, targets, rank, vrank, u, s, du, search);
         const uint32_t max_dv = split && du >= 2 ? du : 0xFFFFFFFFu;
         for (uint32_t c = next_chunk(&s_chunk); c < du; c = next_chunk(&s_chunk))
             wedge_chunk(
                 offsets, tab.values, ulist, du, c, s_excl[warp], s_start[warp], max_dv,
-                [&](uint32_t w) { return cta_find<kPos>(tab, s_keys, pos, ulist, du, w); },
+                [&](uint32_t w) { return cta_find(tab, s_keys, ulist, du, w); },
                 [&](uint32_t pv, uint32_t pw, uint32_t evw) { sink.hit(s, pv, pw, evw); });
         sink.end_vertex(u);
         __syncthreads();  // the table and s_item are reused by the next list
@@ -466,7 +441,7 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_head_warp_kernel(
             if (use_table) {
                 for (uint32_t k = lane; k < (1u << bits); k += 32) keys[k] = kEmptyKey;
                 __syncwarp();
-                for (uint32_t k = lane; k < dv; k += 32) hash_insert<false>(keys, nullptr, bits, vlist[k], k);
+                for (uint32_t k = lane; k < dv; k += 32) hash_insert(keys, bits, vlist[k]);
                 __syncwarp();
             }
             const uint32_t* tails;
@@ -476,7 +451,7 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_head_warp_kernel(
                 wedge_chunk(
                     offsets, targets, tails, count, c, s_excl[warp], s_start[warp], 0xFFFFFFFFu,
                     [&](uint32_t w) {
-                        return use_table ? hash_find<false>(keys, nullptr, bits, w) : sorted_find(vlist, dv, w);
+                        return use_table ? hash_find(keys, bits, w) : sorted_find(vlist, dv, w);
                     },
                     [&](uint32_t pu, uint32_t pw, uint32_t e) { sink.hit(s, pu, pw, e); });
         }
@@ -507,40 +482,18 @@ __global__ void __launch_bounds__(kWedgeThreads) wedge_head_cta_kernel(
         const uint2 item = items[h];
         const uint32_t s = offsets[item.x], dv = offsets[item.x + 1] - s;
         const uint32_t* vlist = targets + s;
-        const CtaTable tab = build_cta_table<false>(s_keys, nullptr, targets, rank, vrank, item.x, s, dv, search);
+        const CtaTable tab = build_cta_table(s_keys, targets, rank, vrank, item.x, s, dv, search);
         const uint32_t* tails;
         uint32_t count;
         head_slice(item, in_off, in_src, kHeadCtaSlice, tails, count);
         for (uint32_t c = next_chunk(&s_chunk); c < count; c = next_chunk(&s_chunk))
             wedge_chunk(
                 offsets, tab.values, tails, count, c, s_excl[warp], s_start[warp], 0xFFFFFFFFu,
-                [&](uint32_t w) { return cta_find<false>(tab, s_keys, nullptr, vlist, dv, w); },
+                [&](uint32_t w) { return cta_find(tab, s_keys, vlist, dv, w); },
                 [&](uint32_t pu, uint32_t pw, uint32_t e) { sink.hit(s, pu, pw, e); });
         __syncthreads();  // the table and s_item are reused by the next item
     }
     sink.finish();
-}
-
-// Runs both wedge kernels over a DAG CSR: long out-lists by CTAs first (they
-// hold the heaviest work), then everything else by warps.
-template <class Sink>
-Error run_wedges(DeviceImpl& dev, const uint32_t* d_offsets, const uint32_t* d_targets, uint32_t V, uint32_t min_deg,
-                 Sink sink, const char* tag) {
-    (void)tag;
-    // scratch: [0] next vertex, [1] long-list count, [2] next long list, then the long lists
-    DeviceBuffer<uint32_t> scratch;
-    GCU_TRY(scratch.allocate(dev, 4 + static_cast<uint64_t>(V)));
-    GCU_CUDA(cudaMemsetAsync(scratch.ptr, 0, 4 * sizeof(uint32_t), dev.stream), "memset");
-    const unsigned grid = static_cast<unsigned>(dev.sm_count) * 8;
-    const unsigned collect_blocks =
-        static_cast<unsigned>(std::min<uint64_t>(ceil_div_u64(V, 256), static_cast<uint64_t>(dev.sm_count) * 8));
-    GCU_LAUNCH(dev, "wedge_collect_long", wedge_collect_long_kernel, collect_blocks, 256, 0, d_offsets, V,
-               scratch.ptr + 4, scratch.ptr + 1);
-    GCU_LAUNCH(dev, "wedge_cta", wedge_cta_kernel<Sink>, grid, kWedgeThreads, 0, d_offsets, d_targets,
-               scratch.ptr + 4, scratch.ptr + 1, scratch.ptr + 2, sink);
-    GCU_LAUNCH(dev, "wedge_warp", wedge_warp_kernel<Sink>, grid, kWedgeThreads, 0, d_offsets, d_targets, V, min_deg,
-               scratch.ptr, sink);
-    return ok();
 }
 
 }  // namespace gcu
