@@ -7,9 +7,9 @@
 // from_edge_pairs_oriented (:299-350: undirected dedup without self-loops,
 // each edge oriented from the lower (degree, id) end, sort). Keys are
 // (source << 32) | target; the stable LSD radix sort of sort.cu runs over the
-// bits the ids actually use, the target bits first and the source bits second
-// (two digit runs of one LSD sort). Deduplication and the row pointers come
-// from one scan over "key differs from its predecessor" flags.
+// bits the ids actually use, the target bits first and the source bits second.
+// Deduplication and the row pointers come from a scan of the keys that differ
+// from their predecessor.
 //
 // The generators (R-MAT, Erdos-Renyi, 2D grid with edge dropout, random
 // geometric, Watts-Strogatz) append their keys straight into the key buffer
@@ -72,6 +72,21 @@ __device__ __forceinline__ void append_undirected(unsigned long long* count, uin
     }
 }
 
+// Exclusive scan in place, from `first`, of at most 64 counts in shared memory,
+// by one warp; the sum of the counts to every lane.
+template <int kCounts>
+__device__ __forceinline__ uint32_t scan_counts(uint32_t* c, uint32_t first) {
+    static_assert(kCounts <= 64 && kCounts % 2 == 0, "two counts per lane");
+    const unsigned at = 2 * lane_id();
+    const uint32_t c0 = at < kCounts ? c[at] : 0u, c1 = at < kCounts ? c[at + 1] : 0u;
+    const uint32_t upto = warp_inclusive_scan(c0 + c1);
+    if (at < kCounts) {
+        c[at] = first + upto - c0 - c1;
+        c[at + 1] = first + upto - c1;
+    }
+    return __shfl_sync(kFullMask, upto, 31);
+}
+
 // Grid-stride loop whose trip count is the same for the 32 lanes of a warp
 // (the warp-wide helpers above need every lane).
 #define GCU_WARP_UNIFORM_LOOP(i, n)                                                                            \
@@ -84,44 +99,66 @@ enum PairMode : int { kDirected = 0, kSymmetric = 1, kUndirected = 2 };
 // per pair, kSymmetric the reverse too (a self-loop once), kUndirected
 // (min, max) without self-loops. Records the first pair whose source (or,
 // unless kDirected, target) is >= num_nodes, and the largest target.
-__global__ void __launch_bounds__(kBuildThreads) pairs_to_keys_kernel(const uint32_t* __restrict__ pairs,
+//
+// A block takes tiles of kPairLoads pairs per thread and one place in the key
+// buffer per tile: an atomic per warp step was what bounded it (16.7 M pairs:
+// 378 us, now 69).
+constexpr int kPairLoads = 8;
+__global__ void __launch_bounds__(kBuildThreads) pairs_to_keys_kernel(const uint2* __restrict__ pairs,
                                                                       uint64_t n_pairs, uint32_t num_nodes, int mode,
                                                                       uint64_t* __restrict__ keys,
                                                                       unsigned long long* __restrict__ count,
                                                                       unsigned long long* __restrict__ first_bad,
                                                                       unsigned* __restrict__ max_target) {
+    __shared__ uint32_t s_count[kPairLoads][kBuildThreads / 32];
+    __shared__ unsigned long long s_base;
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5, below = (1u << lane) - 1;
+    constexpr uint32_t kTile = kPairLoads * kBuildThreads;
     uint32_t local_max = 0;
-    GCU_WARP_UNIFORM_LOOP(i, n_pairs) {
-        const bool valid = i < n_pairs;
-        uint32_t s = 0, d = 0;
-        if (valid) {
-            s = pairs[2 * i];
-            d = pairs[2 * i + 1];
+    for (uint64_t i0 = static_cast<uint64_t>(blockIdx.x) * kTile; i0 < n_pairs;
+         i0 += static_cast<uint64_t>(gridDim.x) * kTile) {
+        uint2 p[kPairLoads];
+#pragma unroll
+        for (int q = 0; q < kPairLoads; ++q) {
+            const uint64_t i = i0 + q * kBuildThreads + threadIdx.x;
+            p[q] = i < n_pairs ? __ldg(pairs + i) : make_uint2(0u, 0u);
         }
-        const bool bad = valid && (s >= num_nodes || (mode != kDirected && d >= num_nodes));
-        if (bad) atomicMin(first_bad, static_cast<unsigned long long>(i));
-        uint32_t want = 0;
-        if (valid && !bad) {
-            if (mode == kDirected)
-                want = 1;
-            else if (mode == kSymmetric)
-                want = s == d ? 1 : 2;
-            else
-                want = s == d ? 0 : 1;
-            local_max = max(local_max, d);
+        unsigned one[kPairLoads], two[kPairLoads];  // lanes with a key, with a second key
+#pragma unroll
+        for (int q = 0; q < kPairLoads; ++q) {
+            const uint64_t i = i0 + q * kBuildThreads + threadIdx.x;
+            const uint32_t s = p[q].x, d = p[q].y;
+            const bool valid = i < n_pairs;
+            const bool bad = valid && (s >= num_nodes || (mode != kDirected && d >= num_nodes));
+            if (bad) atomicMin(first_bad, static_cast<unsigned long long>(i));
+            const bool keep = valid && !bad;
+            if (keep) local_max = max(local_max, d);
+            one[q] = __ballot_sync(kFullMask, keep && !(mode == kUndirected && s == d));
+            two[q] = __ballot_sync(kFullMask, keep && mode == kSymmetric && s != d);
+            if (lane == 0) s_count[q][warp] = __popc(one[q]) + __popc(two[q]);
         }
-        const unsigned long long slot = warp_append(count, want);
-        if (want) {
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t total = scan_counts<kPairLoads * kBuildThreads / 32>(&s_count[0][0], 0);
+            if (lane == 0) s_base = total ? atomicAdd(count, static_cast<unsigned long long>(total)) : 0ull;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kPairLoads; ++q) {
+            if (!((one[q] >> lane) & 1u)) continue;
+            const uint32_t s = p[q].x, d = p[q].y;
+            const unsigned long long slot = s_base + s_count[q][warp] + __popc(one[q] & below) + __popc(two[q] & below);
             if (mode == kUndirected) {
                 keys[slot] = key_of(min(s, d), max(s, d));
             } else {
                 keys[slot] = key_of(s, d);
-                if (want == 2) keys[slot + 1] = key_of(d, s);
+                if ((two[q] >> lane) & 1u) keys[slot + 1] = key_of(d, s);
             }
         }
+        __syncthreads();  // s_count and s_base are the next tile's
     }
     local_max = __reduce_max_sync(kFullMask, local_max);
-    if (lane_id() == 0 && local_max) atomicMax(max_target, local_max);
+    if (lane == 0 && local_max) atomicMax(max_target, local_max);
 }
 
 // R-MAT pairs as host_csr.cpp generate_rmat draws them: `scale` quadrant
@@ -290,19 +327,92 @@ __global__ void mark_first_kernel(const uint64_t* __restrict__ keys, uint64_t n,
         flags[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1u : 0u;
 }
 
-// Unique keys -> targets at their scanned positions; rows s_prev < r <= s
-// (s_prev = source of key i - 1, s = source of key i, or num_nodes past the
-// end) start at pos[i]. Every row gets exactly one writer.
-__global__ void keys_to_csr_kernel(const uint64_t* __restrict__ keys, uint64_t n, const uint32_t* __restrict__ pos,
-                                   uint32_t num_nodes, uint32_t* __restrict__ offsets,
-                                   uint32_t* __restrict__ targets) {
-    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i <= n;
-         i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const int64_t prev = i == 0 ? -1 : static_cast<int64_t>(keys[i - 1] >> 32);
-        const int64_t cur = i < n ? static_cast<int64_t>(keys[i] >> 32) : static_cast<int64_t>(num_nodes);
-        const uint32_t p = pos[i];
-        if (i < n && (i == 0 || keys[i] != keys[i - 1])) targets[p] = static_cast<uint32_t>(keys[i]);
-        for (int64_t r = prev + 1; r <= cur; ++r) offsets[r] = p;
+// firsts[t] = keys of tile t that differ from their predecessor.
+// kLoads keys per thread: kCsrLoads, or one where that leaves SMs without a tile.
+constexpr int kCsrLoads = 8;
+constexpr uint32_t kManyRows = 64;  // without a key, in a run: written by the warp
+
+template <int kLoads>
+__global__ void __launch_bounds__(kBuildThreads) count_first_kernel(const uint64_t* __restrict__ keys, uint64_t n,
+                                                                    uint32_t* __restrict__ firsts) {
+    constexpr uint32_t kTile = kBuildThreads * kLoads;
+    __shared__ uint32_t scratch[32];
+    for (uint64_t t = blockIdx.x; t * kTile < n; t += gridDim.x) {
+        uint64_t key[kLoads], before[kLoads];
+#pragma unroll
+        for (int q = 0; q < kLoads; ++q) {
+            const uint64_t i = t * kTile + q * kBuildThreads + threadIdx.x;
+            key[q] = i < n ? __ldg(keys + i) : 0;
+            before[q] = i <= n && i > 0 ? __ldg(keys + i - 1) : ~key[q];
+        }
+        uint32_t mine = 0;
+#pragma unroll
+        for (int q = 0; q < kLoads; ++q) {
+            const uint64_t i = t * kTile + q * kBuildThreads + threadIdx.x;
+            mine += i < n && key[q] != before[q] ? 1u : 0u;
+        }
+        const uint32_t sum = block_sum(mine, scratch);
+        if (threadIdx.x == 0) firsts[t] = sum;
+    }
+}
+
+// Unique keys -> targets, in order, from each tile's first position; rows
+// s_prev < r <= s (s_prev = source of key i - 1, s = source of key i, or
+// num_nodes past the end) start at the position of key i. Every row gets exactly
+// one writer. Reading the sorted keys twice, here and in the count, moves half
+// the bytes that a position per key did (31 M keys: 221 us for both, 373 with
+// flags, their scan and the positions). The key before comes from the L1: a
+// shuffle waits for the load (10 us more in either kernel).
+template <int kLoads>
+__global__ void __launch_bounds__(kBuildThreads) keys_to_csr_kernel(const uint64_t* __restrict__ keys, uint64_t n,
+                                                                    const uint32_t* __restrict__ tile_pos,
+                                                                    uint32_t num_nodes,
+                                                                    uint32_t* __restrict__ offsets,
+                                                                    uint32_t* __restrict__ targets) {
+    constexpr uint32_t kTile = kBuildThreads * kLoads;
+    __shared__ uint32_t s_count[kLoads][kBuildThreads / 32];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    // Tile t takes keys [t * kTile, ...) and, past the last key, index n.
+    for (uint64_t t = blockIdx.x; t * kTile <= n; t += gridDim.x) {
+        uint64_t key[kLoads], before[kLoads];
+#pragma unroll
+        for (int q = 0; q < kLoads; ++q) {
+            const uint64_t i = t * kTile + q * kBuildThreads + threadIdx.x;
+            key[q] = i < n ? __ldg(keys + i) : 0;
+            before[q] = i <= n && i > 0 ? __ldg(keys + i - 1) : ~key[q];
+        }
+        unsigned first[kLoads];
+#pragma unroll
+        for (int q = 0; q < kLoads; ++q) {
+            const uint64_t i = t * kTile + q * kBuildThreads + threadIdx.x;
+            first[q] = __ballot_sync(kFullMask, i < n && key[q] != before[q]);
+            if (lane == 0) s_count[q][warp] = __popc(first[q]);
+        }
+        __syncthreads();
+        if (warp == 0) scan_counts<kLoads * kBuildThreads / 32>(&s_count[0][0], __ldg(tile_pos + t));
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kLoads; ++q) {
+            const uint32_t p = s_count[q][warp] + __popc(first[q] & ((1u << lane) - 1));
+            const uint64_t i = t * kTile + q * kBuildThreads + threadIdx.x;
+            if ((first[q] >> lane) & 1u) targets[p] = static_cast<uint32_t>(key[q]);
+            // Rows [r0, r1), by the warp where they are many.
+            uint64_t r0 = 0, r1 = 0;
+            if (i <= n) {
+                r0 = i == 0 ? 0 : (before[q] >> 32) + 1;
+                r1 = (i < n ? key[q] >> 32 : static_cast<uint64_t>(num_nodes)) + 1;
+            }
+            const bool many = r1 > r0 + kManyRows;
+            if (!many)
+                for (uint64_t r = r0; r < r1; ++r) offsets[r] = p;
+            for (unsigned todo = __ballot_sync(kFullMask, many); todo; todo &= todo - 1) {
+                const int l = __ffs(todo) - 1;
+                const uint64_t end = __shfl_sync(kFullMask, r1, l);
+                const uint32_t at_row = __shfl_sync(kFullMask, p, l);
+                for (uint64_t r = __shfl_sync(kFullMask, r0, l) + lane; r < end; r += 32) offsets[r] = at_row;
+            }
+        }
+        __syncthreads();  // s_count is the next tile's
     }
 }
 
@@ -376,33 +486,38 @@ struct KeyScratch {
 // [32, 32 + source_bits); *sorted is whichever buffer holds the result.
 Error sort_keys(DeviceImpl& dev, uint64_t* keys, uint64_t* tmp, uint64_t n, uint32_t target_bits,
                 uint32_t source_bits, uint64_t** sorted, uint64_t** other) {
-    uint64_t* s1 = nullptr;
-    GCU_TRY(radix_sort_u64(dev, keys, tmp, n, 0, target_bits, &s1));
-    uint64_t* o1 = s1 == keys ? tmp : keys;
-    uint64_t* s2 = nullptr;
-    GCU_TRY(radix_sort_u64(dev, s1, o1, n, 32, 32 + source_bits, &s2));
-    *sorted = s2;
-    *other = s2 == s1 ? o1 : s1;
+    GCU_TRY(radix_sort_pairs(dev, keys, tmp, n, target_bits, source_bits, sorted));
+    *other = *sorted == keys ? tmp : keys;
     return ok();
 }
 
-// CSR of the sorted keys (repeats dropped) into a new graph's buffers.
-Error csr_from_sorted_keys(DeviceImpl& dev, const uint64_t* sorted, uint64_t n, uint32_t num_nodes, GraphImpl& g) {
+template <int kLoads>
+Error fill_csr(DeviceImpl& dev, const uint64_t* sorted, uint64_t n, uint32_t num_nodes, GraphImpl& g) {
+    // Positions of the tiles' first unique keys; [tiles] = unique keys.
+    const uint64_t tiles = ceil_div_u64(n, kBuildThreads * kLoads);
     DeviceBuffer<uint32_t> pos;
-    GCU_TRY(pos.allocate(dev, n + 1));
-    GCU_LAUNCH(dev, "build_mark_first", mark_first_kernel, grid_for(dev, n), kBuildThreads, 0, sorted, n, pos.ptr);
-    GCU_TRY(exclusive_scan_u32(dev, pos.ptr, pos.ptr, n));
+    GCU_TRY(pos.allocate(dev, tiles + 1));
+    const unsigned grid = static_cast<unsigned>(
+        std::max<uint64_t>(1, std::min<uint64_t>(tiles + 1, static_cast<uint64_t>(dev.sm_count) * 8)));
+    GCU_LAUNCH(dev, "build_count_first", count_first_kernel<kLoads>, grid, kBuildThreads, 0, sorted, n, pos.ptr);
+    GCU_TRY(exclusive_scan_u32(dev, pos.ptr, pos.ptr, tiles));
     uint32_t total = 0;
-    GCU_CUDA(cudaMemcpyAsync(&total, pos.ptr + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
+    GCU_CUDA(cudaMemcpyAsync(&total, pos.ptr + tiles, sizeof(uint32_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
     GCU_TRY(dev.sync());
     g.num_nodes = num_nodes;
     g.num_edges = total;
     GCU_TRY(g.offsets.allocate(dev, static_cast<uint64_t>(num_nodes) + 1));
     GCU_TRY(g.targets.allocate(dev, total));
-    GCU_LAUNCH(dev, "build_keys_to_csr", keys_to_csr_kernel, grid_for(dev, n + 1), kBuildThreads, 0, sorted, n,
-               pos.ptr, num_nodes, g.offsets.ptr, g.targets.ptr);
+    GCU_LAUNCH(dev, "build_keys_to_csr", keys_to_csr_kernel<kLoads>, grid, kBuildThreads, 0, sorted, n, pos.ptr, num_nodes,
+               g.offsets.ptr, g.targets.ptr);
     GCU_TRY(dev.sync());  // scratch is freed on return
     return ok();
+}
+
+// CSR of the sorted keys (repeats dropped) into a new graph's buffers.
+Error csr_from_sorted_keys(DeviceImpl& dev, const uint64_t* sorted, uint64_t n, uint32_t num_nodes, GraphImpl& g) {
+    const uint64_t wide = static_cast<uint64_t>(dev.sm_count) * kBuildThreads * kCsrLoads;
+    return n < wide ? fill_csr<1>(dev, sorted, n, num_nodes, g) : fill_csr<kCsrLoads>(dev, sorted, n, num_nodes, g);
 }
 
 Error check_capacity(uint64_t keys) {
@@ -423,7 +538,8 @@ Error build_graph_from_pairs(DeviceImpl& dev, const uint32_t* host_pairs, uint64
     GCU_TRY(copy_to_device(dev, d_pairs.ptr, host_pairs, 8 * n_pairs, dev.stream));
     KeyScratch ks;
     GCU_TRY(ks.allocate(dev, capacity));
-    GCU_LAUNCH(dev, "build_pairs_to_keys", pairs_to_keys_kernel, grid_for(dev, n_pairs), kBuildThreads, 0, d_pairs.ptr,
+    GCU_LAUNCH(dev, "build_pairs_to_keys", pairs_to_keys_kernel, grid_for(dev, ceil_div_u64(n_pairs, kPairLoads)),
+               kBuildThreads, 0, reinterpret_cast<const uint2*>(d_pairs.ptr),
                n_pairs, num_nodes, mode, ks.keys.ptr, ks.meta.ptr, ks.meta.ptr + 1, ks.max_target.ptr);
     uint64_t count = 0, bad = 0;
     uint32_t maxt = 0;

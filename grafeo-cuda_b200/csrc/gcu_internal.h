@@ -329,6 +329,9 @@ uint64_t scan_device_n_tiles(uint64_t max_n);
 // pass, ping-ponging between keys and tmp; *sorted is whichever holds the result.
 Error radix_sort_u64(DeviceImpl& dev, uint64_t* keys, uint64_t* tmp, uint64_t n, uint32_t low_bit, uint32_t high_bit,
                      uint64_t** sorted);
+// The same by bits [0, low_bits) and then [32, 32 + high_bits).
+Error radix_sort_pairs(DeviceImpl& dev, uint64_t* keys, uint64_t* tmp, uint64_t n, uint32_t low_bits,
+                       uint32_t high_bits, uint64_t** sorted);
 
 // In-lists of a CSR (the transpose), every in-list ordered by source.
 Error transpose_csr(DeviceImpl& dev, const uint32_t* offsets, const uint32_t* targets, uint32_t V, uint32_t E,
