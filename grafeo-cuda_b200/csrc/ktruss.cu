@@ -359,6 +359,14 @@ __global__ void __launch_bounds__(256) kt_live_fill_kernel(const LiveCsr lv, uin
 struct LiveBuffers {
     DeviceBuffer<uint32_t> offsets, targets, eid;
     uint32_t entries = 0;
+    // Dense form (live_matrix): the vertices with entries numbered in order, and
+    // a row of neighbour bits for each.
+    DeviceBuffer<uint32_t> number;   // of every vertex
+    DeviceBuffer<uint32_t> bits;     // n_rows x words
+    DeviceBuffer<uint16_t> before;   // bits of the row in the words before
+    DeviceBuffer<ushort2> span;      // the row's words [x, y) hold all its bits
+    DeviceBuffer<uint16_t> numbers;  // of the live entries' vertices
+    uint32_t words = 0;              // 0: not built
 };
 
 static Error compact_live(DeviceImpl& dev, uint32_t V, const LiveCsr& lv, uint32_t L, const uint32_t* rev,
@@ -384,6 +392,94 @@ static Error compact_live(DeviceImpl& dev, uint32_t V, const LiveCsr& lv, uint32
         GCU_LAUNCH(dev, "kt_live_fill", kt_live_fill_kernel, tiles, 256, 0, lv, V, L, rev, pos.ptr, out->targets.ptr,
                    out->eid.ptr);
     GCU_TRY(dev.sync());  // pos is freed on return
+    return ok();
+}
+
+// Number and row bit of every live entry.
+__global__ void __launch_bounds__(256) kt_matrix_bits_kernel(const uint32_t* __restrict__ offsets,
+                                                             const uint32_t* __restrict__ targets, uint32_t V,
+                                                             uint32_t L, const uint32_t* __restrict__ number,
+                                                             uint32_t words, uint16_t* __restrict__ numbers,
+                                                             uint32_t* __restrict__ bits) {
+    for_each_entry<256, 4>(offsets, V, L, [&](uint32_t p, uint32_t u) {
+        const uint32_t w = number[targets[p]];
+        numbers[p] = static_cast<uint16_t>(w);
+        atomicOr(bits + static_cast<uint64_t>(number[u]) * words + (w >> 5), 1u << (w & 31));
+    });
+}
+
+// A warp per row: the bits before each word, and the words between its first
+// and last bits.
+__global__ void __launch_bounds__(256) kt_matrix_before_kernel(const uint32_t* __restrict__ bits, uint32_t rows,
+                                                               uint32_t words, uint16_t* __restrict__ before,
+                                                               ushort2* __restrict__ span) {
+    const unsigned lane = lane_id();
+    for (uint64_t r = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < rows;
+         r += (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5) {
+        uint32_t total = 0, first = words, last = 0;
+        for (uint32_t j0 = 0; j0 < words; j0 += 32) {
+            const uint32_t j = j0 + lane;
+            const uint32_t n = j < words ? __popc(bits[r * words + j]) : 0u;
+            const uint32_t upto = warp_inclusive_scan(n);
+            if (j < words) before[r * words + j] = static_cast<uint16_t>(total + upto - n);
+            if (n) {
+                first = min(first, j);
+                last = j + 1;
+            }
+            total += __shfl_sync(kFullMask, upto, 31);
+        }
+        first = __reduce_min_sync(kFullMask, first);
+        last = __reduce_max_sync(kFullMask, last);
+        if (lane == 0) span[r] = make_ushort2(static_cast<uint16_t>(first), static_cast<uint16_t>(last));
+    }
+}
+
+__global__ void kt_has_entries_kernel(const uint32_t* __restrict__ offsets, uint32_t V, uint32_t* __restrict__ has) {
+    for (uint64_t u = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; u < V;
+         u += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+        has[u] = offsets[u + 1] > offsets[u] ? 1u : 0u;
+}
+
+// The dense form of the live lists, where intersecting two rows' words is less
+// work than searching: W words of two rows are 2 W / 32 coalesced loads of a
+// warp, d entries searched in a list of their kind d / 32 walks of 10 or more
+// dependent, scattered ones. Left out (words = 0) for more vertices than 16-bit
+// positions allow, for rows of more than kDenseWords words per live neighbour,
+// and where there is no memory for it.
+constexpr uint32_t kDenseRows = 65535;
+constexpr uint32_t kDenseWords = 8;
+
+static Error live_matrix(DeviceImpl& dev, uint32_t V, LiveBuffers* lv) {
+    lv->words = 0;
+    if (lv->entries == 0) return ok();
+    const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
+    GCU_TRY(lv->number.allocate(dev, static_cast<uint64_t>(V) + 1));
+    GCU_LAUNCH(dev, "kt_has_entries", kt_has_entries_kernel,
+               static_cast<unsigned>(std::min<uint64_t>(ceil_div_u64(V, 256), cap)), 256, 0, lv->offsets.ptr, V,
+               lv->number.ptr);
+    GCU_TRY(exclusive_scan_u32(dev, lv->number.ptr, lv->number.ptr, V));
+    uint32_t rows = 0;
+    GCU_CUDA(cudaMemcpyAsync(&rows, lv->number.ptr + V, sizeof(uint32_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
+    GCU_TRY(dev.sync());
+    const uint32_t words = static_cast<uint32_t>(ceil_div_u64(rows, 32));
+    if (rows > kDenseRows || static_cast<uint64_t>(words) * rows > static_cast<uint64_t>(kDenseWords) * lv->entries)
+        return ok();
+    const uint64_t all = static_cast<uint64_t>(rows) * words;
+    if (!lv->bits.allocate(dev, all).ok() || !lv->before.allocate(dev, all).ok() ||
+        !lv->span.allocate(dev, rows).ok() || !lv->numbers.allocate(dev, lv->entries).ok()) {
+        lv->bits.reset();
+        lv->before.reset();
+        return ok();
+    }
+    GCU_CUDA(cudaMemsetAsync(lv->bits.ptr, 0, sizeof(uint32_t) * all, dev.stream), "memset");
+    GCU_LAUNCH(dev, "kt_matrix_bits", kt_matrix_bits_kernel,
+               static_cast<unsigned>(std::min<uint64_t>(ceil_div_u64(lv->entries, 1024), cap)), 256, 0,
+               lv->offsets.ptr, lv->targets.ptr, V, lv->entries, lv->number.ptr, words,
+               lv->numbers.ptr, lv->bits.ptr);
+    GCU_LAUNCH(dev, "kt_matrix_before", kt_matrix_before_kernel,
+               static_cast<unsigned>(std::min<uint64_t>(ceil_div_u64(rows, 8), cap)), 256, 0, lv->bits.ptr, rows,
+               words, lv->before.ptr, lv->span.ptr);
+    lv->words = words;
     return ok();
 }
 
@@ -647,6 +743,12 @@ struct TrussLoop {
     const uint32_t* offsets;  // live CSR
     const uint32_t* targets;
     const uint32_t* eid;      // u < v entry (in the graph's CSR) of each live entry
+    const uint32_t* number;   // the dense form (words > 0)
+    const uint32_t* bits;
+    const uint16_t* before;
+    const ushort2* span;
+    const uint16_t* numbers;
+    uint32_t words;
     const uint32_t* g_targets;
     const uint32_t* src;
     uint32_t* state;
@@ -661,23 +763,60 @@ struct TrussLoop {
 
 // What bounds the loop: R-MAT scale 19 (14.3 M entries, trussness up to 187,
 // 1,697 rounds) takes 132 scans and about 1,300 peels. A round of a few edges is
-// one peel's chain of dependent loads and the barrier, 6 to 8 us; rounds of 1 K
-// to 12 K edges, most of the time, are bound by the searches, which take the
-// SM's issue slots and bank conflicts rather than bandwidth. Measured there:
-// 40.7 ms for the whole decomposition after the support, 109.5 ms when each
-// round was four launches and a count read by the host. 1,024 staged entries
-// take 40.1 ms, one or four walked entries in flight 40 to 41 ms, so the smaller
-// stage stays, which leaves the L1 the rest.
+// one peel's chain of dependent loads and the barrier, 4 to 8 us; in larger rounds
+// it is the triangles' scattered loads and atomics, and before the dense form
+// (first 108 rounds) the searches. Measured there, the whole decomposition after
+// the support: 109.5 ms when each round was four launches and a count read by the
+// host, 40.7 in this loop with searched lists only (nine in ten were too long for
+// the stage), 35.1 with rows intersected, 28.7 with short lists looked up in rows,
+// 28.0 with a scan's four edges per lane taken with one atomic. With 1, 2, 3 or 8
+// words intersected per walked entry saved 28.6, 28.7, 28.7, 31.5 ms.
 constexpr int kTrussThreads = 1024;
 constexpr uint32_t kStage = 512;  // entries of the searched list a warp stages in shared memory
 constexpr int kTrussUnroll = 2;   // walked entries per lane in flight
+constexpr int kScanLoads = 4;     // listed edges per lane in flight in a scan
+
+// Removes, with edge e, the triangles it makes with the live entries p1 and p2
+// (where hit). A triangle with several edges removed in this round is handled
+// once, by the one with the smallest id; the edges of it that survive the round
+// lose one support, and one that falls below the threshold is listed for the
+// next round.
+__device__ __forceinline__ void truss_remove(const TrussLoop& a, uint32_t e, const bool (&hit)[kTrussUnroll],
+                                             const uint32_t (&p1)[kTrussUnroll], const uint32_t (&p2)[kTrussUnroll],
+                                             uint32_t round, uint32_t k, uint32_t* next, uint32_t* next_count) {
+    uint32_t e1[kTrussUnroll], e2[kTrussUnroll], s1[kTrussUnroll], s2[kTrussUnroll];
+#pragma unroll
+    for (int c = 0; c < kTrussUnroll; ++c) {
+        e1[c] = ld_nc_if(hit[c], a.eid + p1[c], 0u);
+        e2[c] = ld_nc_if(hit[c], a.eid + p2[c], 0u);
+    }
+#pragma unroll
+    for (int c = 0; c < kTrussUnroll; ++c) {
+        s1[c] = ld_if(hit[c], a.state + e1[c], 1u);
+        s2[c] = ld_if(hit[c], a.state + e2[c], 1u);
+    }
+#pragma unroll
+    for (int c = 0; c < kTrussUnroll; ++c) {
+        if (!hit[c]) continue;
+        const bool live1 = s1[c] == 0 || s1[c] == round + 1, live2 = s2[c] == 0 || s2[c] == round + 1;
+        if ((!live1 && s1[c] != round) || (!live2 && s2[c] != round)) continue;   // destroyed earlier
+        if ((!live1 && e1[c] < e) || (!live2 && e2[c] < e)) continue;             // another edge's triangle
+        if (live1 && atomicSub(a.support + e1[c], 1u) == k - 2) {
+            a.state[e1[c]] = round + 1;
+            a.truss[e1[c]] = k - 1;
+            next[atomicAdd(next_count, 1u)] = e1[c];
+        }
+        if (live2 && atomicSub(a.support + e2[c], 1u) == k - 2) {
+            a.state[e2[c]] = round + 1;
+            a.truss[e2[c]] = k - 1;
+            next[atomicAdd(next_count, 1u)] = e2[c];
+        }
+    }
+}
 
 // One removed edge (or the part-th of 2^log_parts slices of its walk): the
 // shorter live list is walked, the longer one searched, in shared memory where
-// it fits kStage entries. A triangle with several edges removed in this round is
-// handled once, by the one with the smallest id; the edges of it that survive
-// the round lose one support, and one that falls below the threshold is listed
-// for the next round.
+// it fits kStage entries.
 __device__ __forceinline__ void truss_peel(const TrussLoop& a, uint32_t e, uint32_t part, uint32_t log_parts,
                                            uint32_t round, uint32_t k, uint32_t* s_y, uint32_t* next,
                                            uint32_t* next_count) {
@@ -718,42 +857,128 @@ __device__ __forceinline__ void truss_peel(const TrussLoop& a, uint32_t e, uint3
 #pragma unroll
         for (int c = 0; c < kTrussUnroll; ++c)
             hit[c] = hit[c] && q[c] < yn && (staged ? s_y[q[c]] : __ldg(a.targets + ys + q[c])) == w[c];
-        uint32_t e1[kTrussUnroll], e2[kTrussUnroll], s1[kTrussUnroll], s2[kTrussUnroll];
 #pragma unroll
         for (int c = 0; c < kTrussUnroll; ++c) {
-            e1[c] = ld_nc_if(hit[c], a.eid + xs + i0 + c * stride, 0u);
-            e2[c] = ld_nc_if(hit[c], a.eid + ys + q[c], 0u);
+            w[c] = xs + i0 + c * stride;
+            q[c] += ys;
         }
-#pragma unroll
-        for (int c = 0; c < kTrussUnroll; ++c) {
-            s1[c] = ld_if(hit[c], a.state + e1[c], 1u);
-            s2[c] = ld_if(hit[c], a.state + e2[c], 1u);
-        }
-#pragma unroll
-        for (int c = 0; c < kTrussUnroll; ++c) {
-            if (!hit[c]) continue;
-            const bool live1 = s1[c] == 0 || s1[c] == round + 1, live2 = s2[c] == 0 || s2[c] == round + 1;
-            if ((!live1 && s1[c] != round) || (!live2 && s2[c] != round)) continue;   // destroyed earlier
-            if ((!live1 && e1[c] < e) || (!live2 && e2[c] < e)) continue;             // another edge's triangle
-            if (live1 && atomicSub(a.support + e1[c], 1u) == k - 2) {
-                a.state[e1[c]] = round + 1;
-                a.truss[e1[c]] = k - 1;
-                next[atomicAdd(next_count, 1u)] = e1[c];
-            }
-            if (live2 && atomicSub(a.support + e2[c], 1u) == k - 2) {
-                a.state[e2[c]] = round + 1;
-                a.truss[e2[c]] = k - 1;
-                next[atomicAdd(next_count, 1u)] = e2[c];
-            }
-        }
+        truss_remove(a, e, hit, w, q, round, k, next, next_count);
     }
 }
 
+// The same on the dense form. Where the words that both rows have bits in are
+// few, they are intersected; else the shorter live list is walked and each of its
+// vertices looked up in the other end's row, one load where a search takes ten or
+// more. kDenseLoads words or entries per lane are in flight, and the common
+// neighbours' positions in the two live lists are queued in shared memory, from
+// where all lanes take them.
+constexpr int kDenseLoads = 4;
+constexpr uint32_t kWalkWords = 2;  // words intersected per walked entry saved
+constexpr uint32_t kDenseBatch = 32 * kTrussUnroll;
+constexpr uint32_t kQueue = 32 * 32 + kDenseBatch;  // positions a warp queues: a word per lane beyond a batch
+
+__device__ __forceinline__ void truss_peel_dense(const TrussLoop& a, uint32_t e, uint32_t part, uint32_t log_parts,
+                                                 uint32_t round, uint32_t k, uint32_t* s_queue, uint32_t* next,
+                                                 uint32_t* next_count) {
+    const unsigned lane = lane_id();
+    uint32_t u = __ldg(a.src + e), v = __ldg(a.g_targets + e);
+    uint32_t pu = __ldg(a.offsets + u), du = __ldg(a.offsets + u + 1) - pu;
+    uint32_t pv = __ldg(a.offsets + v), dv = __ldg(a.offsets + v + 1) - pv;
+    uint32_t nu = __ldg(a.number + u), nv = __ldg(a.number + v);
+    if (du > dv) {  // u: the shorter list
+        uint32_t t = pu; pu = pv; pv = t;
+        t = du; du = dv; dv = t;
+        t = nu; nu = nv; nv = t;
+    }
+    const ushort2 su = __ldg(a.span + nu), sv = __ldg(a.span + nv);
+    const uint64_t rv = static_cast<uint64_t>(nv) * a.words;
+    const uint32_t first = max(su.x, sv.x), last = max(first, static_cast<uint32_t>(min(su.y, sv.y)));
+    uint32_t queued = 0;
+    auto take = [&](uint32_t n) {  // the last n queued, at most kDenseBatch
+        queued -= n;
+        __syncwarp();
+        bool hit[kTrussUnroll];
+        uint32_t p1[kTrussUnroll], p2[kTrussUnroll];
+#pragma unroll
+        for (int c = 0; c < kTrussUnroll; ++c) {
+            hit[c] = lane + c * 32 < n;
+            const uint32_t x = hit[c] ? s_queue[queued + lane + c * 32] : 0u;
+            p1[c] = pu + (x >> 16);
+            p2[c] = pv + (x & 0xFFFFu);
+        }
+        __syncwarp();
+        truss_remove(a, e, hit, p1, p2, round, k, next, next_count);
+    };
+    const bool intersect = last - first <= kWalkWords * du;
+    const uint32_t all = intersect ? last - first : du;
+    const uint32_t share = (all + (1u << log_parts) - 1) >> log_parts;  // of this part
+    const uint32_t begin = min(part * share, all), end = min(begin + share, all);
+    if (intersect) {
+        const uint64_t ru = static_cast<uint64_t>(nu) * a.words;
+        for (uint32_t j0 = begin; j0 < end; j0 += kDenseLoads * 32) {
+            uint32_t x[kDenseLoads], y[kDenseLoads], bx[kDenseLoads], by[kDenseLoads];
+#pragma unroll
+            for (int c = 0; c < kDenseLoads; ++c) {
+                const uint32_t j = j0 + c * 32 + lane;
+                x[c] = ld_nc_if(j < end, a.bits + ru + first + j, 0u);
+                y[c] = ld_nc_if(j < end, a.bits + rv + first + j, 0u);
+            }
+#pragma unroll
+            for (int c = 0; c < kDenseLoads; ++c) {
+                const uint32_t j = j0 + c * 32 + lane;
+                bx[c] = x[c] & y[c] ? __ldg(a.before + ru + first + j) : 0u;
+                by[c] = x[c] & y[c] ? __ldg(a.before + rv + first + j) : 0u;
+            }
+#pragma unroll
+            for (int c = 0; c < kDenseLoads; ++c) {
+                uint32_t m = x[c] & y[c];
+                if (!__any_sync(kFullMask, m)) continue;
+                const uint32_t n = __popc(m);
+                const uint32_t upto = warp_inclusive_scan(n);
+                uint32_t at = queued + upto - n;
+                for (; m; m &= m - 1) {
+                    const uint32_t below = (m & (0u - m)) - 1;
+                    s_queue[at++] = (bx[c] + __popc(x[c] & below)) << 16 | (by[c] + __popc(y[c] & below));
+                }
+                queued += __shfl_sync(kFullMask, upto, 31);
+                while (queued >= kDenseBatch) take(kDenseBatch);
+            }
+        }
+    } else {
+        for (uint32_t i0 = begin; i0 < end; i0 += kDenseLoads * 32) {
+            uint32_t w[kDenseLoads], y[kDenseLoads], by[kDenseLoads];
+#pragma unroll
+            for (int c = 0; c < kDenseLoads; ++c) {
+                const uint32_t i = i0 + c * 32 + lane;
+                w[c] = i < end ? __ldg(a.numbers + pu + i) : 0u;
+            }
+#pragma unroll
+            for (int c = 0; c < kDenseLoads; ++c)
+                y[c] = ld_nc_if(i0 + c * 32 + lane < end, a.bits + rv + (w[c] >> 5), 0u);
+#pragma unroll
+            for (int c = 0; c < kDenseLoads; ++c)
+                by[c] = (y[c] >> (w[c] & 31)) & 1u ? __ldg(a.before + rv + (w[c] >> 5)) : 0u;
+#pragma unroll
+            for (int c = 0; c < kDenseLoads; ++c) {
+                const bool hit = (y[c] >> (w[c] & 31)) & 1u;
+                const unsigned hits = __ballot_sync(kFullMask, hit);
+                if (hit)
+                    s_queue[queued + __popc(hits & ((1u << lane) - 1))] =
+                        (i0 + c * 32 + lane) << 16 | (by[c] + __popc(y[c] & ((1u << (w[c] & 31)) - 1)));
+                queued += __popc(hits);
+                if (queued >= kDenseBatch) take(kDenseBatch);
+            }
+        }
+    }
+    if (queued) take(queued);
+}
+
+template <bool kDense>
 __global__ void __launch_bounds__(kTrussThreads, 1) kt_truss_loop_kernel(const TrussLoop a) {
     extern __shared__ uint32_t s_stage[];
     __shared__ uint32_t s_count, s_least;
     const unsigned lane = lane_id();
-    uint32_t* s_y = s_stage + (threadIdx.x >> 5) * kStage;
+    uint32_t* s_warp = s_stage + (threadIdx.x >> 5) * (kDense ? kQueue : kStage);
     const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     const uint32_t nwarps = static_cast<uint32_t>(nthreads >> 5);
@@ -782,24 +1007,39 @@ __global__ void __launch_bounds__(kTrussThreads, 1) kt_truss_loop_kernel(const T
         ++round;
         if (level_start) {
             uint32_t least = 0xFFFFFFFFu;
-            for (uint64_t b = tid & ~31ull; b < a.listed; b += nthreads) {
-                const uint64_t i = b + lane;
-                bool take = false;
-                uint32_t j = 0;
-                if (i < a.listed) {
-                    j = __ldg(a.active + i);
-                    if (a.state[j] == 0) {
-                        const uint32_t s = a.support[j];
-                        take = s < k - 2;
-                        if (take) {
-                            a.state[j] = round;
-                            a.truss[j] = k - 1;
-                        } else {
-                            least = min(least, s);
-                        }
-                    }
+            for (uint64_t b = tid & ~31ull; b < a.listed; b += kScanLoads * nthreads) {
+                uint32_t j[kScanLoads], alive_state[kScanLoads], s[kScanLoads];
+#pragma unroll
+                for (int c = 0; c < kScanLoads; ++c) {
+                    const uint64_t i = b + c * nthreads + lane;
+                    j[c] = ld_nc_if(i < a.listed, a.active + i, kNone);
                 }
-                kt_append(take, j, list ? a.list1 : a.list0, a.st->count + phase % 3);
+#pragma unroll
+                for (int c = 0; c < kScanLoads; ++c) {
+                    alive_state[c] = ld_if(j[c] != kNone, a.state + j[c], 1u);
+                    s[c] = ld_if(j[c] != kNone, a.support + j[c], 0u);
+                }
+                unsigned below[kScanLoads];
+                uint32_t taken = 0;
+#pragma unroll
+                for (int c = 0; c < kScanLoads; ++c) {
+                    below[c] = __ballot_sync(kFullMask, alive_state[c] == 0 && s[c] < k - 2);
+                    taken += __popc(below[c]);
+                    if (alive_state[c] == 0 && s[c] >= k - 2) least = min(least, s[c]);
+                }
+                if (taken == 0) continue;
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(a.st->count + phase % 3, taken);
+                at = __shfl_sync(kFullMask, at, 0);
+#pragma unroll
+                for (int c = 0; c < kScanLoads; ++c) {
+                    if ((below[c] >> lane) & 1u) {
+                        a.state[j[c]] = round;
+                        a.truss[j[c]] = k - 1;
+                        (list ? a.list1 : a.list0)[at + __popc(below[c] & ((1u << lane) - 1))] = j[c];
+                    }
+                    at += __popc(below[c]);
+                }
             }
             least = __reduce_min_sync(kFullMask, least);
             if (lane == 0 && least != 0xFFFFFFFFu) atomicMin(a.st->least + phase % 3, least);
@@ -822,10 +1062,14 @@ __global__ void __launch_bounds__(kTrussThreads, 1) kt_truss_loop_kernel(const T
         alive -= n;
         // With fewer edges than warps, up to 16 warps share one.
         const uint32_t log_parts = n >= nwarps ? 0u : min(4u, 31 - __clz(nwarps / n));
-        for (uint64_t w = warp; w < static_cast<uint64_t>(n) << log_parts; w += nwarps)
-            truss_peel(a, __ldcg((list ? a.list1 : a.list0) + (w >> log_parts)),
-                       static_cast<uint32_t>(w) & ((1u << log_parts) - 1), log_parts, round, k, s_y,
-                       list ? a.list0 : a.list1, a.st->count + phase % 3);
+        for (uint64_t w = warp; w < static_cast<uint64_t>(n) << log_parts; w += nwarps) {
+            const uint32_t e = __ldcg((list ? a.list1 : a.list0) + (w >> log_parts));
+            // An edge's support is its triangles alive at the round's start.
+            if (__ldcg(a.support + e) == 0) continue;
+            (kDense ? truss_peel_dense : truss_peel)(a, e, static_cast<uint32_t>(w) & ((1u << log_parts) - 1),
+                                                     log_parts, round, k, s_warp, list ? a.list0 : a.list1,
+                                                     a.st->count + phase % 3);
+        }
         if (!end_phase()) return;
         n = s_count;
         list ^= 1u;
@@ -903,14 +1147,24 @@ Error truss_decomposition(GraphImpl& g, uint32_t* host_truss, uint32_t* max_trus
     LiveBuffers live[2];
     GCU_TRY(compact_live(dev, g.num_nodes, LiveCsr{g.offsets.ptr, g.targets.ptr, nullptr}, E, rev, state.ptr, &live[0]));
 
-    constexpr size_t kSmem = sizeof(uint32_t) * kStage * (kTrussThreads / 32);
-    GCU_CUDA(cudaFuncSetAttribute(kt_truss_loop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(kSmem)),
+    GCU_TRY(live_matrix(dev, g.num_nodes, &live[0]));
+    constexpr size_t kListSmem = sizeof(uint32_t) * kStage * (kTrussThreads / 32);
+    constexpr size_t kDenseSmem = sizeof(uint32_t) * kQueue * (kTrussThreads / 32);
+    GCU_CUDA(cudaFuncSetAttribute(kt_truss_loop_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(kListSmem)),
              "cudaFuncSetAttribute");
-    int per_sm = 0;
-    GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kt_truss_loop_kernel, kTrussThreads, kSmem),
+    GCU_CUDA(cudaFuncSetAttribute(kt_truss_loop_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(kDenseSmem)),
+             "cudaFuncSetAttribute");
+    int per_sm = 0, per_sm_dense = 0;
+    GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kt_truss_loop_kernel<false>, kTrussThreads,
+                                                           kListSmem),
              "occupancy");
-    if (per_sm < 1) return kernel_error("truss decomposition: the loop kernel does not fit an SM");
+    GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_dense, kt_truss_loop_kernel<true>, kTrussThreads,
+                                                           kDenseSmem),
+             "occupancy");
+    if (per_sm < 1 || per_sm_dense < 1)
+        return kernel_error("truss decomposition: the loop kernel does not fit an SM");
     TrussState st{};
     st.k = 3;
     st.top = edges > 0 ? 2 : 0;
@@ -924,12 +1178,16 @@ Error truss_decomposition(GraphImpl& g, uint32_t* host_truss, uint32_t* max_trus
         std::fill(st.least, st.least + 3, 0xFFFFFFFFu);
         st.phase = 0;
         GCU_CUDA(cudaMemcpyAsync(loop_state.ptr, &st, sizeof(st), cudaMemcpyHostToDevice, dev.stream), "copy");
-        const TrussLoop a{live[cur].offsets.ptr, live[cur].targets.ptr, live[cur].eid.ptr, g.targets.ptr, src, state.ptr,
-                          support.ptr, truss.ptr, active[cur].ptr, listed, lists[0].ptr, lists[1].ptr, loop_state.ptr};
+        const LiveBuffers& lv = live[cur];
+        const TrussLoop a{lv.offsets.ptr, lv.targets.ptr, lv.eid.ptr,    lv.number.ptr,  lv.bits.ptr,
+                          lv.before.ptr,  lv.span.ptr,    lv.numbers.ptr, lv.words,      g.targets.ptr,  src,
+                          state.ptr,      support.ptr,    truss.ptr,     active[cur].ptr, listed,
+                          lists[0].ptr,   lists[1].ptr,   loop_state.ptr};
         // One block per SM; fewer for a core too small to use them.
         const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(
             1, std::min<uint64_t>(dev.sm_count, ceil_div_u64(listed, kTrussThreads / 32))));
-        GCU_LAUNCH_COOP(dev, "kt_truss_loop", kt_truss_loop_kernel, grid, kTrussThreads, kSmem, a);
+        if (lv.words) GCU_LAUNCH_COOP(dev, "kt_truss_dense", kt_truss_loop_kernel<true>, grid, kTrussThreads, kDenseSmem, a);
+        else GCU_LAUNCH_COOP(dev, "kt_truss_loop", kt_truss_loop_kernel<false>, grid, kTrussThreads, kListSmem, a);
         GCU_CUDA(cudaMemcpyAsync(&st, loop_state.ptr, sizeof(st), cudaMemcpyDeviceToHost, dev.stream), "copy");
         GCU_TRY(dev.sync());
         if (st.bar.failed) return kernel_error("truss decomposition: a block did not reach the grid barrier");
@@ -944,6 +1202,7 @@ Error truss_decomposition(GraphImpl& g, uint32_t* host_truss, uint32_t* max_trus
         GCU_TRY(compact_live(dev, g.num_nodes,
                              LiveCsr{live[cur].offsets.ptr, live[cur].targets.ptr, live[cur].eid.ptr},
                              live[cur].entries, rev, state.ptr, &live[cur ^ 1], st.n > 0 ? st.round + 1 : 0));
+        GCU_TRY(live_matrix(dev, g.num_nodes, &live[cur ^ 1]));
         cur ^= 1;
     }
     *max_truss = st.top;

@@ -1,8 +1,9 @@
 """The truss decomposition's loop kernel at the edges of its paths.
 
 Its rounds, level skips and compactions run in one kernel; searched lists are
-staged in shared memory up to 512 entries, and a round of few edges shares each
-edge's walk among warps. Every result is a whole number: trussness, the largest
+staged in shared memory up to 512 entries, or looked up in rows of bits where
+those are dense enough, and a round of few edges shares each edge's walk among
+warps. Every result is a whole number: trussness, the largest
 and the round count equal the oracle's peeling of the same CSR.
 """
 from __future__ import annotations
@@ -50,6 +51,18 @@ def hubs(leaves: int) -> tuple[int, np.ndarray]:
     return leaves + 2, np.concatenate([[[0, 1]], np.stack([0 * v, v], 1), np.stack([0 * v + 1, v], 1), clique(2, 12)])
 
 
+def fringed(n: int, core: int, seed: int) -> tuple[int, np.ndarray]:
+    """A dense core and low-degree vertices across all ids: rows of bits in which
+    short lists are looked up."""
+    rng = np.random.default_rng(seed)
+    members = rng.choice(n, size=core, replace=False)
+    a, b = np.triu_indices(core, 1)
+    keep = rng.random(len(a)) < 0.5
+    fringe = np.stack([np.repeat(np.arange(n), 6), rng.choice(members, size=6 * n)], 1)
+    p = np.sort(np.concatenate([np.stack([members[a[keep]], members[b[keep]]], 1), fringe]), axis=1)
+    return n, np.unique(p[p[:, 0] != p[:, 1]], axis=0)
+
+
 GRAPHS = {
     "stage-1": lambda: disjoint_cliques([512]),  # live lists of 511
     "stage": lambda: disjoint_cliques([513, 5]),
@@ -57,6 +70,11 @@ GRAPHS = {
     "levels": lambda: disjoint_cliques([3, 3, 4, 9, 33, 34, 70, 2, 2]),
     "halves": lambda: disjoint_cliques([3] * 6000 + [6] * 700 + [14] * 60 + [40] * 4),  # a compaction per level
     "dense": lambda: dense(900, 0.62, 3),
+    "rows-1": lambda: dense(1023, 0.1, 7),  # of bits: one word less than a warp's 32
+    "rows": lambda: dense(1024, 0.1, 8),
+    "rows+1": lambda: dense(1025, 0.1, 9),
+    "fringe": lambda: fringed(4000, 600, 10),
+    "wide fringe": lambda: fringed(20000, 1500, 11),
     "sparse": lambda: dense(3000, 0.02, 5),
     "ladder": lambda: ladder(301),
     "hubs": lambda: hubs(5000),
