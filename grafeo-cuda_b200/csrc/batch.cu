@@ -99,18 +99,21 @@ __global__ void batch_extract_kernel(const uint32_t* __restrict__ offsets, const
 // ---------------------------------------------------------------- passes over the union's entries
 
 constexpr uint32_t kBatchChunk = 256;     // entries per warp step
-constexpr int kBatchThreads = 512;
-constexpr int kBatchCtasPerSm = 3;
+constexpr int kBatchThreads = 256;
+constexpr int kBatchCtasPerSm = 5;
 constexpr uint32_t kBatchRun = 2;         // consecutive chunks per warp turn (neighbouring chunks share their graph's lines)
 constexpr uint32_t kNoGraph = 0xFFFFFFFFu;
 
 // Measured on one B200, 256 graphs of the generated corpus (6 M vertices, 106 M
-// entries), a CTA per graph before: BFS from 16 sources 49.1 -> 3.7 ms (the four
+// entries), a CTA per graph before: BFS from 16 sources 49.1 -> 3.5 ms (the four
 // or five graphs of 4 M entries ran alone at the end), 20 PageRank iterations
-// 74.1 -> 8.1 ms (260 G entries/s; the bound is the L1's rate of scattered
-// gathers, as in the single-graph SpMV, plus eight words per finished row). CTA
-// shapes: 2 x 512 threads (64 registers) 8.8 / 4.0 ms, 3 x 512 (40) 8.1 / 3.7;
-// turns of 1 / 4 / 16 chunks 8.9 / 8.8 / 9.6 ms with two CTAs.
+// 74.1 -> 6.9 ms (307 G entries/s). Finishing rows in the lanes where they end, one
+// after another and their inputs loaded behind the gathers, took 8.0 ms for the
+// PageRank (40 registers, 3 x 512 threads). What bounds it now is half issue (57 %
+// of the slots), half the L1 (56 %, 44 % hits). CTA shapes, PageRank / BFS: 5 x 256
+// threads (48 registers) 6.9 / 3.5 ms, 4 x 256 (64) 7.1 / 3.8, 6 x 256 (40) 7.7 /
+// 3.8, 3 x 512 (40) 7.6 / 3.6; turns of 1 / 4 chunks 7.6 / 7.5 ms; a contiguous
+// stretch per SM instead of interleaved turns 7.8 / 4.4.
 
 // The union's rows with entries, packed ("rows" below are indices into this
 // list), and its vertices without.
@@ -202,14 +205,19 @@ __global__ void __launch_bounds__(256) batch_delta_kernel(const uint32_t* __rest
 //   begin(g0, g1)      whether a graph in [g0, g1] is at work (else the chunk is skipped)
 //   want(row)          whether the row's entries have to be gathered
 //   gather(target), add(x, y), zero()
-//   finish(row, x)     the row's result
+//   load(row), more(in)  what finish needs besides the result: loads, and those
+//                      that depend on them
+//   finish(row, x, in) the row's result
 //   part(i, x)         part i of a row that crosses chunks: 2c for the end of a row
 //                      begun before chunk c, 2c + 1 for a row that goes on after it
 //   flush()            after every turn (all lanes)
 // Runs of equal rows are joined per lane, then across lanes by a segmented
-// scan; the lane where a row ends finishes it.
+// scan; the lane where a row ends puts its result into s_row (kBatchChunk of the
+// warp's own), from where consecutive lanes finish consecutive rows. The first 32
+// rows' inputs are loaded beside the gathers: loads that follow them wait in the
+// queue behind them.
 template <class Op>
-__device__ __forceinline__ void batch_pass(const BatchRows& R, Op& op) {
+__device__ __forceinline__ void batch_pass(const BatchRows& R, Op& op, typename Op::T* s_row) {
     using T = typename Op::T;
     const unsigned lane = lane_id();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
@@ -245,9 +253,12 @@ __device__ __forceinline__ void batch_pass(const BatchRows& R, Op& op) {
             }
             uint32_t t[8] = {};
             if (Op::kSkips ? some : any) ld_stream8(R.targets + eb, t);
+            const uint32_t n_rows = rlast - rbase + 1;
+            auto in = op.load(rbase + min(lane, n_rows - 1));
             T val[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) val[i] = op.gather(want[i], t[i]);
+            op.more(in);
             T head = Op::zero(), acc = Op::zero();
             bool multi = false;
 #pragma unroll
@@ -258,7 +269,7 @@ __device__ __forceinline__ void batch_pass(const BatchRows& R, Op& op) {
                         head = acc;
                         multi = true;
                     } else {
-                        op.finish(row[i], acc);
+                        s_row[row[i] - rbase] = acc;
                     }
                     acc = Op::zero();
                 }
@@ -279,17 +290,21 @@ __device__ __forceinline__ void batch_pass(const BatchRows& R, Op& op) {
                 }
             }
             const T carry = __shfl_up_sync(kFullMask, S, 1);
-            if (multi && rf != kNoGraph) {  // the first run ends in this lane
-                const T total = carry_in ? Op::add(head, carry) : head;
-                if (rf == rbase && first_split) op.part(2 * static_cast<uint64_t>(c), total);
-                else op.finish(rf, total);
-            }
+            if (multi && rf != kNoGraph) s_row[rf - rbase] = carry_in ? Op::add(head, carry) : head;
             const bool continues = lane < 31 && next_first == rl;
-            if (!continues && rl != kNoGraph) {  // the last run ends at this lane's end
-                if (rl == rlast && last_split) op.part(2 * static_cast<uint64_t>(c) + 1, S);
-                else if (rl == rbase && first_split) op.part(2 * static_cast<uint64_t>(c), S);
-                else op.finish(rl, S);
+            if (!continues && rl != kNoGraph) s_row[rl - rbase] = S;  // the last run ends at this lane's end
+            __syncwarp();
+            for (uint32_t r = lane; r < n_rows; r += 32) {
+                if (r >= 32) {
+                    in = op.load(rbase + r);
+                    op.more(in);
+                }
+                const T x = s_row[r];
+                if (r == n_rows - 1 && last_split) op.part(2 * static_cast<uint64_t>(c) + 1, x);
+                else if (r == 0 && first_split) op.part(2 * static_cast<uint64_t>(c), x);
+                else op.finish(rbase + r, x, in);
             }
+            __syncwarp();  // s_row is the next chunk's
         }
         op.flush();
     }
@@ -309,7 +324,9 @@ __device__ __forceinline__ void batch_split_pass(const BatchRows& R, Op& op) {
                 T x = op.parts(2 * static_cast<uint64_t>(s.y) + 1);
                 for (uint32_t c = s.y + 1; c < s.z; ++c) x = Op::add(x, op.parts(2 * static_cast<uint64_t>(c) + 1));
                 x = Op::add(x, op.parts(2 * static_cast<uint64_t>(s.z)));
-                op.finish(s.x, x);
+                auto in = op.load(s.x);
+                op.more(in);
+                op.finish(s.x, x, in);
             }
         }
         op.flush();
@@ -360,15 +377,21 @@ struct BfsOp {
     __device__ __forceinline__ T gather(bool p, uint32_t t) const { return ld_if(p, in + t, 0u); }
     __device__ __forceinline__ void part(uint64_t i, T x) { a.parts[i] = x; }
     __device__ __forceinline__ T parts(uint64_t i) const { return a.parts[i]; }
-    __device__ __forceinline__ void finish(uint32_t r, T m) {
-        const uint32_t v = __ldg(a.rows.row_vertex + r);
-        const uint32_t old = in[v], now = (m & ~old);
+    struct In {
+        uint32_t v, g, old;
+    };
+    __device__ __forceinline__ In load(uint32_t r) const {
+        return In{__ldg(a.rows.row_vertex + r), __ldg(a.rows.row_graph + r), 0u};
+    }
+    __device__ __forceinline__ void more(In& x) const { x.old = ld_if(true, in + x.v, 0u); }
+    __device__ __forceinline__ void finish(uint32_t, T m, const In& x) {
+        const uint32_t v = x.v, old = x.old, now = (m & ~old);
         out[v] = old | m;
         if (!now) return;
         if (a.dist)
             for (uint32_t bits = now; bits; bits &= bits - 1)
                 a.dist[static_cast<uint64_t>(__ffs(bits) - 1) * a.V + v] = static_cast<int32_t>(level) + 1;
-        const uint32_t g = __ldg(a.rows.row_graph + r);
+        const uint32_t g = x.g;
         if (g != my_graph) {
             if (my_fresh) atomicOr(fresh + my_graph, my_fresh);
             my_graph = g;
@@ -392,6 +415,7 @@ struct BfsOp {
 __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_bfs_kernel(const BatchBfs a) {
     __shared__ uint32_t s_active;
     __shared__ uint32_t s_count[kMaxBatchSources];
+    __shared__ uint32_t s_rows[kBatchThreads / 32][kBatchChunk];
     const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     unsigned barriers = 0;
@@ -437,7 +461,7 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_bfs_kern
             atomicAdd(a.st->active + level % 3, 1u);
         }
         if (tid == 0) a.st->active[(level + 1) % 3] = 0;
-        batch_pass(a.rows, op);
+        batch_pass(a.rows, op, s_rows[threadIdx.x >> 5]);
         if (!grid_barrier(&a.st->bar, gridDim.x, barriers, [&] { s_active = __ldcg(a.st->active + level % 3); })) return;
         if (s_active == 0) break;
         batch_split_pass(a.rows, op);
@@ -539,25 +563,36 @@ struct PprOp {
         my_diff = 0;
         my_dangle = 0;
     }
-    __device__ __forceinline__ float update(uint32_t v, double sum) {
-        const double p = a.tele[v];
+    __device__ __forceinline__ float update(uint32_t v, double sum, float tele, float old) {
+        const double p = tele;
         const float x = static_cast<float>((1.0 - a.damp) * p + a.damp * (sum + my_mass * p));
-        my_diff += batch_fixed(fabs(static_cast<double>(x) - static_cast<double>(a.ranks[v])));
+        my_diff += batch_fixed(fabs(static_cast<double>(x) - static_cast<double>(old)));
         a.ranks[v] = x;
         return x;
     }
-    __device__ __forceinline__ void finish(uint32_t r, T sum) {
-        enter(__ldg(a.rows.row_graph + r));
+    struct In {
+        uint32_t v, g, len;
+        float tele, old;
+    };
+    __device__ __forceinline__ In load(uint32_t r) const {
+        return In{__ldg(a.rows.row_vertex + r), __ldg(a.rows.row_graph + r),
+                  __ldg(a.rows.row_start + r + 1) - __ldg(a.rows.row_start + r), 0.f, 0.f};
+    }
+    __device__ __forceinline__ void more(In& x) const {
+        x.tele = __ldg(a.tele + x.v);
+        x.old = __uint_as_float(ld_if(true, reinterpret_cast<const uint32_t*>(a.ranks) + x.v, 0u));
+    }
+    __device__ __forceinline__ void finish(uint32_t, T sum, const In& in) {
+        enter(in.g);
         if (!my_works) return;
-        const uint32_t v = __ldg(a.rows.row_vertex + r);
-        const float x = update(v, sum);
-        out[v] = x / static_cast<float>(__ldg(a.rows.row_start + r + 1) - __ldg(a.rows.row_start + r));
+        out[in.v] = update(in.v, sum, in.tele, in.old) / static_cast<float>(in.len);
     }
     // A vertex without entries: its rank is dangling mass.
     __device__ __forceinline__ void finish_lone(uint32_t i) {
         enter(__ldg(a.rows.lone_graph + i));
         if (!my_works) return;
-        my_dangle += batch_fixed(static_cast<double>(update(__ldg(a.rows.lone + i), 0.0)));
+        const uint32_t v = __ldg(a.rows.lone + i);
+        my_dangle += batch_fixed(static_cast<double>(update(v, 0.0, a.tele[v], a.ranks[v])));
     }
     __device__ __forceinline__ void flush() {
         const unsigned has = __ballot_sync(kFullMask, my_graph != kNoGraph);
@@ -583,6 +618,7 @@ struct PprOp {
 
 __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kernel(const BatchPpr a) {
     __shared__ uint32_t s_active;
+    __shared__ double s_rows[kBatchThreads / 32][kBatchChunk];
     const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     unsigned barriers = 0;
@@ -628,7 +664,7 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kern
             if (b + lane_id() < a.rows.n_lone) op.finish_lone(static_cast<uint32_t>(b + lane_id()));
             op.flush();
         }
-        batch_pass(a.rows, op);
+        batch_pass(a.rows, op, s_rows[threadIdx.x >> 5]);
         if (!grid_barrier(&a.st->bar, gridDim.x, barriers, [&] { s_active = __ldcg(a.st->active + it % 3); })) return;
         if (s_active == 0) break;
         batch_split_pass(a.rows, op);
