@@ -6,11 +6,10 @@
 // plain symmetric CSR and graph i's entries are [offsets[vbase[i]],
 // offsets[vbase[i + 1]]).
 //
-//  * Triangles: one degree-oriented DAG of the union and its out-degree
-//    buckets, one variant per bucket (the installed learned schedule's pick,
-//    else the fastest of the valid variants timed once on the batch); the
-//    wedge kernels add each DAG source's triangles into a per-vertex counter
-//    and a block per graph sums its vertices.
+//  * Triangles: word lists of the union, counted per owner (tri_words.cu), or,
+//    with a learned schedule installed, one degree-oriented DAG of the union and
+//    its out-degree buckets, the schedule's variant per bucket; a block per graph
+//    sums its vertices.
 //  * BFS and PageRank run over the union as a whole, one cooperative launch
 //    each: every level or iteration is one pass over the entries of all graphs
 //    that are still at work, and the blocks meet at a grid barrier. The entries

@@ -143,8 +143,8 @@ class GpuDevice:
         lib.gcu_device_set_kernel_timing(self._h, 1 if on else 0)
 
     def set_bfs_device_loop(self, on: bool) -> None:
-        """BFS level loop on the device (default) or driven from the host;
-        the host drives it whenever per-kernel timing is on."""
+        """BFS levels on the device, in one launch (default), or driven from
+        the host; the host drives them whenever per-kernel timing is on."""
         lib.gcu_device_set_bfs_device_loop(self._h, 1 if on else 0)
 
     def kernel_stats(self) -> dict:

@@ -82,9 +82,10 @@ GCU_API uint64_t gcu_device_launch_count(const gcu_device* dev);
 /* When on, every kernel launch is bracketed by CUDA events and its device time
  * is accumulated per kernel name. */
 GCU_API void gcu_device_set_kernel_timing(gcu_device* dev, int on);
-/* BFS level loop on the device (default, on = 1): a search is one CUDA-graph
- * launch whose WHILE node runs decide + step until the frontier is empty, with
- * no host round trip per level. on = 0 (or per-kernel timing on) drives the
+/* BFS levels on the device (default, on = 1): a search is one cooperative
+ * launch that runs every level or, with a schedule installed, one CUDA-graph
+ * launch whose WHILE node runs decide + step until the frontier is empty; no
+ * host round trip per level. on = 0 (or per-kernel timing on) drives the
  * levels from the host, reading the counters back after each step. Results
  * are the same either way. No reference counterpart (bfs.rs:42-131 syncs
  * every level). */
@@ -343,15 +344,15 @@ GCU_API gcu_status gcu_batch_set_pagerank_seeds(gcu_batch* b, const uint32_t* se
  * (num_graphs each, may be NULL). */
 GCU_API gcu_status gcu_batch_personalized_pagerank(gcu_batch* b, float* ranks, uint32_t* iterations,
                                                    uint8_t* converged, double* seconds);
-/* Plans, autotunes and captures triangles + BFS + PageRank into one CUDA
+/* Plans and captures triangles + BFS + PageRank into one CUDA
  * graph; gcu_batch_replay enqueues it on the device stream (asynchronous);
  * gcu_batch_results synchronizes and copies any of the results (NULL skips). */
 GCU_API gcu_status gcu_batch_capture(gcu_batch* b);
 GCU_API gcu_status gcu_batch_replay(gcu_batch* b);
 GCU_API gcu_status gcu_batch_results(gcu_batch* b, uint64_t* triangles, int32_t* distances, uint32_t* reachable,
                                      int32_t* max_depth, float* ranks, uint32_t* iterations, uint8_t* converged);
-/* JSON of the autotuned choices (variant per bucket, CTA sizes with their
- * timings); returns the length, writes up to buflen bytes. */
+/* JSON of the choices made (intersection form, block sizes with the time of
+ * one run); returns the length, writes up to buflen bytes. */
 GCU_API size_t gcu_batch_tuning(const gcu_batch* b, char* buf, size_t buflen);
 
 #define GCU_SCHEDULE_FEATURES 12
