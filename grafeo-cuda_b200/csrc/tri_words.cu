@@ -24,8 +24,8 @@
 // Only the owner's words are ever set and cleared, not the whole bitmap.
 //
 // Measured on one B200 against the oriented-CSR form (triangle.cu): R-MAT 16
-// 3.13 -> 0.21 ms, R-MAT 22 30.7 -> 12.1 ms (count 9.9, lists 1.8), the triangles
-// of 256 batched graphs 9.5 -> 3.7 ms. On the way, R-MAT 22 count: one word per
+// 3.13 -> 0.19 ms, R-MAT 22 30.7 -> 11.7 ms (count 9.6, lists 1.9), the triangles
+// of 256 batched graphs 9.5 -> 3.6 ms. On the way, R-MAT 22 count: one word per
 // lane and four lists in flight, 256-thread blocks 14.9 ms (76 instructions per
 // 32 words, 24 % of the stalls at the items' block barriers); two words per lane
 // 11.5; 128-thread blocks with a 16 KB bitmap 10.7; two lists in flight, 40
@@ -332,11 +332,15 @@ __global__ void tw_owners_kernel(const uint32_t* __restrict__ offsets, const uin
         }
         const bool alone = n <= warp_words && d <= kWarpOwnerRow;  // a warp's
         append_vertex(n > 0 && alone, static_cast<uint32_t>(v), warp_list, warp_count);
-        if (n > 0 && !alone) {
-            const uint32_t slices = (d + kSlice - 1) / kSlice;
-            const uint32_t at = atomicAdd(item_count, slices);
-            for (uint32_t k = 0; k < slices; ++k) items[at + k] = make_uint2(static_cast<uint32_t>(v), k);
-        }
+        // One place per warp step: an atomic per vertex on the one counter bounded
+        // this kernel (R-MAT 22 262 -> 121 us).
+        const uint32_t slices = n > 0 && !alone ? (d + kSlice - 1) / kSlice : 0u;
+        const uint32_t upto = warp_inclusive_scan(slices), all = __shfl_sync(kFullMask, upto, 31);
+        if (all == 0) continue;
+        uint32_t at = 0;
+        if (lane_id() == 0) at = atomicAdd(item_count, all);
+        at = __shfl_sync(kFullMask, at, 0) + upto - slices;
+        for (uint32_t k = 0; k < slices; ++k) items[at + k] = make_uint2(static_cast<uint32_t>(v), k);
     }
 }
 
