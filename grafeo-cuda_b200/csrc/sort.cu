@@ -42,7 +42,7 @@ static_assert(kSortThreads == kRadix, "one thread per digit in the block scans")
 static_assert(kSliceKeys % 32 == 0, "whole warp rounds per slice");
 static_assert(kKeysPerLane % 2 == 0, "two keys' rank words per register");
 constexpr int kScatterCtasPerSm = 4;
-constexpr uint32_t kMaxTilesPerCta = 16, kScatterWaves = 7;
+constexpr uint32_t kTilesPerCta = 16, kScatterWaves = 7;  // tiles at most
 
 // A digit of up to 8 bits: low_mask's bits of (key >> shift), and above them,
 // where the digit goes on into the key's high word, that word's lowest ones.
@@ -101,7 +101,7 @@ __device__ __forceinline__ unsigned same_digit_lanes(uint32_t d) {
 // order, then in digit order, kSortTile each.
 constexpr size_t kSmemScatterBytes = 2 * sizeof(uint64_t) * kSortTile;
 
-__global__ void __launch_bounds__(kSortThreads, kScatterCtasPerSm) radix_scatter_kernel(
+__global__ void __launch_bounds__(kSortThreads, kScatterCtasPerSm) radix_scatter_smem_kernel(
     const uint64_t* __restrict__ in, uint64_t* __restrict__ out, uint64_t n, RadixDigit field, uint32_t tiles,
     uint32_t nctas, const uint32_t* __restrict__ bases) {
     extern __shared__ uint64_t s_dyn[];
@@ -217,13 +217,13 @@ static Error radix_passes(DeviceImpl& dev, uint64_t* keys, uint64_t* tmp, uint64
     // Few keys are spread over all SMs (a million: 17 us, 62 with 16 tiles).
     const uint64_t all = ceil_div_u64(n, kSortTile);
     const uint64_t most = static_cast<uint64_t>(dev.sm_count) * kScatterCtasPerSm * kScatterWaves;
-    const uint32_t tiles = static_cast<uint32_t>(std::min<uint64_t>(kMaxTilesPerCta, ceil_div_u64(all, most)));
+    const uint32_t tiles = static_cast<uint32_t>(std::min<uint64_t>(kTilesPerCta, ceil_div_u64(all, most)));
     const uint32_t nctas = static_cast<uint32_t>(ceil_div_u64(all, tiles));
     DeviceBuffer<uint32_t> hist, bases;
     GCU_TRY(hist.allocate(dev, static_cast<uint64_t>(nctas) * kRadix));
     GCU_TRY(bases.allocate(dev, static_cast<uint64_t>(nctas) * kRadix + 1));
     if (kSmemScatterBytes > 48 * 1024)
-        GCU_CUDA(cudaFuncSetAttribute(radix_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        GCU_CUDA(cudaFuncSetAttribute(radix_scatter_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kSmemScatterBytes)),
                  "cudaFuncSetAttribute");
     uint64_t* src = keys;
@@ -231,7 +231,7 @@ static Error radix_passes(DeviceImpl& dev, uint64_t* keys, uint64_t* tmp, uint64
     for (const RadixDigit& d : digits) {
         GCU_LAUNCH(dev, "radix_hist", radix_hist_kernel, nctas, kSortThreads, 0, src, n, d, tiles, nctas, hist.ptr);
         GCU_TRY(exclusive_scan_u32(dev, hist.ptr, bases.ptr, static_cast<uint64_t>(nctas) * kRadix));
-        GCU_LAUNCH(dev, "radix_scatter", radix_scatter_kernel, nctas, kSortThreads, kSmemScatterBytes, src, dst, n, d,
+        GCU_LAUNCH(dev, "radix_scatter", radix_scatter_smem_kernel, nctas, kSortThreads, kSmemScatterBytes, src, dst, n, d,
                    tiles, nctas, bases.ptr);
         std::swap(src, dst);
     }
