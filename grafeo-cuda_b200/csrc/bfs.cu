@@ -585,7 +585,7 @@ struct BfsSearch {
     uint2* queue0;
     uint2* queue1;
     uint4* segments;  // the group's items: [2][kGroupBlocks][kGroupItems] (start, end, phase, epoch)
-    uint32_t epoch;   // differs from search to search on the same buffers
+    uint32_t epoch;   // of this search among those of its segments, never 0
     BfsSearchState* st;
 };
 
@@ -854,10 +854,14 @@ __device__ __forceinline__ void local_level(const BfsSearch& a, const uint2* g_i
 // The group: block b's new items go to its segment of `out` (and, past
 // kGroupItems, to g_out at positions from the shared counter `overflow`).
 // Warp w of block b reads segment (b + w) % group, so every segment is read by
-// warps of every block, whichever block filled it. An item carries the phase
-// that wrote it; a reader that comes before the item is there polls it, so the
-// group's barrier needs no memory fence (a release waits about a microsecond
-// for the level's scattered stores).
+// warps of every block, whichever block filled it. An item carries the phase and
+// the search that wrote it; a reader that comes before the item is there polls
+// it, so the group's barrier needs no memory fence (a release waits about a
+// microsecond for the level's scattered stores). What a reader may find instead
+// of the item is an older one of the same segments, whose tag differs: the
+// segments are cleared when they are allocated (the pool hands out memory in
+// which another graph's searches left their items, whose tags repeat), the
+// searches on them are numbered and so are a search's phases.
 __device__ __forceinline__ void group_level(const BfsSearch& a, const uint2* queue, const uint4* in,
                                             const uint32_t* counts, bool first, uint32_t q, unsigned log_group, uint4* out,
                                             uint2* g_out, uint32_t phase, BfsLocal* c, int32_t next_level) {
@@ -874,7 +878,10 @@ __device__ __forceinline__ void group_level(const BfsSearch& a, const uint2* que
             if (first) return __ldcg(queue + i);
             const uint4* p = in + static_cast<size_t>(seg) * kGroupItems + i;
             uint4 v = ld_relaxed_16(p);
-            for (unsigned k = 0; (v.z != phase - 1 || v.w != a.epoch) && k < kGridSpinLimit; ++k) v = ld_relaxed_16(p);
+            for (unsigned k = 0; (v.z != phase - 1 || v.w != a.epoch) && k < kGridSpinLimit; ++k) {
+                if ((k & 1023u) == 1023u && ld_relaxed(&a.st->bar.failed)) break;  // given up elsewhere
+                v = ld_relaxed_16(p);
+            }
             if (v.z != phase - 1 || v.w != a.epoch) {
                 atomicExch(&a.st->bar.failed, 1u);
                 return make_uint2(0u, 0u);
@@ -1527,6 +1534,12 @@ __global__ void bfs_active_scatter_kernel(const uint32_t* __restrict__ offsets, 
         if (offsets[v + 1] > offsets[v]) active[pos[v]] = static_cast<uint32_t>(v);
 }
 
+// No item of these segments has a tag that a search looks for (see group_level).
+static Error clear_segments(DeviceImpl& dev, BfsWork& w) {
+    GCU_CUDA(cudaMemsetAsync(w.search_segments.ptr, 0, sizeof(uint4) * w.search_segments.count, dev.stream), "memset");
+    return ok();
+}
+
 static Error ensure_work(GraphImpl& g) {
     if (g.bfs_work) return ok();
     DeviceImpl& dev = *g.dev;
@@ -1542,6 +1555,7 @@ static Error ensure_work(GraphImpl& g) {
     GCU_TRY(w->queue[0].allocate(dev, queue_words));
     GCU_TRY(w->queue[1].allocate(dev, queue_words));
     GCU_TRY(w->search_segments.allocate(dev, 2 * static_cast<size_t>(kGroupBlocks) * kGroupItems));
+    GCU_TRY(clear_segments(dev, *w));
     GCU_TRY(w->search.allocate(dev, 1));
     GCU_TRY(w->degree_scan.allocate(dev, V + 1));
     GCU_TRY(w->counters.allocate(dev, 1));
@@ -1886,7 +1900,11 @@ Error run_search(GraphImpl& g, BfsWork& w, uint32_t source) {
     a.queue0 = reinterpret_cast<uint2*>(w.queue[0].ptr);
     a.queue1 = reinterpret_cast<uint2*>(w.queue[1].ptr);
     a.segments = w.search_segments.ptr;
-    a.epoch = ++w.search_epoch;
+    if (++w.search_epoch == 0) {  // the numbers begin again
+        GCU_TRY(clear_segments(dev, w));
+        w.search_epoch = 1;
+    }
+    a.epoch = w.search_epoch;
     a.st = w.search.ptr;
     GCU_CUDA(cudaMemsetAsync(w.search.ptr, 0, sizeof(BfsSearchState), dev.stream), "memset");
     GCU_LAUNCH_COOP(dev, "bfs_search", kernel, w.search_grid, kSearchThreads, 0, a);
