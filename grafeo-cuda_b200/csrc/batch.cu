@@ -54,7 +54,7 @@ __global__ void batch_check_kernel(const uint32_t* __restrict__ offsets, const u
     for (uint32_t g = blockIdx.x; g < G; g += gridDim.x) {
         const uint32_t vb = vbase[g], ve = vbase[g + 1];
         const uint32_t e0 = offsets[vb], e1 = offsets[ve];
-        for (uint32_t j = e0 + threadIdx.x; j < e1; j += blockDim.x) {
+        for (uint64_t j = static_cast<uint64_t>(e0) + threadIdx.x; j < e1; j += blockDim.x) {
             const uint32_t t = targets[j];
             if (t < vb || t >= ve) atomicMin(first_bad, static_cast<unsigned long long>(j));
         }
@@ -67,7 +67,8 @@ __global__ void batch_graph_sum_kernel(const unsigned long long* __restrict__ pe
     __shared__ unsigned long long scratch[32];
     for (uint32_t g = blockIdx.x; g < G; g += gridDim.x) {
         unsigned long long acc = 0;
-        for (uint32_t v = vbase[g] + threadIdx.x; v < vbase[g + 1]; v += blockDim.x) acc += per_vertex[v];
+        for (uint64_t v = static_cast<uint64_t>(vbase[g]) + threadIdx.x; v < vbase[g + 1]; v += blockDim.x)
+            acc += per_vertex[v];
         acc = block_sum(acc, scratch);
         if (threadIdx.x == 0) totals[g] = acc;
     }
@@ -474,8 +475,8 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_bfs_kern
         __syncthreads();
         uint32_t cnt = 0;
         const uint32_t ve = a.vbase[g + 1];
-        for (uint32_t base = a.vbase[g] + warp * 32; base < ve; base += kBatchThreads) {
-            const uint32_t v = base + lane;
+        for (uint64_t base = static_cast<uint64_t>(a.vbase[g]) + warp * 32; base < ve; base += kBatchThreads) {
+            const uint64_t v = base + lane;
             const uint32_t vis = v < ve ? a.mask_a[v] : 0u;
             for (uint32_t k = 0; k < a.S; ++k) {
                 const unsigned b = __ballot_sync(kFullMask, (vis >> k) & 1u);

@@ -223,10 +223,10 @@ __device__ __forceinline__ void topdown_tile(const uint32_t* __restrict__ offset
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < kTdItems; ++q) {
-        const uint32_t e = static_cast<uint32_t>(e0) + q * kTdThreads + threadIdx.x;
+        const uint32_t o = q * kTdThreads + threadIdx.x, e = static_cast<uint32_t>(e0) + o;
         bool found = false;
         uint32_t v = 0;
-        if (e < e1) {
+        if (o < e1 - static_cast<uint32_t>(e0)) {
             uint32_t lo = 0, hi = window;
             while (hi - lo > 1) {
                 uint32_t mid = (lo + hi) >> 1;
@@ -533,6 +533,11 @@ constexpr uint32_t kLocalMaxLevels = 32768;  // levels per local or group stretc
 constexpr int kPushUnroll = 4;               // edges per lane in flight in a push
 constexpr int kPullTiles = 1;                // 32-vertex tiles per warp in flight in a pull
 
+// Item c of a list of d entries from s.
+__device__ __forceinline__ uint2 list_item(uint32_t s, uint32_t d, uint32_t c) {
+    return make_uint2(range_begin(s, kItemEdges, c), range_end(s, d, kItemEdges, c));
+}
+
 struct alignas(16) BfsSlot {
     unsigned long long edges;     // out-edges of the new frontier
     uint32_t discovered;          // vertices of the new frontier
@@ -627,9 +632,7 @@ __device__ __forceinline__ void push_items(const BfsSearch& a, const uint2* g_in
         if (lane < k && i < q) {
             it = __ldcg(g_in + i);
             if (parts > 1) {
-                const uint32_t piece = (it.y - it.x + parts - 1) / parts;
-                it.x = min(it.y, it.x + part * piece);
-                it.y = min(it.y, it.x + piece);
+                take_piece(it.x, it.y, part, (it.y - it.x + parts - 1) / parts);
             }
         }
         const uint32_t len = it.y - it.x;
@@ -679,7 +682,7 @@ __device__ __forceinline__ void push_items(const BfsSearch& a, const uint2* g_in
                     tally.found += 1;
                     tally.edges += deg[u];
                 }
-                mine += (deg[u] + kItemEdges - 1) / kItemEdges;
+                mine += range_count(deg[u], kItemEdges);
             }
             const uint32_t upto = warp_inclusive_scan(mine);
             const uint32_t all = __shfl_sync(kFullMask, upto, 31);
@@ -689,10 +692,9 @@ __device__ __forceinline__ void push_items(const BfsSearch& a, const uint2* g_in
             pos = __shfl_sync(kFullMask, pos, 0) + upto - mine;
 #pragma unroll
             for (int u = 0; u < kPushUnroll; ++u) {
-                const uint32_t n = (deg[u] + kItemEdges - 1) / kItemEdges;
+                const uint32_t n = range_count(deg[u], kItemEdges);
                 if (n <= kLaneItems)
-                    for (uint32_t c = 0; c < n; ++c)
-                        g_out[pos + c] = make_uint2(ls[u] + c * kItemEdges, ls[u] + min(deg[u], (c + 1) * kItemEdges));
+                    for (uint32_t c = 0; c < n; ++c) g_out[pos + c] = list_item(ls[u], deg[u], c);
                 // Longer lists: the warp writes their items together.
                 unsigned longs = __ballot_sync(kFullMask, n > kLaneItems);
                 while (longs) {
@@ -700,8 +702,7 @@ __device__ __forceinline__ void push_items(const BfsSearch& a, const uint2* g_in
                     longs &= longs - 1;
                     const uint32_t s = __shfl_sync(kFullMask, ls[u], l), d = __shfl_sync(kFullMask, deg[u], l);
                     const uint32_t p = __shfl_sync(kFullMask, pos, l);
-                    for (uint32_t c = lane; c * kItemEdges < d; c += 32)
-                        g_out[p + c] = make_uint2(s + c * kItemEdges, s + min(d, (c + 1) * kItemEdges));
+                    for (uint32_t c = lane; c < range_count(d, kItemEdges); c += 32) g_out[p + c] = list_item(s, d, c);
                 }
                 pos += n;
             }
@@ -760,7 +761,7 @@ __device__ __forceinline__ void stretch_items(const BfsSearch& a, uint32_t n, ui
                 found_n += 1;
                 found_m += deg[u];
             }
-            mine += (deg[u] + kItemEdges - 1) / kItemEdges;
+            mine += range_count(deg[u], kItemEdges);
         }
         if (__ballot_sync(kFullMask, mine) == 0) return;
         const uint32_t upto = warp_inclusive_scan(mine);
@@ -780,18 +781,22 @@ __device__ __forceinline__ void stretch_items(const BfsSearch& a, uint32_t n, ui
         }
 #pragma unroll
         for (int u = 0; u < kPushUnroll; ++u) {
-            const uint32_t n = (deg[u] + kItemEdges - 1) / kItemEdges;
+            const uint32_t n = range_count(deg[u], kItemEdges);
             if (n <= kLaneItems)
-                for (uint32_t k = 0; k < n; ++k)
-                    put(pos + k, ls[u] + k * kItemEdges, ls[u] + min(deg[u], (k + 1) * kItemEdges));
+                for (uint32_t k = 0; k < n; ++k) {
+                    const uint2 it = list_item(ls[u], deg[u], k);
+                    put(pos + k, it.x, it.y);
+                }
             unsigned longs = __ballot_sync(kFullMask, n > kLaneItems);
             while (longs) {
                 const int l = __ffs(longs) - 1;
                 longs &= longs - 1;
                 const uint32_t s = __shfl_sync(kFullMask, ls[u], l), d = __shfl_sync(kFullMask, deg[u], l);
                 const uint32_t p = __shfl_sync(kFullMask, pos, l);
-                for (uint32_t k = lane; k * kItemEdges < d; k += 32)
-                    put(p + k, s + k * kItemEdges, s + min(d, (k + 1) * kItemEdges));
+                for (uint32_t k = lane; k < range_count(d, kItemEdges); k += 32) {
+                    const uint2 it = list_item(s, d, k);
+                    put(p + k, it.x, it.y);
+                }
             }
             pos += n;
         }
@@ -808,9 +813,7 @@ __device__ __forceinline__ void stretch_items(const BfsSearch& a, uint32_t n, ui
         if (slot < k && base + slot < n) {
             it = read(base + slot);
             if (log_parts) {
-                const uint32_t piece = ((it.y - it.x) >> log_parts) + 1;
-                it.x = min(it.y, it.x + part * piece);
-                it.y = min(it.y, it.x + piece);
+                take_piece(it.x, it.y, part, ((it.y - it.x) >> log_parts) + 1);
             }
         }
         const uint32_t len = it.y - it.x;
@@ -818,15 +821,14 @@ __device__ __forceinline__ void stretch_items(const BfsSearch& a, uint32_t n, ui
         const uint32_t end = together ? it.x : it.y;
         const uint32_t longest = __reduce_max_sync(kFullMask, end - it.x);
         for (uint32_t o = 0; o < longest; o += lanes * kStretchUnroll) {
-            const uint32_t at = it.x + o + mine;
-            expand(min(at, end), end, lanes);
+            expand(entry_or_end(it.x, end, min(o, end - it.x), mine), end, lanes);
         }
         unsigned longs = __ballot_sync(kFullMask, together && mine == 0);
         while (longs) {
             const int l = __ffs(longs) - 1;
             longs &= longs - 1;
             const uint32_t s = __shfl_sync(kFullMask, it.x, l), e = __shfl_sync(kFullMask, it.y, l);
-            for (uint32_t b = s; b < e; b += 32 * kStretchUnroll) expand(min(b + lane, e), e, 32);
+            walk_entries(s, e, 32 * kStretchUnroll, [&](uint32_t b) { expand(entry_or_end(s, e, b, lane), e, 32); });
         }
     }
     found_n = __reduce_add_sync(kFullMask, found_n);
@@ -1129,10 +1131,9 @@ __global__ void __launch_bounds__(kSearchThreads, kSearchCtasPerSm) bfs_search_k
         }
     }
     const uint32_t s0 = __ldg(a.offsets + a.source), d0 = __ldg(a.offsets + a.source + 1) - s0;
-    uint32_t items = (d0 + kItemEdges - 1) / kItemEdges;
+    uint32_t items = range_count(d0, kItemEdges);
     if (blockIdx.x == 0)
-        for (uint32_t c = threadIdx.x; c < items; c += blockDim.x)
-            a.queue0[c] = make_uint2(s0 + c * kItemEdges, s0 + min(d0, (c + 1) * kItemEdges));
+        for (uint32_t c = threadIdx.x; c < items; c += blockDim.x) a.queue0[c] = list_item(s0, d0, c);
     if (!grid_barrier(&a.st->bar, barriers)) {
         a.st->failed = 1;
         return;
@@ -1208,13 +1209,12 @@ __global__ void __launch_bounds__(kSearchThreads, kSearchCtasPerSm) bfs_search_k
                             s = __ldg(a.offsets + v);
                             d = __ldg(a.offsets + v + 1) - s;
                         }
-                        const uint32_t mine = (d + kItemEdges - 1) / kItemEdges;
+                        const uint32_t mine = range_count(d, kItemEdges);
                         const uint32_t upto = warp_inclusive_scan(mine);
                         uint32_t at = 0;
                         if (lane == 31 && upto) at = atomicAdd(&slot->items, upto);
                         at = __shfl_sync(kFullMask, at, 31) + upto - mine;
-                        for (uint32_t c = 0; c < mine; ++c)
-                            search_queue(a, cur)[at + c] = make_uint2(s + c * kItemEdges, s + min(d, (c + 1) * kItemEdges));
+                        for (uint32_t c = 0; c < mine; ++c) search_queue(a, cur)[at + c] = list_item(s, d, c);
                     }
                 }
                 if (!end_phase()) return;

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "entry_index.h"
+
 namespace gcu {
 
 constexpr int kWarp = 32;

@@ -101,12 +101,12 @@ __global__ void __launch_bounds__(256) kt_support_kernel(const uint32_t* __restr
                 t = ae; ae = be; be = t;
             }
             uint32_t hits = 0;
-            for (uint32_t i = as + lane; i < ae; i += 32) {
-                if (!live[i]) continue;
-                const uint32_t x = targets[i];
+            walk_entries(as, ae, 32, [&](uint32_t o) {
+                if (ae - as - o <= lane || !live[as + o + lane]) return;
+                const uint32_t x = targets[as + o + lane];
                 const uint32_t p = lower_bound_u32(targets, bs, be, x);
                 if (p < be && targets[p] == x && live[p]) ++hits;
-            }
+            });
             hits = warp_sum(hits);
             if (lane == 0) {
                 const uint64_t ej = base + l;
@@ -315,9 +315,11 @@ __global__ void __launch_bounds__(256) kt_peel_kernel(const uint32_t* __restrict
         }
         const uint32_t e = removed[lo];
         const PeelEdge pe = peel_edge(offsets, targets, src, e);
-        const uint32_t begin = pe.xs + (static_cast<uint32_t>(w) - chunk_start[lo]) * kPeelChunk;
-        const uint32_t end = min(begin + kPeelChunk, pe.xe);
-        for (uint32_t p = begin + lane; p < end; p += 32) {
+        const uint32_t chunk = static_cast<uint32_t>(w) - chunk_start[lo];
+        const uint32_t begin = range_begin(pe.xs, kPeelChunk, chunk);
+        const uint32_t count = range_end(pe.xs, pe.xe - pe.xs, kPeelChunk, chunk) - begin;
+        for (uint32_t o = lane; o < count; o += 32) {
+            const uint32_t p = begin + o;
             const uint32_t wv = targets[p];
             if (wv == pe.a || wv == pe.b) continue;
             const uint32_t e1 = pe.x < wv ? p : rev[p];

@@ -555,20 +555,21 @@ __global__ void __launch_bounds__(kPrThreads, kRowCtasPerSm) pr_rows_kernel(
                 const uint2 unit = units[b - ph.first_block];
                 const uint32_t row_start = poff[unit.x], row_end = poff[unit.x + 1];
                 const uint32_t s0 = row_start + unit.y * kSegment;
-                const uint32_t s1 = min(s0 + kSegment, row_end);
+                const uint32_t n = min(kSegment, row_end - s0);
                 float acc = 0.f, comp = 0.f;
-                uint32_t j = s0 + lane;
-                for (; j + 7 * 32 < s1; j += 8 * 32) {
+                uint32_t j = lane;
+                for (; j + 7 * 32 < n; j += 8 * 32) {
                     uint32_t t[8];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) t[q] = ld_stream(ptgt + j + q * 32);
+                    for (int q = 0; q < 8; ++q) t[q] = ld_stream(ptgt + s0 + j + q * 32);
                     float c[8];
 #pragma unroll
                     for (int q = 0; q < 8; ++q) c[q] = gather_contrib(s_hub, contrib_in, t[q]);
 #pragma unroll
                     for (int q = 0; q < 8; ++q) kahan_add(acc, comp, c[q]);
                 }
-                for (; j < s1; j += 32) kahan_add(acc, comp, gather_contrib(s_hub, contrib_in, ld_stream(ptgt + j)));
+                for (; j < n; j += 32)
+                    kahan_add(acc, comp, gather_contrib(s_hub, contrib_in, ld_stream(ptgt + s0 + j)));
                 const double part = warp_sum(static_cast<double>(acc) - static_cast<double>(comp));
                 if (lane == 0) seg_partial[b - ph.first_block] = part;
             } else if (ph.kind == kPhaseGroup) {
@@ -595,8 +596,8 @@ __global__ void __launch_bounds__(kPrThreads, kRowCtasPerSm) pr_rows_kernel(
                     for (int u = 0; u < kUnroll; ++u) {
 #pragma unroll
                         for (int q = 0; q < kRowsPerGroup; ++q) {
-                            const uint32_t j = rs[q] + off + u * g;
-                            t[u][q] = j < re[q] ? ld_stream(ptgt + j) : 0xFFFFFFFFu;
+                            const uint32_t o = off + u * g;
+                            t[u][q] = o < re[q] - rs[q] ? ld_stream(ptgt + rs[q] + o) : 0xFFFFFFFFu;
                         }
                     }
 #pragma unroll

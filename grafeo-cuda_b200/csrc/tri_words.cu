@@ -580,13 +580,14 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) tw_count_kernel(
             }
             __syncwarp();
             uint32_t hits = 0;
-            for (uint32_t j = s; j < e; j += 32) {
-                const bool valid = e - j > lane;
-                const uint32_t v = valid ? ld_stream(targets + j + lane) : 0u;
+            walk_entries(s, e, 32, [&](uint32_t o) {
+                const bool valid = e - s - o > lane;
+                const uint32_t j = s + o + lane;
+                const uint32_t v = valid ? ld_stream(targets + j) : 0u;
                 hits += count_neighbours<kSupport>(
-                    valid, j + lane, v, u, own.y, lists, words, out.rev, s_box[warp],
+                    valid, j, v, u, own.y, lists, words, out.rev, s_box[warp],
                     [&](uint32_t w) { return table_mask(table, bits, w); }, store);
-            }
+            });
             if (!kSupport) add_owner(u, hits, out.per_vertex, sum);
         }
     }
