@@ -485,8 +485,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) tw_count_kernel(
     const uint2* __restrict__ lists, const uint2* __restrict__ words, const uint2* __restrict__ items,
     const uint32_t* __restrict__ owners, const uint32_t* __restrict__ counts, uint32_t* __restrict__ next,
     uint32_t batch, const WordCount out) {
-    __shared__ uint32_t s_fixed[kSupport ? 1 : kBitmapWords];
-    extern __shared__ uint32_t s_dynamic[];
+    // Words as a bitmap, pairs of words as a table: 8-byte accesses.
+    __shared__ __align__(16) uint32_t s_fixed[kSupport ? 1 : kBitmapWords];
+    extern __shared__ __align__(16) uint32_t s_dynamic[];
     __shared__ ListBox<kSupport> s_box[kThreads / 32];
     __shared__ uint32_t s_item, s_chunk;
     uint32_t* s_bits = kSupport ? s_dynamic : s_fixed;
