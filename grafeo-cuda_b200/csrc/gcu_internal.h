@@ -96,6 +96,7 @@ struct DeviceImpl {
     cudaEvent_t timer_start = nullptr;
     cudaEvent_t timer_stop = nullptr;
     cudaStream_t copy_stream = nullptr;  // chunked host-to-device copies that overlap the checks
+    std::mutex copy_mu;                  // guards copy_event (order_streams)
     cudaEvent_t copy_event = nullptr;
 
     std::atomic<uint64_t> launches{0};
@@ -130,6 +131,10 @@ struct DeviceImpl {
     Error activate() const;
     // Synchronizes the stream and folds pending per-kernel timings into stats.
     Error sync();
+    // What `after` is given from here on waits for what `before` holds. Under a
+    // lock: an event that another thread records in between would stand for that
+    // thread's work, and `after` would not wait for this one's.
+    Error order_streams(cudaStream_t before, cudaStream_t after);
     // Called around each kernel launch by GCU_LAUNCH.
     void before_launch(const char* name, cudaEvent_t* start);
     void after_launch(const char* name, cudaEvent_t start);

@@ -228,6 +228,13 @@ Error DeviceImpl::activate() const {
     return ok();
 }
 
+Error DeviceImpl::order_streams(cudaStream_t before, cudaStream_t after) {
+    std::lock_guard<std::mutex> lock(copy_mu);
+    GCU_CUDA(cudaEventRecord(copy_event, before), "cudaEventRecord");
+    GCU_CUDA(cudaStreamWaitEvent(after, copy_event, 0), "cudaStreamWaitEvent");
+    return ok();
+}
+
 Error DeviceImpl::sync() {
     cudaError_t e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return kernel_error(std::string("synchronize failed: ") + cudaGetErrorString(e));

@@ -102,19 +102,12 @@ static Error check_csr(DeviceImpl& dev, const uint32_t* d_offsets, uint32_t* d_t
         // The copy stream starts once the buffers above exist (they are
         // stream-ordered allocations of dev.stream); dev.stream then waits for
         // each chunk before checking it.
-        GCU_CUDA(cudaEventRecord(dev.copy_event, dev.stream), "cudaEventRecord");
-        GCU_CUDA(cudaStreamWaitEvent(dev.copy_stream, dev.copy_event, 0), "cudaStreamWaitEvent");
-        Error err = ok();
+        Error err = dev.order_streams(dev.stream, dev.copy_stream);
         for (uint64_t c0 = 0; c0 < num_edges && err.ok(); c0 += kUploadChunk) {
             const uint64_t c1 = std::min<uint64_t>(c0 + kUploadChunk, num_edges);
             err = copy_to_device(dev, d_targets + c0, h_targets + c0, sizeof(uint32_t) * (c1 - c0), dev.copy_stream);
+            if (err.ok()) err = dev.order_streams(dev.copy_stream, dev.stream);
             if (!err.ok()) break;
-            cudaError_t c = cudaEventRecord(dev.copy_event, dev.copy_stream);
-            if (c == cudaSuccess) c = cudaStreamWaitEvent(dev.stream, dev.copy_event, 0);
-            if (c != cudaSuccess) {
-                err = driver_error(c, "copy CSR to device");
-                break;
-            }
             const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>(ceil_div_u64(c1 - c0, 256), cap)));
             err = [&]() -> Error {
                 GCU_LAUNCH(dev, "csr_check_entries", csr_check_entries_kernel, grid, 256, 0, d_offsets, d_targets,
