@@ -667,14 +667,17 @@ Error build_word_lists(GraphImpl& g, bool full, WordLists* w) {
 
 namespace {
 
-template <bool kSupport, int kThreads, int kCtasPerSm>
+// kMaxSmem: the most dynamic shared memory that a graph of this form asks for. The
+// kernel's limit is set to it, not to this graph's need: it belongs to the kernel,
+// and another thread may launch it on a graph with another need.
+template <bool kSupport, int kThreads, int kCtasPerSm, size_t kMaxSmem>
 Error launch_count(GraphImpl& g, const WordLists& w, uint32_t* next, const WordCount& out) {
     DeviceImpl& dev = *g.dev;
     constexpr int kWarps = kThreads / 32;
     const size_t smem = sizeof(uint32_t) * out.bitmap_words;
     const auto kernel = tw_count_kernel<kSupport, kThreads, kCtasPerSm>;
-    if (smem)
-        GCU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+    if (kMaxSmem)
+        GCU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxSmem)),
                  "cudaFuncSetAttribute");
     GCU_CUDA(cudaMemsetAsync(next, 0, 2 * sizeof(uint32_t), dev.stream), "memset");
     const uint64_t want = std::max<uint64_t>(w.max_items, ceil_div_u64(g.num_nodes, kWarps));
@@ -692,7 +695,7 @@ Error launch_count(GraphImpl& g, const WordLists& w, uint32_t* next, const WordC
 
 Error count_words(GraphImpl& g, const WordLists& w, uint32_t* next, unsigned long long* total,
                   unsigned long long* per_vertex) {
-    return launch_count<false, kCountThreads, kCountCtasPerSm>(
+    return launch_count<false, kCountThreads, kCountCtasPerSm, 0>(
         g, w, next, WordCount{total, per_vertex, g.num_nodes, 0, nullptr, nullptr});
 }
 
@@ -704,10 +707,10 @@ Error edge_support(GraphImpl& g, const uint32_t* rev, uint32_t* support) {
     GCU_TRY(next.allocate(dev, 2));
     WordCount out{nullptr, nullptr, g.num_nodes, support_bitmap_words(g.num_nodes), rev, support};
     const size_t bytes = sizeof(uint32_t) * out.bitmap_words;
-    if (bytes <= kBitmap128) GCU_TRY((launch_count<true, 128, 12>(g, w, next.ptr, out)));
-    else if (bytes <= kBitmap256) GCU_TRY((launch_count<true, 256, 6>(g, w, next.ptr, out)));
-    else if (bytes <= kBitmap512) GCU_TRY((launch_count<true, 512, 3>(g, w, next.ptr, out)));
-    else GCU_TRY((launch_count<true, 1024, 1>(g, w, next.ptr, out)));
+    if (bytes <= kBitmap128) GCU_TRY((launch_count<true, 128, 12, kBitmap128>(g, w, next.ptr, out)));
+    else if (bytes <= kBitmap256) GCU_TRY((launch_count<true, 256, 6, kBitmap256>(g, w, next.ptr, out)));
+    else if (bytes <= kBitmap512) GCU_TRY((launch_count<true, 512, 3, kBitmap512>(g, w, next.ptr, out)));
+    else GCU_TRY((launch_count<true, 1024, 1, sizeof(uint32_t) * kMaxBitmapWords>(g, w, next.ptr, out)));
     return dev.sync();  // the lists are freed on return
 }
 
