@@ -800,8 +800,11 @@ Error finish_layout(BatchImpl& b) {
     b.rows = BatchRows{b.u.targets.ptr, b.row_vertex.ptr, b.row_graph.ptr, b.row_start.ptr, b.chunk_row.ptr,
                        b.delta.ptr, b.split.ptr, b.lone.ptr, b.lone_graph.ptr, E, n_rows, n_chunks, n_split,
                        V - n_rows};
-    GCU_TRY(b.bfs_state.allocate(dev, 1));
-    GCU_TRY(b.ppr_state.allocate(dev, 1));
+    // Zero until a pass kernel runs: results may be read before.
+    for (auto* st : {&b.bfs_state, &b.ppr_state}) {
+        GCU_TRY(st->allocate(dev, 1));
+        GCU_CUDA(cudaMemsetAsync(st->ptr, 0, sizeof(BatchRunState), dev.stream), "memset");
+    }
     return dev.sync();
 }
 
