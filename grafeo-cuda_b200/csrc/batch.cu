@@ -26,9 +26,11 @@
 //    already.)
 //  * Personalised PageRank from K seeds per graph (teleport 1/K per seed,
 //    repeats add up; the formula of gcu_personalized_pagerank): every graph
-//    iterates to its own convergence (L1 change < tol; the change and the
-//    dangling mass are summed per graph as 64-bit fixed-point integers, so the
-//    result does not depend on which warp did what), FP64 row sums.
+//    iterates to its own convergence (L1 change < tol), FP64 row sums. The change
+//    is summed per graph in integers, as a multiple of the tolerance, and the
+//    dangling mass in a fixed order, so the result does not depend on which warp
+//    did what. Neither has a range: a CSR that is not symmetric, pulled over its
+//    own lists, does not conserve mass, nor does a damping outside [0, 1].
 // No reference counterpart: the reference runs one graph per call.
 #include <algorithm>
 
@@ -82,6 +84,24 @@ __global__ void batch_tele_kernel(const uint32_t* __restrict__ seeds, const uint
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         const uint32_t g = static_cast<uint32_t>(i / K);
         atomicAdd(tele + vbase[g] + seeds[i], 1.0f / static_cast<float>(K));
+    }
+}
+
+// Teleport of every seed without entries, 0 for the others (and for kNoSeed).
+constexpr uint32_t kNoSeed = 0xFFFFFFFFu;
+
+__global__ void batch_lone_tele_kernel(const uint32_t* __restrict__ seeds, const uint32_t* __restrict__ vbase,
+                                       const uint32_t* __restrict__ offsets, const float* __restrict__ tele, uint32_t G,
+                                       uint32_t K, float* __restrict__ lone_tele) {
+    const uint64_t total = static_cast<uint64_t>(G) * K;
+    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+         i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        float p = 0.f;
+        if (seeds[i] != kNoSeed) {
+            const uint32_t v = vbase[static_cast<uint32_t>(i / K)] + seeds[i];
+            if (offsets[v + 1] == offsets[v]) p = tele[v];
+        }
+        lone_tele[i] = p;
     }
 }
 
@@ -492,25 +512,41 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_bfs_kern
 
 // ---------------------------------------------------------------- personalised PageRank
 
-// Sums of values in [0, 2] as 64-bit fixed-point integers (units of 2^-62).
-__device__ __forceinline__ unsigned long long batch_fixed(double x) { return __double2ull_rz(x * 4611686018427387904.0); }
-__device__ __forceinline__ double batch_from_fixed(unsigned long long q) {
-    return static_cast<double>(q) * (1.0 / 4611686018427387904.0);
+// A graph's L1 change, of which only whether it is below the tolerance is asked:
+// the sum of the warps' parts in units of 2^-62 of the tolerance, the low 32 bits
+// of each part in one word and the rest in the other, so that no sum of 2^32 parts
+// overflows. A part that is not below the tolerance itself (NaN, or any part where
+// the tolerance is not positive) counts as twice the tolerance.
+struct alignas(16) ChangeSum {
+    unsigned long long low, high;
+};
+constexpr double kChangeUnits = 4611686018427387904.0;  // 2^62
+constexpr unsigned long long kChangeLimit = 1ull << 30;  // of the high parts
+
+__device__ __forceinline__ void add_change(ChangeSum* sum, double part, double tolerance, double scale) {
+    if (!(part < tolerance)) {
+        atomicAdd(&sum->high, 2 * kChangeLimit);
+    } else if (const unsigned long long q = __double2ull_rz(part * scale)) {
+        if (q & 0xFFFFFFFFull) atomicAdd(&sum->low, q & 0xFFFFFFFFull);
+        if (q >> 32) atomicAdd(&sum->high, q >> 32);
+    }
 }
+__device__ __forceinline__ bool below_tolerance(const ChangeSum& c) { return c.high + (c.low >> 32) < kChangeLimit; }
 
 struct BatchPpr {
     BatchRows rows;
     const uint32_t* vbase;
     const uint32_t* lone_count;  // [G]
     const float* tele;
-    uint32_t G, V;
-    double damp, tolerance;
+    const float* lone_tele;      // [G][K] of the seeds without entries (each once), 0 for the others
+    uint32_t G, V, K, log_lanes; // 2^log_lanes lanes sum a graph's dangling mass
+    double damp, tolerance, scale;
     uint32_t max_iterations;
     float *contrib_a, *contrib_b;
     float* ranks;
     double* parts;
-    unsigned long long* diff;    // [3][G], rotating by iteration
-    unsigned long long* dangle;  // [3][G]
+    ChangeSum* change;           // [3][G], rotating by iteration
+    double* mass;                // [2][G]: dangling mass, alternating
     uint32_t* stop;              // [G]: iterations a graph has run when it stopped
     uint32_t* iterations;
     uint8_t* converged;
@@ -523,20 +559,18 @@ struct PprOp {
     const BatchPpr& a;
     const float* in;
     float* out;
-    const unsigned long long* prev_diff;    // [G], the iteration before
-    const unsigned long long* prev_dangle;  // [G]
-    unsigned long long* diff;
-    unsigned long long* dangle;
+    const ChangeSum* prev_change;  // [G], the iteration before
+    const double* mass;            // [G]
+    ChangeSum* change;
     uint32_t it;
     uint32_t my_graph = kNoGraph;
     bool my_works = false;
-    double my_mass = 0.0;
-    unsigned long long my_diff = 0, my_dangle = 0;
+    double my_mass = 0.0, my_change = 0.0;
 
     static __device__ __forceinline__ T zero() { return 0.0; }
     static __device__ __forceinline__ T add(T x, T y) { return x + y; }
     __device__ __forceinline__ bool works(uint32_t g) const {
-        return a.stop[g] > it && (it == 0 || !(batch_from_fixed(prev_diff[g]) < a.tolerance));
+        return a.stop[g] > it && (it == 0 || !below_tolerance(prev_change[g]));
     }
     __device__ __forceinline__ bool begin(uint32_t g0, uint32_t g1) const {
         for (uint32_t g = g0; g <= g1; ++g)
@@ -555,18 +589,16 @@ struct PprOp {
         if (my_graph != kNoGraph) spill();
         my_graph = g;
         my_works = works(g);
-        my_mass = batch_from_fixed(prev_dangle[g]);
+        my_mass = mass[g];
     }
     __device__ __forceinline__ void spill() {
-        if (my_diff) atomicAdd(diff + my_graph, my_diff);
-        if (my_dangle) atomicAdd(dangle + my_graph, my_dangle);
-        my_diff = 0;
-        my_dangle = 0;
+        add_change(change + my_graph, my_change, a.tolerance, a.scale);
+        my_change = 0.0;
     }
     __device__ __forceinline__ float update(uint32_t v, double sum, float tele, float old) {
         const double p = tele;
         const float x = static_cast<float>((1.0 - a.damp) * p + a.damp * (sum + my_mass * p));
-        my_diff += batch_fixed(fabs(static_cast<double>(x) - static_cast<double>(old)));
+        my_change += fabs(static_cast<double>(x) - static_cast<double>(old));
         a.ranks[v] = x;
         return x;
     }
@@ -587,34 +619,53 @@ struct PprOp {
         if (!my_works) return;
         out[in.v] = update(in.v, sum, in.tele, in.old) / static_cast<float>(in.len);
     }
-    // A vertex without entries: its rank is dangling mass.
     __device__ __forceinline__ void finish_lone(uint32_t i) {
         enter(__ldg(a.rows.lone_graph + i));
         if (!my_works) return;
         const uint32_t v = __ldg(a.rows.lone + i);
-        my_dangle += batch_fixed(static_cast<double>(update(v, 0.0, a.tele[v], a.ranks[v])));
+        update(v, 0.0, a.tele[v], a.ranks[v]);
     }
     __device__ __forceinline__ void flush() {
         const unsigned has = __ballot_sync(kFullMask, my_graph != kNoGraph);
         if (has) {
-            // One graph per warp turn nearly always: one pair of atomics.
+            // One graph per warp turn nearly always.
             const uint32_t g = __shfl_sync(kFullMask, my_graph, __ffs(has) - 1);
             const bool same = my_graph == g;
-            const unsigned long long d = warp_sum(same ? my_diff : 0ull), m = warp_sum(same ? my_dangle : 0ull);
-            if (lane_id() == static_cast<unsigned>(__ffs(has) - 1)) {
-                if (d) atomicAdd(diff + g, d);
-                if (m) atomicAdd(dangle + g, m);
-            }
-            if (same) {
-                my_diff = 0;
-                my_dangle = 0;
-            } else if (my_graph != kNoGraph) {
-                spill();
-            }
+            const double part = warp_sum(same ? my_change : 0.0);
+            if (lane_id() == static_cast<unsigned>(__ffs(has) - 1)) add_change(change + g, part, a.tolerance, a.scale);
+            if (same) my_change = 0.0;
+            else if (my_graph != kNoGraph) spill();
         }
         my_graph = kNoGraph;
     }
 };
+
+// The dangling mass of the ranks that an iteration makes from the mass before it: a
+// vertex without entries gets nothing but its teleport, so its rank follows from
+// that mass alone (update() with an empty sum), and is 0 unless it is a seed. A
+// group of lanes per graph, in a fixed order.
+__device__ __forceinline__ void batch_next_mass(const BatchPpr& a, const double* mass, double* next, uint64_t tid,
+                                                uint64_t nthreads) {
+    const uint32_t lanes = 1u << a.log_lanes, at = static_cast<uint32_t>(tid) & (lanes - 1);
+    for (uint64_t b = (tid & ~31ull) >> a.log_lanes; b < a.G; b += nthreads >> a.log_lanes) {
+        const uint64_t g = b + (lane_id() >> a.log_lanes);
+        double sum = 0.0;
+        if (g < a.G) {
+            const double m = mass[g];
+            auto rank = [&](double p) {
+                return static_cast<double>(static_cast<float>((1.0 - a.damp) * p + a.damp * (0.0 + m * p)));
+            };
+            for (uint32_t k = at; k < a.K; k += lanes) {
+                const float p = __ldg(a.lone_tele + g * a.K + k);
+                if (p != 0.f) sum += rank(static_cast<double>(p));
+            }
+            // The others' rank is 0, or NaN once the mass is no number.
+            if (at == 0 && a.lone_count[g] > 0) sum += rank(0.0);
+        }
+        for (uint32_t d = lanes / 2; d > 0; d /= 2) sum += __shfl_xor_sync(kFullMask, sum, d);
+        if (g < a.G && at == 0) next[g] = sum;
+    }
+}
 
 __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kernel(const BatchPpr a) {
     __shared__ uint32_t s_active;
@@ -638,12 +689,8 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kern
     }
     for (uint64_t g = tid; g < a.G; g += nthreads) {
         const bool some = a.vbase[g + 1] > a.vbase[g];
-        for (uint64_t q = 0; q < 3; ++q) {
-            a.diff[q * a.G + g] = 0;
-            a.dangle[q * a.G + g] = 0;
-        }
-        // Iteration 0 reads slot 2.
-        if (some) a.dangle[2ull * a.G + g] = batch_fixed(static_cast<double>(a.lone_count[g]) * static_cast<double>(start(static_cast<uint32_t>(g))));
+        for (uint64_t q = 0; q < 3; ++q) a.change[q * a.G + g] = ChangeSum{0, 0};
+        a.mass[g] = some ? static_cast<double>(a.lone_count[g]) * static_cast<double>(start(static_cast<uint32_t>(g))) : 0.0;
         a.stop[g] = some ? 0xFFFFFFFFu : 0u;
     }
     if (!grid_barrier(&a.st->bar, barriers)) return;
@@ -651,14 +698,14 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kern
         const uint64_t cur = static_cast<uint64_t>(it % 3) * a.G, prev = static_cast<uint64_t>((it + 2) % 3) * a.G;
         const uint64_t next = static_cast<uint64_t>((it + 1) % 3) * a.G;
         PprOp op{a, (it & 1) ? a.contrib_b : a.contrib_a, (it & 1) ? a.contrib_a : a.contrib_b,
-                 a.diff + prev, a.dangle + prev, a.diff + cur, a.dangle + cur, it};
+                 a.change + prev, a.mass + static_cast<uint64_t>(it & 1) * a.G, a.change + cur, it};
         for (uint64_t g = tid; g < a.G; g += nthreads) {
-            a.diff[next + g] = 0;  // last read an iteration ago
-            a.dangle[next + g] = 0;
+            a.change[next + g] = ChangeSum{0, 0};  // last read an iteration ago
             if (a.stop[g] <= it) continue;
-            if (it && batch_from_fixed(op.prev_diff[g]) < a.tolerance) a.stop[g] = it;
+            if (it && below_tolerance(op.prev_change[g])) a.stop[g] = it;
             else atomicAdd(a.st->active + it % 3, 1u);
         }
+        batch_next_mass(a, op.mass, a.mass + static_cast<uint64_t>(~it & 1) * a.G, tid, nthreads);
         if (tid == 0) a.st->active[(it + 1) % 3] = 0;
         for (uint64_t b = tid & ~31ull; b < a.rows.n_lone; b += nthreads) {
             if (b + lane_id() < a.rows.n_lone) op.finish_lone(static_cast<uint32_t>(b + lane_id()));
@@ -676,7 +723,7 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kern
         bool conv = n != 0xFFFFFFFFu;
         if (!conv) {
             n = a.max_iterations;
-            conv = n > 0 && batch_from_fixed(a.diff[static_cast<uint64_t>((n + 2) % 3) * a.G + g]) < a.tolerance;
+            conv = n > 0 && below_tolerance(a.change[static_cast<uint64_t>((n + 2) % 3) * a.G + g]);
         }
         a.iterations[g] = n;
         a.converged[g] = conv ? 1 : 0;
@@ -714,9 +761,9 @@ struct BatchImpl {
     bool ppr_timed = false;
     DeviceBuffer<uint32_t> seeds, iterations, ppr_stop;
     DeviceBuffer<uint8_t> converged;
-    DeviceBuffer<float> tele, contrib_a, contrib_b, ranks;
-    DeviceBuffer<double> ppr_parts;
-    DeviceBuffer<unsigned long long> sums;  // diff then dangle, [3][G] each
+    DeviceBuffer<float> tele, lone_tele, contrib_a, contrib_b, ranks;
+    DeviceBuffer<double> ppr_parts, mass;
+    DeviceBuffer<ChangeSum> change;
     // captured replay of the three
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -861,17 +908,21 @@ Error launch_ppr(BatchImpl& b) {
     a.vbase = b.d_vbase.ptr;
     a.lone_count = b.lone_count.ptr;
     a.tele = b.tele.ptr;
+    a.lone_tele = b.lone_tele.ptr;
     a.G = b.G;
     a.V = b.u.num_nodes;
+    a.K = b.K;
+    while (a.log_lanes < 5 && (1u << a.log_lanes) < b.K) ++a.log_lanes;
     a.damp = static_cast<double>(b.damping);
     a.tolerance = static_cast<double>(b.tolerance);
+    a.scale = kChangeUnits / a.tolerance;
     a.max_iterations = b.max_iterations;
     a.contrib_a = b.contrib_a.ptr;
     a.contrib_b = b.contrib_b.ptr;
     a.ranks = b.ranks.ptr;
     a.parts = b.ppr_parts.ptr;
-    a.diff = b.sums.ptr;
-    a.dangle = b.sums.ptr + 3 * static_cast<size_t>(b.G);
+    a.change = b.change.ptr;
+    a.mass = b.mass.ptr;
     a.stop = b.ppr_stop.ptr;
     a.iterations = b.iterations.ptr;
     a.converged = b.converged.ptr;
@@ -1089,7 +1140,9 @@ Error batch_set_ppr(BatchImpl& b, const uint32_t* seeds, uint32_t K, float dampi
     GCU_CUDA(cudaMemcpyAsync(b.seeds.ptr, seeds, 4ull * b.G * K, cudaMemcpyHostToDevice, dev.stream), "copy");
     GCU_TRY(b.tele.allocate(dev, V));
     GCU_TRY(b.ppr_parts.allocate(dev, 2ull * b.rows.n_chunks));
-    GCU_TRY(b.sums.allocate(dev, 6ull * b.G));
+    GCU_TRY(b.change.allocate(dev, 3ull * b.G));
+    GCU_TRY(b.mass.allocate(dev, 2ull * b.G));
+    GCU_TRY(b.lone_tele.allocate(dev, static_cast<uint64_t>(b.G) * K));
     GCU_TRY(b.ppr_stop.allocate(dev, b.G));
     GCU_TRY(b.contrib_a.allocate(dev, V));
     GCU_TRY(b.contrib_b.allocate(dev, V));
@@ -1099,6 +1152,16 @@ Error batch_set_ppr(BatchImpl& b, const uint32_t* seeds, uint32_t K, float dampi
     GCU_CUDA(cudaMemsetAsync(b.tele.ptr, 0, 4 * std::max<uint64_t>(V, 1), dev.stream), "memset");
     GCU_LAUNCH(dev, "batch_tele", batch_tele_kernel, small_grid(dev, static_cast<uint64_t>(b.G) * K, 256), 256, 0,
                b.seeds.ptr, b.d_vbase.ptr, b.G, K, b.tele.ptr);
+    // Each graph's seeds once, in order, then their teleports where they have no entries.
+    std::vector<uint32_t> once(seeds, seeds + static_cast<uint64_t>(b.G) * K);
+    for (uint32_t g = 0; g < b.G; ++g) {
+        const auto first = once.begin() + static_cast<int64_t>(g) * K, last = first + K;
+        std::sort(first, last);
+        std::fill(std::unique(first, last), last, kNoSeed);
+    }
+    GCU_CUDA(cudaMemcpyAsync(b.seeds.ptr, once.data(), 4ull * b.G * K, cudaMemcpyHostToDevice, dev.stream), "copy");
+    GCU_LAUNCH(dev, "batch_lone_tele", batch_lone_tele_kernel, small_grid(dev, static_cast<uint64_t>(b.G) * K, 256), 256,
+               0, b.seeds.ptr, b.d_vbase.ptr, b.u.offsets.ptr, b.tele.ptr, b.G, K, b.lone_tele.ptr);
     b.ppr_timed = false;
     return dev.sync();
 }
