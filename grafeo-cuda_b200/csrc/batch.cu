@@ -187,13 +187,61 @@ struct BatchRows {
     const uint8_t* delta;        // per entry of a chunk: its row minus the chunk's first row
     const uint4* split;          // (row, first chunk, last chunk, graph) of the rows that cross chunks
     const uint2* lone;           // (vertex without entries, graph)
+    uint32_t* lists;             // [2][n_chunks]: the chunks of a pass (ChunkList)
     uint32_t n_graphs, n_rows, n_chunks, n_split, n_lone;
 };
 
+constexpr uint32_t kMaxLists = 33;
 struct BatchRunState {
     GridBarrier bar;
-    uint32_t active[3];  // graphs at work in this pass, rotating
+    uint32_t active[3];          // chunks of the graphs at work in this pass (and one per graph), rotating
+    uint32_t listed[kMaxLists];  // chunks of each list made
 };
+
+// The chunks that a pass goes through: all of them, and once half are of graphs
+// that have stopped, a list of the others, made anew each time it has halved. A
+// deep graph among large ones is then not charged with theirs: BFS on 121 graphs of
+// which one is a path of 20,000 vertices 443 -> 249 ms (a block per graph: 304); a
+// whole batch that stops at about the same time 1 % slower to 2 % faster. Not worth
+// it below two chunks a warp.
+struct ChunkList {  // in shared memory: the passes are short of registers
+    const uint32_t* list;  // NULL: chunk i is i
+    uint32_t n, made;
+};
+__device__ __forceinline__ uint32_t list_chunk(const uint32_t* list, uint32_t i) { return list ? list[i] : i; }
+
+__device__ __forceinline__ bool list_halved(const ChunkList& l, uint32_t active) {
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    return l.n > 2 * warps && 2ull * active <= l.n && l.made < kMaxLists;
+}
+
+// All threads of the grid, between two barriers; then list_take with the count.
+template <class Op>
+__device__ __forceinline__ void list_make(const BatchRows& R, const ChunkList& l, const Op& op, BatchRunState* st) {
+    uint32_t* to = R.lists + static_cast<size_t>(l.made & 1) * R.n_chunks;
+    const uint32_t* from = l.list;
+    for (uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; b < l.n; b += gridDim.x * blockDim.x) {
+        const uint32_t i = b + lane_id();
+        const uint32_t c = i < l.n ? list_chunk(from, i) : 0u;
+        const bool keep = i < l.n && op.works(__ldg(&R.chunks[c].graph));
+        const unsigned kept = __ballot_sync(kFullMask, keep);
+        uint32_t place = 0;
+        if (lane_id() == 0 && kept) place = atomicAdd(st->listed + l.made, static_cast<uint32_t>(__popc(kept)));
+        place = __shfl_sync(kFullMask, place, 0) + __popc(kept & ((1u << lane_id()) - 1));
+        if (keep) to[place] = c;
+    }
+}
+
+// By one thread of the block, before a block barrier.
+__device__ __forceinline__ void list_take(const BatchRows& R, ChunkList& l, const BatchRunState* st) {
+    l.list = R.lists + static_cast<size_t>(l.made & 1) * R.n_chunks;
+    l.n = __ldcg(st->listed + l.made);
+    ++l.made;
+}
+
+__device__ __forceinline__ uint32_t batch_chunk_count(const BatchRows& R, uint64_t g) {
+    return (g + 1 < R.n_graphs ? R.graphs[g + 1].chunk : R.n_chunks) - R.graphs[g].chunk;
+}
 
 // The last of the graphs that begins at or before x (`first` picks where).
 template <class First>
@@ -313,15 +361,14 @@ __global__ void batch_split_rows_kernel(const uint32_t* __restrict__ offsets, co
 // rows' inputs are loaded beside the gathers: loads that follow them wait in the
 // queue behind them.
 template <class Op>
-__device__ __forceinline__ void batch_pass(const BatchRows& R, Op& op, typename Op::T* s_row) {
+__device__ __forceinline__ void batch_pass(const BatchRows& R, const ChunkList& list, Op& op, typename Op::T* s_row) {
     using T = typename Op::T;
     const unsigned lane = lane_id();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    for (uint64_t c0 = static_cast<uint64_t>(warp) * kBatchRun; c0 < R.n_chunks;
-         c0 += static_cast<uint64_t>(warps) * kBatchRun) {
-        const uint32_t c1 = static_cast<uint32_t>(min_u64(c0 + kBatchRun, R.n_chunks));
-        for (uint32_t c = static_cast<uint32_t>(c0); c < c1; ++c) {
+    for (uint32_t i0 = warp * kBatchRun; i0 < list.n; i0 += warps * kBatchRun) {  // chunks: far below 2^32
+        for (uint32_t ci = i0; ci < min(i0 + kBatchRun, list.n); ++ci) {
+            const uint32_t c = list_chunk(list.list, ci);
             const uint4 meta = __ldg(reinterpret_cast<const uint4*>(R.chunks) + c);
             const uint2 dl =
                 ld_stream2(reinterpret_cast<const uint2*>(R.delta + static_cast<uint64_t>(c) * kBatchChunk + 8 * lane));
@@ -502,6 +549,8 @@ struct BfsOp {
 
 __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_bfs_kernel(const BatchBfs a) {
     __shared__ uint32_t s_active;
+    __shared__ ChunkList s_list;
+    if (threadIdx.x == 0) s_list = ChunkList{nullptr, a.rows.n_chunks, 0};  // before the first barrier
     __shared__ uint32_t s_count[kMaxBatchSources];
     __shared__ uint32_t s_rows[kBatchThreads / 32][kBatchChunk];
     const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -551,14 +600,16 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_bfs_kern
                 const uint64_t base = static_cast<uint64_t>(a.rows.graphs[g].id) * a.S;
                 for (; bits; bits &= bits - 1) a.max_depth[base + __ffs(bits) - 1] = static_cast<int32_t>(level);
             }
-            atomicAdd(a.st->active + level % 3, 1u);
+            atomicAdd(a.st->active + level % 3, 1u + batch_chunk_count(a.rows, g));
         }
         if (tid == 0) a.st->active[(level + 1) % 3] = 0;
-        batch_pass(a.rows, op, s_rows[threadIdx.x >> 5]);
+        batch_pass(a.rows, s_list, op, s_rows[threadIdx.x >> 5]);
         if (!grid_barrier(&a.st->bar, gridDim.x, barriers, [&] { s_active = __ldcg(a.st->active + level % 3); })) return;
         if (s_active == 0) break;
+        const bool halved = list_halved(s_list, s_active);
+        if (halved) list_make(a.rows, s_list, op, a.st);
         batch_split_pass(a.rows, op);
-        if (!grid_barrier(&a.st->bar, barriers)) return;
+        if (!grid_barrier(&a.st->bar, gridDim.x, barriers, [&] { if (halved) list_take(a.rows, s_list, a.st); })) return;
     }
     // Reached vertices per source: lane k of every warp counts bit k of its
     // graph's vertices. A graph that has stopped has the same masks in both arrays.
@@ -732,6 +783,8 @@ __device__ __forceinline__ void batch_next_mass(const BatchPpr& a, const double*
 
 __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kernel(const BatchPpr a) {
     __shared__ uint32_t s_active;
+    __shared__ ChunkList s_list;
+    if (threadIdx.x == 0) s_list = ChunkList{nullptr, a.rows.n_chunks, 0};  // before the first barrier
     __shared__ double s_rows[kBatchThreads / 32][kBatchChunk];
     const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
@@ -770,7 +823,7 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kern
             a.change[next + g] = ChangeSum{0, 0};  // last read an iteration ago
             if (a.stop[g] <= it) continue;
             if (it && below_tolerance(op.prev_change[g])) a.stop[g] = it;
-            else atomicAdd(a.st->active + it % 3, 1u);
+            else atomicAdd(a.st->active + it % 3, 1u + batch_chunk_count(a.rows, g));
         }
         batch_next_mass(a, op.mass, a.mass + static_cast<uint64_t>(~it & 1) * G, tid, nthreads);
         if (tid == 0) a.st->active[(it + 1) % 3] = 0;
@@ -786,11 +839,13 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kern
             }
             op.flush_lanes(g);
         }
-        batch_pass(a.rows, op, s_rows[threadIdx.x >> 5]);
+        batch_pass(a.rows, s_list, op, s_rows[threadIdx.x >> 5]);
         if (!grid_barrier(&a.st->bar, gridDim.x, barriers, [&] { s_active = __ldcg(a.st->active + it % 3); })) return;
         if (s_active == 0) break;
+        const bool halved = list_halved(s_list, s_active);
+        if (halved) list_make(a.rows, s_list, op, a.st);
         batch_split_pass(a.rows, op);
-        if (!grid_barrier(&a.st->bar, barriers)) return;
+        if (!grid_barrier(&a.st->bar, gridDim.x, barriers, [&] { if (halved) list_take(a.rows, s_list, a.st); })) return;
     }
     // A graph whose last iteration met the tolerance has not been marked yet.
     for (uint64_t g = tid; g < G; g += nthreads) {
@@ -1030,7 +1085,7 @@ struct BatchImpl {
     DeviceBuffer<BatchGraph> large, small;
     DeviceBuffer<uint2> row_list, lone;
     DeviceBuffer<BatchChunk> chunks;
-    DeviceBuffer<uint32_t> lone_count, next_small;
+    DeviceBuffer<uint32_t> lone_count, chunk_lists, next_small;
     DeviceBuffer<uint8_t> delta;
     DeviceBuffer<uint4> split;
     uint32_t n_small[kSmallClasses] = {};  // by block size
@@ -1179,6 +1234,7 @@ Error part_graphs(BatchImpl& b) {
         GCU_TRY(b.lone.allocate(dev, n_vertices - n_rows));
         GCU_TRY(chunk_rows.allocate(dev, n_chunks));
         GCU_TRY(b.chunks.allocate(dev, n_chunks));
+        GCU_TRY(b.chunk_lists.allocate(dev, 2 * n_chunks));
         GCU_TRY(b.delta.allocate(dev, n_chunks * kBatchChunk));
         GCU_CUDA(cudaMemsetAsync(b.lone_count.ptr, 0, 4ull * n_graphs, dev.stream), "memset");
         GCU_LAUNCH(dev, "batch_rows", batch_rows_kernel, small_grid(dev, n_vertices, 256), 256, 0, b.u.offsets.ptr,
@@ -1198,7 +1254,7 @@ Error part_graphs(BatchImpl& b) {
             GCU_LAUNCH(dev, "batch_split_rows", batch_split_rows_kernel, small_grid(dev, n_rows, 256), 256, 0,
                        b.u.offsets.ptr, b.large.ptr, n_rows, b.row_list.ptr, row_graph.ptr, split_pos.ptr, b.split.ptr);
         b.rows = BatchRows{b.u.targets.ptr, b.large.ptr, b.row_list.ptr, b.chunks.ptr, b.delta.ptr, b.split.ptr, b.lone.ptr,
-                           n_graphs, n_rows, static_cast<uint32_t>(n_chunks), n_split,
+                           b.chunk_lists.ptr, n_graphs, n_rows, static_cast<uint32_t>(n_chunks), n_split,
                            static_cast<uint32_t>(n_vertices - n_rows)};
         GCU_TRY(dev.sync());
     }
