@@ -770,6 +770,7 @@ struct TrussState {
     GridBarrier bar;
     uint32_t count[3];  // entries listed by the phase, rotating (slot p % 3 is phase p's)
     uint32_t least[3];  // smallest support a scan left alive
+    uint32_t longs[3];  // edges put off by the phase
     // carried from launch to launch
     uint32_t k, round, top, phase, level_start, list, n;
     uint32_t alive;
@@ -794,6 +795,7 @@ struct TrussLoop {
     uint32_t listed;
     uint32_t* list0;
     uint32_t* list1;
+    uint32_t* longs;          // edges put off
     TrussState* st;
 };
 
@@ -811,6 +813,13 @@ constexpr int kTrussThreads = 1024;
 constexpr uint32_t kStage = 512;  // entries of the searched list a warp stages in shared memory
 constexpr int kTrussUnroll = 2;   // walked entries per lane in flight
 constexpr int kScanLoads = 4;     // listed edges per lane in flight in a scan
+// An edge of which a warp would walk more than this many entries is put off, and
+// the round's edges of that kind are then shared by all warps. Else a hub's edge is
+// one warp's while the others wait at the barrier: 4 hubs of 600,000 leaves, joined
+// to one another, 44.9 -> 11.7 ms. Limits of 2,048, 8,192 and 32,768 entries are alike
+// (R-MAT 19 30.6 to 31.9 ms with and without).
+constexpr uint32_t kLongWalk = 8192;
+constexpr uint32_t kMaxLogParts = 12;
 
 // Removes, with edge e, the triangles it makes with the live entries p1 and p2
 // (where hit). A triangle with several edges removed in this round is handled
@@ -852,10 +861,10 @@ __device__ __forceinline__ void truss_remove(const TrussLoop& a, uint32_t e, con
 
 // One removed edge (or the part-th of 2^log_parts slices of its walk): the
 // shorter live list is walked, the longer one searched, in shared memory where
-// it fits kStage entries.
+// it fits kStage entries. With `put_off`, a long walk is only listed there.
 __device__ __forceinline__ void truss_peel(const TrussLoop& a, uint32_t e, uint32_t part, uint32_t log_parts,
                                            uint32_t round, uint32_t k, uint32_t* s_y, uint32_t* next,
-                                           uint32_t* next_count) {
+                                           uint32_t* next_count, uint32_t* put_off) {
     const unsigned lane = lane_id();
     const uint32_t u = __ldg(a.src + e), v = __ldg(a.g_targets + e);
     uint32_t xs = __ldg(a.offsets + u), xn = __ldg(a.offsets + u + 1) - xs;
@@ -863,6 +872,10 @@ __device__ __forceinline__ void truss_peel(const TrussLoop& a, uint32_t e, uint3
     if (xn > yn) {
         uint32_t t = xs; xs = ys; ys = t;
         t = xn; xn = yn; yn = t;
+    }
+    if (put_off && xn >> log_parts > kLongWalk) {
+        if (part == 0 && lane == 0) a.longs[atomicAdd(put_off, 1u)] = e;
+        return;
     }
     const bool staged = yn <= kStage;
     if (staged) {
@@ -915,7 +928,7 @@ constexpr uint32_t kQueue = 32 * 32 + kDenseBatch;  // positions a warp queues: 
 
 __device__ __forceinline__ void truss_peel_dense(const TrussLoop& a, uint32_t e, uint32_t part, uint32_t log_parts,
                                                  uint32_t round, uint32_t k, uint32_t* s_queue, uint32_t* next,
-                                                 uint32_t* next_count) {
+                                                 uint32_t* next_count, uint32_t*) {
     const unsigned lane = lane_id();
     uint32_t u = __ldg(a.src + e), v = __ldg(a.g_targets + e);
     uint32_t pu = __ldg(a.offsets + u), du = __ldg(a.offsets + u + 1) - pu;
@@ -1012,7 +1025,7 @@ __device__ __forceinline__ void truss_peel_dense(const TrussLoop& a, uint32_t e,
 template <bool kDense>
 __global__ void __launch_bounds__(kTrussThreads, 1) kt_truss_loop_kernel(const TrussLoop a) {
     extern __shared__ uint32_t s_stage[];
-    __shared__ uint32_t s_count, s_least;
+    __shared__ uint32_t s_count, s_least, s_long;
     const unsigned lane = lane_id();
     uint32_t* s_warp = s_stage + (threadIdx.x >> 5) * (kDense ? kQueue : kStage);
     const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -1029,12 +1042,14 @@ __global__ void __launch_bounds__(kTrussThreads, 1) kt_truss_loop_kernel(const T
         const bool ok = grid_barrier(&a.st->bar, gridDim.x, barriers, [&] {
             s_count = __ldcg(a.st->count + slot);
             s_least = __ldcg(a.st->least + slot);
+            s_long = __ldcg(a.st->longs + slot);
         });
         ++phase;
         // Slot (phase + 1) % 3 was read two barriers ago.
         if (tid == 0) {
             a.st->count[(phase + 1) % 3] = 0;
             a.st->least[(phase + 1) % 3] = 0xFFFFFFFFu;
+            a.st->longs[(phase + 1) % 3] = 0;
         }
         return ok;
     };
@@ -1104,10 +1119,21 @@ __global__ void __launch_bounds__(kTrussThreads, 1) kt_truss_loop_kernel(const T
             if (__ldcg(a.support + e) == 0) continue;
             (kDense ? truss_peel_dense : truss_peel)(a, e, static_cast<uint32_t>(w) & ((1u << log_parts) - 1),
                                                      log_parts, round, k, s_warp, list ? a.list0 : a.list1,
-                                                     a.st->count + phase % 3);
+                                                     a.st->count + phase % 3, a.st->longs + phase % 3);
         }
         if (!end_phase()) return;
         n = s_count;
+        if (!kDense && s_long) {
+            // The edges put off, in as many parts as give every warp a few.
+            const uint32_t longs = s_long;
+            const uint32_t share = 4 * nwarps / longs;
+            const uint32_t parts = min(kMaxLogParts, share ? max(4u, 31 - __clz(share)) : 4u);
+            for (uint64_t w = warp; w < static_cast<uint64_t>(longs) << parts; w += nwarps)
+                truss_peel(a, __ldcg(a.longs + (w >> parts)), static_cast<uint32_t>(w) & ((1u << parts) - 1), parts, round, k,
+                           s_warp, (list ? a.list0 : a.list1) + n, a.st->count + phase % 3, nullptr);
+            if (!end_phase()) return;
+            n += s_count;
+        }
         list ^= 1u;
         level_start = false;
     }
@@ -1212,13 +1238,14 @@ Error truss_decomposition(GraphImpl& g, uint32_t* host_truss, uint32_t* max_trus
         st.bar = GridBarrier{};
         std::fill(st.count, st.count + 3, 0u);
         std::fill(st.least, st.least + 3, 0xFFFFFFFFu);
+        std::fill(st.longs, st.longs + 3, 0u);
         st.phase = 0;
         GCU_CUDA(cudaMemcpyAsync(loop_state.ptr, &st, sizeof(st), cudaMemcpyHostToDevice, dev.stream), "copy");
         const LiveBuffers& lv = live[cur];
         const TrussLoop a{lv.offsets.ptr, lv.targets.ptr, lv.eid.ptr,    lv.number.ptr,  lv.bits.ptr,
                           lv.before.ptr,  lv.span.ptr,    lv.numbers.ptr, lv.words,      g.targets.ptr,  src,
                           state.ptr,      support.ptr,    truss.ptr,     active[cur].ptr, listed,
-                          lists[0].ptr,   lists[1].ptr,   loop_state.ptr};
+                          lists[0].ptr,   lists[1].ptr,   active[cur ^ 1].ptr, loop_state.ptr};
         // One block per SM; fewer for a core too small to use them.
         const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(
             1, std::min<uint64_t>(dev.sm_count, ceil_div_u64(listed, kTrussThreads / 32))));
