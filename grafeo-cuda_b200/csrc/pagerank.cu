@@ -263,12 +263,14 @@ __global__ void pr_perm_degree_kernel(const uint32_t* __restrict__ offsets, cons
     }
 }
 
-Error degree_class_order(DeviceImpl& dev, const uint32_t* offsets, uint32_t V, DeviceBuffer<uint32_t>* inv) {
+Error degree_class_order(DeviceImpl& dev, const uint32_t* offsets, uint32_t V, DeviceBuffer<uint32_t>* inv,
+                         DeviceBuffer<uint32_t>* order) {
     GCU_TRY(inv->allocate(dev, std::max<uint32_t>(V, 1)));
     if (V == 0) return ok();
     const uint32_t nblk = static_cast<uint32_t>(ceil_div_u64(V, kClassBlock));
     const uint64_t ncount = static_cast<uint64_t>(kDegClasses) * nblk;
-    DeviceBuffer<uint32_t> counts, cpos, perm;
+    DeviceBuffer<uint32_t> counts, cpos, own;
+    DeviceBuffer<uint32_t>& perm = order ? *order : own;
     GCU_TRY(counts.allocate(dev, ncount));
     GCU_TRY(cpos.allocate(dev, ncount + 1));
     GCU_TRY(perm.allocate(dev, V));

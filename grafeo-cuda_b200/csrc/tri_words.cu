@@ -241,10 +241,17 @@ __global__ void tw_long_rows_kernel(const uint32_t* __restrict__ offsets, uint32
 
 // Longer rows, a CTA each: the ranks of the list are set in a bitmap,
 // bitmap_words * 32 of them at a time, and its non-zero words written out. Two
-// sweeps of the row where it has more than one window: the first counts.
+// sweeps of the row where it has more than one window: the first counts. A row is
+// read kRowLoads entries per thread at a time (one at a time, a hub of 2 M entries
+// took 5 ms). The longest rows are those of the lowest ranks, and the vertices that
+// rank below them few: where there are kSearchRatio times more entries than those,
+// they are looked up in the row instead (triangles of that star 5.8 -> 0.9 ms).
+constexpr int kRowLoads = 8;
+constexpr uint32_t kSearchRatio = 32;
+
 __global__ void __launch_bounds__(1024) tw_build_cta_kernel(
     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ rank,
-    uint32_t V, bool full, uint32_t bitmap_words, const uint32_t* __restrict__ rows,
+    const uint32_t* __restrict__ at_rank, uint32_t V, bool full, uint32_t bitmap_words, const uint32_t* __restrict__ rows,
     const uint32_t* __restrict__ n_rows, uint32_t* __restrict__ next, uint2* __restrict__ lists,
     uint2* __restrict__ words, unsigned long long* __restrict__ cursor) {
     extern __shared__ uint32_t s_bits[];
@@ -270,9 +277,27 @@ __global__ void __launch_bounds__(1024) tw_build_cta_kernel(
         for (uint32_t sweep = windows > 1 ? 0 : 1; sweep < 2; ++sweep) {
             for (uint32_t w = 0; w < max(windows, 1u); ++w) {
                 const uint32_t lo = w * window, hi = min(end - lo, window) + lo;
-                for (uint64_t j = static_cast<uint64_t>(s) + threadIdx.x; j < e; j += blockDim.x) {
-                    const uint32_t x = __ldg(rank + ld_stream(targets + j));
-                    if (x >= lo && x < hi && x != r) atomicOr(s_bits + ((x - lo) >> 5), 1u << (x & 31));
+                if (!full && (e - s) / kSearchRatio > r) {
+                    for (uint32_t x = lo + threadIdx.x; x < hi; x += blockDim.x) {
+                        const uint32_t v = __ldg(at_rank + x), p = lower_bound_u32(targets, s, e, v);
+                        if (p < e && targets[p] == v) atomicOr(s_bits + ((x - lo) >> 5), 1u << (x & 31));
+                    }
+                } else {
+                    for (uint64_t j = static_cast<uint64_t>(s) + threadIdx.x; j < e; j += kRowLoads * blockDim.x) {
+                        uint32_t x[kRowLoads];
+#pragma unroll
+                        for (int q = 0; q < kRowLoads; ++q) {
+                            const uint64_t i = j + static_cast<uint64_t>(q) * blockDim.x;
+                            x[q] = ld_nc_if(i < e, targets + i, 0u);
+                        }
+#pragma unroll
+                        for (int q = 0; q < kRowLoads; ++q)
+                            x[q] = ld_nc_if(j + static_cast<uint64_t>(q) * blockDim.x < e, rank + x[q], r);
+#pragma unroll
+                        for (int q = 0; q < kRowLoads; ++q)
+                            if (x[q] >= lo && x[q] < hi && x[q] != r)
+                                atomicOr(s_bits + ((x[q] - lo) >> 5), 1u << (x[q] & 31));
+                    }
                 }
                 __syncthreads();
                 const uint32_t used = (hi - lo + 31) / 32;
@@ -618,7 +643,8 @@ Error build_word_lists(GraphImpl& g, bool full, WordLists* w) {
     DeviceImpl& dev = *g.dev;
     const uint32_t V = g.num_nodes, E = g.num_edges;
     const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
-    GCU_TRY(degree_class_order(dev, g.offsets.ptr, V, &w->rank));
+    DeviceBuffer<uint32_t> at_rank;
+    GCU_TRY(degree_class_order(dev, g.offsets.ptr, V, &w->rank, &at_rank));
     GCU_TRY(w->lists.allocate(dev, V));
     // An edge's ranks are kept at one end, or at both: E / 2 or E words at most,
     // and a padding word per list (lists without words take no room).
@@ -653,7 +679,7 @@ Error build_word_lists(GraphImpl& g, bool full, WordLists* w) {
     const unsigned cgrid = static_cast<unsigned>(
         std::max<uint64_t>(1, std::min<uint64_t>(E / kWarpRow, static_cast<uint64_t>(dev.sm_count) * resident)));
     GCU_LAUNCH(dev, "tw_build_cta", tw_build_cta_kernel, cgrid, threads, smem, g.offsets.ptr, g.targets.ptr,
-               w->rank.ptr, V, full, bitmap_words, w->warp_owners.ptr, w->counts.ptr, w->counts.ptr + 1, w->lists.ptr,
+               w->rank.ptr, at_rank.ptr, V, full, bitmap_words, w->warp_owners.ptr, w->counts.ptr, w->counts.ptr + 1, w->lists.ptr,
                w->words.ptr, cursor.ptr);
     // Items: at most one per kSlice entries plus one per vertex with more words,
     // so more neighbours, than a warp owner.
