@@ -277,7 +277,7 @@ Error upload_and_validate_csr(DeviceImpl& dev, const uint32_t* d_offsets, uint32
 // New id of every vertex in the stable partition by degree class (class c:
 // list lengths in [2^(c-1), 2^c)), highest class first: the order the
 // PageRank plan relabels by, and the triangle count orients by. With `order`, also
-// the vertex of every new id.
+// the vertex of every new id and, at [V], the first new id of one entry or none.
 Error degree_class_order(DeviceImpl& dev, const uint32_t* offsets, uint32_t V, DeviceBuffer<uint32_t>* inv,
                          DeviceBuffer<uint32_t>* order = nullptr);
 
