@@ -651,7 +651,7 @@ uint32_t support_bitmap_words(uint32_t V) {
 
 }  // namespace
 
-Error build_word_lists(GraphImpl& g, bool full, WordLists* w) {
+Error build_word_lists(GraphImpl& g, bool full, WordLists* w, uint64_t* n_words) {
     DeviceImpl& dev = *g.dev;
     const uint32_t V = g.num_nodes, E = g.num_edges;
     const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
@@ -701,6 +701,10 @@ Error build_word_lists(GraphImpl& g, bool full, WordLists* w) {
     GCU_TRY(w->items.allocate(dev, w->max_items));
     GCU_LAUNCH(dev, "tw_owners", tw_owners_kernel, vgrid, 256, 0, g.offsets.ptr, w->lists.ptr, V, warp_words,
                w->warp_owners.ptr, w->counts.ptr + 2, w->items.ptr, w->counts.ptr + 3);
+    if (n_words) {
+        GCU_CUDA(cudaMemcpyAsync(n_words, cursor.ptr, sizeof(uint64_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
+        GCU_TRY(dev.sync());
+    }
     return ok();
 }
 
