@@ -515,7 +515,9 @@ struct WordCount {
 };
 
 // Blocks take the CTA items first, then their warps take the warp owners: the
-// end of the one fills the idle warps with the other.
+// end of the one fills the idle warps with the other. Everyone's first turn is its
+// own number and only what is beyond those is handed out by counters: on a small graph
+// the atomics on them were a third of a count (8 graphs of 1,000 vertices 27 -> 21 us).
 template <bool kSupport, int kThreads, int kCtasPerSm>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) tw_count_kernel(
     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ targets, const uint32_t* __restrict__ rank,
@@ -535,9 +537,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) tw_count_kernel(
     unsigned long long sum = 0;
     if (n_items)
         for (uint32_t k = threadIdx.x; k < bitmap_words; k += kThreads) s_bits[k] = 0;
-    while (true) {
+    for (uint32_t turn = 0;; ++turn) {
         __syncthreads();
-        if (threadIdx.x == 0) s_item = atomicAdd(next, 1u);
+        if (threadIdx.x == 0)
+            s_item = turn == 0 ? blockIdx.x : gridDim.x < n_items ? gridDim.x + atomicAdd(next, 1u) : n_items;
         __syncthreads();
         if (s_item >= n_items) break;
         const uint2 item = items[s_item];
@@ -597,11 +600,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) tw_count_kernel(
     }
     table += warp << kWarpBits;  // the warps' own tables from here on (after the loop's block barrier)
     auto store = [&](uint32_t entry, uint32_t h) { out.support[entry] = h; };
-    while (true) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(next + 1, batch);
-        base = __shfl_sync(kFullMask, base, 0);
-        if (base >= n_owners) break;
+    const uint32_t own_turns = gridDim.x * (kThreads / 32) * batch;
+    for (uint32_t base = (blockIdx.x * (kThreads / 32) + warp) * batch; base < n_owners;) {
         const uint32_t last = min(base + batch, n_owners);
         for (uint32_t h = base; h < last; ++h) {
             const uint32_t u = owners[h];
@@ -628,6 +628,9 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) tw_count_kernel(
             });
             if (!kSupport) add_owner(u, hits, out.per_vertex, sum);
         }
+        if (own_turns >= n_owners) break;
+        if (lane == 0) base = own_turns + atomicAdd(next + 1, batch);
+        base = __shfl_sync(kFullMask, base, 0);
     }
     if (!kSupport) {
         sum = warp_sum(sum);
