@@ -427,8 +427,7 @@ static Error compact_live(DeviceImpl& dev, uint32_t V, const LiveCsr& lv, uint32
     if (out->entries > 0)
         GCU_LAUNCH(dev, "kt_live_fill", kt_live_fill_kernel, tiles, 256, 0, lv, V, L, rev, pos.ptr, out->targets.ptr,
                    out->eid.ptr);
-    GCU_TRY(dev.sync());  // pos is freed on return
-    return ok();
+    return ok();  // pos is freed in stream order
 }
 
 // Number and row bit of every live entry.
@@ -484,10 +483,11 @@ __global__ void kt_has_entries_kernel(const uint32_t* __restrict__ offsets, uint
 // and where there is no memory for it.
 constexpr uint32_t kDenseRows = 65535;
 constexpr uint32_t kDenseWords = 8;
+constexpr uint32_t kDenseEntries = 65536;  // live entries that are worth its launches
 
 static Error live_matrix(DeviceImpl& dev, uint32_t V, LiveBuffers* lv) {
     lv->words = 0;
-    if (lv->entries == 0) return ok();
+    if (lv->entries < kDenseEntries) return ok();
     const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
     GCU_TRY(lv->number.allocate(dev, static_cast<uint64_t>(V) + 1));
     GCU_LAUNCH(dev, "kt_has_entries", kt_has_entries_kernel,
@@ -819,6 +819,10 @@ constexpr int kScanLoads = 4;     // listed edges per lane in flight in a scan
 // to one another, 44.9 -> 11.7 ms. Limits of 2,048, 8,192 and 32,768 entries are alike
 // (R-MAT 19 30.6 to 31.9 ms with and without).
 constexpr uint32_t kLongWalk = 8192;
+// Active edges that are not worth a compaction (some 100 us of launches and waits):
+// 2,000 vertices and 16,000 edges 0.49 -> 0.17 ms with kDenseEntries, R-MAT 14 5.5 ->
+// 4.5; with 32,768 edges 0.17 and 4.7, with 524,288 0.17 and 5.0.
+constexpr uint32_t kCompactEdges = 131072;
 constexpr uint32_t kMaxLogParts = 12;
 
 // Removes, with edge e, the triangles it makes with the live entries p1 and p2
@@ -1053,8 +1057,8 @@ __global__ void __launch_bounds__(kTrussThreads, 1) kt_truss_loop_kernel(const T
         }
         return ok;
     };
-    // Half of the active list gone: the host compacts it and the live lists.
-    while (alive > 0 && 2ull * alive >= a.listed) {
+    // Half of a long active list gone: the host compacts it and the live lists.
+    while (alive > 0 && (a.listed <= kCompactEdges || 2ull * alive >= a.listed)) {
         ++round;
         if (level_start) {
             uint32_t least = 0xFFFFFFFFu;
@@ -1161,6 +1165,16 @@ __global__ void kt_truss_spread_kernel(const uint32_t* __restrict__ targets, con
     }
 }
 
+template <class Kernel>
+static Error fit_truss_loop(Kernel kernel, size_t smem) {
+    GCU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+             "cudaFuncSetAttribute");
+    int per_sm = 0;
+    GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTrussThreads, smem), "occupancy");
+    if (per_sm < 1) return kernel_error("truss decomposition: the loop kernel does not fit an SM");
+    return ok();
+}
+
 // Trussness of every edge of a symmetric CSR: the peeling of k_truss_symmetric
 // continued level by level without restarting. At level k the rounds remove
 // every alive edge with fewer than k - 2 alive triangles until none is left
@@ -1212,21 +1226,6 @@ Error truss_decomposition(GraphImpl& g, uint32_t* host_truss, uint32_t* max_trus
     GCU_TRY(live_matrix(dev, g.num_nodes, &live[0]));
     constexpr size_t kListSmem = sizeof(uint32_t) * kStage * (kTrussThreads / 32);
     constexpr size_t kDenseSmem = sizeof(uint32_t) * kQueue * (kTrussThreads / 32);
-    GCU_CUDA(cudaFuncSetAttribute(kt_truss_loop_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(kListSmem)),
-             "cudaFuncSetAttribute");
-    GCU_CUDA(cudaFuncSetAttribute(kt_truss_loop_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(kDenseSmem)),
-             "cudaFuncSetAttribute");
-    int per_sm = 0, per_sm_dense = 0;
-    GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kt_truss_loop_kernel<false>, kTrussThreads,
-                                                           kListSmem),
-             "occupancy");
-    GCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_dense, kt_truss_loop_kernel<true>, kTrussThreads,
-                                                           kDenseSmem),
-             "occupancy");
-    if (per_sm < 1 || per_sm_dense < 1)
-        return kernel_error("truss decomposition: the loop kernel does not fit an SM");
     TrussState st{};
     st.k = 3;
     st.top = edges > 0 ? 2 : 0;
@@ -1249,8 +1248,13 @@ Error truss_decomposition(GraphImpl& g, uint32_t* host_truss, uint32_t* max_trus
         // One block per SM; fewer for a core too small to use them.
         const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(
             1, std::min<uint64_t>(dev.sm_count, ceil_div_u64(listed, kTrussThreads / 32))));
-        if (lv.words) GCU_LAUNCH_COOP(dev, "kt_truss_dense", kt_truss_loop_kernel<true>, grid, kTrussThreads, kDenseSmem, a);
-        else GCU_LAUNCH_COOP(dev, "kt_truss_loop", kt_truss_loop_kernel<false>, grid, kTrussThreads, kListSmem, a);
+        if (lv.words) {
+            GCU_TRY(fit_truss_loop(kt_truss_loop_kernel<true>, kDenseSmem));
+            GCU_LAUNCH_COOP(dev, "kt_truss_dense", kt_truss_loop_kernel<true>, grid, kTrussThreads, kDenseSmem, a);
+        } else {
+            GCU_TRY(fit_truss_loop(kt_truss_loop_kernel<false>, kListSmem));
+            GCU_LAUNCH_COOP(dev, "kt_truss_loop", kt_truss_loop_kernel<false>, grid, kTrussThreads, kListSmem, a);
+        }
         GCU_CUDA(cudaMemcpyAsync(&st, loop_state.ptr, sizeof(st), cudaMemcpyDeviceToHost, dev.stream), "copy");
         GCU_TRY(dev.sync());
         if (st.bar.failed) return kernel_error("truss decomposition: a block did not reach the grid barrier");
