@@ -34,6 +34,9 @@ count ride along (computed outside the timed region).
          k-truss sweep k = 3..8 on R-MAT 22 (seed 2) and Erdos-Renyi 2^22
          (seed 3).
 
+The algorithms and harness blocks, and what else explains the line's figures, go
+to stderr as one more JSON document ("details"); the line itself stays short.
+
 `--impl reference` times the reference's CPU implementation of the path (the
 oracle port; Grafeo's own Rust crate cannot be built here) on the same metric
 and configuration; its graph comes from the oracle's own generator, so it
@@ -98,6 +101,27 @@ def parse_args():
                          "degree-class relabelling) of the R-MAT directed copy at --scale (24: seed 5, 22: seed 2), "
                          "device ms per kernel, median of 4 builds; one JSON document")
     return ap.parse_args()
+
+
+# What a line says beyond its figures: on stderr, so that the last line of stdout
+# stays short enough for readers that keep its tail only.
+DETAILS = (("algorithms",), ("harness",), ("kernel_ms_per_step",), ("graph_preparation_s",), ("e2e", "what"),
+           ("e2e", "breakdown"), ("accuracy", "oracle"), ("roofline", "traffic_is"),
+           ("roofline", "kernel_ms_per_step"), ("roofline", "frac_of_8tbs_spec"), ("roofline", "share_of_step"),
+           ("roofline", "launches_per_step"), ("roofline", "working_launches_per_step"))
+
+
+def split_details(line: dict) -> tuple[dict, dict]:
+    """The line without DETAILS, and those, under the same keys."""
+    short = {k: dict(v) if isinstance(v, dict) else v for k, v in line.items()}
+    details: dict = {}
+    for path in DETAILS:
+        at, to = short, details
+        for key in path[:-1]:
+            at, to = at.get(key, {}), to.setdefault(key, {})
+        if path[-1] in at:
+            to[path[-1]] = at.pop(path[-1])
+    return short, {k: v for k, v in details.items() if v != {}}
 
 
 # ---------------------------------------------------------------- distributed plumbing
@@ -899,6 +923,8 @@ def main():
     try:
         line = run_reference(args, d) if args.impl == "reference" else run_ours(args, d)
         if d.rank == 0 and line is not None:
+            line, details = split_details(line)
+            print(json.dumps({"details": details}), file=sys.stderr, flush=True)
             print(json.dumps(line), flush=True)
     finally:
         d.close()
