@@ -863,7 +863,9 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtasPerSm) batch_ppr_kern
 // ---------------------------------------------------------------- small graphs: a block each
 
 // The small graphs, largest first; a block takes the next one when it is done. A
-// row of up to kSoloRow entries is a lane's, a longer one its warp's.
+// row of up to kSoloRow entries is a lane's, a longer one its warp's. The walks
+// count from a graph's first vertex and a row's first entry: a union may end
+// within a block's step of 2^32 vertices or entries.
 struct BatchSmall {
     const uint32_t* offsets;
     const uint32_t* targets;
@@ -905,7 +907,8 @@ __global__ void __launch_bounds__(kThreads) batch_small_bfs_kernel(const BatchSm
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     for_each_small(a.small, [&](const BatchGraph& g) {
         const uint64_t base = static_cast<uint64_t>(g.id) * a.S;
-        for (uint32_t v = g.v_begin + threadIdx.x; v < g.v_end; v += kThreads) a.mask_a[v] = 0;
+        const uint32_t n = g.v_end - g.v_begin;
+        for (uint32_t i = threadIdx.x; i < n; i += kThreads) a.mask_a[g.v_begin + i] = 0;
         if (threadIdx.x < kMaxBatchSources) s_count[threadIdx.x] = 0;
         __syncthreads();
         if (threadIdx.x < a.S) {
@@ -919,10 +922,11 @@ __global__ void __launch_bounds__(kThreads) batch_small_bfs_kernel(const BatchSm
         int32_t depth = 0;  // of source threadIdx.x
         for (int32_t level = 0;; ++level) {
             uint32_t fresh = 0;
-            for (uint32_t b = g.v_begin + warp * 32; b < g.v_end; b += kThreads) {
-                const uint32_t v = b + lane;
+            for (uint32_t b = warp * 32; b < n; b += kThreads) {
+                const bool real = b + lane < n;
+                const uint32_t v = g.v_begin + b + lane;
                 uint32_t old = a.full, s = 0, e = 0;
-                if (v < g.v_end) {
+                if (real) {
                     old = in[v];
                     s = __ldg(a.small.offsets + v);
                     e = __ldg(a.small.offsets + v + 1);
@@ -933,17 +937,18 @@ __global__ void __launch_bounds__(kThreads) batch_small_bfs_kernel(const BatchSm
                     for (uint32_t j = s; j < e && (m | old) != a.full; ++j) m |= in[__ldg(a.small.targets + j)];
                 for (unsigned longs = __ballot_sync(kFullMask, open && e - s > kSoloRow); longs; longs &= longs - 1) {
                     const int l = __ffs(longs) - 1;
-                    const uint32_t ls = __shfl_sync(kFullMask, s, l), le = __shfl_sync(kFullMask, e, l);
+                    const uint32_t len = __shfl_sync(kFullMask, e - s, l);
+                    const uint32_t* list = a.small.targets + __shfl_sync(kFullMask, s, l);
                     const uint32_t lold = __shfl_sync(kFullMask, old, l);
                     uint32_t got = 0;
-                    for (uint32_t j = ls; j < le && (got | lold) != a.full; j += 64) {
-                        uint32_t x = j + lane < le ? in[__ldg(a.small.targets + j + lane)] : 0u;
-                        if (j + 32 + lane < le) x |= in[__ldg(a.small.targets + j + 32 + lane)];
+                    for (uint32_t o = lane; o - lane < len && (got | lold) != a.full; o += 64) {
+                        uint32_t x = o < len ? in[__ldg(list + o)] : 0u;
+                        if (o + 32 < len) x |= in[__ldg(list + o + 32)];
                         got |= __reduce_or_sync(kFullMask, x);
                     }
                     if (static_cast<int>(lane) == l) m = got;
                 }
-                if (v < g.v_end) {
+                if (real) {
                     const uint32_t now = m & ~old;
                     out[v] = old | m;
                     batch_label(a.dist, a.V, v, now, level + 1);
@@ -963,11 +968,11 @@ __global__ void __launch_bounds__(kThreads) batch_small_bfs_kernel(const BatchSm
         }
         // Reached vertices per source: lane k of every warp counts bit k.
         uint32_t cnt = 0;
-        for (uint32_t b = g.v_begin + warp * 32; b < g.v_end; b += kThreads) {
-            const uint32_t vis = b + lane < g.v_end ? in[b + lane] : 0u;
+        for (uint32_t b = warp * 32; b < n; b += kThreads) {
+            const uint32_t vis = b + lane < n ? in[g.v_begin + b + lane] : 0u;
             for (uint32_t k = 0; k < a.S; ++k) {
-                const unsigned n = __ballot_sync(kFullMask, (vis >> k) & 1u);
-                if (lane == k) cnt += __popc(n);
+                const unsigned some = __ballot_sync(kFullMask, (vis >> k) & 1u);
+                if (lane == k) cnt += __popc(some);
             }
         }
         if (lane < a.S && cnt) atomicAdd(&s_count[lane], cnt);
@@ -1010,9 +1015,11 @@ __global__ void __launch_bounds__(kThreads) batch_small_ppr_kernel(const BatchSm
         parity ^= 1u;
     };
     for_each_small(a.small, [&](const BatchGraph& g) {
-        const float r0 = 1.0f / static_cast<float>(g.v_end - g.v_begin);
+        const uint32_t n = g.v_end - g.v_begin;
+        const float r0 = 1.0f / static_cast<float>(n);
         double mass = 0.0, change = 0.0;
-        for (uint32_t v = g.v_begin + threadIdx.x; v < g.v_end; v += kThreads) {
+        for (uint32_t i = threadIdx.x; i < n; i += kThreads) {
+            const uint32_t v = g.v_begin + i;
             const uint32_t deg = __ldg(a.small.offsets + v + 1) - __ldg(a.small.offsets + v);
             a.ranks[v] = r0;
             a.contrib_a[v] = deg ? r0 / static_cast<float>(deg) : 0.f;
@@ -1022,15 +1029,16 @@ __global__ void __launch_bounds__(kThreads) batch_small_ppr_kernel(const BatchSm
         const float* in = a.contrib_a;
         float* out = a.contrib_b;
         uint32_t it = 0;
-        bool conv = g.v_end == g.v_begin;
+        bool conv = n == 0;
         while (!conv && it < a.max_iterations) {
             double dangling = 0.0;
             change = 0.0;
-            for (uint32_t b = g.v_begin + warp * 32; b < g.v_end; b += kThreads) {
-                const uint32_t v = b + lane;
+            for (uint32_t b = warp * 32; b < n; b += kThreads) {
+                const bool real = b + lane < n;
+                const uint32_t v = g.v_begin + b + lane;
                 uint32_t s = 0, e = 0;
                 float tele = 0.f, old = 0.f;
-                if (v < g.v_end) {
+                if (real) {
                     s = __ldg(a.small.offsets + v);
                     e = __ldg(a.small.offsets + v + 1);
                     tele = __ldg(a.tele + v);
@@ -1041,14 +1049,14 @@ __global__ void __launch_bounds__(kThreads) batch_small_ppr_kernel(const BatchSm
                     for (uint32_t j = s; j < e; ++j) sum += static_cast<double>(in[__ldg(a.small.targets + j)]);
                 for (unsigned longs = __ballot_sync(kFullMask, e - s > kSoloRow); longs; longs &= longs - 1) {
                     const int l = __ffs(longs) - 1;
-                    const uint32_t ls = __shfl_sync(kFullMask, s, l), le = __shfl_sync(kFullMask, e, l);
+                    const uint32_t len = __shfl_sync(kFullMask, e - s, l);
+                    const uint32_t* list = a.small.targets + __shfl_sync(kFullMask, s, l);
                     double part = 0.0;
-                    for (uint32_t j = ls + lane; j < le; j += 32)
-                        part += static_cast<double>(in[__ldg(a.small.targets + j)]);
+                    for (uint32_t o = lane; o < len; o += 32) part += static_cast<double>(in[__ldg(list + o)]);
                     part = warp_sum(part);
                     if (static_cast<int>(lane) == l) sum = part;
                 }
-                if (v < g.v_end) {
+                if (real) {
                     const float x = batch_rank(a.damp, sum, static_cast<double>(tele), mass);
                     change += fabs(static_cast<double>(x) - static_cast<double>(old));
                     a.ranks[v] = x;
