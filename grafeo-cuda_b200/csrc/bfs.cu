@@ -81,17 +81,14 @@ struct BfsSearchState;
 struct BfsWork {
     DeviceBuffer<int32_t> dist;
     DeviceBuffer<uint32_t> visited;
-    DeviceBuffer<uint32_t> bitmap[2];
-    DeviceBuffer<uint32_t> queue[2];       // vertices, or the one-launch search's items (uint2)
-    DeviceBuffer<uint32_t> degree_scan;  // V + 1
-    DeviceBuffer<BfsCounters> counters;
-    BfsCounters host_counters{};  // host copy, read after a synchronisation (plain memory)
     int symmetric = -1;                    // -1 unknown, 0 no, 1 yes
     DeviceBuffer<uint32_t> active;         // vertices with edges, ascending (symmetric graphs)
     uint32_t n_active = 0;
     bool pull_list = false;                // the pull walks `active` instead of every bitmap word
-    // one-launch search
+    // one-launch search (ensure_search)
+    bool search_ready = false;
     DeviceBuffer<uint32_t> search_bitmaps;  // three
+    DeviceBuffer<uint2> items[2];
     DeviceBuffer<uint4> search_segments;
     uint32_t search_epoch = 0;
     DeviceBuffer<BfsSearchState> search;
@@ -101,6 +98,13 @@ struct BfsWork {
         int32_t level;
         uint32_t failed;
     } host_search{};
+    // level by level, driven by the device or the host, and the trace (ensure_levels)
+    bool levels_ready = false;
+    DeviceBuffer<uint32_t> bitmap[2];
+    DeviceBuffer<uint32_t> queue[2];
+    DeviceBuffer<uint32_t> degree_scan;  // V + 1
+    DeviceBuffer<BfsCounters> counters;
+    BfsCounters host_counters{};  // host copy, read after a synchronisation (plain memory)
     // device-driven level loop (built on first use, per schedule network)
     DeviceBuffer<BfsDevState> loop_state;
     DeviceBuffer<uint32_t> loop_scan_sums;
@@ -1547,42 +1551,60 @@ static Error ensure_work(GraphImpl& g) {
     const uint64_t V = g.num_nodes, words = ceil_div_u64(V, 32);
     GCU_TRY(w->dist.allocate(dev, V));
     GCU_TRY(w->visited.allocate(dev, words));
-    GCU_TRY(w->bitmap[0].allocate(dev, words));
-    GCU_TRY(w->bitmap[1].allocate(dev, words));
-    GCU_TRY(w->search_bitmaps.allocate(dev, 3 * words));
-    // At most one item per labelled vertex plus one per kItemEdges entries.
-    const uint64_t queue_words = 2 * (V + static_cast<uint64_t>(g.num_edges) / kItemEdges + 1);
-    GCU_TRY(w->queue[0].allocate(dev, queue_words));
-    GCU_TRY(w->queue[1].allocate(dev, queue_words));
-    GCU_TRY(w->search_segments.allocate(dev, 2 * static_cast<size_t>(kGroupBlocks) * kGroupItems));
-    GCU_TRY(clear_segments(dev, *w));
-    GCU_TRY(w->search.allocate(dev, 1));
-    GCU_TRY(w->degree_scan.allocate(dev, V + 1));
-    GCU_TRY(w->counters.allocate(dev, 1));
     // Bottom-up steps read in-neighbours; they equal the CSR lists only when
     // the CSR is symmetric (checked once per graph).
     bool sym = false;
     GCU_TRY(graph_symmetry(g, &sym));
     w->symmetric = sym ? 1 : 0;
     if (sym && V > 0) {
-        // degree_scan is free until the first balanced push: flags, then positions.
+        DeviceBuffer<uint32_t> pos;  // flags, then positions
+        GCU_TRY(pos.allocate(dev, V + 1));
         const unsigned grid = static_cast<unsigned>(
             std::min<uint64_t>(ceil_div_u64(V, 256), static_cast<uint64_t>(dev.sm_count) * 16));
         GCU_LAUNCH(dev, "bfs_has_edges", bfs_has_edges_kernel, grid, 256, 0, g.offsets.ptr, static_cast<uint32_t>(V),
-                   w->degree_scan.ptr);
-        GCU_TRY(exclusive_scan_u32(dev, w->degree_scan.ptr, w->degree_scan.ptr, V));
+                   pos.ptr);
+        GCU_TRY(exclusive_scan_u32(dev, pos.ptr, pos.ptr, V));
         uint32_t n = 0;
-        GCU_CUDA(cudaMemcpyAsync(&n, w->degree_scan.ptr + V, sizeof(n), cudaMemcpyDeviceToHost, dev.stream), "copy");
+        GCU_CUDA(cudaMemcpyAsync(&n, pos.ptr + V, sizeof(n), cudaMemcpyDeviceToHost, dev.stream), "copy");
         GCU_TRY(dev.sync());
         w->n_active = n;
         w->pull_list = V - n >= V / kBuListFraction;
         if (w->pull_list) {
             GCU_TRY(w->active.allocate(dev, std::max<uint32_t>(n, 1)));
             GCU_LAUNCH(dev, "bfs_active_scatter", bfs_active_scatter_kernel, grid, 256, 0, g.offsets.ptr,
-                       static_cast<uint32_t>(V), w->degree_scan.ptr, w->active.ptr);
+                       static_cast<uint32_t>(V), pos.ptr, w->active.ptr);
         }
     }
     g.bfs_work = w.release();
+    return ok();
+}
+
+// What the one-launch search works in, and what the levels by themselves do: a
+// program that runs one form does not hold the other's (up to 24 bytes per vertex and
+// 20; 36 with both).
+static Error ensure_search(GraphImpl& g, BfsWork& w) {
+    if (w.search_ready) return ok();
+    DeviceImpl& dev = *g.dev;
+    const uint64_t V = g.num_nodes;
+    GCU_TRY(w.search_bitmaps.allocate(dev, 3 * ceil_div_u64(V, 32)));
+    // At most one item per labelled vertex plus one per kItemEdges entries.
+    for (auto& q : w.items) GCU_TRY(q.allocate(dev, V + g.num_edges / kItemEdges + 1));
+    GCU_TRY(w.search_segments.allocate(dev, 2 * static_cast<size_t>(kGroupBlocks) * kGroupItems));
+    GCU_TRY(clear_segments(dev, w));
+    GCU_TRY(w.search.allocate(dev, 1));
+    w.search_ready = true;
+    return ok();
+}
+
+static Error ensure_levels(GraphImpl& g, BfsWork& w) {
+    if (w.levels_ready) return ok();
+    DeviceImpl& dev = *g.dev;
+    const uint64_t V = g.num_nodes;
+    for (auto& b : w.bitmap) GCU_TRY(b.allocate(dev, ceil_div_u64(V, 32)));
+    for (auto& q : w.queue) GCU_TRY(q.allocate(dev, V));
+    GCU_TRY(w.degree_scan.allocate(dev, V + 1));
+    GCU_TRY(w.counters.allocate(dev, 1));
+    w.levels_ready = true;
     return ok();
 }
 
@@ -1897,8 +1919,8 @@ Error run_search(GraphImpl& g, BfsWork& w, uint32_t source) {
     a.visited = w.visited.ptr;
     a.bitmaps = w.search_bitmaps.ptr;
     a.bitmap_words = static_cast<uint32_t>(ceil_div_u64(g.num_nodes, 32));
-    a.queue0 = reinterpret_cast<uint2*>(w.queue[0].ptr);
-    a.queue1 = reinterpret_cast<uint2*>(w.queue[1].ptr);
+    a.queue0 = w.items[0].ptr;
+    a.queue1 = w.items[1].ptr;
     a.segments = w.search_segments.ptr;
     if (++w.search_epoch == 0) {  // the numbers begin again
         GCU_TRY(clear_segments(dev, w));
@@ -1933,15 +1955,21 @@ Error bfs(GraphImpl& g, uint32_t source, int32_t* host_distances, uint32_t* reac
     if (net) GCU_TRY(degree_stats(g, &stats));
 
     if (dev.bfs_device_loop && !dev.kernel_timing && !net) {
-        GCU_TRY(run_search(g, w, source));
-        if (host_distances)
-            GCU_TRY(copy_to_host(dev, host_distances, w.dist.ptr, sizeof(int32_t) * g.num_nodes));
-        GCU_TRY(dev.sync());
-        if (w.host_search.failed) return kernel_error("BFS stopped on an impossible state");
-        *reachable = w.host_search.reached;
-        *max_depth = w.host_search.level;
-        return ok();
+        const Error ready = ensure_search(g, w);
+        if (ready.ok()) {
+            GCU_TRY(run_search(g, w, source));
+            if (host_distances)
+                GCU_TRY(copy_to_host(dev, host_distances, w.dist.ptr, sizeof(int32_t) * g.num_nodes));
+            GCU_TRY(dev.sync());
+            if (w.host_search.failed) return kernel_error("BFS stopped on an impossible state");
+            *reachable = w.host_search.reached;
+            *max_depth = w.host_search.level;
+            return ok();
+        }
+        if (ready.status != GCU_ERR_OUT_OF_MEMORY) return ready;
+        for (auto& q : w.items) q.reset();  // the levels need less
     }
+    GCU_TRY(ensure_levels(g, w));
     if (dev.bfs_device_loop && !dev.kernel_timing && !w.loop_unavailable) {
         if (!w.loop_exec || w.loop_net != static_cast<const void*>(net)) {
             // A driver that cannot build the conditional graph leaves the
@@ -1998,6 +2026,7 @@ Error bfs_trace(GraphImpl& g, uint32_t source, uint64_t explore_seed, std::vecto
     DeviceImpl& dev = *g.dev;
     GCU_TRY(ensure_work(g));
     BfsWork& w = *g.bfs_work;
+    GCU_TRY(ensure_levels(g, w));
     const bool sym = w.symmetric == 1;
     const unsigned valid = valid_variants(sym);
     DegreeStats stats;
