@@ -12,10 +12,10 @@
 #include <cstring>
 #include <functional>
 #include <sstream>
-#include <system_error>
 #include <thread>
 
 #include "gcu_internal.h"
+#include "host_workers.h"
 
 namespace gcu {
 
@@ -82,24 +82,7 @@ namespace {
 constexpr size_t kStageMin = size_t(4) << 20;
 constexpr size_t kStageUploadMin = size_t(16) << 20;
 constexpr size_t kStageUploadFew = size_t(64) << 20;
-constexpr unsigned kStageWorkers = 8;
-
-// Runs work(worker, workers) on the calling thread and up to workers - 1 others;
-// fewer where a thread cannot be started (each takes chunks until none is left).
-template <class Work>
-void run_workers(unsigned workers, const Work& work) {
-    std::thread pool[kStageWorkers];
-    for (unsigned t = 1; t < workers; ++t) {
-        try {
-            pool[t] = std::thread([&work, t] { work(t); });
-        } catch (const std::system_error&) {
-            break;
-        }
-    }
-    work(0);
-    for (auto& t : pool)
-        if (t.joinable()) t.join();
-}
+constexpr unsigned kStageWorkers = kMaxWorkers;
 
 unsigned stage_workers(unsigned wanted) {
     return std::min({wanted, kStageWorkers, std::max(1u, std::thread::hardware_concurrency())});
