@@ -547,7 +547,7 @@ struct alignas(16) BfsSlot {
     uint32_t discovered;          // vertices of the new frontier
     uint32_t items;               // its items (push)
     unsigned long long explored;  // stretch: out-edges of every vertex it labelled
-    uint32_t levels;              // stretch: levels it advanced
+    uint32_t levels;              // stretch: levels it advanced; items: whether some list made several
     uint32_t reached;             // stretch: vertices it labelled
 };
 
@@ -619,19 +619,24 @@ __device__ __forceinline__ uint32_t* search_bitmap(const BfsSearch& a, uint32_t 
 __device__ __forceinline__ uint2* search_queue(const BfsSearch& a, uint32_t i) { return i ? a.queue1 : a.queue0; }
 
 // Expands the q items of the frontier with the warps warp, warp + nwarps, ...
-// of the blocks at work; new items go to slot `*count` onwards of g_out.
-__device__ __forceinline__ void push_items(const BfsSearch& a, const uint2* g_in, uint32_t q, uint2* g_out,
-                                           uint32_t* count, int32_t next_level, uint32_t warp, uint32_t nwarps,
+// of the blocks at work; new items go to the slot's `items` onwards of g_out. A warp
+// takes consecutive items, whose lists are often neighbours in memory, but with
+// `spread` items that are far apart: the items of a long list are consecutive, and
+// 32 of them were one warp's while the others waited (a directed CSR of 4 hubs and
+// 600,000 leaves: 700 of the level's 740 us).
+__device__ __forceinline__ void push_items(const BfsSearch& a, const uint2* g_in, uint32_t q, bool spread, uint2* g_out,
+                                           BfsSlot* slot, int32_t next_level, uint32_t warp, uint32_t nwarps,
                                            Tally& tally) {
     const unsigned lane = lane_id();
+    uint32_t* const count = &slot->items;
     // Up to 32 items per warp at a time; with fewer items than warps, up to
     // 2^kLogItemParts warps share each.
     const uint32_t k = min(32u, max(1u, (q + nwarps - 1) / nwarps));
     const uint32_t parts = q ? min(1u << kLogItemParts, max(1u, nwarps / q)) : 1u;
     const uint32_t part = warp % parts;
-    for (uint64_t base = static_cast<uint64_t>(warp / parts) * k; base < q;
-         base += static_cast<uint64_t>(nwarps / parts) * k) {
-        const uint64_t i = base + lane;
+    const uint32_t turns = range_count(q, k);
+    for (uint32_t turn = warp / parts; turn < turns; turn += nwarps / parts) {
+        const uint64_t i = spread ? turn + static_cast<uint64_t>(lane) * turns : static_cast<uint64_t>(turn) * k + lane;
         uint2 it = make_uint2(0u, 0u);
         if (lane < k && i < q) {
             it = __ldcg(g_in + i);
@@ -691,6 +696,10 @@ __device__ __forceinline__ void push_items(const BfsSearch& a, const uint2* g_in
             const uint32_t upto = warp_inclusive_scan(mine);
             const uint32_t all = __shfl_sync(kFullMask, upto, 31);
             if (all == 0) continue;
+            bool several = false;
+#pragma unroll
+            for (int u = 0; u < kPushUnroll; ++u) several = several || deg[u] > kItemEdges;
+            if (several) slot->levels = 1;
             uint32_t pos = 0;
             if (lane == 0) pos = atomicAdd(count, all);
             pos = __shfl_sync(kFullMask, pos, 0) + upto - mine;
@@ -1146,7 +1155,7 @@ __global__ void __launch_bounds__(kSearchThreads, kSearchCtasPerSm) bfs_search_k
     unsigned long long m = d0, unexplored = a.E - d0;  // frontier edges, edges of unlabelled vertices
     uint32_t n = 1, reached = 1, cur = 0, bm = 0, phase = 0, group_phase = 0;
     int32_t level = 0;
-    bool bottom_up = false, failed = false;
+    bool bottom_up = false, failed = false, spread = true;
     // Ends a phase: barrier, the phase's slot into shared memory.
     auto end_phase = [&]() -> bool {
         BfsSlot* slot = a.st->slot + phase % 3;
@@ -1214,6 +1223,7 @@ __global__ void __launch_bounds__(kSearchThreads, kSearchCtasPerSm) bfs_search_k
                             d = __ldg(a.offsets + v + 1) - s;
                         }
                         const uint32_t mine = range_count(d, kItemEdges);
+                        if (mine > 1) slot->levels = 1;
                         const uint32_t upto = warp_inclusive_scan(mine);
                         uint32_t at = 0;
                         if (lane == 31 && upto) at = atomicAdd(&slot->items, upto);
@@ -1223,12 +1233,13 @@ __global__ void __launch_bounds__(kSearchThreads, kSearchCtasPerSm) bfs_search_k
                 }
                 if (!end_phase()) return;
                 items = sh.slot.items;
+                spread = sh.slot.levels != 0;
                 slot = a.st->slot + phase % 3;
             }
             local = m <= kGroupEdges;
             if (!local) {
-                push_items(a, search_queue(a, cur), items, search_queue(a, cur ^ 1), &slot->items, level + 1,
-                                  warp, nwarps, tally);
+                push_items(a, search_queue(a, cur), items, spread, search_queue(a, cur ^ 1), slot, level + 1, warp, nwarps,
+                           tally);
                 flush_block_tally(tally, sh, slot);
             } else {
                 // A stretch of levels by block 0 or by the group, until the
@@ -1314,7 +1325,9 @@ __global__ void __launch_bounds__(kSearchThreads, kSearchCtasPerSm) bfs_search_k
             reached += r.reached;
             unexplored -= r.explored;
             cur ^= r.levels & 1u;
+            spread = true;  // not known
         } else {
+            spread = r.levels != 0;
             if (r.discovered == 0) break;  // the step labelled nothing: level and reached stay
             level += 1;
             reached += r.discovered;
