@@ -11,8 +11,8 @@
 //
 // The count is the sum over edges {u, v} of |N+(u) ∩ N+(v)|: every triangle
 // once, at the edge of its two highest-ranked vertices. Each edge is counted
-// from the end whose list has more words (ties: the larger id), the owner: the
-// owner's words go into a table in shared memory and the other end's words are
+// from the end whose list has more words (ties: the larger id, or, with one word
+// each, the higher rank), the owner: the owner's words go into a table in shared memory and the other end's words are
 // streamed against it, 4, 16 or 32 lanes per list. An owner reads its neighbours
 // from its own CSR row, so there are no in-lists and no oriented CSR to build.
 //  * owners of up to kWarpWords words and kWarpOwnerRow neighbours: a warp each,
@@ -351,12 +351,20 @@ __global__ void __launch_bounds__(1024) tw_build_cta_kernel(
     }
 }
 
+// First word of a list.
+__device__ __forceinline__ const uint2* list_words(const uint2* __restrict__ words, const uint2 l) {
+    return words + 2ull * l.x;
+}
+
 // ---------------------------------------------------------------- owners
 
 // Vertices with words: to the warp kernel's list, or as (vertex, slice) items
-// to the CTA kernel's.
-__global__ void tw_owners_kernel(const uint32_t* __restrict__ offsets, const uint2* __restrict__ lists, uint32_t V,
-                                 uint32_t warp_words,
+// to the CTA kernel's. A list of one neighbour shares none with that one's, and
+// edges between lists of one word belong to the higher rank, which has both ends
+// of a triangle's third edge in its own: such a vertex owns nothing (all vertices of
+// a forest).
+__global__ void tw_owners_kernel(const uint32_t* __restrict__ offsets, const uint2* __restrict__ lists,
+                                 const uint2* __restrict__ words, uint32_t V, uint32_t warp_words,
                                  uint32_t* __restrict__ warp_list, uint32_t* __restrict__ warp_count,
                                  uint2* __restrict__ items, uint32_t* __restrict__ item_count) {
     for (uint64_t b = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) & ~31ull; b < V;
@@ -364,8 +372,10 @@ __global__ void tw_owners_kernel(const uint32_t* __restrict__ offsets, const uin
         const uint64_t v = b + lane_id();
         uint32_t n = 0, d = 0;
         if (v < V) {
-            n = lists[v].y;
+            const uint2 l = lists[v];
+            n = l.y;
             d = offsets[v + 1] - offsets[v];
+            if (n == 1 && __popc(__ldg(list_words(words, l)).y) == 1) n = 0;
         }
         const bool alone = n <= warp_words && d <= kWarpOwnerRow;  // a warp's
         append_vertex(n > 0 && alone, static_cast<uint32_t>(v), warp_list, warp_count);
@@ -387,11 +397,6 @@ __global__ void tw_owners_kernel(const uint32_t* __restrict__ offsets, const uin
 // words.
 __device__ __forceinline__ uint4 word_pair(const uint2* __restrict__ words, const uint2 l, uint32_t at) {
     return __ldg(reinterpret_cast<const uint4*>(words) + (l.x + at / 2));
-}
-
-// First word of a list.
-__device__ __forceinline__ const uint2* list_words(const uint2* __restrict__ words, const uint2 l) {
-    return words + 2ull * l.x;
 }
 
 // The warp's neighbours in hand: their lists and, for the support, the entries
@@ -475,16 +480,18 @@ __device__ __forceinline__ uint32_t stream_lists(bool take, const uint2 l, uint3
 
 // Up to 32 neighbours (v per lane, `valid`) of an owner with id u and n words:
 // the lists of those it owns the edge to (fewer words, or as many and a smaller
-// id), by length: up to 8 words 4 lanes each, up to 32 words 16, the others 32.
+// id; one word each: a lower rank), by length: up to 8 words 4 lanes each, up to 32 words 16, the others 32.
 // j: the CSR entry of the neighbour; the support of an edge is kept at its
 // entry in the smaller vertex's row.
 template <bool kSupport, class Mask, class Store>
 __device__ __forceinline__ uint32_t count_neighbours(bool valid, uint32_t j, uint32_t v, uint32_t u, uint32_t n,
                                                      const uint2* __restrict__ lists, const uint2* __restrict__ words,
-                                                     const uint32_t* __restrict__ rev, ListBox<kSupport>& box,
-                                                     Mask mask, Store store) {
+                                                     const uint32_t* __restrict__ rank, const uint32_t* __restrict__ rev,
+                                                     ListBox<kSupport>& box, Mask mask, Store store) {
     const uint2 l = valid ? __ldg(lists + v) : make_uint2(0u, 0u);
-    const bool take = l.y > 0 && (l.y < n || (l.y == n && v < u));
+    bool below = v < u;
+    if (n == 1) below = valid && __ldg(rank + v) < __ldg(rank + u);
+    const bool take = l.y > 0 && (l.y < n || (l.y == n && below));
     uint32_t entry = 0;
     if constexpr (kSupport) entry = take ? (u < v ? j : __ldg(rev + j)) : 0u;
     return stream_lists<2, kSupport>(take && l.y <= 8, l, entry, words, box, mask, store) +
@@ -578,11 +585,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) tw_count_kernel(
                 const uint32_t v = valid ? ld_stream(targets + j) : 0u;
                 if (hash)
                     hits += count_neighbours<kSupport>(
-                        valid, j, v, u, own.y, lists, words, out.rev, s_box[warp],
+                        valid, j, v, u, own.y, lists, words, rank, out.rev, s_box[warp],
                         [&](uint32_t w) { return table_mask(table, kHashBits, w); }, store);
                 else
                     hits += count_neighbours<kSupport>(
-                        valid, j, v, u, own.y, lists, words, out.rev, s_box[warp],
+                        valid, j, v, u, own.y, lists, words, rank, out.rev, s_box[warp],
                         [&](uint32_t w) { return w - lo < bitmap_words ? s_bits[w - lo] : 0u; }, store);
             }
             __syncthreads();
@@ -623,7 +630,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) tw_count_kernel(
                 const uint32_t j = s + o + lane;
                 const uint32_t v = valid ? ld_stream(targets + j) : 0u;
                 hits += count_neighbours<kSupport>(
-                    valid, j, v, u, own.y, lists, words, out.rev, s_box[warp],
+                    valid, j, v, u, own.y, lists, words, rank, out.rev, s_box[warp],
                     [&](uint32_t w) { return table_mask(table, bits, w); }, store);
             });
             if (!kSupport) add_owner(u, hits, out.per_vertex, sum);
@@ -702,7 +709,7 @@ Error build_word_lists(GraphImpl& g, bool full, WordLists* w, uint64_t* n_words)
     const uint32_t warp_words = !full && V < kSmallGraph ? kWarpWordsSmall : kWarpWords;
     w->max_items = E / kSlice + E / warp_words + 1;
     GCU_TRY(w->items.allocate(dev, w->max_items));
-    GCU_LAUNCH(dev, "tw_owners", tw_owners_kernel, vgrid, 256, 0, g.offsets.ptr, w->lists.ptr, V, warp_words,
+    GCU_LAUNCH(dev, "tw_owners", tw_owners_kernel, vgrid, 256, 0, g.offsets.ptr, w->lists.ptr, w->words.ptr, V, warp_words,
                w->warp_owners.ptr, w->counts.ptr + 2, w->items.ptr, w->counts.ptr + 3);
     if (n_words) {
         GCU_CUDA(cudaMemcpyAsync(n_words, cursor.ptr, sizeof(uint64_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
