@@ -6,18 +6,18 @@
 // plain symmetric CSR and graph i's entries are [offsets[vbase[i]],
 // offsets[vbase[i + 1]]).
 //
-//  * Triangles: word lists of the union, counted per owner (tri_words.cu), or,
-//    with a learned schedule installed, one degree-oriented DAG of the union and
-//    its out-degree buckets, the schedule's variant per bucket; a block per graph
+//  * Triangles: word lists of the union, counted per owner (tri_words.cu), or one
+//    degree-oriented DAG of the union and its out-degree buckets, with a learned
+//    schedule installed or where that is faster (batch_tc_plan); a block per graph
 //    sums its vertices.
-//  * BFS and PageRank run over the union as a whole, one cooperative launch
-//    each: every level or iteration is one pass over the entries of all graphs
-//    that are still at work, and the blocks meet at a grid barrier. The entries
-//    are read as a stream of 256-entry chunks (8 consecutive entries per lane,
-//    a byte per entry says which row it belongs to), so a pass is spread evenly
-//    over the GPU whatever the sizes of the graphs; a graph has no CTA of its
-//    own to wait for. Rows that cross chunks leave parts that are joined after
-//    the pass.
+//  * BFS and PageRank of the larger graphs are one cooperative launch each: every
+//    level or iteration is one pass over the entries of all of them that are still
+//    at work, and the blocks meet at a grid barrier. The entries are read as a
+//    stream of 256-entry chunks (8 consecutive entries per lane, a byte per entry
+//    says which row it belongs to), so a pass is spread evenly over the GPU
+//    whatever the sizes of the graphs. Rows that cross chunks leave parts that are
+//    joined after the pass. A small graph is a block's, with one block barrier per
+//    level or iteration (batch_small_*).
 //  * BFS from S <= 32 sources per graph: multi-source BFS (Then et al., VLDB
 //    2015) with one S-bit mask per vertex. A level ORs the neighbours' masks
 //    into the vertex's own, from one mask array into another; a bit that is new
@@ -1692,7 +1692,7 @@ Error batch_read_ppr(BatchImpl& b, float* ranks, uint32_t* iterations, uint8_t* 
 }
 
 // Captures triangle counts, BFS and PageRank of the whole batch into one CUDA
-// graph (plans and autotunes first: nothing in the capture allocates or syncs).
+// graph (planned and run once first: nothing in the capture allocates or syncs).
 Error batch_capture(BatchImpl& b) {
     DeviceImpl& dev = *b.dev;
     if (!b.S || !b.K) return kernel_error("set the batch BFS sources and PageRank seeds before capturing");

@@ -535,7 +535,6 @@ constexpr uint32_t kPullMinEdges = 8192;     // a push with fewer frontier edges
 constexpr uint32_t kLocalItems = 2048;       // items of a local level kept in shared memory (the rest spill)
 constexpr uint32_t kLocalMaxLevels = 32768;  // levels per local or group stretch (the other blocks wait at a barrier)
 constexpr int kPushUnroll = 4;               // edges per lane in flight in a push
-constexpr int kPullTiles = 1;                // 32-vertex tiles per warp in flight in a pull
 
 // Item c of a list of d entries from s.
 __device__ __forceinline__ uint2 list_item(uint32_t s, uint32_t d, uint32_t c) {
@@ -974,7 +973,7 @@ __device__ __forceinline__ bool probe_sector(uint32_t at, uint32_t s, uint32_t e
     return (w[4] | w[5] | w[6] | w[7]) & 1u;
 }
 
-// Pull level: kPullTiles tiles of 32 vertices per warp at a time. A lane reads
+// Pull level: a tile of 32 vertices per warp at a time. A lane reads
 // its list in whole 32-byte sectors (8 entries, 8 frontier probes in flight),
 // up to kSoloSectors of them; the lists still open after that are walked by
 // the warp, 128 entries per step.
@@ -985,101 +984,79 @@ __device__ __forceinline__ void pull_level(const BfsSearch& a, const uint32_t* f
                                            int32_t next_level, uint32_t warp, uint32_t nwarps, Tally& tally) {
     const unsigned lane = lane_id();
     const uint64_t tiles = kList ? ceil_div_u64(a.n_active, 32) : ceil_div_u64(a.V, 32);
-    const uint64_t step = static_cast<uint64_t>(nwarps) * kPullTiles;
-    uint32_t nv[kPullTiles], ns[kPullTiles], ne[kPullTiles], nvis[kPullTiles];
-    // The next tiles' vertices, visited words and list bounds are loaded while
-    // the current ones are probed.
+    uint32_t nv, ns, ne, nvis;
+    // The next tile's vertices, visited words and list bounds are loaded while
+    // the current one is probed.
     auto fetch = [&](uint64_t t) {
-#pragma unroll
-        for (int q = 0; q < kPullTiles; ++q) {
-            nv[q] = 0;
-            ns[q] = 0;
-            ne[q] = 0;
-            nvis[q] = 0xFFFFFFFFu;
-            const uint64_t i = (t + q) * 32 + lane;
-            if (i < (kList ? a.n_active : a.V)) {
-                nv[q] = kList ? __ldg(a.active + i) : static_cast<uint32_t>(i);
-                nvis[q] = a.visited[nv[q] >> 5];
-                ns[q] = __ldg(a.offsets + nv[q]);
-                ne[q] = __ldg(a.offsets + nv[q] + 1);
-            }
+        nv = 0;
+        ns = 0;
+        ne = 0;
+        nvis = 0xFFFFFFFFu;
+        const uint64_t i = t * 32 + lane;
+        if (i < (kList ? a.n_active : a.V)) {
+            nv = kList ? __ldg(a.active + i) : static_cast<uint32_t>(i);
+            nvis = a.visited[nv >> 5];
+            ns = __ldg(a.offsets + nv);
+            ne = __ldg(a.offsets + nv + 1);
         }
     };
-    fetch(static_cast<uint64_t>(warp) * kPullTiles);
-    for (uint64_t t0 = static_cast<uint64_t>(warp) * kPullTiles; t0 < tiles; t0 += step) {
-        uint32_t v[kPullTiles], s[kPullTiles], e[kPullTiles], vis[kPullTiles];
-        bool found[kPullTiles];
-#pragma unroll
-        for (int q = 0; q < kPullTiles; ++q) {
-            v[q] = nv[q];
-            s[q] = ns[q];
-            e[q] = ne[q];
-            vis[q] = nvis[q];
+    fetch(warp);
+    for (uint64_t tile = warp; tile < tiles; tile += nwarps) {
+        const uint32_t v = nv, s = ns, vis = nvis;
+        uint32_t e = ne, t[8];
+        if ((vis >> (v & 31)) & 1u) e = s;
+        if (e > s) ld_stream8(a.targets + (s & ~7u), t);
+        fetch(tile + nwarps);
+        bool found = e > s && probe_sector(s & ~7u, s, e, t, frontier);
+        // Rounded up in 64 bits: lists may end within a sector of 2^32.
+        uint64_t at = (static_cast<uint64_t>(s) & ~7ull) + 8;
+        for (uint32_t k = 1; k < kSoloSectors && at < e && !found; ++k, at += 8) {
+            ld_stream8(a.targets + at, t);
+            found = probe_sector(static_cast<uint32_t>(at), s, e, t, frontier);
         }
-        uint32_t t[kPullTiles][8];
-#pragma unroll
-        for (int q = 0; q < kPullTiles; ++q) {
-            if ((vis[q] >> (v[q] & 31)) & 1u) e[q] = s[q];
-            if (e[q] > s[q]) ld_stream8(a.targets + (s[q] & ~7u), t[q]);
+        unsigned pending = __ballot_sync(kFullMask, !found && at < e);
+        while (pending) {
+            const int p = __ffs(pending) - 1;
+            pending &= pending - 1;
+            const uint64_t ps = __shfl_sync(kFullMask, static_cast<uint32_t>(at), p);
+            const uint64_t pe = __shfl_sync(kFullMask, e, p);
+            bool hit = false;
+            for (uint64_t b = ps; b < pe && !hit; b += 128) {
+                const uint64_t j = b + 4 * lane;
+                uint32_t h = 0;
+                if (j < pe) {
+                    const uint4 z = ld_stream4(reinterpret_cast<const uint4*>(a.targets + j));
+                    const uint32_t h0 = ld_if(true, frontier + (z.x >> 5), 0u);
+                    const uint32_t h1 = ld_if(j + 1 < pe, frontier + (z.y >> 5), 0u);
+                    const uint32_t h2 = ld_if(j + 2 < pe, frontier + (z.z >> 5), 0u);
+                    const uint32_t h3 = ld_if(j + 3 < pe, frontier + (z.w >> 5), 0u);
+                    h = (h0 >> (z.x & 31)) | (h1 >> (z.y & 31)) | (h2 >> (z.z & 31)) | (h3 >> (z.w & 31));
+                }
+                hit = __any_sync(kFullMask, h & 1u);
+            }
+            if (static_cast<int>(lane) == p) found = hit;
         }
-        fetch(t0 + step);
-#pragma unroll
-        for (int q = 0; q < kPullTiles; ++q) {
-            found[q] = false;
-            if (e[q] > s[q]) found[q] = probe_sector(s[q] & ~7u, s[q], e[q], t[q], frontier);
+        if (found) {
+            a.dist[v] = next_level;
+            tally.found += 1;
+            tally.edges += e - s;
         }
-#pragma unroll
-        for (int q = 0; q < kPullTiles; ++q) {
-            // Rounded up in 64 bits: lists may end within a sector of 2^32.
-            uint64_t at = (static_cast<uint64_t>(s[q]) & ~7ull) + 8;
-            for (uint32_t k = 1; k < kSoloSectors && at < e[q] && !found[q]; ++k, at += 8) {
-                ld_stream8(a.targets + at, t[q]);
-                found[q] = probe_sector(static_cast<uint32_t>(at), s[q], e[q], t[q], frontier);
-            }
-            unsigned pending = __ballot_sync(kFullMask, !found[q] && at < e[q]);
-            while (pending) {
-                const int p = __ffs(pending) - 1;
-                pending &= pending - 1;
-                const uint64_t ps = __shfl_sync(kFullMask, static_cast<uint32_t>(at), p);
-                const uint64_t pe = __shfl_sync(kFullMask, e[q], p);
-                bool hit = false;
-                for (uint64_t b = ps; b < pe && !hit; b += 128) {
-                    const uint64_t j = b + 4 * lane;
-                    uint32_t h = 0;
-                    if (j < pe) {
-                        const uint4 z = ld_stream4(reinterpret_cast<const uint4*>(a.targets + j));
-                        const uint32_t h0 = ld_if(true, frontier + (z.x >> 5), 0u);
-                        const uint32_t h1 = ld_if(j + 1 < pe, frontier + (z.y >> 5), 0u);
-                        const uint32_t h2 = ld_if(j + 2 < pe, frontier + (z.z >> 5), 0u);
-                        const uint32_t h3 = ld_if(j + 3 < pe, frontier + (z.w >> 5), 0u);
-                        h = (h0 >> (z.x & 31)) | (h1 >> (z.y & 31)) | (h2 >> (z.z & 31)) | (h3 >> (z.w & 31));
-                    }
-                    hit = __any_sync(kFullMask, h & 1u);
+        if (kList) {
+            // The tile's vertices ascend, so they share a few words: one
+            // pair of atomics per word.
+            if (__any_sync(kFullMask, found)) {
+                const unsigned peers = __match_any_sync(kFullMask, v >> 5);
+                const uint32_t bits = __reduce_or_sync(peers, found ? 1u << (v & 31) : 0u);
+                if (bits && lane == static_cast<unsigned>(__ffs(peers) - 1)) {
+                    atomicOr(next_frontier + (v >> 5), bits);
+                    atomicOr(a.visited + (v >> 5), bits);
                 }
-                if (static_cast<int>(lane) == p) found[q] = hit;
             }
-            if (found[q]) {
-                a.dist[v[q]] = next_level;
-                tally.found += 1;
-                tally.edges += e[q] - s[q];
-            }
-            if (kList) {
-                // The tile's vertices ascend, so they share a few words: one
-                // pair of atomics per word.
-                if (__any_sync(kFullMask, found[q])) {
-                    const unsigned peers = __match_any_sync(kFullMask, v[q] >> 5);
-                    const uint32_t bits = __reduce_or_sync(peers, found[q] ? 1u << (v[q] & 31) : 0u);
-                    if (bits && lane == static_cast<unsigned>(__ffs(peers) - 1)) {
-                        atomicOr(next_frontier + (v[q] >> 5), bits);
-                        atomicOr(a.visited + (v[q] >> 5), bits);
-                    }
-                }
-            } else {
-                const unsigned mask = __ballot_sync(kFullMask, found[q]);
-                if (lane == 0 && t0 + q < tiles) {
-                    next_frontier[t0 + q] = mask;
-                    if (mask) a.visited[t0 + q] = vis[q] | mask;
-                }
+        } else {
+            const unsigned mask = __ballot_sync(kFullMask, found);
+            if (lane == 0) {
+                next_frontier[tile] = mask;
+                if (mask) a.visited[tile] = vis | mask;
             }
         }
     }
