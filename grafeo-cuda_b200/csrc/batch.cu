@@ -984,6 +984,23 @@ __global__ void __launch_bounds__(kThreads) batch_small_bfs_kernel(const BatchSm
     });
 }
 
+// sum + the contributions of entries o, o + stride, ... of a list, in that order,
+// kLoads of them in flight.
+template <int kLoads>
+__device__ __forceinline__ double add_entries(double sum, const uint32_t* list, const float* in, uint32_t o,
+                                              uint32_t stride, uint32_t len) {
+    uint32_t x[kLoads];
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) x[q] = ld_nc_if(o + q * stride < len, list + o + q * stride, 0u);
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q)
+        x[q] = ld_if(o + q * stride < len, reinterpret_cast<const uint32_t*>(in) + x[q], 0u);
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) sum += static_cast<double>(__uint_as_float(x[q]));
+    return sum;
+}
+constexpr int kSoloLoads = 4, kWarpLoads = 8;
+
 struct BatchSmallPpr {
     BatchSmall small;
     const float* tele;
@@ -1046,13 +1063,15 @@ __global__ void __launch_bounds__(kThreads) batch_small_ppr_kernel(const BatchSm
                 }
                 double sum = 0.0;
                 if (e - s <= kSoloRow)
-                    for (uint32_t j = s; j < e; ++j) sum += static_cast<double>(in[__ldg(a.small.targets + j)]);
+                    for (uint32_t o = 0; o < e - s; o += kSoloLoads)
+                        sum = add_entries<kSoloLoads>(sum, a.small.targets + s, in, o, 1, e - s);
                 for (unsigned longs = __ballot_sync(kFullMask, e - s > kSoloRow); longs; longs &= longs - 1) {
                     const int l = __ffs(longs) - 1;
                     const uint32_t len = __shfl_sync(kFullMask, e - s, l);
                     const uint32_t* list = a.small.targets + __shfl_sync(kFullMask, s, l);
                     double part = 0.0;
-                    for (uint32_t o = lane; o < len; o += 32) part += static_cast<double>(in[__ldg(list + o)]);
+                    for (uint32_t o = lane; o < len; o += 32 * kWarpLoads)
+                        part = add_entries<kWarpLoads>(part, list, in, o, 32, len);
                     part = warp_sum(part);
                     if (static_cast<int>(lane) == l) sum = part;
                 }
@@ -1215,6 +1234,20 @@ Error part_graphs(BatchImpl& b) {
             b.n_small[c] = 0;
         }
     }
+    // Warps beyond a graph's vertices have nothing to do: a class whose graphs are all
+    // that small has smaller blocks, unless those have graphs of their own.
+    uint32_t widest[kSmallClasses] = {};
+    for (const BatchGraph& g : small) {
+        uint32_t& w = widest[joins[class_of(g)]];
+        w = std::max(w, g.v_end - g.v_begin);
+    }
+    for (int c = 0; c + 1 < kSmallClasses; ++c)
+        for (int k = kSmallClasses - 1; k > c && b.n_small[c]; --k)
+            if (!b.n_small[k] && widest[c] <= static_cast<uint32_t>(kSmallThreads[k])) {
+                std::swap(b.n_small[c], b.n_small[k]);
+                for (int& j : joins)
+                    if (j == c) j = k;
+            }
     std::stable_sort(small.begin(), small.end(), [&](const BatchGraph& x, const BatchGraph& y) {
         const int cx = joins[class_of(x)], cy = joins[class_of(y)];
         return cx != cy ? cx < cy : x.e_end - x.e_begin > y.e_end - y.e_begin;
