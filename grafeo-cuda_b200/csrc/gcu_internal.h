@@ -300,8 +300,12 @@ struct WordLists {
     DeviceBuffer<uint32_t> counts;       // [2] warp owners, [3] items
     uint64_t max_items = 0;
 };
-// n_words (may be NULL): words of all lists, their padding among them (synchronises).
-Error build_word_lists(GraphImpl& g, bool full, WordLists* w, uint64_t* n_words = nullptr);
+struct WordListSizes {
+    uint64_t words = 0;   // of all lists, their padding among them
+    uint64_t owners = 0;  // warp owners and items
+};
+// size (may be NULL) synchronises.
+Error build_word_lists(GraphImpl& g, bool full, WordLists* w, WordListSizes* size = nullptr);
 // Adds the triangles to *total, or to per_vertex[owner] where that is given
 // (device memory). next: two words of scratch. Only enqueues (capturable).
 Error count_words(GraphImpl& g, const WordLists& w, uint32_t* next, unsigned long long* total,

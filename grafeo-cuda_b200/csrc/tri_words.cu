@@ -661,7 +661,7 @@ uint32_t support_bitmap_words(uint32_t V) {
 
 }  // namespace
 
-Error build_word_lists(GraphImpl& g, bool full, WordLists* w, uint64_t* n_words) {
+Error build_word_lists(GraphImpl& g, bool full, WordLists* w, WordListSizes* size) {
     DeviceImpl& dev = *g.dev;
     const uint32_t V = g.num_nodes, E = g.num_edges;
     const uint64_t cap = static_cast<uint64_t>(dev.sm_count) * 16;
@@ -711,9 +711,12 @@ Error build_word_lists(GraphImpl& g, bool full, WordLists* w, uint64_t* n_words)
     GCU_TRY(w->items.allocate(dev, w->max_items));
     GCU_LAUNCH(dev, "tw_owners", tw_owners_kernel, vgrid, 256, 0, g.offsets.ptr, w->lists.ptr, w->words.ptr, V, warp_words,
                w->warp_owners.ptr, w->counts.ptr + 2, w->items.ptr, w->counts.ptr + 3);
-    if (n_words) {
-        GCU_CUDA(cudaMemcpyAsync(n_words, cursor.ptr, sizeof(uint64_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
+    if (size) {
+        uint32_t counts[2];
+        GCU_CUDA(cudaMemcpyAsync(&size->words, cursor.ptr, sizeof(uint64_t), cudaMemcpyDeviceToHost, dev.stream), "copy");
+        GCU_CUDA(cudaMemcpyAsync(counts, w->counts.ptr + 2, sizeof(counts), cudaMemcpyDeviceToHost, dev.stream), "copy");
         GCU_TRY(dev.sync());
+        size->owners = static_cast<uint64_t>(counts[0]) + counts[1];
     }
     return ok();
 }

@@ -641,6 +641,7 @@ struct BatchTcPlan {
     // Counted over word lists (symmetric union, no learned schedule), else over the DAG.
     GraphImpl* word_graph = nullptr;
     WordLists words;
+    bool no_owners = false;  // no triangles: nothing to launch
     DeviceBuffer<uint32_t> dag_offsets, dag_targets;
     uint32_t m = 0;
     BucketPlan buckets;
@@ -650,6 +651,11 @@ struct BatchTcPlan {
 
 void destroy_batch_tc_plan(BatchTcPlan* p) { delete p; }
 
+// Buckets that take the warp variant untimed: the other variants have a block per
+// vertex, which is slower wherever there are many vertices of few out-neighbours, and
+// timing it was most of the plan (30 grids of 150 x 150: first count 4.7 -> 2.0 ms).
+static bool untimed_bucket(int c, uint32_t vertices) { return bucket_fixed(c) == 0 && (c <= 4 || vertices >= 65536); }
+
 static Error plan_dag(GraphImpl& u, BatchTcPlan* p, std::string* tuning) {
     DeviceImpl& dev = *u.dev;
     GCU_TRY(build_dag(u, true, &p->dag_offsets, &p->dag_targets, &p->m));
@@ -657,8 +663,8 @@ static Error plan_dag(GraphImpl& u, BatchTcPlan* p, std::string* tuning) {
     if (dev.schedule) GCU_TRY(degree_stats(u, &stats));
     GCU_TRY(plan_buckets(dev, p->dag_offsets.ptr, u.num_nodes, 2, p->m, stats, false, p->buckets));
     GCU_TRY(p->next.allocate(dev, kBuckets * kSchedOut));
-    // Variant per bucket: the learned schedule's pick when one is installed,
-    // else the fastest valid variant timed once on this batch (autotune).
+    // Variant per bucket: the learned schedule's pick when one is installed, else
+    // the fastest valid variant timed once on this batch (see untimed_bucket).
     DeviceBuffer<unsigned long long> scratch;
     GCU_TRY(scratch.allocate(dev, std::max<uint32_t>(u.num_nodes, 1)));
     GCU_CUDA(cudaMemsetAsync(p->next.ptr, 0, sizeof(uint32_t) * kBuckets * kSchedOut, dev.stream), "memset");
@@ -681,6 +687,8 @@ static Error plan_dag(GraphImpl& u, BatchTcPlan* p, std::string* tuning) {
         if (learned >= 0 && ((valid >> learned) & 1u)) {
             pick = learned;
             how = "learned";
+        } else if (untimed_bucket(c, p->buckets.host_counts[c])) {
+            how = "fixed";
         } else {
             bool first = true;
             for (int v = 0; v < kSchedOut; ++v) {
@@ -740,7 +748,8 @@ static Error time_plan(GraphImpl& u, BatchTcPlan& p, float* ms) {
 // words for 10 kept entries or more: sparse graphs without hubs), both forms are
 // tried on the batch and the faster one is kept: 120 Erdos-Renyi graphs of 59 M
 // entries 2.45 ms over word lists, 1.61 over the DAG; 256 corpus graphs (0.5 words
-// an entry) 3.6 and 9.5. Below kTryBoth entries either takes some 10 us.
+// an entry) 3.6 and 9.5. Below kTryBoth entries either takes some 10 us, and lists
+// without owners (paths) are not counted at all.
 constexpr uint32_t kTryBoth = 1u << 16;
 
 Error batch_tc_plan(GraphImpl& u, BatchTcPlan** out, std::string* tuning) {
@@ -752,10 +761,12 @@ Error batch_tc_plan(GraphImpl& u, BatchTcPlan** out, std::string* tuning) {
     if (words) {
         p->word_graph = &u;
         GCU_TRY(p->next.allocate(dev, 2));
-        uint64_t n_words = 0;
-        GCU_TRY(build_word_lists(u, false, &p->words, &n_words));
+        WordListSizes size;
+        GCU_TRY(build_word_lists(u, false, &p->words, &size));
         *tuning = "{\"variant\": \"word lists\"}";
-        if (u.num_edges < kTryBoth || 10 * n_words < 9 * static_cast<uint64_t>(u.num_edges / 2)) {
+        p->no_owners = size.owners == 0;
+        if (u.num_edges < kTryBoth || p->no_owners ||
+            10 * size.words < 9 * static_cast<uint64_t>(u.num_edges / 2)) {
             *out = p.release();
             return ok();
         }
@@ -784,6 +795,7 @@ Error batch_tc_plan(GraphImpl& u, BatchTcPlan** out, std::string* tuning) {
 Error batch_tc_launch(DeviceImpl& dev, BatchTcPlan& p, unsigned long long* per_vertex, uint32_t num_nodes) {
     GCU_CUDA(cudaMemsetAsync(per_vertex, 0, sizeof(unsigned long long) * std::max<uint32_t>(num_nodes, 1), dev.stream),
              "memset");
+    if (p.no_owners) return ok();
     if (p.word_graph) return count_words(*p.word_graph, p.words, p.next.ptr, nullptr, per_vertex);
     GCU_CUDA(cudaMemsetAsync(p.next.ptr, 0, sizeof(uint32_t) * kBuckets, dev.stream), "memset");
     for (int c = kBuckets - 1; c >= 0; --c) {
